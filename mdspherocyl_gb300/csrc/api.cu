@@ -22,11 +22,12 @@
 namespace mdsc {
 void launch_real_pairs(const Batch& b, bool multi, cudaStream_t s);
 cudaError_t prepare_real_pairs();
+cudaError_t prepare_kspace();
+cudaError_t prepare_wca();
 void launch_real_sum(const Batch& b, cudaStream_t s);
 // the cutoff systems' neighbour pass: real space (1), WCA screen (2), both (3)
 void launch_near_pass(const Batch& b, int mode, cudaStream_t s);
-void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner,
-                   double* kE, cudaStream_t s);
+void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, cudaStream_t s);
 void launch_derive(const Batch& b, cudaStream_t s);
 void launch_integrate_first(const Batch& b, cudaStream_t s);
 void launch_finalize(const Batch& b, int mode, cudaStream_t s);
@@ -46,8 +47,8 @@ void launch_cluster_compress(const Batch& b, cudaStream_t s);
 void launch_reset_iter(const Batch& b, cudaStream_t s);
 // copies systems (dst slot, src slot) between batches on the destination's stream
 cudaError_t launch_transfer(const Batch& dst, const Batch& src, const std::vector<int2>& pairs, cudaStream_t s);
-void launch_kspace_parts(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner,
-                         double* kE, int part, cudaStream_t s);
+void launch_kspace_parts(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, int part,
+                         cudaStream_t s);
 void launch_correlations(const Batch& b, const CorrSys* cs, const unsigned char* species, double bar_w,
                          int max_bins, unsigned long long* hist, cudaStream_t s);
 void launch_order_sums(const Batch& b, double* out, cudaStream_t s);
@@ -67,6 +68,12 @@ using namespace mdsc;
 namespace {
 
 constexpr int kNoiseChunk = 256;  // steps of thermostat noise per upload
+// Batches of at most this many particle blocks (2 per SM) gather one k tile
+// per block: 2048 rods (16 blocks) 85 us per step with whole walks and 80
+// split, 24 systems of 128 to 2048 rods (140 blocks) 144 and 135; 64 systems
+// (400 blocks) 226 and 231, 256 systems 693 and 701 (the tiles' sums through
+// memory then cost more than the added blocks gain).
+constexpr int kGatherSplitMax = 300;
 // the reference's table covers r <= 0.5 * 200.2 (v25/functions.cpp:1563,1681)
 constexpr double kTableRmax = 0.5 * 200 * 1.001;
 constexpr double kLh = 0.5 * (200 * 1.001) / 32768;
@@ -80,7 +87,8 @@ struct Layout {
   std::vector<double> kval, kpre, kvec;
   std::vector<int2> blk, kowner;
   std::vector<int2> bstrips;  // strips of the systems whose tile energies are summed per strip
-  std::vector<int2> kgwork;   // (particle block, part) of the k-space gather
+  std::vector<int2> kgwork;   // (particle block, tile) of the k-space gather
+  std::vector<int2> ktile;    // (system, k tile)
   std::vector<int2> cellblk;  // (system, first cell) of every block of the cell-binned list build
   std::vector<int4> rpwork;   // runs of tiles whose table is staged in shared memory
   std::vector<int> gtile;     // tiles of the one-tile-per-warp kernel (analytic or global table)
@@ -344,16 +352,16 @@ void make_layout(const mdsc_system_desc* descs, int nsys, Layout& Lo) {
     P.blk_off = blk;
     P.nblk = cdiv(d.n, kPartBlock);
     for (int k = 0; k < P.nblk; ++k) Lo.blk.push_back(make_int2(s, part + k * kPartBlock));
-    // the k-space gather of a large single-dipole system runs its k tiles in
-    // parts on separate blocks (a function of the system only, so the same
-    // bits alone and in any batch); smaller systems fill the GPU as they
-    // are (split for every single-dipole system, the 256-replica mix's
-    // gather went from 0.107 to 0.117 ms: the parts' partial sums and their
-    // combination cost more than the added blocks gained)
+    // the k-space gather of a large single-dipole system adds its k tiles in
+    // parts (a function of the system only, so the same bits alone and in
+    // any batch)
     const int ktiles = cdiv(P.nk, kKBlock);
     P.kgs = (d.nd == 1 && d.n >= 4096 && ktiles > 1) ? std::min(8, ktiles) : 1;
+    P.kt_off = (int)Lo.ktile.size();
+    P.nkt = ktiles;
+    for (int q = 0; q < ktiles; ++q) Lo.ktile.push_back(make_int2(s, q));
     P.kgp_off = (int)Lo.kgsets;
-    if (P.kgs > 1) Lo.kgsets += (long long)P.nblk * P.kgs;
+    Lo.kgsets += (long long)P.nblk * ktiles * d.nd;
     blk += P.nblk;
     P.cl_fr = d.cl_fr;
     for (int a = 0; a < 3; ++a) {
@@ -424,10 +432,18 @@ void make_layout(const mdsc_system_desc* descs, int nsys, Layout& Lo) {
   // order.
   std::stable_sort(Lo.blk.begin(), Lo.blk.end(),
                    [&](const int2& u, const int2& v) { return descs[u.x].n > descs[v.x].n; });
-  // the k-space gather's blocks: every part of every particle block, in the
-  // launch order above (entries index the sorted block list)
-  for (int g = 0; g < (int)Lo.blk.size(); ++g)
-    for (int q = 0; q < Lo.sys[Lo.blk[g].x].kgs; ++q) Lo.kgwork.push_back(make_int2(g, q));
+  // the k-space gather's blocks, in the launch order above (entries index
+  // the sorted block list): one per particle block where those fill the GPU,
+  // one per particle block and k tile where they do not (and always for
+  // systems that add their tiles in parts)
+  const bool split = (int)Lo.blk.size() <= kGatherSplitMax;
+  for (int s = 0; s < nsys; ++s) Lo.sys[s].kgt = (split || Lo.sys[s].kgs > 1) ? std::max(Lo.sys[s].nkt, 1) : 1;
+  for (int g = 0; g < (int)Lo.blk.size(); ++g) {
+    const SysDev& P = Lo.sys[Lo.blk[g].x];
+    if (P.kgt == 1) Lo.kgwork.push_back(make_int2(g, -1));
+    else
+      for (int q = 0; q < P.kgt; ++q) Lo.kgwork.push_back(make_int2(g, q));
+  }
   Lo.ntot = part;
   Lo.ndtot = dip;
   Lo.nktot = (int)Lo.kn.size();
@@ -483,7 +499,7 @@ void carve(Arena& A, const Layout& Lo, int nsys, Batch& b, int4** kwork, int2** 
   b.stripE = A.take<double>(10 * (size_t)std::max(Lo.nstrips, 1));
   b.bstrips = A.take<int2>(std::max<size_t>(Lo.bstrips.size(), 1));
   b.kgwork = A.take<int2>(std::max<size_t>(Lo.kgwork.size(), 1));
-  b.kgpart = A.take<float>(std::max<long long>(Lo.kgsets, 1) * kPartBlock * 12);
+  b.kgpart = A.take<float>(std::max<long long>(Lo.kgsets, 1) * kPartBlock * 6);
   b.kgdone = A.take<int>(nb);
   b.rnb = A.take<int>(Lo.any_rc ? n * kMaxR : 1);
   b.rnbc = A.take<int>(n);
@@ -510,10 +526,9 @@ void carve(Arena& A, const Layout& Lo, int nsys, Batch& b, int4** kwork, int2** 
   b.kpart = A.take<float>(10 * std::max<long long>(Lo.kpart, 1));
   b.ksum = A.take<double>(10 * nk);
   b.kS = A.take<float2>(nk);
-  b.kE = A.take<double>(10 * nk);
+  b.kE = A.take<double>(10 * std::max<size_t>(Lo.ktile.size(), 1));
+  b.ktile = A.take<int2>(std::max<size_t>(Lo.ktile.size(), 1));
   b.kG = A.take<double>(6 * (size_t)std::max(Lo.nchunks, 1));
-  b.kGs = A.take<double>(6 * (size_t)std::max(nsys, 1));
-  b.kgcnt = A.take<int>(std::max(nsys, 1));
   b.icnt = A.take<int>(std::max(nsys, 1));
   b.Fk = A.take<float2>(3 * nd);
   b.Tk = A.take<float2>(3 * nd);
@@ -549,8 +564,8 @@ struct mdsc_batch {
   int device = 0;
   int num_sms = 0;  // streaming multiprocessors of the device
   int nsys = 0;
-  cudaStream_t st = nullptr, s2 = nullptr, s3 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_j2 = nullptr, ev_j3 = nullptr;
+  cudaStream_t st = nullptr, s2 = nullptr, s3 = nullptr, s4 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_j2 = nullptr, ev_j3 = nullptr, ev_j4 = nullptr, ev_k = nullptr;
   // mdsc_step_io: the stream that takes positions and orientations home
   // while a step's forces are computed, and the event its graph records
   // once they are final
@@ -628,7 +643,7 @@ mdsc_status eval_forces(mdsc_batch* B, int force_list, const int* skip = nullptr
   launch_wca(b, 1, B->st);  // with the cutoff systems' real space, in the same neighbour pass
   launch_real_pairs(b, B->lo.multi, B->st);
   launch_real_sum(b, B->st);
-  launch_kspace(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, b.kE, B->st);
+  launch_kspace(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, B->st);
   launch_finalize(b, kMaskAll, B->st);
   launch_order_terms(b, B->st);
   launch_reduce_obs(b, kRedEnergies, B->st);
@@ -724,11 +739,11 @@ mdsc_status autotune(mdsc_batch* B, int force, int reps) {
   }
   // k-space gather form (single-dipole systems)
   if (b.nktot > 0 && B->lo.maxnd <= 1) {
-    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, b.kE, 0, B->st);
-    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, b.kE, 1, B->st);
+    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 0, B->st);
+    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 1, B->st);
     const int cand[2] = {0, 1};
     pick("kg_scalar", cand, 2, b.tune.kg_scalar, [&] {
-      launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, b.kE, 2, B->st);
+      launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 2, B->st);
     });
   }
   CU(cudaStreamSynchronize(B->st));
@@ -758,7 +773,6 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   cudaEventRecord(B->ev_fork, B->st);
   cudaStreamWaitEvent(B->s2, B->ev_fork, 0);
   cudaStreamWaitEvent(B->s3, B->ev_fork, 0);
-  launch_order_terms(b, B->st);
   launch_list_build(b, 0, B->st);
   launch_wca(b, 1, B->st);  // the cutoff systems' real space in their neighbour pass, after their list
   // order terms, the list build's decision and scan (+ the cell binning),
@@ -767,14 +781,27 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   launch_real_pairs(b, B->lo.multi, B->s2);
   launch_real_sum(b, B->s2);
   launches += b.ntiles > 0 ? 2 + (b.nbstrips > 0 ? 1 : 0) : 0;
-  launch_kspace(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, b.kE, B->s3);
-  launches += b.nktot > 0 ? (B->lo.maxnd > 1 ? 5 : 3) : 0;  // multi-dipole batches: both ksum and kgather forms
+  auto kpart = [&](int part, cudaStream_t s) {
+    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, part, s);
+  };
+  kpart(0, B->s3);
+  kpart(1, B->s3);
+  cudaEventRecord(B->ev_k, B->s3);
+  kpart(2, B->s3);
+  // what only the per-system sums at the end of the step read
+  cudaStreamWaitEvent(B->s4, B->ev_fork, 0);
+  launch_order_terms(b, B->s4);
+  cudaStreamWaitEvent(B->s4, B->ev_k, 0);
+  kpart(3, B->s4);
+  cudaEventRecord(B->ev_j4, B->s4);
+  launches += b.nktot > 0 ? (B->lo.maxnd > 1 ? 6 : 4) : 0;  // multi-dipole batches: both ksum and kgather forms
   cudaEventRecord(B->ev_j2, B->s2);
   cudaEventRecord(B->ev_j3, B->s3);
   cudaStreamWaitEvent(B->st, B->ev_j2, 0);
   cudaStreamWaitEvent(B->st, B->ev_j3, 0);
   launch_finalize(b, kMaskAll | kFlagMoveP, B->st);
   if (io) cudaEventRecordWithFlags(B->ev_f, B->st, cudaEventRecordExternal);
+  cudaStreamWaitEvent(B->st, B->ev_j4, 0);
   launch_reduce_obs(b, kRedStep, B->st);
   launches += 2;
   cudaError_t e = cudaStreamEndCapture(B->st, &g);
@@ -1165,7 +1192,8 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   B->desc.assign(descs, descs + nsys);
   cudaSetDevice(device);
   if (cudaDeviceGetAttribute(&B->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-      B->num_sms <= 0 || prepare_real_pairs() != cudaSuccess) {
+      B->num_sms <= 0 || prepare_real_pairs() != cudaSuccess || prepare_kspace() != cudaSuccess ||
+      prepare_wca() != cudaSuccess) {
     delete B;
     return MDSC_ERR_NO_DEVICE;
   }
@@ -1193,6 +1221,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   b.nbstrips = (int)lo.bstrips.size();
   b.any_rc = lo.any_rc ? 1 : 0;
   b.nkgwork = (int)lo.kgwork.size();
+  b.nktile = (int)lo.ktile.size();
   b.nblk = (int)lo.blk.size();
   b.ncellblk = (int)lo.cellblk.size();
   b.nrpwork = (int)lo.rpwork.size();
@@ -1211,9 +1240,12 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   if (cudaStreamCreateWithPriority(&B->st, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
       cudaStreamCreateWithPriority(&B->s2, cudaStreamNonBlocking, prio_lo) != cudaSuccess ||
       cudaStreamCreateWithPriority(&B->s3, cudaStreamNonBlocking, prio_hi) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&B->s4, cudaStreamNonBlocking, prio_lo) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_j2, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_j3, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&B->ev_j4, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&B->ev_k, cudaEventDisableTiming) != cudaSuccess ||
       cudaStreamCreateWithFlags(&B->sio, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_x, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_f, cudaEventDisableTiming) != cudaSuccess ||
@@ -1236,6 +1268,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   if (!lo.gtile.empty()) up(b.gtile, lo.gtile.data(), sizeof(int) * lo.gtile.size());
   if (!lo.bstrips.empty()) up(b.bstrips, lo.bstrips.data(), sizeof(int2) * lo.bstrips.size());
   if (!lo.kgwork.empty()) up(b.kgwork, lo.kgwork.data(), sizeof(int2) * lo.kgwork.size());
+  if (!lo.ktile.empty()) up(b.ktile, lo.ktile.data(), sizeof(int2) * lo.ktile.size());
   up(b.blk, lo.blk.data(), sizeof(int2) * lo.blk.size());
   if (!lo.cellblk.empty()) up(b.cellblk, lo.cellblk.data(), sizeof(int2) * lo.cellblk.size());
   up(b.kn, lo.kn.data(), sizeof(int4) * lo.kn.size());
@@ -1269,7 +1302,6 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   cudaMemsetAsync(b.ccnt, 0, sizeof(int) * std::max(lo.ncellcap, 1), B->st);
   cudaMemsetAsync(b.kgdone, 0, sizeof(int) * std::max<size_t>(lo.blk.size(), 1), B->st);
   cudaMemsetAsync(b.rlE, 0, sizeof(double) * 10 * std::max<size_t>(lo.blk.size(), 1), B->st);
-  cudaMemsetAsync(b.kgcnt, 0, sizeof(int) * std::max(nsys, 1), B->st);
   cudaMemsetAsync(b.icnt, 0, sizeof(int) * std::max(nsys, 1), B->st);
   cudaMemsetAsync(b.F, 0, sizeof(double) * 3 * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(b.T, 0, sizeof(double) * 3 * std::max(lo.ntot, 1), B->st);
@@ -1324,6 +1356,8 @@ mdsc_status mdsc_destroy(mdsc_batch* B) {
   if (B->ev_fork) cudaEventDestroy(B->ev_fork);
   if (B->ev_j2) cudaEventDestroy(B->ev_j2);
   if (B->ev_j3) cudaEventDestroy(B->ev_j3);
+  if (B->ev_j4) cudaEventDestroy(B->ev_j4);
+  if (B->ev_k) cudaEventDestroy(B->ev_k);
   if (B->ev_x) cudaEventDestroy(B->ev_x);
   if (B->ev_f) cudaEventDestroy(B->ev_f);
   if (B->sio) cudaStreamDestroy(B->sio);
@@ -1332,6 +1366,7 @@ mdsc_status mdsc_destroy(mdsc_batch* B) {
   if (B->st) cudaStreamDestroy(B->st);
   if (B->s2) cudaStreamDestroy(B->s2);
   if (B->s3) cudaStreamDestroy(B->s3);
+  if (B->s4) cudaStreamDestroy(B->s4);
   delete B;
   return MDSC_OK;
 }
@@ -1640,7 +1675,7 @@ mdsc_status mdsc_force_dipK(mdsc_batch* B, double* U, double* PT) {
   mdsc_status st = need_state(B);
   if (st) return st;
   launch_derive(B->b, B->st);
-  launch_kspace(B->b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, B->b.kE, B->st);
+  launch_kspace(B->b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, B->st);
   launch_finalize(B->b, kMaskK | kFlagAccum, B->st);
   launch_order_terms(B->b, B->st);
   launch_reduce_obs(B->b, kRedEnergies, B->st);
@@ -2476,12 +2511,13 @@ mdsc_status mdsc_profile_steps(mdsc_batch* B, int nsteps, int max_kernels, char*
     cudaEventRecord(ev[6], B->st);
     launch_near_pass(b, 1, B->st);
     cudaEventRecord(ev[7], B->st);
-    // the three k-space kernels, timed one by one
-    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, b.kE, 0, B->st);
+    // the k-space kernels, timed one by one (the energies with the chunk sums)
+    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 0, B->st);
     cudaEventRecord(ev[8], B->st);
-    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, b.kE, 1, B->st);
+    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 1, B->st);
+    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 3, B->st);
     cudaEventRecord(ev[9], B->st);
-    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, b.kE, 2, B->st);
+    launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 2, B->st);
     cudaEventRecord(ev[10], B->st);
     launch_finalize(b, kMaskAll | kFlagMoveP, B->st);
     cudaEventRecord(ev[11], B->st);

@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
   {
     // the rows of one per-system table, column by column: real-space tiles
     // (U, PT; FP32) or, in large systems, strips (each strip's tiles summed
-    // in float-float by strip_energy), k-vectors (U, PT), WCA blocks (U, W, PT), kinetic
+    // in float-float by strip_energy), k tiles (U, PT), WCA blocks (U, W, PT), kinetic
     // blocks (K_t, K_r, PT_kin, U_ext) or order-parameter blocks.  One code
     // path for the five keeps the kernel small: its blocks are short, and a
     // larger kernel waited on instruction fetch.
@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
       nrow = P.ntile;
       ncol = 10;
     } else if (grp == 1) {
-      dsrc = b.kE + (long long)P.k_off * 10;
-      nrow = P.nk;
+      dsrc = b.kE + (long long)P.kt_off * 10;
+      nrow = P.nkt;
       ncol = 10;
     } else if (grp == 2) {
       dsrc = b.wcaE + (long long)P.blk_off * 11;

@@ -18,13 +18,22 @@
 // wraps modulo 2^32 exactly: the phase is reduced exactly to [-pi, pi) for
 // any box size and any k, and only the final sine/cosine is rounded.
 //
-// Kernels: ksum (partial sums over chunks of kKChunk particles, one k per
-// thread), kcombine (chunks -> FP64 sums per k, energy and pressure-tensor
-// terms per k), kgather (per particle over all k: force and torque).
+// Kernels: ksum (partial sums over chunks of kKChunk particles), kstruct
+// (chunks -> FP64 sums per k and val S(k), all the gather waits for), kenergy
+// (energy and pressure tensor of each k tile, beside the gather), kgather (per
+// particle over all k: force and torque).
+#include <initializer_list>
+
 #include "mdsc_dev.cuh"
 #include "reduce.cuh"
 
 namespace mdsc {
+
+// Batches of at most this many structure-factor blocks (4 per SM) run ksum1s:
+// a system of 256 rods 65.7 us per step with ksum1 and 62.4 with ksum1s, 24
+// systems of 128 to 2048 rods (330 blocks) 144 and 135; 64 systems (900) 229
+// and 226, 256 systems 693 and 696.
+constexpr int kKsumScalarMax = 4 * 152;
 
 __device__ __forceinline__ void phase_cs(uint32_t ph, float& c, float& s) {
   // (int)ph * 2^-31 * pi: the phase, already reduced to [-pi, pi); the
@@ -47,19 +56,60 @@ __device__ __forceinline__ uint32_t phase_next(uint32_t ph, bool have, uint32_t 
   return (have && n.w) ? ph + ux : phase_of(ux, uy, uz, n);
 }
 
-// grid: one block per (system, particle chunk, k tile); work list kwork.
-// With one dipole per particle the per-particle self terms need no per-k
-// work: |S_i(k)|^2 = (m_i.k)^2 and Re(conj(S_i) U_ic) = (m_i.k) m_ic, so
-// self(k) = k^T G k and uvslf(k) = G k with G = sum_i m_i m_i^T, which the
-// first k tile of every chunk sums once.
+// The moment tensor of one particle chunk, sum of m m^T (one dipole per
+// particle), for the self terms of kenergy.  Float-float: the products exact
+// (one FMA each for the low half), 48-bit sums -- in FP64 the six sums cost
+// 64 cycles an instruction and a warp (the FP64 unit's issue rate on this GPU,
+// whatever the number of independent chains).
+// The block's first two warps take the chunk, whatever the block's size: one
+// order of the sums for both forms of the kernel.
+template <class M>
+__device__ __forceinline__ void chunk_tensor(const Batch& b, long long row, int np, FF (*sh)[6], M&& moment) {
+  const int w = threadIdx.x >> 5;
+  if (w < 2) {
+    FF g[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) g[c] = ff_of(0.f);
+    for (int q = threadIdx.x; q < np; q += 64) {
+      const float4 m = moment(q);
+      const float u[6] = {m.x, m.x, m.x, m.y, m.y, m.z}, v[6] = {m.x, m.y, m.z, m.y, m.z, m.z};
+#pragma unroll
+      for (int c = 0; c < 6; ++c) {
+        FF t;
+        t.hi = __fmul_rn(u[c], v[c]);
+        t.lo = __fmaf_rn(u[c], v[c], -t.hi);
+        g[c] = ff_add(g[c], t);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      g[c] = ff_warp_sum(g[c]);
+      if ((threadIdx.x & 31) == 0) sh[w][c] = g[c];
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    const FF g = ff_add(sh[0][threadIdx.x], sh[1][threadIdx.x]);
+    b.kG[row * 6 + threadIdx.x] = soft_f2d(g.hi) + soft_f2d(g.lo);
+  }
+}
+
+// Structure-factor partials, component-major so that a warp's 32 k-vectors
+// are consecutive: partial c of k-vector kl in a chunk, nv values per k.
+__device__ __forceinline__ float* ksum_part(const Batch& b, const SysDev& P, int chunk, int nv) {
+  return b.kpart + ((long long)P.kchunk_off * 10 + (long long)chunk * P.nk * nv);
+}
+
+// Several dipoles per particle: one block per (system, particle chunk, k
+// tile) of the work list kwork, one k per thread.  The particle's own terms
+// per k (S_i over its dipoles) need the per-k work here.
 template <int ND>
 __global__ void __launch_bounds__(kKBlock) ksum_kernel(Batch b, const int4* __restrict__ kwork) {
   __shared__ uint32_t sx[kKChunk * ND], sy[kKChunk * ND], sz[kKChunk * ND];
   __shared__ float smx[kKChunk * ND], smy[kKChunk * ND], smz[kKChunk * ND];
-  __shared__ double shG[6 * kKBlock / 32];
   const int4 w = kwork[blockIdx.x];
   const SysDev& P = b.sys[w.x];
-  if ((ND > 1 && P.nd <= 1) || at_limit(b, w.x)) return;  // single-dipole systems: ksum1_kernel
+  if (P.nd <= 1 || at_limit(b, w.x)) return;  // single-dipole systems: ksum1_kernel, ksum1s_kernel
   const int chunk = w.y;
   const int kl = w.z * kKBlock + threadIdx.x;
   const int ND_all = b.ndtot;
@@ -76,122 +126,83 @@ __global__ void __launch_bounds__(kKBlock) ksum_kernel(Batch b, const int4* __re
     smz[q] = b.dm[2 * ND_all + g];
   }
   __syncthreads();
-  if (ND == 1 && w.z == 0) {
-    double gl[6] = {0, 0, 0, 0, 0, 0};
-    for (int q = threadIdx.x; q < np; q += kKBlock) {
-      const double mx = smx[q], my = smy[q], mz = smz[q];
-      gl[0] += mx * mx; gl[1] += mx * my; gl[2] += mx * mz;
-      gl[3] += my * my; gl[4] += my * mz; gl[5] += mz * mz;
-    }
-    double tot[6];
-    block_sum<6, kKBlock>(gl, shG, tot);
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) b.kG[((long long)P.gch_off + chunk) * 6 + c] = tot[c];
-    }
-  }
   if (kl >= P.nk) return;
   const int4 n = b.kn[P.k_off + kl];
   const float4 kv = b.kv[P.k_off + kl];
   float acc[10];
 #pragma unroll
   for (int c = 0; c < 10; ++c) acc[c] = 0.f;
-  if (ND == 1) {
-    for (int p = 0; p < np; ++p) {
-      float c, s;
-      phase_exp(sx[p], sy[p], sz[p], n, c, s);
-      // E = exp(-i k.r) = (c, -s); U_c += m_c E
-      const float mx = smx[p], my = smy[p], mz = smz[p];
-      acc[0] += mx * c; acc[1] -= mx * s;
-      acc[2] += my * c; acc[3] -= my * s;
-      acc[4] += mz * c; acc[5] -= mz * s;
-    }
-  } else {
-    for (int p = 0; p < np; ++p) {
-      float Sr = 0.f, Si = 0.f, Ur[3] = {0.f, 0.f, 0.f}, Ui[3] = {0.f, 0.f, 0.f};
+  for (int p = 0; p < np; ++p) {
+    float Sr = 0.f, Si = 0.f, Ur[3] = {0.f, 0.f, 0.f}, Ui[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-      for (int d = 0; d < ND; ++d) {
-        if (d < nd) {
-          const int q = p * nd + d;
-          float c, s;
-          phase_exp(sx[q], sy[q], sz[q], n, c, s);
-          const float mx = smx[q], my = smy[q], mz = smz[q];
-          const float a = mx * kv.x + my * kv.y + mz * kv.z;
-          Sr += a * c;
-          Si -= a * s;
-          Ur[0] += mx * c; Ui[0] -= mx * s;
-          Ur[1] += my * c; Ui[1] -= my * s;
-          Ur[2] += mz * c; Ui[2] -= mz * s;
-        }
+    for (int d = 0; d < ND; ++d) {
+      if (d < nd) {
+        const int q = p * nd + d;
+        float c, s;
+        phase_exp(sx[q], sy[q], sz[q], n, c, s);
+        const float mx = smx[q], my = smy[q], mz = smz[q];
+        const float a = mx * kv.x + my * kv.y + mz * kv.z;
+        Sr += a * c;
+        Si -= a * s;
+        Ur[0] += mx * c; Ui[0] -= mx * s;
+        Ur[1] += my * c; Ui[1] -= my * s;
+        Ur[2] += mz * c; Ui[2] -= mz * s;
       }
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        acc[2 * c] += Ur[c];
-        acc[2 * c + 1] += Ui[c];
-        acc[7 + c] += Sr * Ur[c] + Si * Ui[c];
-      }
-      acc[6] += Sr * Sr + Si * Si;
     }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      acc[2 * c] += Ur[c];
+      acc[2 * c + 1] += Ui[c];
+      acc[7 + c] += Sr * Ur[c] + Si * Ui[c];
+    }
+    acc[6] += Sr * Sr + Si * Si;
   }
-  float* out = b.kpart + ((long long)P.kchunk_off + (long long)chunk * P.nk + kl) * 10;
-  const int nout = ND == 1 ? 6 : 10;
+  float* out = ksum_part(b, P, chunk, 10) + kl;
 #pragma unroll
-  for (int c = 0; c < 10; ++c)
-    if (c < nout) out[c] = acc[c];
+  for (int c = 0; c < 10; ++c) out[(long long)c * P.nk] = acc[c];
 }
 
-// Single-dipole systems: as ksum_kernel<1>, with each thread taking two
-// k-vectors (kl and kl + 64 of the block's k tile) in the halves of float2
-// values, so every particle read from shared memory serves two k's and the
-// six multiply-adds of U(k) issue once for both.
+// Single-dipole systems.  The particle's own terms need no per-k work:
+// |S_i(k)|^2 = (m_i.k)^2 and Re(conj(S_i) U_ic) = (m_i.k) m_ic, so
+// self(k) = k^T G k and uvslf(k) = G k with G = sum_i m_i m_i^T
+// (chunk_tensor, by the first k tile of every chunk).
+//
+// Two forms, the same IEEE operations in the same order per (particle, k)
+// and so the same bits.  ksum1: two k-vectors per thread (kl and kl + 64 of
+// the block's k tile) in the halves of float2 values, so every particle
+// read from shared memory serves two k's and the six multiply-adds of U(k)
+// issue once for both -- for batches that fill the GPU.  ksum1s: one k per
+// thread, twice the warps -- for the others, where one warp's chain of
+// sines and cosines over the chunk (the special-function unit takes a warp
+// 16 cycles per particle and k) is the time.
+struct KChunk {
+  uint4 u[kKChunk];   // fixed-point x, y, z
+  float4 m[kKChunk];  // moment
+  FF sh[2][6];
+};
+
+template <int NT>
+__device__ __forceinline__ int stage_chunk(const Batch& b, const SysDev& P, int4 w, KChunk& c) {
+  const int N = b.ndtot, p0 = w.y * kKChunk;
+  const int np = min(kKChunk, P.n - p0);
+  for (int q = threadIdx.x; q < np; q += NT) {
+    const int g = P.dip_off + p0 + q;
+    c.u[q] = make_uint4(b.dfx[g], b.dfx[N + g], b.dfx[2 * N + g], 0u);
+    c.m[q] = make_float4(b.dm[g], b.dm[N + g], b.dm[2 * N + g], 0.f);
+  }
+  __syncthreads();
+  if (w.z == 0)
+    chunk_tensor(b, (long long)P.gch_off + w.y, np, c.sh, [&](int q) { return c.m[q]; });
+  return np;
+}
+
 __global__ void __launch_bounds__(kKBlock / 2) ksum1_kernel(Batch b, const int4* __restrict__ kwork) {
-  __shared__ uint32_t sx[kKChunk], sy[kKChunk], sz[kKChunk];
-  __shared__ float4 sm[kKChunk];
-  __shared__ double shG[6 * (kKBlock / 2) / 32];
+  __shared__ KChunk ck;
   const int4 w = kwork[blockIdx.x];
   const SysDev& P = b.sys[w.x];
   if (P.nd != 1 || at_limit(b, w.x)) return;  // other systems: ksum_kernel<ND>
-  const int chunk = w.y;
-  const int t = threadIdx.x;
-  const int kl0 = w.z * kKBlock + t, kl1 = kl0 + kKBlock / 2;
-  const int ND_all = b.ndtot;
-  const int p0 = chunk * kKChunk;
-  const int np = min(kKChunk, P.n - p0);
-  for (int q = t; q < np; q += kKBlock / 2) {
-    const int g = P.dip_off + p0 + q;
-    sx[q] = b.dfx[g];
-    sy[q] = b.dfx[ND_all + g];
-    sz[q] = b.dfx[2 * ND_all + g];
-    sm[q] = make_float4(b.dm[g], b.dm[ND_all + g], b.dm[2 * ND_all + g], 0.f);
-  }
-  __syncthreads();
-  if (w.z == 0) {
-    double gl[6] = {0, 0, 0, 0, 0, 0};
-    for (int q = t; q < np; q += kKBlock / 2) {
-      const double mx = soft_f2d(sm[q].x), my = soft_f2d(sm[q].y), mz = soft_f2d(sm[q].z);
-      gl[0] += mx * mx; gl[1] += mx * my; gl[2] += mx * mz;
-      gl[3] += my * my; gl[4] += my * mz; gl[5] += mz * mz;
-    }
-    double tot[6];
-    block_sum<6, kKBlock / 2>(gl, shG, tot);
-    if (t == 0) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) b.kG[((long long)P.gch_off + chunk) * 6 + c] = tot[c];
-      // the last chunk of the system to finish adds all chunks in chunk
-      // order (the same bits whichever block it is) and rearms the counter
-      __threadfence();
-      if (atomicAdd(&b.kgcnt[w.x], 1) == P.nkchunk - 1) {
-        __threadfence();
-        double g[6] = {0, 0, 0, 0, 0, 0};
-        for (int ch = 0; ch < P.nkchunk; ++ch)
-#pragma unroll
-          for (int c = 0; c < 6; ++c) g[c] += __ldcg(&b.kG[((long long)P.gch_off + ch) * 6 + c]);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) b.kGs[6 * w.x + c] = g[c];
-        b.kgcnt[w.x] = 0;
-      }
-    }
-  }
+  const int np = stage_chunk<kKBlock / 2>(b, P, w, ck);
+  const int kl0 = w.z * kKBlock + threadIdx.x, kl1 = kl0 + kKBlock / 2;
   const bool v0 = kl0 < P.nk, v1 = kl1 < P.nk;
   if (!v0) return;
   const int4 n0 = b.kn[P.k_off + kl0];
@@ -202,11 +213,12 @@ __global__ void __launch_bounds__(kKBlock / 2) ksum1_kernel(Batch b, const int4*
 #pragma unroll 2
   for (int p = 0; p < np; ++p) {
     float c0, s0, c1, s1;
-    phase_exp(sx[p], sy[p], sz[p], n0, c0, s0);
-    phase_exp(sx[p], sy[p], sz[p], n1, c1, s1);
+    const uint4 u = ck.u[p];
+    phase_exp(u.x, u.y, u.z, n0, c0, s0);
+    phase_exp(u.x, u.y, u.z, n1, c1, s1);
     const float2 c = make_float2(c0, c1), sn = make_float2(-s0, -s1);
     // E = exp(-i k.r) = (c, -s); U_c += m_c E
-    const float4 m = sm[p];
+    const float4 m = ck.m[p];
     acc[0] = __ffma2_rn(make_float2(m.x, m.x), c, acc[0]);
     acc[1] = __ffma2_rn(make_float2(m.x, m.x), sn, acc[1]);
     acc[2] = __ffma2_rn(make_float2(m.y, m.y), c, acc[2]);
@@ -214,89 +226,173 @@ __global__ void __launch_bounds__(kKBlock / 2) ksum1_kernel(Batch b, const int4*
     acc[4] = __ffma2_rn(make_float2(m.z, m.z), c, acc[4]);
     acc[5] = __ffma2_rn(make_float2(m.z, m.z), sn, acc[5]);
   }
-  float* out0 = b.kpart + ((long long)P.kchunk_off + (long long)chunk * P.nk + kl0) * 10;
+  float* out = ksum_part(b, P, w.y, 6);
 #pragma unroll
-  for (int c = 0; c < 6; ++c) out0[c] = acc[c].x;
-  if (v1) {
-    float* out1 = b.kpart + ((long long)P.kchunk_off + (long long)chunk * P.nk + kl1) * 10;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) out1[c] = acc[c].y;
+  for (int c = 0; c < 6; ++c) {
+    out[(long long)c * P.nk + kl0] = acc[c].x;
+    if (v1) out[(long long)c * P.nk + kl1] = acc[c].y;
   }
+}
+
+__global__ void __launch_bounds__(kKBlock) ksum1s_kernel(Batch b, const int4* __restrict__ kwork) {
+  __shared__ KChunk ck;
+  const int4 w = kwork[blockIdx.x];
+  const SysDev& P = b.sys[w.x];
+  if (P.nd != 1 || at_limit(b, w.x)) return;  // other systems: ksum_kernel<ND>
+  const int np = stage_chunk<kKBlock>(b, P, w, ck);
+  const int kl = w.z * kKBlock + threadIdx.x;
+  if (kl >= P.nk) return;
+  const int4 n = b.kn[P.k_off + kl];
+  float acc[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) acc[c] = 0.f;
+#pragma unroll 8
+  for (int p = 0; p < np; ++p) {
+    float c, s;
+    const uint4 u = ck.u[p];
+    phase_exp(u.x, u.y, u.z, n, c, s);
+    const float4 m = ck.m[p];
+    acc[0] = __fmaf_rn(m.x, c, acc[0]);
+    acc[1] = __fmaf_rn(m.x, -s, acc[1]);
+    acc[2] = __fmaf_rn(m.y, c, acc[2]);
+    acc[3] = __fmaf_rn(m.y, -s, acc[3]);
+    acc[4] = __fmaf_rn(m.z, c, acc[4]);
+    acc[5] = __fmaf_rn(m.z, -s, acc[5]);
+  }
+  float* out = ksum_part(b, P, w.y, 6) + kl;
+#pragma unroll
+  for (int c = 0; c < 6; ++c) out[(long long)c * P.nk] = acc[c];
 }
 
 template <int ND>
 static void launch_ksum(const Batch& b, const int4* kwork, int nkwork, cudaStream_t s) {
-  // every single-dipole system through the single-dipole kernel, in any
+  // every single-dipole system through a single-dipole kernel, in any
   // batch, so that it gives the same bits alone and beside multi-dipole ones
-  ksum1_kernel<<<nkwork, kKBlock / 2, 0, s>>>(b, kwork);
-  if (ND > 1) ksum_kernel<ND><<<nkwork, kKBlock, 0, s>>>(b, kwork);
+  if (nkwork <= kKsumScalarMax)
+    ksum1s_kernel<<<nkwork, kKBlock, 0, s>>>(b, kwork);
+  else
+    ksum1_kernel<<<nkwork, kKBlock / 2, 0, s>>>(b, kwork);
+  if constexpr (ND > 1) ksum_kernel<ND><<<nkwork, kKBlock, 0, s>>>(b, kwork);
 }
 
-// one thread per k over the whole batch: chunk sums in FP64, S(k), and the
-// energy and pressure-tensor terms of that k (v25/functions.cpp:1839-1952)
-template <int ND>
-__global__ void kcombine_kernel(Batch b, const int2* __restrict__ kowner, double* __restrict__ kE) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= b.nktot) return;
-  const int2 ow = kowner[k];  // (system, k index within the system)
-  if (at_limit(b, ow.x)) return;
+// Chunk sums per k and val S(k): all the gather needs, nothing more.  A
+// block takes 32 consecutive k-vectors of the batch, its four warps the
+// chunks w, w + 4, ... of each (float-float); warp 0 adds the four in order.
+__global__ void __launch_bounds__(128) kstruct_kernel(Batch b, const int2* __restrict__ kowner) {
+  __shared__ FF sh[3][10][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  bool on = k < b.nktot;
+  const int2 ow = on ? kowner[k] : make_int2(0, 0);  // (system, k index within the system)
+  on = on && !at_limit(b, ow.x);
   const SysDev& P = b.sys[ow.x];
-  const int kl = ow.y;
-  // single-dipole systems (all of them when ND = 1): 6 sums per chunk and
-  // the self terms from the moment tensor, as ksum1_kernel leaves them
-  const bool one = ND == 1 || P.nd == 1;
-  const int nv = one ? 6 : 10;
-  // chunk sums in float-float (FP32 instructions; ~48 bits), then FP64
+  const int nv = P.nd == 1 ? 6 : 10;
   FF sf[10];
 #pragma unroll
-  for (int c = 0; c < 10; ++c) sf[c].hi = sf[c].lo = 0.f;
-  for (int ch = 0; ch < P.nkchunk; ++ch) {
-    const float* in = b.kpart + ((long long)P.kchunk_off + (long long)ch * P.nk + kl) * 10;
+  for (int c = 0; c < 10; ++c) sf[c] = ff_of(0.f);
+  if (on) {
+    for (int ch = w; ch < P.nkchunk; ch += 4) {
+      const float* in = ksum_part(b, P, ch, nv) + ow.y;
 #pragma unroll
-    for (int c = 0; c < 10; ++c)
-      if (c < nv) {
-        FF v;
-        v.hi = in[c];
-        v.lo = 0.f;
-        sf[c] = ff_add(sf[c], v);
-      }
+      for (int c = 0; c < 10; ++c)
+        if (c < nv) sf[c] = ff_add(sf[c], ff_of(in[(long long)c * P.nk]));
+    }
   }
+  if (w > 0) {
+#pragma unroll
+    for (int c = 0; c < 10; ++c) sh[w - 1][c][lane] = sf[c];
+  }
+  __syncthreads();
+  if (w > 0 || !on) return;
   double s[10];
 #pragma unroll
-  for (int c = 0; c < 10; ++c) s[c] = c < nv ? soft_f2d(sf[c].hi) + soft_f2d(sf[c].lo) : 0.0;
-  const double kx = b.kvec[3 * k], ky = b.kvec[3 * k + 1], kz = b.kvec[3 * k + 2];
-  if (one) {
-    const double* G = b.kGs + 6 * ow.x;
-    const double gx = G[0] * kx + G[1] * ky + G[2] * kz;
-    const double gy = G[1] * kx + G[3] * ky + G[4] * kz;
-    const double gz = G[2] * kx + G[4] * ky + G[5] * kz;
-    s[6] = kx * gx + ky * gy + kz * gz;
-    s[7] = gx;
-    s[8] = gy;
-    s[9] = gz;
-  }
-  double* ks = b.ksum + (long long)k * 10;
+  for (int c = 0; c < 10; ++c) {
+    if (c < nv) {
 #pragma unroll
-  for (int c = 0; c < 10; ++c) ks[c] = s[c];
+      for (int q = 0; q < 3; ++q) sf[c] = ff_add(sf[c], sh[q][c][lane]);
+      s[c] = soft_f2d(sf[c].hi) + soft_f2d(sf[c].lo);
+    }
+  }
+  const double kx = b.kvec[3 * k], ky = b.kvec[3 * k + 1], kz = b.kvec[3 * k + 2];
+  const double val = b.kval[k];
   const double Sr = kx * s[0] + ky * s[2] + kz * s[4];
   const double Si = kx * s[1] + ky * s[3] + kz * s[5];
-  const double val = b.kval[k];
-  const double nrm = Sr * Sr + Si * Si;
-  const double self = s[6];
-  const double en = val * 0.5 * (nrm - self);
   b.kS[k] = make_float2(soft_d2f_rn(val * Sr), soft_d2f_rn(val * Si));
-  const double pval = b.kpre[k];
-  const double kk[3] = {kx, ky, kz};
-  double* e = kE + (long long)k * 10;
-  e[0] = en;
+  double* ks = b.ksum + (long long)k * 10;
 #pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    // Re(conj(S) U_j) - uvslf_j
-    const double re = Sr * s[2 * j] + Si * s[2 * j + 1] - s[7 + j];
+  for (int c = 0; c < 10; ++c)
+    if (c < nv) ks[c] = s[c];
+}
+
+// Energy and pressure tensor of one k tile (v25/functions.cpp:1839-1952),
+// the tile's k-vectors summed in float-float into one row of kE.  Off the
+// path the forces wait for: it runs beside the gather.
+__global__ void __launch_bounds__(kKBlock) kenergy_kernel(Batch b) {
+  __shared__ double sh[10 * kKBlock / 32];
+  __shared__ double sG[6];
+  const int2 kt = b.ktile[blockIdx.x];  // (system, k tile)
+  if (at_limit(b, kt.x)) return;
+  const SysDev& P = b.sys[kt.x];
+  const bool one = P.nd == 1;
+  if (one) {  // the moment tensor over the system's chunks
+    FF g[6];
 #pragma unroll
-    for (int q = 0; q < 3; ++q)
-      e[1 + 3 * j + q] =
-          val * 0.5 * (((j == q ? 1.0 : 0.0) - pval * kk[j] * kk[q]) * (nrm - self) + 2.0 * re * kk[q]);
+    for (int c = 0; c < 6; ++c) g[c] = ff_of(0.f);
+    for (int ch = threadIdx.x; ch < P.nkchunk; ch += kKBlock) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) g[c] = ff_add(g[c], ff_from(b.kG[((long long)P.gch_off + ch) * 6 + c]));
+    }
+    double tot[6];
+    block_sum<6, kKBlock>(g, sh, tot);
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) sG[c] = tot[c];
+    }
+    __syncthreads();
+  }
+  FF e[10];
+#pragma unroll
+  for (int c = 0; c < 10; ++c) e[c] = ff_of(0.f);
+  const int kl = kt.y * kKBlock + threadIdx.x;
+  if (kl < P.nk) {
+    const long long k = P.k_off + kl;
+    const double* ks = b.ksum + k * 10;
+    const double kk[3] = {b.kvec[3 * k], b.kvec[3 * k + 1], b.kvec[3 * k + 2]};
+    double s[6], slf, uv[3];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) s[c] = ks[c];
+    if (one) {
+      uv[0] = sG[0] * kk[0] + sG[1] * kk[1] + sG[2] * kk[2];
+      uv[1] = sG[1] * kk[0] + sG[3] * kk[1] + sG[4] * kk[2];
+      uv[2] = sG[2] * kk[0] + sG[4] * kk[1] + sG[5] * kk[2];
+      slf = kk[0] * uv[0] + kk[1] * uv[1] + kk[2] * uv[2];
+    } else {
+      slf = ks[6];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) uv[c] = ks[7 + c];
+    }
+    const double Sr = kk[0] * s[0] + kk[1] * s[2] + kk[2] * s[4];
+    const double Si = kk[0] * s[1] + kk[1] * s[3] + kk[2] * s[5];
+    const double val = b.kval[k];
+    // val/2 ((delta_jq - pval k_j k_q)(|S|^2 - self) + 2 re_j k_q) with
+    // re_j = Re(conj(S) U_j) - uvslf_j
+    const double en = val * 0.5 * (Sr * Sr + Si * Si - slf);
+    const double pen = b.kpre[k] * en;
+    e[0] = ff_from(en);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const double re = Sr * s[2 * j] + Si * s[2 * j + 1] - uv[j];
+      const double row = val * re - pen * kk[j];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) e[1 + 3 * j + q] = ff_from(j == q ? row * kk[q] + en : row * kk[q]);
+    }
+  }
+  double out[10];
+  block_sum<10, kKBlock>(e, sh, out);
+  if (threadIdx.x == 0) {
+    double* dst = b.kE + (long long)blockIdx.x * 10;
+#pragma unroll
+    for (int c = 0; c < 10; ++c) dst[c] = out[c];
   }
 }
 
@@ -314,15 +410,115 @@ __device__ __forceinline__ void store_kout(const Batch& b, int g, const float* f
   b.Tk[3 * g + 2] = make_float2(mx * gy - my * gx, mx * ly - my * lx);
 }
 
-// per particle over all k of its system: force and torque (:1853-1925)
+// The gathers: per particle over all k of its system, force and torque
+// (:1853-1925).  The sums of a k tile are plain FP32, the tiles are added in
+// order (Kahan), and a system of SysDev::kgs > 1 parts adds its parts'
+// sums the same way -- the order of every addition is the system's own.
+//
+// The work of one particle block goes to one block (it walks every tile) or
+// to one block per tile (SysDev::kgt > 1): each leaves its tile's sums in the
+// partial set of (particle block, tile) and the block that finishes last
+// adds the tiles, in the same order, so the bits are the same either way and
+// whichever block ends last.
+constexpr int kSet = kPartBlock * 6;  // floats of a partial set per dipole: 6 components x kPartBlock particles
+__device__ __forceinline__ float* ktile_set(const Batch& b, const SysDev& P, int slot, int tile) {
+  const long long tiles = cdiv(P.nk, kKBlock);
+  return b.kgpart + ((long long)P.kgp_off + ((slot - P.blk_off) * tiles + tile) * P.nd) * kSet;
+}
+
+// one Kahan addition: (fo, fc) += v
+__device__ __forceinline__ void kahan(float& fo, float& fc, float v) {
+  const float y = __fadd_rn(v, -fc);
+  const float t = __fadd_rn(fo, y);
+  fc = __fadd_rn(__fadd_rn(t, -fo), -y);
+  fo = t;
+}
+
+// the tile sums of local particle p, dipole d, in the order described above
+__device__ __forceinline__ void ktile_combine(const Batch& b, const SysDev& P, int slot, int p, int d, float* fo,
+                                              float* fc) {
+  const int tiles = cdiv(P.nk, kKBlock), tpk = cdiv(tiles, P.kgs);
+  float cs[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) fo[c] = fc[c] = cs[c] = 0.f;
+  for (int q = 0; q < P.kgs; ++q) {
+    float po[6], pc[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) po[c] = pc[c] = 0.f;
+    const int t1 = min(tiles, (q + 1) * tpk);
+#pragma unroll 4
+    for (int t = q * tpk; t < t1; ++t) {
+      const float* set = ktile_set(b, P, slot, t) + d * kSet + p;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) kahan(po[c], pc[c], __ldcg(set + c * kPartBlock));
+    }
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      if (P.kgs == 1) {
+        fo[c] = po[c];
+        fc[c] = pc[c];
+      } else {
+        kahan(fo[c], fc[c], po[c]);
+        cs[c] = __fadd_rn(cs[c], pc[c]);
+      }
+    }
+  }
+  if (P.kgs > 1) {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) fc[c] = __fadd_rn(fc[c], cs[c]);
+  }
+}
+
+// Counts a tile of a particle block done; true for every thread of the block
+// that finishes last, which then sees every other block's sums (each thread
+// fences its own before the count, and again after it).
+__device__ __forceinline__ bool ktile_last(const Batch& b, const SysDev& P, int slot, int* last) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int tiles = cdiv(P.nk, kKBlock);
+    *last = atomicAdd(&b.kgdone[slot], 1) == tiles - 1;
+    if (*last) b.kgdone[slot] = 0;
+  }
+  __syncthreads();
+  if (!*last) return false;
+  __threadfence();
+  return true;
+}
+
+// the k-vectors of a work item: tile wk.y, or all of them (wk.y < 0)
+__device__ __forceinline__ void ktile_range(const SysDev& P, int2 wk, int& kb, int& ke) {
+  kb = wk.y < 0 ? 0 : wk.y * kKBlock;
+  ke = wk.y < 0 ? P.nk : min(P.nk, kb + kKBlock);
+}
+
+struct KTile {
+  int4 n[kKBlock];
+  float4 v[kKBlock];  // kx, ky, kz, val
+  float2 S[kKBlock];  // val * S(k)
+  int last;
+};
+template <int NT>
+__device__ __forceinline__ int stage_ktile(const Batch& b, const SysDev& P, int k0, int ke, KTile& kt) {
+  const int nk = min(kKBlock, ke - k0);
+  __syncthreads();
+  for (int q = threadIdx.x; q < nk; q += NT) {
+    kt.n[q] = b.kn[P.k_off + k0 + q];
+    kt.v[q] = b.kv[P.k_off + k0 + q];
+    kt.S[q] = b.kS[P.k_off + k0 + q];
+  }
+  __syncthreads();
+  return nk;
+}
+
+// several dipoles per particle, one particle per thread
 template <int ND>
 __global__ void __launch_bounds__(kPartBlock) kgather_kernel(Batch b) {
-  __shared__ int4 skn[kKBlock];
-  __shared__ float4 skv[kKBlock];
-  __shared__ float2 sks[kKBlock];
-  const int2 bk = b.blk[blockIdx.x];
+  __shared__ KTile kt;
+  const int2 wk = b.kgwork[blockIdx.x];  // (particle block, tile)
+  const int2 bk = b.blk[wk.x];
   const SysDev& P = b.sys[bk.x];
-  if ((ND > 1 && P.nd <= 1) || at_limit(b, bk.x)) return;  // single-dipole systems: kgather1 / kgather1s
+  if (P.nd <= 1 || at_limit(b, bk.x)) return;  // single-dipole systems: kgather1 / kgather1s
   const int i = bk.y + threadIdx.x;  // batch particle index
   const bool ok = i < P.part_off + P.n;
   const int nd = P.nd;
@@ -341,35 +537,28 @@ __global__ void __launch_bounds__(kPartBlock) kgather_kernel(Batch b) {
     my[d] = v ? b.dm[ND_all + g] : 0.f;
     mz[d] = v ? b.dm[2 * ND_all + g] : 0.f;
   }
-  // outer accumulators (Kahan-compensated) and per-tile FP32 sums
-  float fo[ND][6], fc[ND][6];
+  float fo[ND][6], fc[ND][6], ft[ND][6];
 #pragma unroll
   for (int d = 0; d < ND; ++d)
 #pragma unroll
-    for (int c = 0; c < 6; ++c) fo[d][c] = fc[d][c] = 0.f;
+    for (int c = 0; c < 6; ++c) fo[d][c] = fc[d][c] = ft[d][c] = 0.f;
 
   uint32_t ph[ND];
 #pragma unroll
   for (int d = 0; d < ND; ++d) ph[d] = 0u;
   bool have = false;
-  for (int k0 = 0; k0 < P.nk; k0 += kKBlock) {
-    const int nk = min(kKBlock, P.nk - k0);
-    __syncthreads();
-    for (int q = threadIdx.x; q < nk; q += blockDim.x) {
-      skn[q] = b.kn[P.k_off + k0 + q];
-      skv[q] = b.kv[P.k_off + k0 + q];
-      sks[q] = b.kS[P.k_off + k0 + q];
-    }
-    __syncthreads();
-    float ft[ND][6];
+  int kb, ke;
+  ktile_range(P, wk, kb, ke);
+  for (int k0 = kb; k0 < ke; k0 += kKBlock) {
+    const int nk = stage_ktile<kPartBlock>(b, P, k0, ke, kt);
 #pragma unroll
     for (int d = 0; d < ND; ++d)
 #pragma unroll
       for (int c = 0; c < 6; ++c) ft[d][c] = 0.f;
     for (int q = 0; q < nk; ++q) {
-      const int4 n = skn[q];
-      const float4 kv = skv[q];  // kx, ky, kz, val
-      const float2 vS = sks[q];  // val * S(k)
+      const int4 n = kt.n[q];
+      const float4 kv = kt.v[q];
+      const float2 vS = kt.S[q];
       float Ec[ND], Es[ND], a[ND];
       float Sr = 0.f, Si = 0.f;
 #pragma unroll
@@ -406,52 +595,26 @@ __global__ void __launch_bounds__(kPartBlock) kgather_kernel(Batch b) {
 #pragma unroll
     for (int d = 0; d < ND; ++d)
 #pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        const float y = ft[d][c] - fc[d][c];
-        const float t = fo[d][c] + y;
-        fc[d][c] = (t - fo[d][c]) - y;
-        fo[d][c] = t;
+      for (int c = 0; c < 6; ++c) kahan(fo[d][c], fc[d][c], ft[d][c]);
+  }
+  if (wk.y >= 0) {  // one tile: leave its sums, the last block combines
+    const int slot = blk_slot(P, bk);
+    float* mine = ktile_set(b, P, slot, wk.y) + threadIdx.x;
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+      if (d < nd) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) mine[d * kSet + c * kPartBlock] = ft[d][c];
       }
+    if (!ktile_last(b, P, slot, &kt.last)) return;
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+      if (d < nd) ktile_combine(b, P, slot, threadIdx.x, d, fo[d], fc[d]);
   }
   if (!ok) return;
 #pragma unroll
   for (int d = 0; d < ND; ++d)
     if (d < nd) store_kout(b, gd0 + d, fo[d], fc[d], mx[d], my[d], mz[d]);
-}
-
-// Split gathers (large single-dipole systems, SysDev::kgs > 1): block part
-// ks of a particle block takes the k tiles [ks tpk, (ks + 1) tpk), tpk =
-// ceil(tiles / kgs), and leaves its Kahan sums (fo, fc per component) in
-// its partial set; the block that finishes last adds the parts in part
-// order (Kahan over the sums, the compensations apart) and stores the
-// result, so the order of the sums does not depend on which block ends last.
-__device__ __forceinline__ void kpart_range(const SysDev& P, int ks, int& k0, int& k1) {
-  const int tpk = cdiv(cdiv(P.nk, kKBlock), P.kgs) * kKBlock;
-  k0 = min(P.nk, ks * tpk);
-  k1 = min(P.nk, (ks + 1) * tpk);
-}
-__device__ __forceinline__ float* kpart_set(const Batch& b, const SysDev& P, int slot, int ks) {
-  return b.kgpart + ((long long)P.kgp_off + (long long)(slot - P.blk_off) * P.kgs + ks) * kPartBlock * 12;
-}
-// the parts of local particle p of a particle block, added in part order
-__device__ __forceinline__ void kpart_combine(const Batch& b, const SysDev& P, int slot, int p, float* fo,
-                                              float* fc) {
-  float cs[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) fo[c] = fc[c] = cs[c] = 0.f;
-  for (int q = 0; q < P.kgs; ++q) {
-    const float* part = kpart_set(b, P, slot, q) + p * 12;
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      const float y = __fadd_rn(__ldcg(part + c), -fc[c]);
-      const float tt = __fadd_rn(fo[c], y);
-      fc[c] = __fadd_rn(__fadd_rn(tt, -fo[c]), -y);
-      fo[c] = tt;
-      cs[c] = __fadd_rn(cs[c], __ldcg(part + 6 + c));
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < 6; ++c) fc[c] = __fadd_rn(fc[c], cs[c]);
 }
 
 // Single-dipole systems: a thread takes two particles, i and i + 64 of its
@@ -467,16 +630,13 @@ __device__ __forceinline__ float2 bc(float a) { return make_float2(a, a); }
 }  // namespace
 
 __global__ void __launch_bounds__(kPartBlock / 2) kgather1_kernel(Batch b) {
-  __shared__ int4 skn[kKBlock];
-  __shared__ float4 skv[kKBlock];
-  __shared__ float2 sks[kKBlock];
-  __shared__ int last;
-  const int2 wk = b.kgwork[blockIdx.x];  // (particle block, part)
+  __shared__ KTile kt;
+  const int2 wk = b.kgwork[blockIdx.x];  // (particle block, tile)
   const int2 bk = b.blk[wk.x];
   const SysDev& P = b.sys[bk.x];
   if (P.nd != 1 || at_limit(b, bk.x)) return;  // other systems: kgather_kernel<ND>
   int kb, ke;
-  kpart_range(P, wk.y, kb, ke);
+  ktile_range(P, wk, kb, ke);
   const int t = threadIdx.x;
   const int i0 = bk.y + t, i1 = i0 + kPartBlock / 2;
   const int iend = P.part_off + P.n;
@@ -491,29 +651,21 @@ __global__ void __launch_bounds__(kPartBlock / 2) kgather1_kernel(Batch b) {
   const float2 my = pk(ok0 ? b.dm[ND_all + g0] : 0.f, ok1 ? b.dm[ND_all + g1] : 0.f);
   const float2 mz = pk(ok0 ? b.dm[2 * ND_all + g0] : 0.f, ok1 ? b.dm[2 * ND_all + g1] : 0.f);
   // outer accumulators (Kahan-compensated) of the per-tile sums
-  float2 fo[6], fc[6];
+  float2 fo[6], fc[6], ft[6];
 #pragma unroll
-  for (int c = 0; c < 6; ++c) fo[c] = fc[c] = bc(0.f);
+  for (int c = 0; c < 6; ++c) fo[c] = fc[c] = ft[c] = bc(0.f);
 
   uint32_t ph0 = 0u, ph1 = 0u;
   bool have = false;  // a phase from the previous k-vector (the first of the range computes its own)
   for (int k0 = kb; k0 < ke; k0 += kKBlock) {
-    const int nk = min(kKBlock, ke - k0);
-    __syncthreads();
-    for (int q = t; q < nk; q += kPartBlock / 2) {
-      skn[q] = b.kn[P.k_off + k0 + q];
-      skv[q] = b.kv[P.k_off + k0 + q];
-      sks[q] = b.kS[P.k_off + k0 + q];
-    }
-    __syncthreads();
-    float2 ft[6];
+    const int nk = stage_ktile<kPartBlock / 2>(b, P, k0, ke, kt);
 #pragma unroll
     for (int c = 0; c < 6; ++c) ft[c] = bc(0.f);
 #pragma unroll 2
     for (int q = 0; q < nk; ++q) {
-      const int4 n = skn[q];
-      const float4 kv = skv[q];  // kx, ky, kz, val
-      const float2 vS = sks[q];  // val * S(k)
+      const int4 n = kt.n[q];
+      const float4 kv = kt.v[q];
+      const float2 vS = kt.S[q];
       float c0, s0, c1, s1;
       ph0 = phase_next(ph0, have, ux0, uy0, uz0, n);
       ph1 = phase_next(ph1, have, ux1, uy1, uz1, n);
@@ -543,32 +695,25 @@ __global__ void __launch_bounds__(kPartBlock / 2) kgather1_kernel(Batch b) {
     }
   }
   float a0[6], c0[6], a1[6], c1[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) {
-    a0[c] = fo[c].x;
-    c0[c] = fc[c].x;
-    a1[c] = fo[c].y;
-    c1[c] = fc[c].y;
-  }
-  if (P.kgs > 1) {  // a part: leave the sums, the last part combines
+  if (wk.y >= 0) {  // one tile: leave its sums, the last block combines
     const int slot = blk_slot(P, bk);
-    float* mine = kpart_set(b, P, slot, wk.y);
+    float* mine = ktile_set(b, P, slot, wk.y) + t;
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      mine[t * 12 + c] = a0[c];
-      mine[t * 12 + 6 + c] = c0[c];
-      mine[(t + kPartBlock / 2) * 12 + c] = a1[c];
-      mine[(t + kPartBlock / 2) * 12 + 6 + c] = c1[c];
+      mine[c * kPartBlock] = ft[c].x;
+      mine[c * kPartBlock + kPartBlock / 2] = ft[c].y;
     }
-    __threadfence();
-    __syncthreads();
-    if (t == 0) last = atomicAdd(&b.kgdone[slot], 1) == P.kgs - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    kpart_combine(b, P, slot, t, a0, c0);
-    kpart_combine(b, P, slot, t + kPartBlock / 2, a1, c1);
-    if (t == 0) b.kgdone[slot] = 0;
+    if (!ktile_last(b, P, slot, &kt.last)) return;
+    ktile_combine(b, P, slot, t, 0, a0, c0);
+    ktile_combine(b, P, slot, t + kPartBlock / 2, 0, a1, c1);
+  } else {
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      a0[c] = fo[c].x;
+      c0[c] = fc[c].x;
+      a1[c] = fo[c].y;
+      c1[c] = fc[c].y;
+    }
   }
   if (ok0) store_kout(b, g0, a0, c0, mx.x, my.x, mz.x);
   if (ok1) store_kout(b, g1, a1, c1, mx.y, my.y, mz.y);
@@ -580,16 +725,13 @@ __global__ void __launch_bounds__(kPartBlock / 2) kgather1_kernel(Batch b) {
 // the packed kernel (explicit _rn intrinsics, no contraction), so the two
 // forms give identical bits and the autotuner may pick either.
 __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
-  __shared__ int4 skn[kKBlock];
-  __shared__ float4 skv[kKBlock];
-  __shared__ float2 sks[kKBlock];
-  __shared__ int last;
-  const int2 wk = b.kgwork[blockIdx.x];  // (particle block, part)
+  __shared__ KTile kt;
+  const int2 wk = b.kgwork[blockIdx.x];  // (particle block, tile)
   const int2 bk = b.blk[wk.x];
   const SysDev& P = b.sys[bk.x];
   if (P.nd != 1 || at_limit(b, bk.x)) return;  // other systems: kgather_kernel<ND>
   int kb, ke;
-  kpart_range(P, wk.y, kb, ke);
+  ktile_range(P, wk, kb, ke);
   const int t = threadIdx.x;
   const int i0 = bk.y + t;
   const bool ok0 = i0 < P.part_off + P.n;
@@ -598,28 +740,20 @@ __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
   const uint32_t ux0 = b.dfx[g0], uy0 = b.dfx[ND_all + g0], uz0 = b.dfx[2 * ND_all + g0];
   const float mx = ok0 ? b.dm[g0] : 0.f, my = ok0 ? b.dm[ND_all + g0] : 0.f,
               mz = ok0 ? b.dm[2 * ND_all + g0] : 0.f;
-  float fo[6], fc[6];
+  float fo[6], fc[6], ft[6];
 #pragma unroll
-  for (int c = 0; c < 6; ++c) fo[c] = fc[c] = 0.f;
+  for (int c = 0; c < 6; ++c) fo[c] = fc[c] = ft[c] = 0.f;
   uint32_t ph = 0u;
   bool have = false;
   for (int k0 = kb; k0 < ke; k0 += kKBlock) {
-    const int nk = min(kKBlock, ke - k0);
-    __syncthreads();
-    for (int q = t; q < nk; q += kPartBlock) {
-      skn[q] = b.kn[P.k_off + k0 + q];
-      skv[q] = b.kv[P.k_off + k0 + q];
-      sks[q] = b.kS[P.k_off + k0 + q];
-    }
-    __syncthreads();
-    float ft[6];
+    const int nk = stage_ktile<kPartBlock>(b, P, k0, ke, kt);
 #pragma unroll
     for (int c = 0; c < 6; ++c) ft[c] = 0.f;
-#pragma unroll 2
+#pragma unroll 4
     for (int q = 0; q < nk; ++q) {
-      const int4 n = skn[q];
-      const float4 kv = skv[q];
-      const float2 vS = sks[q];
+      const int4 n = kt.n[q];
+      const float4 kv = kt.v[q];
+      const float2 vS = kt.S[q];
       float c, sn;
       ph = phase_next(ph, have, ux0, uy0, uz0, n);
       have = true;
@@ -638,29 +772,15 @@ __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
       ft[5] = __fmaf_rn(fT, kv.z, ft[5]);
     }
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      const float y = __fadd_rn(ft[c], -fc[c]);
-      const float tt = __fadd_rn(fo[c], y);
-      fc[c] = __fadd_rn(__fadd_rn(tt, -fo[c]), -y);
-      fo[c] = tt;
-    }
+    for (int c = 0; c < 6; ++c) kahan(fo[c], fc[c], ft[c]);
   }
-  if (P.kgs > 1) {  // a part: leave the sums, the last part combines
+  if (wk.y >= 0) {  // one tile: leave its sums, the last block combines
     const int slot = blk_slot(P, bk);
-    float* mine = kpart_set(b, P, slot, wk.y) + t * 12;
+    float* mine = ktile_set(b, P, slot, wk.y) + t;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      mine[c] = fo[c];
-      mine[6 + c] = fc[c];
-    }
-    __threadfence();
-    __syncthreads();
-    if (t == 0) last = atomicAdd(&b.kgdone[slot], 1) == P.kgs - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    kpart_combine(b, P, slot, t, fo, fc);
-    if (t == 0) b.kgdone[slot] = 0;
+    for (int c = 0; c < 6; ++c) mine[c * kPartBlock] = ft[c];
+    if (!ktile_last(b, P, slot, &kt.last)) return;
+    ktile_combine(b, P, slot, t, 0, fo, fc);
   }
   if (ok0) store_kout(b, g0, fo, fc, mx, my, mz);
 }
@@ -671,46 +791,39 @@ static void launch_kgather(const Batch& b, cudaStream_t s) {
     kgather1s_kernel<<<b.nkgwork, kPartBlock, 0, s>>>(b);
   else
     kgather1_kernel<<<b.nkgwork, kPartBlock / 2, 0, s>>>(b);
-  if (ND > 1) kgather_kernel<ND><<<b.nblk, kPartBlock, 0, s>>>(b);
+  if constexpr (ND > 1) kgather_kernel<ND><<<b.nkgwork, kPartBlock, 0, s>>>(b);
 }
 
 template <int ND>
-static void launch_kspace_nd(const Batch& b, const int4* kwork, int nkwork, const int2* kowner,
-                             double* kE, cudaStream_t s) {
-  if (b.nktot == 0) return;
-  if (nkwork > 0) launch_ksum<ND>(b, kwork, nkwork, s);
-  kcombine_kernel<ND><<<cdiv(b.nktot, 128), 128, 0, s>>>(b, kowner, kE);
-  launch_kgather<ND>(b, s);
-}
-
-template <int ND>
-static void kspace_part_nd(const Batch& b, const int4* kwork, int nkwork, const int2* kowner,
-                           double* kE, int part, cudaStream_t s) {
+static void kspace_part_nd(const Batch& b, const int4* kwork, int nkwork, const int2* kowner, int part,
+                           cudaStream_t s) {
   if (b.nktot == 0) return;
   if (part == 0 && nkwork > 0) launch_ksum<ND>(b, kwork, nkwork, s);
-  if (part == 1) kcombine_kernel<ND><<<cdiv(b.nktot, 128), 128, 0, s>>>(b, kowner, kE);
+  if (part == 1) kstruct_kernel<<<cdiv(b.nktot, 32), 128, 0, s>>>(b, kowner);
   if (part == 2) launch_kgather<ND>(b, s);
+  if (part == 3) kenergy_kernel<<<b.nktile, kKBlock, 0, s>>>(b);
 }
 
-// one of the three k-space kernels (0: ksum, 1: kcombine, 2: kgather)
-void launch_kspace_parts(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner,
-                         double* kE, int part, cudaStream_t s) {
+// one of the four k-space stages (0: ksum, 1: kstruct, 2: kgather, 3:
+// kenergy; 2 and 3 need 0 and 1 before them, and may run side by side)
+void launch_kspace_parts(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, int part,
+                         cudaStream_t s) {
   if (maxnd <= 1)
-    kspace_part_nd<1>(b, kwork, nkwork, kowner, kE, part, s);
+    kspace_part_nd<1>(b, kwork, nkwork, kowner, part, s);
   else if (maxnd == 2)
-    kspace_part_nd<2>(b, kwork, nkwork, kowner, kE, part, s);
+    kspace_part_nd<2>(b, kwork, nkwork, kowner, part, s);
   else
-    kspace_part_nd<4>(b, kwork, nkwork, kowner, kE, part, s);
+    kspace_part_nd<4>(b, kwork, nkwork, kowner, part, s);
 }
 
-void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner,
-                   double* kE, cudaStream_t s) {
-  if (maxnd <= 1)
-    launch_kspace_nd<1>(b, kwork, nkwork, kowner, kE, s);
-  else if (maxnd == 2)
-    launch_kspace_nd<2>(b, kwork, nkwork, kowner, kE, s);
-  else
-    launch_kspace_nd<4>(b, kwork, nkwork, kowner, kE, s);
+// once per device: the step's memory split
+cudaError_t prepare_kspace() {
+  return set_carveout(ksum1_kernel, ksum1s_kernel, ksum_kernel<2>, ksum_kernel<4>, kstruct_kernel, kenergy_kernel,
+                      kgather1_kernel, kgather1s_kernel, kgather_kernel<2>, kgather_kernel<4>);
+}
+
+void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, cudaStream_t s) {
+  for (int part : {0, 1, 3, 2}) launch_kspace_parts(b, maxnd, kwork, nkwork, kowner, part, s);
 }
 
 }  // namespace mdsc

@@ -856,12 +856,18 @@ size_t real_pairs_smem_bytes(int tn) {
 }
 
 // Once per device, outside any stream capture: the largest dynamic shared
-// memory a shared-table tile launch may ask for.
+// memory a shared-table tile launch may ask for, and the step's memory split.
 cudaError_t prepare_real_pairs() {
   const int most = (int)real_pairs_smem_bytes(kSmemTableMax);
   cudaError_t e = cudaFuncSetAttribute(real_pairs_smem_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(real_pairs_smem_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+  // not near_pass: its table lookups want the L1, and no tiles run beside it
+  if (e == cudaSuccess)
+    e = set_carveout(real_sum_kernel, strip_energy_kernel, real_pairs_kernel<true, 1, kAnalytic>,
+                     real_pairs_kernel<false, 1, kAnalytic>, real_pairs_kernel<true, 2, kAnalytic>,
+                     real_pairs_kernel<false, 2, kAnalytic>, real_pairs_kernel<true, 4, kAnalytic>,
+                     real_pairs_kernel<false, 4, kAnalytic>);
   return e;
 }
 

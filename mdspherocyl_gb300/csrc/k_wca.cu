@@ -673,6 +673,10 @@ void launch_list_build(const Batch& b, int force_all, cudaStream_t s) {
   if (ncb) cell_bin_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
   list_build_kernel<<<b.nblk + ncb, kPartBlock, 0, s>>>(b);
 }
+// once per device: the step's memory split
+cudaError_t prepare_wca() {
+  return set_carveout(list_prep_kernel, cell_bin_kernel, list_build_kernel, wca_screen_kernel, wca_eval_kernel);
+}
 void launch_near_pass(const Batch& b, int mode, cudaStream_t s);  // k_real.cu
 
 void launch_wca(const Batch& b, int near_mode, cudaStream_t s) {

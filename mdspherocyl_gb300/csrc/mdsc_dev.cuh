@@ -59,6 +59,26 @@ constexpr int kRedGroups = 5;  // blocks per system of the reduction kernel
 // modes of the per-system reduction kernel
 enum : int { kRedEnergies = 1, kRedStep = 2 };
 
+// The kernels that run side by side in the step (tiles, k-space, lists and
+// WCA) ask for one split of the SM's memory between shared memory and L1, in
+// percent shared: half holds the tiles' 20 blocks per SM.  A block whose
+// kernel prefers another split than the SM has waits until the SM is empty,
+// so a chain beside the tiles could start behind them: 1500 rods with two
+// dipoles each took 0.213 ms per step with the driver's own choices, 0.120
+// this way (0.112 to 0.117 with only some of them set, but then 0.7060 for
+// the 256-replica mix against 0.688).  A quarter: 0.747 ms on the mix (fewer
+// tiles per SM); all shared: 0.703.
+constexpr int kStepCarveout = 50;
+template <class... K>
+cudaError_t set_carveout(K... kernels) {
+  cudaError_t e = cudaSuccess;
+  ((e = e == cudaSuccess
+            ? cudaFuncSetAttribute(kernels, cudaFuncAttributePreferredSharedMemoryCarveout, kStepCarveout)
+            : e),
+   ...);
+  return e;
+}
+
 // Per-system constants (read-only during a step).
 struct SysDev {
   int n, nd, ndip;
@@ -71,8 +91,10 @@ struct SysDev {
   int k_off, nk;        // k-vector range
   int rt_off, rt_n;     // real-space table entries (A, B, C of the reference's tabul)
   int kchunk_off, nkchunk;  // structure-factor partial range (chunks of kKChunk particles)
-  int kgs;                  // k-space gather parts: the k tiles split over kgs blocks per particle block
-  int kgp_off;              // first partial set of the system (kgs > 1)
+  int kgs;                  // k-space gather: the tiles' sums are added in kgs parts (arithmetic only)
+  int kgt;                  // blocks per particle block of the gather: 1 (it walks every tile) or one per tile
+  int kgp_off;              // first partial set of the system
+  int kt_off, nkt;          // k tiles: the system's energy rows
   int gch_off, pad_g;       // first chunk of the system in the G-tensor partials
   int blk_off, nblk;        // per-particle block range
   int cl_fr;
@@ -242,18 +264,18 @@ struct Batch {
   double* kval;  // val per k (FP64)
   double* kvec;  // 3 per k: the k vector in FP64
   double* kpre;  // pval per k (2 (a4 + 1/k^2)) for the pressure tensor
-  float* kpart;  // structure-factor partials: 10 per (chunk, k)
-  double* ksum;  // 10 per k: uve (6), self, uvslf (3) -- FP64
+  float* kpart;  // structure-factor partials per (chunk, component, k): 6 or 10 components
+  double* ksum;  // 10 per k: uve (6), and for several dipoles self, uvslf (3) -- FP64
   float2* kS;    // val * S(k) per k, FP32 for the gather
-  double* kE;    // 10 per k: energy and pressure-tensor terms
+  double* kE;    // 10 per k tile: energy and pressure tensor
+  int2* ktile;   // (system, tile) of every k tile
+  int nktile;
   double* kG;    // 6 per particle chunk: sum of m m^T (one dipole per particle)
-  double* kGs;   // 6 per system: the chunk sums added in chunk order
-  int* kgcnt;    // per system: chunks done this step (the last one adds them)
   int* icnt;     // per system: first-half blocks done this step (the last one sets xi_mid)
-  int2* kgwork;  // (particle block, part) of every k-space gather block
+  int2* kgwork;  // (particle block, k tile or -1: all) of every k-space gather block
   int nkgwork;
-  float* kgpart; // partial gather sums of split systems: per (particle block, part) kPartBlock x 12
-  int* kgdone;   // per particle block: parts done this launch (the last one combines them)
+  float* kgpart; // tile sums of split gathers: per (particle block, tile, dipole) 6 x kPartBlock
+  int* kgdone;   // per particle block: tiles done this launch (the last one combines them)
   float2* Fk;    // 3 ndip: k-space force on each dipole, float-float (hi, lo)
   float2* Tk;    // 3 ndip: k-space torque m x G, float-float
   // integrator partials, per block

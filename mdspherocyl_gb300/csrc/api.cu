@@ -30,6 +30,7 @@ void launch_near_pass(const Batch& b, int mode, cudaStream_t s);
 void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, cudaStream_t s);
 void launch_derive(const Batch& b, cudaStream_t s);
 void launch_integrate_first(const Batch& b, cudaStream_t s);
+void launch_xi_mid(const Batch& b, cudaStream_t s);
 void launch_finalize(const Batch& b, int mode, cudaStream_t s);
 void launch_reduce_obs(const Batch& b, int mode, cudaStream_t s);
 void launch_order_terms(const Batch& b, cudaStream_t s);
@@ -85,7 +86,7 @@ struct Layout {
   std::vector<float4> rtab;  // real-space tables of every system (filled by fill_tables)
   size_t rtab_n = 0;         // float4 slots the tables take (2 per entry)
   std::vector<double> kval, kpre, kvec;
-  std::vector<int2> blk, kowner;
+  std::vector<int2> blk, wblk, kowner;
   std::vector<int2> bstrips;  // strips of the systems whose tile energies are summed per strip
   std::vector<int2> kgwork;   // (particle block, tile) of the k-space gather
   std::vector<int2> ktile;    // (system, k tile)
@@ -352,6 +353,9 @@ void make_layout(const mdsc_system_desc* descs, int nsys, Layout& Lo) {
     P.blk_off = blk;
     P.nblk = cdiv(d.n, kPartBlock);
     for (int k = 0; k < P.nblk; ++k) Lo.blk.push_back(make_int2(s, part + k * kPartBlock));
+    P.w_off = (int)Lo.wblk.size();
+    P.nw = cdiv(d.n, 32);
+    for (int k = 0; k < P.nw; ++k) Lo.wblk.push_back(make_int2(s, part + k * 32));
     // the k-space gather of a large single-dipole system adds its k tiles in
     // parts (a function of the system only, so the same bits alone and in
     // any batch)
@@ -430,8 +434,8 @@ void make_layout(const mdsc_system_desc* descs, int nsys, Layout& Lo) {
   // be the last wave on the GPU.  Kernels find a block's partial-sum slot
   // from its particle range (blk_slot), so results do not depend on this
   // order.
-  std::stable_sort(Lo.blk.begin(), Lo.blk.end(),
-                   [&](const int2& u, const int2& v) { return descs[u.x].n > descs[v.x].n; });
+  for (std::vector<int2>* w : {&Lo.blk, &Lo.wblk})
+    std::stable_sort(w->begin(), w->end(), [&](const int2& u, const int2& v) { return descs[u.x].n > descs[v.x].n; });
   // the k-space gather's blocks, in the launch order above (entries index
   // the sorted block list): one per particle block where those fill the GPU,
   // one per particle block and k tile where they do not (and always for
@@ -511,7 +515,6 @@ void carve(Arena& A, const Layout& Lo, int nsys, Batch& b, int4** kwork, int2** 
   b.wlist_n = A.take<int>(1);
   b.wown = A.take<double>(n * kMaxC * 6);
   b.wev = A.take<double>(n * kMaxC * 11);
-  b.wcaE = A.take<double>(11 * nb);
   b.wcand = A.take<int>(n * kMaxC);
   b.wcnt = A.take<int>(n);
   b.win = A.take<int>(n * kMaxC);
@@ -529,12 +532,15 @@ void carve(Arena& A, const Layout& Lo, int nsys, Batch& b, int4** kwork, int2** 
   b.kE = A.take<double>(10 * std::max<size_t>(Lo.ktile.size(), 1));
   b.ktile = A.take<int2>(std::max<size_t>(Lo.ktile.size(), 1));
   b.kG = A.take<double>(6 * (size_t)std::max(Lo.nchunks, 1));
-  b.icnt = A.take<int>(std::max(nsys, 1));
   b.Fk = A.take<float2>(3 * nd);
   b.Tk = A.take<float2>(3 * nd);
-  b.kin1 = A.take<double>(2 * nb);
+  const size_t nw = 3 * std::max<size_t>(Lo.wblk.size(), 1);
+  b.krow = A.take<float2>(2 * nw);
+  b.krow2 = A.take<float2>(5 * nw);
+  b.wrow = A.take<float2>(4 * nw);
+  b.dmax = A.take<float>(nw / 3);
+  b.wblk = A.take<int2>(nw / 3);
   b.kin2 = A.take<double>(9 * nb);
-  b.dmax = A.take<double>(nb);
   b.obk = A.take<double>(12 * nb);
   b.blk = A.take<int2>(nb);
   b.ccnt = A.take<int>(std::max(Lo.ncellcap, 1));
@@ -565,7 +571,8 @@ struct mdsc_batch {
   int num_sms = 0;  // streaming multiprocessors of the device
   int nsys = 0;
   cudaStream_t st = nullptr, s2 = nullptr, s3 = nullptr, s4 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_j2 = nullptr, ev_j3 = nullptr, ev_j4 = nullptr, ev_k = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_j2 = nullptr, ev_j3 = nullptr, ev_j4 = nullptr, ev_k = nullptr,
+              ev_mid = nullptr;
   // mdsc_step_io: the stream that takes positions and orientations home
   // while a step's forces are computed, and the event its graph records
   // once they are final
@@ -775,9 +782,9 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   cudaStreamWaitEvent(B->s3, B->ev_fork, 0);
   launch_list_build(b, 0, B->st);
   launch_wca(b, 1, B->st);  // the cutoff systems' real space in their neighbour pass, after their list
-  // order terms, the list build's decision and scan (+ the cell binning),
-  // the WCA screen and evaluation (+ the cutoff pass)
-  launches += 5 + (b.cells && b.ncellblk ? 1 : 0) + (b.any_rc ? 1 : 0);
+  // xi at mid-step, order terms, the list build's decision and scan (+ the cell
+  // binning), the WCA screen and evaluation (+ the cutoff pass)
+  launches += 6 + (b.cells && b.ncellblk ? 1 : 0) + (b.any_rc ? 1 : 0);
   launch_real_pairs(b, B->lo.multi, B->s2);
   launch_real_sum(b, B->s2);
   launches += b.ntiles > 0 ? 2 + (b.nbstrips > 0 ? 1 : 0) : 0;
@@ -788,8 +795,10 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   kpart(1, B->s3);
   cudaEventRecord(B->ev_k, B->s3);
   kpart(2, B->s3);
-  // what only the per-system sums at the end of the step read
+  // what only the second half kick and the per-system sums read
   cudaStreamWaitEvent(B->s4, B->ev_fork, 0);
+  launch_xi_mid(b, B->s4);
+  cudaEventRecord(B->ev_mid, B->s4);
   launch_order_terms(b, B->s4);
   cudaStreamWaitEvent(B->s4, B->ev_k, 0);
   kpart(3, B->s4);
@@ -799,6 +808,7 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   cudaEventRecord(B->ev_j3, B->s3);
   cudaStreamWaitEvent(B->st, B->ev_j2, 0);
   cudaStreamWaitEvent(B->st, B->ev_j3, 0);
+  cudaStreamWaitEvent(B->st, B->ev_mid, 0);
   launch_finalize(b, kMaskAll | kFlagMoveP, B->st);
   if (io) cudaEventRecordWithFlags(B->ev_f, B->st, cudaEventRecordExternal);
   cudaStreamWaitEvent(B->st, B->ev_j4, 0);
@@ -1223,6 +1233,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   b.nkgwork = (int)lo.kgwork.size();
   b.nktile = (int)lo.ktile.size();
   b.nblk = (int)lo.blk.size();
+  b.nwblk = (int)lo.wblk.size();
   b.ncellblk = (int)lo.cellblk.size();
   b.nrpwork = (int)lo.rpwork.size();
   b.ngtile = (int)lo.gtile.size();
@@ -1246,6 +1257,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
       cudaEventCreateWithFlags(&B->ev_j3, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_j4, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_k, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&B->ev_mid, cudaEventDisableTiming) != cudaSuccess ||
       cudaStreamCreateWithFlags(&B->sio, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_x, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_f, cudaEventDisableTiming) != cudaSuccess ||
@@ -1270,6 +1282,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   if (!lo.kgwork.empty()) up(b.kgwork, lo.kgwork.data(), sizeof(int2) * lo.kgwork.size());
   if (!lo.ktile.empty()) up(b.ktile, lo.ktile.data(), sizeof(int2) * lo.ktile.size());
   up(b.blk, lo.blk.data(), sizeof(int2) * lo.blk.size());
+  up(b.wblk, lo.wblk.data(), sizeof(int2) * lo.wblk.size());
   if (!lo.cellblk.empty()) up(b.cellblk, lo.cellblk.data(), sizeof(int2) * lo.cellblk.size());
   up(b.kn, lo.kn.data(), sizeof(int4) * lo.kn.size());
   up(b.kv, lo.kv.data(), sizeof(float4) * lo.kv.size());
@@ -1302,7 +1315,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   cudaMemsetAsync(b.ccnt, 0, sizeof(int) * std::max(lo.ncellcap, 1), B->st);
   cudaMemsetAsync(b.kgdone, 0, sizeof(int) * std::max<size_t>(lo.blk.size(), 1), B->st);
   cudaMemsetAsync(b.rlE, 0, sizeof(double) * 10 * std::max<size_t>(lo.blk.size(), 1), B->st);
-  cudaMemsetAsync(b.icnt, 0, sizeof(int) * std::max(nsys, 1), B->st);
+  cudaMemsetAsync(b.wrow, 0, sizeof(float2) * 12 * std::max<size_t>(lo.wblk.size(), 1), B->st);
   cudaMemsetAsync(b.F, 0, sizeof(double) * 3 * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(b.T, 0, sizeof(double) * 3 * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(B->noise[0], 0, sizeof(double) * kNoiseChunk * nsys * 4, B->st);
@@ -1358,6 +1371,7 @@ mdsc_status mdsc_destroy(mdsc_batch* B) {
   if (B->ev_j3) cudaEventDestroy(B->ev_j3);
   if (B->ev_j4) cudaEventDestroy(B->ev_j4);
   if (B->ev_k) cudaEventDestroy(B->ev_k);
+  if (B->ev_mid) cudaEventDestroy(B->ev_mid);
   if (B->ev_x) cudaEventDestroy(B->ev_x);
   if (B->ev_f) cudaEventDestroy(B->ev_f);
   if (B->sio) cudaStreamDestroy(B->sio);
@@ -1770,13 +1784,13 @@ mdsc_status mdsc_check_list(mdsc_batch* B, int* rebuild) {
   mdsc_status st = need_state(B);
   if (st) return st;
   launch_derive(B->b, B->st);
-  std::vector<double> dm(B->b.nblk);
-  CU(cudaMemcpyAsync(dm.data(), B->b.dmax, sizeof(double) * dm.size(), cudaMemcpyDeviceToHost, B->st));
+  std::vector<float> dm(std::max(B->b.nwblk, 1));
+  CU(cudaMemcpyAsync(dm.data(), B->b.dmax, sizeof(float) * B->b.nwblk, cudaMemcpyDeviceToHost, B->st));
   CU(cudaStreamSynchronize(B->st));
   for (int s = 0; s < B->nsys; ++s) {
     const SysDev& P = B->lo.sys[s];
-    double m = 0;
-    for (int k = 0; k < P.nblk; ++k) m = std::max(m, dm[P.blk_off + k]);
+    float m = 0;
+    for (int k = 0; k < P.nw; ++k) m = std::max(m, dm[P.w_off + k]);
     if (rebuild) rebuild[s] = (!B->built[s] || 2.0 * m > P.skin) ? 1 : 0;
   }
   return MDSC_OK;
@@ -2498,6 +2512,7 @@ mdsc_status mdsc_profile_steps(mdsc_batch* B, int nsteps, int max_kernels, char*
     launch_reset_iter(b, B->st);
     cudaEventRecord(ev[0], B->st);
     launch_integrate_first(b, B->st);
+    launch_xi_mid(b, B->st);
     cudaEventRecord(ev[1], B->st);
     launch_order_terms(b, B->st);
     cudaEventRecord(ev[2], B->st);

@@ -12,86 +12,13 @@
 // to the FP64 orientation as O += D O.  Kicks, drifts and the thermostat
 // scalars stay in FP64.
 #include <algorithm>
+#include <climits>
 #include <vector>
 
 #include "mdsc_dev.cuh"
 #include "reduce.cuh"
 
 namespace mdsc {
-
-// ---------------------------------------------------------------------
-// working copies: fixed-point positions, FP32 axes and dipole vectors
-// ---------------------------------------------------------------------
-__device__ __forceinline__ void derive_particle(const Batch& b, const SysDev& P, int i,
-                                                const double* r, const double* O, uint32_t* u) {
-  const int N = b.ntot, ND = b.ndtot;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    u[a] = to_fix(r[a], P.invL32[a]);
-    b.pfx[a * N + i] = u[a];
-  }
-  // FP32 copies by integer instructions (the FP64 unit is the scarce one)
-  float Of[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) Of[k] = soft_d2f_rn(O[k]);
-  b.pax[i] = make_float4(Of[6], Of[7], Of[8], soft_d2f_rn(b.len[i]));
-  b.pdia[i] = soft_d2f_rn(b.dia[i]);
-  const int nd = P.nd;
-  const int g0 = P.dip_off + (i - P.part_off) * nd;
-  for (int w = 0; w < nd; ++w) {
-    const int g = g0 + w;
-    const double pc = b.dpc[g];
-    if (pc == 0.0) {
-#pragma unroll
-      for (int a = 0; a < 3; ++a) b.dfx[a * ND + g] = u[a];
-    } else {
-#pragma unroll
-      for (int a = 0; a < 3; ++a) b.dfx[a * ND + g] = to_fix(r[a] + pc * O[6 + a], P.invL32[a]);
-    }
-    // lab direction O^T o_body (Spherocyl::set_dip, v25/classes.cpp:166-170), times the moment
-    const float ox = soft_d2f_rn(b.dob[3 * g]), oy = soft_d2f_rn(b.dob[3 * g + 1]),
-                oz = soft_d2f_rn(b.dob[3 * g + 2]);
-    const float mu = soft_d2f_rn(b.dmu[g]);
-#pragma unroll
-    for (int a = 0; a < 3; ++a) b.dm[a * ND + g] = mu * (Of[a] * ox + Of[3 + a] * oy + Of[6 + a] * oz);
-  }
-}
-
-// how far the rod's ends may have moved since the last list build: the
-// centre's move from the fixed-point coordinates (exact minimum image, no
-// FP64 arithmetic) plus half the length times the axis change
-__device__ __forceinline__ float displacement(const Batch& b, const SysDev& P, int i, const uint32_t* u,
-                                              const double* O) {
-  float dr2 = 0.f, du2 = 0.f;
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const float d = fix_diff(u[a], b.fsave[3 * i + a], P.Lfix[a]);
-    const float e = soft_d2f_rn(O[6 + a]) - b.usave[3 * i + a];
-    dr2 += d * d;
-    du2 += e * e;
-  }
-  return sqrtf(dr2) + 0.5f * soft_d2f_rn(b.len[i]) * sqrtf(du2);
-}
-
-__global__ void __launch_bounds__(kPartBlock) derive_kernel(Batch b) {
-  __shared__ float shm[kPartBlock / 32];
-  const int2 bk = b.blk[blockIdx.x];
-  const SysDev& P = b.sys[bk.x];
-  const int i = bk.y + threadIdx.x;
-  float disp = 0.f;
-  if (i < P.part_off + P.n) {
-    double r[3], O[9];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) r[a] = b.r[3 * i + a];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) O[k] = b.O[9 * i + k];
-    uint32_t u[3];
-    derive_particle(b, P, i, r, O, u);
-    disp = displacement(b, P, i, u, O);
-  }
-  const float m = block_max<kPartBlock>(disp, shm);
-  if (threadIdx.x == 0) b.dmax[blk_slot(P, bk)] = soft_f2d(m);
-}
 
 // Spherocyl::renorm, v25/classes.cpp:307-325
 __device__ __forceinline__ void renorm_O(double* o) {
@@ -130,40 +57,6 @@ __device__ __forceinline__ void plane_rot(float a, int i, int j, float* lb, floa
   }
 }
 
-// translate + rotate (Spherocyl::translate / rotate, v25/classes.cpp:228-304)
-__device__ __forceinline__ void move_x(const Batch& b, int i, double dt, double* r, const double* p,
-                                       double* O, const double* l) {
-  const double im = b.invm[i];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) r[a] += dt * p[a] * im;
-  const float iI0 = soft_d2f_rn(b.invI[3 * i]), iI1 = soft_d2f_rn(b.invI[3 * i + 1]),
-              iI2 = soft_d2f_rn(b.invI[3 * i + 2]);
-  const float fdt = soft_d2f_rn(dt), h = 0.5f * fdt;
-  float lb[3], Of[9];
-  const float lf[3] = {soft_d2f_rn(l[0]), soft_d2f_rn(l[1]), soft_d2f_rn(l[2])};
-#pragma unroll
-  for (int k = 0; k < 9; ++k) Of[k] = soft_d2f_rn(O[k]);
-#pragma unroll
-  for (int a = 0; a < 3; ++a) lb[a] = Of[3 * a] * lf[0] + Of[3 * a + 1] * lf[1] + Of[3 * a + 2] * lf[2];
-  float D[9];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) D[k] = 0.f;
-  plane_rot(-lb[0] * h * iI0, 1, 2, lb, D);   // Rx
-  plane_rot(-lb[1] * h * iI1, 2, 0, lb, D);   // Ry
-  plane_rot(-lb[2] * fdt * iI2, 0, 1, lb, D); // Rz
-  plane_rot(-lb[1] * h * iI1, 2, 0, lb, D);   // Ry
-  plane_rot(-lb[0] * h * iI0, 1, 2, lb, D);   // Rx
-  // O += D O: the increment (|D| ~ 1e-3) in FP32, ~1e-10 absolute like D
-  // itself, added to the FP64 orientation
-  float inc[9];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) inc[3 * a + c] = D[3 * a] * Of[c] + D[3 * a + 1] * Of[3 + c] + D[3 * a + 2] * Of[6 + c];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) O[k] += soft_f2d(inc[k]);
-}
-
 // K_r = l^T (O^T I^-1 O) l = sum_a (O l)_a^2 / I_a  (v25/functions.cpp:2123-2148)
 __device__ __forceinline__ double rot_kin(const Batch& b, int i, const double* O, const double* l) {
   double kr = 0.0;
@@ -175,300 +68,386 @@ __device__ __forceinline__ double rot_kin(const Batch& b, int i, const double* O
   return kr;
 }
 
-// thermostat coordinates used by the second half kick: moveTher 0 then 1
-// (v25/functions.cpp:2193-2206), from the first-half kinetic energies of
-// every block of the system (read from L2: other blocks wrote them)
-__device__ __forceinline__ void xi_mid(const Batch& b, const SysDev& P, const SysState& S, int s,
-                                       double* xi2, double* Kf) {
-  double K0 = 0.0, K1 = 0.0;
-  for (int k = 0; k < P.nblk; ++k) {
-    K0 += __ldcg(&b.kin1[2 * (P.blk_off + k)]);
-    K1 += __ldcg(&b.kin1[2 * (P.blk_off + k) + 1]);
+// ---------------------------------------------------------------------
+// One rod on three lanes.  An FP64 instruction occupies a warp for 64 cycles
+// here, however many independent ones follow it, so the per-particle kernels
+// take a block of 32 rods and three warps, warp a the component a of every
+// vector and row a of the orientation; what a component needs of the others
+// goes through shared memory.  A third of the instructions per warp on three
+// times the warps: one system's step waits for ~20 of them instead of ~60,
+// and a batch that fills the GPU keeps the FP64 unit as busy as before.
+// ---------------------------------------------------------------------
+constexpr int kRows = 32;           // rods per block
+constexpr int kRowBlock = 3 * kRows;
+
+struct Shared3 {
+  double l[3][kRows];
+  double ax[3][kRows];
+  float O[9][kRows];   // orientation before the move
+  float O2[9][kRows];  // and after it
+  float d2[3][kRows];
+};
+
+// Working copies of component a: fixed-point position, dipole positions and
+// moment vectors, and (warp 2, which holds the rod axis) the FP32 axis and
+// length; sh.O2 and sh.ax hold the new orientation.  Returns, in warp 2, how
+// far the rod's ends may have moved since the last list build: the centre's
+// move from the fixed-point coordinates (exact minimum image) plus half the
+// length times the axis change.
+__device__ __forceinline__ float derive_comp(const Batch& b, const SysDev& P, Shared3& sh, int a, int lane, int i,
+                                             bool ok, double r, const double* O) {
+  const int N = b.ntot, ND = b.ndtot;
+  const uint32_t u = to_fix(r, P.invL32[a]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) sh.O2[3 * a + c][lane] = soft_d2f_rn(O[c]);
+  if (a == 2) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sh.ax[c][lane] = O[c];
   }
-  Kf[0] = 0.5 * K0;
-  Kf[1] = 0.5 * K1;
-  const double* nz = b.noise + ((long long)S.iter * b.nsys + s) * 4;
-  const double x1t = P.ex1 * S.xi[0] + P.cnoise * nz[0];
-  const double x1r = P.ex1 * S.xi[1] + P.cnoise * nz[2];
-  xi2[0] = x1t + P.dt * (2. * Kf[0] - P.ntemp3) / P.Q;
-  xi2[1] = x1r + P.dt * (2. * Kf[1] - P.ntemp3) / P.Q;
+  {
+    const float d = fix_diff(u, b.fsave[3 * i + a], P.Lfix[a]);
+    sh.d2[a][lane] = d * d;
+  }
+  __syncthreads();
+  float disp = 0.f;
+  if (ok) {
+    b.pfx[a * N + i] = u;
+    const int nd = P.nd;
+    const int g0 = P.dip_off + (i - P.part_off) * nd;
+    const float o0 = sh.O2[a][lane], o1 = sh.O2[3 + a][lane], o2 = sh.O2[6 + a][lane];
+    for (int w = 0; w < nd; ++w) {
+      const int g = g0 + w;
+      const double pc = b.dpc[g];
+      b.dfx[a * ND + g] = pc == 0.0 ? u : to_fix(r + pc * sh.ax[a][lane], P.invL32[a]);
+      // lab direction O^T o_body (Spherocyl::set_dip, v25/classes.cpp:166-170), times the moment
+      const float ox = soft_d2f_rn(b.dob[3 * g]), oy = soft_d2f_rn(b.dob[3 * g + 1]),
+                  oz = soft_d2f_rn(b.dob[3 * g + 2]);
+      b.dm[a * ND + g] = soft_d2f_rn(b.dmu[g]) * (o0 * ox + o1 * oy + o2 * oz);
+    }
+    if (a == 2) {
+      const float ln = soft_d2f_rn(b.len[i]);
+      const float x[3] = {sh.O2[6][lane], sh.O2[7][lane], sh.O2[8][lane]};
+      b.pax[i] = make_float4(x[0], x[1], x[2], ln);
+      b.pdia[i] = soft_d2f_rn(b.dia[i]);
+      float du2 = 0.f;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const float q = x[c] - b.usave[3 * i + c];
+        du2 += q * q;
+      }
+      disp = sqrtf(sh.d2[0][lane] + sh.d2[1][lane] + sh.d2[2][lane]) + 0.5f * ln * sqrtf(du2);
+    }
+  }
+  return disp;
+}
+
+// the block's largest displacement measure, from warp 2
+__device__ __forceinline__ void store_disp(const Batch& b, int row, int a, float disp) {
+  if (a != 2) return;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) disp = fmaxf(disp, __shfl_xor_sync(0xffffffffu, disp, off));
+  if ((threadIdx.x & 31) == 0) b.dmax[row] = disp;
+}
+
+// the free-rotor move of the step (Spherocyl::rotate, v25/classes.cpp:240-304):
+// row a of the increment D O from the FP32 orientation and angular momentum;
+// every warp composes the rotation
+__device__ __forceinline__ void rotor_row(const Batch& b, const Shared3& sh, int a, int lane, int i, double dt,
+                                          float* inc) {
+  const float iI0 = soft_d2f_rn(b.invI[3 * i]), iI1 = soft_d2f_rn(b.invI[3 * i + 1]),
+              iI2 = soft_d2f_rn(b.invI[3 * i + 2]);
+  const float fdt = soft_d2f_rn(dt), h = 0.5f * fdt;
+  const float lf[3] = {soft_d2f_rn(sh.l[0][lane]), soft_d2f_rn(sh.l[1][lane]), soft_d2f_rn(sh.l[2][lane])};
+  float Of[9], lb[3], D[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) Of[k] = sh.O[k][lane];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) lb[k] = Of[3 * k] * lf[0] + Of[3 * k + 1] * lf[1] + Of[3 * k + 2] * lf[2];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) D[k] = 0.f;
+  plane_rot(-lb[0] * h * iI0, 1, 2, lb, D);   // Rx
+  plane_rot(-lb[1] * h * iI1, 2, 0, lb, D);   // Ry
+  plane_rot(-lb[2] * fdt * iI2, 0, 1, lb, D); // Rz
+  plane_rot(-lb[1] * h * iI1, 2, 0, lb, D);   // Ry
+  plane_rot(-lb[0] * h * iI0, 1, 2, lb, D);   // Rx
+  // O += D O: the increment (|D| ~ 1e-3) in FP32, ~1e-10 absolute like D
+  // itself, added to the FP64 orientation
+  const float d0 = a == 0 ? D[0] : (a == 1 ? D[3] : D[6]), d1 = a == 0 ? D[1] : (a == 1 ? D[4] : D[7]),
+              d2 = a == 0 ? D[2] : (a == 1 ? D[5] : D[8]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) inc[c] = d0 * Of[c] + d1 * Of[3 + c] + d2 * Of[6 + c];
 }
 
 // ---------------------------------------------------------------------
 // first half of the step: moveTher(0), [renorm], moveP(first), moveX
+// (v25/functions.cpp:2071-2149); MOVE_ONLY: moveX alone; DERIVE: only the
+// working copies
 // ---------------------------------------------------------------------
-// 8 blocks per SM (64 registers, 76 B of spills) instead of 6 (80): the
-// state reads' latency is hidden by more warps, 0.047 to 0.045 ms on the
-// 256-replica mix (the same bound on finalize made it 12% slower)
-__global__ void __launch_bounds__(kPartBlock, 8) integrate_first_kernel(Batch b) {
-  __shared__ double sh[2 * kPartBlock / 32];
-  __shared__ float shm[kPartBlock / 32];
+// Measured against one lane per rod in blocks of 128 (with the force assembly
+// below and the per-system sums on lanes): a step of 256 rods 62.4 -> 51.8 us,
+// of 4096 rods 113 -> 93.7, of 32,768 rods 2205 -> 2135, of 64 systems 223 ->
+// 215, of 256 systems 688 -> 688 (FP64 throughput and the state's reads).
+enum : int { kPartDerive = 0, kPartMoveX = 1, kPartStep = 2 };
+
+template <int MODE>
+__global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
+  __shared__ Shared3 sh;
   __shared__ double sfac[2];
-  const int2 bk = b.blk[blockIdx.x];
+  const int2 bk = b.wblk[blockIdx.x];
   const int s = bk.x;
-  if (at_limit(b, s)) return;
+  if (MODE == kPartStep && at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   const SysState& S = b.st[s];
-  const int i = bk.y + threadIdx.x;
-  const bool ok = i < P.part_off + P.n;
-  if (threadIdx.x == 0) {
-    // moveTher mode 0 (v25/functions.cpp:2193-2202); noise drawn on the host
-    const double* nz = b.noise + ((long long)S.iter * b.nsys + s) * 4;
-    const double xt = P.ex1 * S.xi[0] + P.cnoise * nz[0];
-    const double xr = P.ex1 * S.xi[1] + P.cnoise * nz[2];
-    sfac[0] = 1.0 / (1.0 + 0.5 * P.dt * xt);
-    sfac[1] = 1.0 / (1.0 + 0.5 * P.dt * xr);
-  }
-  __syncthreads();
-  double kin[2] = {0.0, 0.0};
-  float disp = 0.f;
-  if (ok) {
-    const double h = 0.5 * P.dt;
-    double r[3], p[3], l[3], O[9];
+  const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool ok = bk.y + lane < P.part_off + P.n;
+  const int i = ok ? bk.y + lane : bk.y;  // lanes past the end repeat the first rod and store nothing
+  const int row = P.w_off + (bk.y - P.part_off) / kRows;
+  double r = b.r[3 * i + a], O[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      r[a] = b.r[3 * i + a];
-      p[a] = b.p[3 * i + a];
-      l[a] = b.l[3 * i + a];
+  for (int c = 0; c < 3; ++c) O[c] = b.O[9 * i + 3 * a + c];
+  if constexpr (MODE != kPartDerive) {
+    double p = b.p[3 * i + a], l = b.l[3 * i + a];
+    const double im = b.invm[i];
+    if constexpr (MODE == kPartStep) {
+      const double h = 0.5 * P.dt, F = b.F[3 * i + a], T = b.T[3 * i + a];
+      if (threadIdx.x < 2) {
+        // moveTher mode 0 (v25/functions.cpp:2193-2202); noise drawn on the host
+        const double* nz = b.noise + ((long long)S.iter * b.nsys + s) * 4;
+        const double x = P.ex1 * S.xi[threadIdx.x] + P.cnoise * nz[2 * threadIdx.x];
+        sfac[threadIdx.x] = 1.0 / (1.0 + 0.5 * P.dt * x);
+      }
+      if (S.step % 100 == 0) {  // v25/main.cpp:556-563
+        double A[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) A[k] = b.O[9 * i + k];
+        renorm_O(A);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) O[c] = a == 0 ? A[c] : (a == 1 ? A[3 + c] : A[6 + c]);
+      }
+      __syncthreads();
+      // moveP first half (v25/functions.cpp:2129-2149)
+      p = (p + h * F) * sfac[0];
+      l = (l + h * T) * sfac[1];
     }
+    sh.l[a][lane] = l;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) O[k] = b.O[9 * i + k];
-    if (S.step % 100 == 0) renorm_O(O);  // v25/main.cpp:556-563
-    // moveP first half (v25/functions.cpp:2129-2149)
-    double psq = 0.0;
+    for (int c = 0; c < 3; ++c) sh.O[3 * a + c][lane] = soft_d2f_rn(O[c]);
+    __syncthreads();
+    if constexpr (MODE == kPartStep) {
+      // the kinetic energies of this component, before the move
+      const double lb = O[0] * sh.l[0][lane] + O[1] * sh.l[1][lane] + O[2] * sh.l[2][lane];
+      FF k[2] = {ff_from(ok ? p * p * im : 0.0), ff_from(ok ? lb * lb * b.invI[3 * i + a] : 0.0)};
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      p[a] = (p[a] + h * b.F[3 * i + a]) * sfac[0];
-      psq += p[a] * p[a];
-      l[a] = (l[a] + h * b.T[3 * i + a]) * sfac[1];
+      for (int c = 0; c < 2; ++c) {
+        k[c] = ff_warp_sum(k[c]);
+        if (lane == 0) b.krow[2 * (3 * row + a) + c] = make_float2(k[c].hi, k[c].lo);
+      }
+      if (ok) {
+        b.p[3 * i + a] = p;
+        b.l[3 * i + a] = l;
+      }
     }
-    kin[0] = psq * b.invm[i];
-    kin[1] = rot_kin(b, i, O, l);
     // moveX (v25/functions.cpp:2071-2092)
-    move_x(b, i, P.dt, r, p, O, l);
+    r += P.dt * p * im;
+    float inc[3];
+    rotor_row(b, sh, a, lane, i, P.dt, inc);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      b.r[3 * i + a] = r[a];
-      b.p[3 * i + a] = p[a];
-      b.l[3 * i + a] = l[a];
-    }
+    for (int c = 0; c < 3; ++c) O[c] += soft_f2d(inc[c]);
+    if (ok) {
+      b.r[3 * i + a] = r;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) b.O[9 * i + k] = O[k];
-    uint32_t u[3];
-    derive_particle(b, P, i, r, O, u);
-    disp = displacement(b, P, i, u, O);
-  }
-  double tot[2];
-  block_sum<2, kPartBlock>(kin, sh, tot);
-  const float m = block_max<kPartBlock>(disp, shm);
-  if (threadIdx.x == 0) {
-    const int lb = blk_slot(P, bk);
-    b.kin1[2 * lb] = tot[0];
-    b.kin1[2 * lb + 1] = tot[1];
-    b.dmax[lb] = soft_f2d(m);
-    // the system's last block to finish computes the second-half thermostat
-    // coordinates once (blocks' sums in block order: the same bits whichever
-    // block is last) and rearms the counter
-    __threadfence();
-    if (atomicAdd(&b.icnt[s], 1) == P.nblk - 1) {
-      __threadfence();
-      SysState& Sw = b.st[s];
-      double xi2[2], Kf[2];
-      xi_mid(b, P, Sw, s, xi2, Kf);
-      Sw.xi_mid[0] = xi2[0];
-      Sw.xi_mid[1] = xi2[1];
-      Sw.K_first[0] = Kf[0];
-      Sw.K_first[1] = Kf[1];
-      b.icnt[s] = 0;
+      for (int c = 0; c < 3; ++c) b.O[9 * i + 3 * a + c] = O[c];
     }
   }
+  const float disp = derive_comp(b, P, sh, a, lane, i, ok, r, O);
+  if constexpr (MODE != kPartMoveX) store_disp(b, row, a, disp);
 }
 
+// Thermostat coordinates of the second half kick, moveTher 0 then 1
+// (v25/functions.cpp:2193-2206), from the first-half kinetic energies: a
+// block per system, beside the force chains (only the second kick reads them).
+__global__ void __launch_bounds__(128) xi_mid_kernel(Batch b) {
+  __shared__ FF sh[2][4];
+  const int s = blockIdx.x;
+  if (at_limit(b, s)) return;
+  const SysDev& P = b.sys[s];
+  SysState& S = b.st[s];
+  FF v[2] = {ff_of(0.f), ff_of(0.f)};
+  for (int t = threadIdx.x; t < 3 * P.nw; t += 128) {
+    const float4 q = reinterpret_cast<const float4*>(b.krow)[3 * P.w_off + t];
+    v[0] = ff_add(v[0], FF{q.x, q.y});
+    v[1] = ff_add(v[1], FF{q.z, q.w});
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    v[c] = ff_warp_sum(v[c]);
+    if ((threadIdx.x & 31) == 0) sh[c][threadIdx.x >> 5] = v[c];
+  }
+  __syncthreads();
+  const int c = threadIdx.x;
+  if (c >= 2) return;
+  const FF t = ff_add(ff_add(ff_add(sh[c][0], sh[c][1]), sh[c][2]), sh[c][3]);
+  const double Kf = 0.5 * (soft_f2d(t.hi) + soft_f2d(t.lo));
+  const double* nz = b.noise + ((long long)S.iter * b.nsys + s) * 4;
+  const double x1 = P.ex1 * S.xi[c] + P.cnoise * nz[2 * c];
+  S.K_first[c] = Kf;
+  S.xi_mid[c] = x1 + P.dt * (2. * Kf - P.ntemp3) / P.Q;
+}
 
 // ---------------------------------------------------------------------
-// force assembly (+ ext_field) and optionally moveP(last)
+// force assembly (+ ext_field) and optionally moveP(last): three lanes per
+// rod as above.  Each warp leaves its sums for the per-system reduction as
+// float-float rows: krow2 (K_t, K_r, two kinetic pressure terms, U_ext) and
+// wrow (the WCA terms a, a + 3, ... of U, W, PT of the rods' own pairs).
 // ---------------------------------------------------------------------
-__global__ void __launch_bounds__(kPartBlock, 6) finalize_kernel(Batch b, int mode) {
-  __shared__ double sh[20 * kPartBlock / 32];
-  const int2 bk = b.blk[blockIdx.x];
+constexpr int kKinCols = 5, kWcaCols = 4;
+// kinetic pressure terms of warp a: (xx, xy), (yy, yz), (zz, zx)
+
+__global__ void __launch_bounds__(kRowBlock) finalize_kernel(Batch b, int mode) {
+  __shared__ double sl[3][kRows];
+  __shared__ double sv[3][kRows];
+  __shared__ float sp[3][kRows];
+  const int2 bk = b.wblk[blockIdx.x];
   const int s = bk.x;
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   const SysState& S = b.st[s];
-  const int i = bk.y + threadIdx.x;
-  const bool ok = i < P.part_off + P.n;
-  // block sums: K_t, K_r, PT_kin (6), U_ext, then the WCA terms U, W, PT (9)
-  // of this block's own candidate pairs
-  FF acc[20];
+  const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool ok = bk.y + lane < P.part_off + P.n;
+  const int i = ok ? bk.y + lane : bk.y;
+  const int row = 3 * (P.w_off + (bk.y - P.part_off) / kRows) + a;
+  const int a1 = a == 2 ? 0 : a + 1, a2 = a == 0 ? 2 : a - 1;  // the cyclic next and previous component
+  double F = (mode & kFlagAccum) ? b.F[3 * i + a] : 0.0;
+  double T = (mode & kFlagAccum) ? b.T[3 * i + a] : 0.0;
+  if (mode & kMaskWca) {
+    FF w[kWcaCols];
 #pragma unroll
-  for (int c = 0; c < 20; ++c) acc[c].hi = acc[c].lo = 0.f;
-  if (ok) {
-    double F[3], T[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      F[a] = (mode & kFlagAccum) ? b.F[3 * i + a] : 0.0;
-      T[a] = (mode & kFlagAccum) ? b.T[3 * i + a] : 0.0;
-    }
-    if (mode & kMaskWca) {
+    for (int c = 0; c < kWcaCols; ++c) w[c] = ff_of(0.f);
+    if (ok) {
       // its own shares of its candidate pairs (higher-index partners), in
       // slot order, as force_sc adds them
-      {
-        const int nc = b.wcnt[i];
-        const double* own = b.wown + (long long)i * kMaxC * 6;
-        const double* ev = b.wev + (long long)i * kMaxC * 11;
-        for (int c = 0; c < nc; ++c) {
+      const int nc = b.wcnt[i];
+      const double* own = b.wown + (long long)i * kMaxC * 6;
+      const double* ev = b.wev + (long long)i * kMaxC * 11;
+      for (int c = 0; c < nc; ++c) {
+        F += own[6 * c + a];
+        T += own[6 * c + 3 + a];
 #pragma unroll
-          for (int a = 0; a < 3; ++a) {
-            F[a] += own[6 * c + a];
-            T[a] += own[6 * c + 3 + a];
-          }
-#pragma unroll
-          for (int q = 0; q < 11; ++q) acc[9 + q] = ff_add(acc[9 + q], ff_from(ev[11 * c + q]));
-        }
+        for (int q = 0; q < kWcaCols; ++q)
+          if (a + 3 * q < 11) w[q] = ff_add(w[q], ff_from(ev[11 * c + a + 3 * q]));
       }
       // shares of the pairs this particle forms with lower-index partners,
       // left by the WCA kernel in the partner's records.  The screen listed
-      // their slots here in arrival order; sorted, the slots ascend with the
-      // partner (slot = partner * kMaxC + c), the order force_sc adds them.
+      // their slots here in arrival order; taken in ascending order the slots
+      // ascend with the partner (slot = partner * kMaxC + c), the order
+      // force_sc adds them.
       const int nin = min(b.wincnt[i], kMaxC);
-      int sl[kMaxC];
+      const int4* win = reinterpret_cast<const int4*>(b.win + (long long)i * kMaxC);
+      int v[kMaxC];
+#pragma unroll
+      for (int q = 0; q < kMaxC / 4; ++q) {
+        const int4 x = 4 * q < nin ? win[q] : make_int4(0, 0, 0, 0);
+        v[4 * q] = 4 * q < nin ? x.x : INT_MAX;
+        v[4 * q + 1] = 4 * q + 1 < nin ? x.y : INT_MAX;
+        v[4 * q + 2] = 4 * q + 2 < nin ? x.z : INT_MAX;
+        v[4 * q + 3] = 4 * q + 3 < nin ? x.w : INT_MAX;
+      }
+      int last = -1;
       for (int k = 0; k < nin; ++k) {
-        const int v = b.win[(long long)i * kMaxC + k];
-        int m = k;
-        while (m > 0 && sl[m - 1] > v) {
-          sl[m] = sl[m - 1];
-          --m;
-        }
-        sl[m] = v;
-      }
-      for (int k = 0; k < nin; ++k) {
-        const double* rec = b.wrec + (long long)sl[k] * 6;
+        int m = INT_MAX;
 #pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          F[a] += rec[a];
-          T[a] += rec[3 + a];
-        }
+        for (int q = 0; q < kMaxC; ++q) m = min(m, v[q] > last ? v[q] : INT_MAX);
+        const double* rec = b.wrec + (long long)m * 6;
+        F += rec[a];
+        T += rec[3 + a];
+        last = m;
       }
     }
-    double ax[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) ax[a] = b.O[9 * i + 6 + a];
-    const int nd = P.nd;
-    const int loc0 = (i - P.part_off) * nd;
-    // the field term needs the FP64 moment; without a field it adds nothing
-    const bool ext = (mode & kMaskExt) && (P.B[0] != 0.0 || P.B[1] != 0.0 || P.B[2] != 0.0);
-    double uext = 0.0;
-    for (int w = 0; w < nd; ++w) {
-      const int loc = loc0 + w;
-      const int g = P.dip_off + loc;
-      // real- and reciprocal-space force and torque of this dipole in
-      // float-float (FP32 instructions), one conversion to FP64 at the end
-      FF acc6[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) acc6[c].hi = acc6[c].lo = 0.f;
-      if (mode & kMaskReal) {
-        // this dipole's tile partials summed over all partner strips
-        // (real_sum_kernel)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-          const float2 v = b.rsum[(long long)c * b.ndtot + g];
-          acc6[c].hi = v.x;
-          acc6[c].lo = v.y;
-        }
-      }
-      if (mode & kMaskK) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const float2 fk = b.Fk[3 * g + c], tk = b.Tk[3 * g + c];
-          FF v;
-          v.hi = fk.x;
-          v.lo = fk.y;
-          acc6[c] = ff_add(acc6[c], v);
-          v.hi = tk.x;
-          v.lo = tk.y;
-          acc6[3 + c] = ff_add(acc6[3 + c], v);
-        }
-      }
-      double f[3], t[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        f[c] = soft_f2d(acc6[c].hi) + soft_f2d(acc6[c].lo);
-        t[c] = soft_f2d(acc6[3 + c].hi) + soft_f2d(acc6[3 + c].lo);
-      }
-      if (ext) {
-        // ext_field: torque mu o x B, energy -mu o.B (v25/functions.cpp:2014-2020),
-        // with the dipole vector mu O^T o_body in FP64
-        const double* O = b.O + 9 * i;
-        const double ox = b.dob[3 * g], oy = b.dob[3 * g + 1], oz = b.dob[3 * g + 2], mu = b.dmu[g];
-        const double mx = mu * (O[0] * ox + O[3] * oy + O[6] * oz);
-        const double my = mu * (O[1] * ox + O[4] * oy + O[7] * oz);
-        const double mz = mu * (O[2] * ox + O[5] * oy + O[8] * oz);
-        t[0] += my * P.B[2] - mz * P.B[1];
-        t[1] += mz * P.B[0] - mx * P.B[2];
-        t[2] += mx * P.B[1] - my * P.B[0];
-        uext -= mx * P.B[0] + my * P.B[1] + mz * P.B[2];
-      }
-      // lever arm of an off-centre dipole: d x f (v25/classes.hpp:135-136)
-      const double pc = b.dpc[g];
-      if (pc != 0.0) {
-        const double d[3] = {pc * ax[0], pc * ax[1], pc * ax[2]};
-        t[0] += d[1] * f[2] - d[2] * f[1];
-        t[1] += d[2] * f[0] - d[0] * f[2];
-        t[2] += d[0] * f[1] - d[1] * f[0];
-      }
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        F[a] += f[a];
-        T[a] += t[a];
-      }
-    }
-    acc[8] = ff_from(uext);
-    double p[3], l[3];
-    if (mode & kFlagMoveP) {
-      // moveP last half (v25/functions.cpp:2150-2173)
-      const double h = 0.5 * P.dt;
-      // xi after moveTher 0 and 1, set by the first-half kernel
-      const double ft = 1. - h * S.xi_mid[0], fr = 1. - h * S.xi_mid[1];
-      double psq = 0.0;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        p[a] = b.p[3 * i + a] * ft + h * F[a];
-        psq += p[a] * p[a];
-        l[a] = b.l[3 * i + a] * fr + h * T[a];
-        b.p[3 * i + a] = p[a];
-        b.l[3 * i + a] = l[a];
-      }
-      double O[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) O[k] = b.O[9 * i + k];
-      const double im = b.invm[i];
-      acc[0] = ff_from(psq * im);
-      acc[1] = ff_from(rot_kin(b, i, O, l));
-      // kinetic pressure tensor p_a p_b / m: FP32 products, float-float sums
-      const float pf[3] = {soft_d2f_rn(p[0]), soft_d2f_rn(p[1]), soft_d2f_rn(p[2])};
-      const float imf = soft_d2f_rn(im);
-      acc[2] = ff_of(pf[0] * pf[0] * imf);
-      acc[3] = ff_of(pf[0] * pf[1] * imf);
-      acc[4] = ff_of(pf[0] * pf[2] * imf);
-      acc[5] = ff_of(pf[1] * pf[1] * imf);
-      acc[6] = ff_of(pf[1] * pf[2] * imf);
-      acc[7] = ff_of(pf[2] * pf[2] * imf);
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      b.F[3 * i + a] = F[a];
-      b.T[3 * i + a] = T[a];
+    for (int c = 0; c < kWcaCols; ++c) {
+      w[c] = ff_warp_sum(w[c]);
+      if (lane == 0) b.wrow[kWcaCols * row + c] = make_float2(w[c].hi, w[c].lo);
     }
   }
-  double tot[20];
-  block_sum<20, kPartBlock>(acc, sh, tot);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int c = 0; c < 9; ++c) b.kin2[9 * blk_slot(P, bk) + c] = tot[c];
-    if (mode & kMaskWca) {
-#pragma unroll
-      for (int c = 0; c < 11; ++c) b.wcaE[11 * blk_slot(P, bk) + c] = tot[9 + c];
+  const int nd = P.nd;
+  // the field term needs the FP64 moment; without a field it adds nothing
+  const bool ext = (mode & kMaskExt) && (P.B[0] != 0.0 || P.B[1] != 0.0 || P.B[2] != 0.0);
+  double uext = 0.0;
+  for (int w = 0; w < nd; ++w) {
+    const int g = P.dip_off + (i - P.part_off) * nd + w;
+    // real- and reciprocal-space force and torque of this dipole in
+    // float-float (FP32 instructions), one conversion to FP64 at the end
+    FF qf = ff_of(0.f), qt = ff_of(0.f);
+    if (mode & kMaskReal) {
+      // this dipole's tile partials summed over all partner strips (real_sum_kernel)
+      const float2 x = b.rsum[(long long)a * b.ndtot + g], y = b.rsum[(long long)(3 + a) * b.ndtot + g];
+      qf = FF{x.x, x.y};
+      qt = FF{y.x, y.y};
     }
+    if (mode & kMaskK) {
+      const float2 x = b.Fk[3 * g + a], y = b.Tk[3 * g + a];
+      qf = ff_add(qf, FF{x.x, x.y});
+      qt = ff_add(qt, FF{y.x, y.y});
+    }
+    const double f = soft_f2d(qf.hi) + soft_f2d(qf.lo);
+    double t = soft_f2d(qt.hi) + soft_f2d(qt.lo);
+    if (ext) {
+      // ext_field: torque mu o x B, energy -mu o.B (v25/functions.cpp:2014-2020),
+      // with the dipole vector mu O^T o_body in FP64
+      const double* O = b.O + 9 * i;
+      const double m = b.dmu[g] * (O[a] * b.dob[3 * g] + O[3 + a] * b.dob[3 * g + 1] + O[6 + a] * b.dob[3 * g + 2]);
+      __syncthreads();
+      sv[a][lane] = m;
+      __syncthreads();
+      t += sv[a1][lane] * P.B[a2] - sv[a2][lane] * P.B[a1];
+      uext -= m * P.B[a];
+    }
+    // lever arm of an off-centre dipole: d x f (v25/classes.hpp:135-136)
+    const double pc = b.dpc[g];
+    if (__syncthreads_or(pc != 0.0)) {
+      sv[a][lane] = f;
+      __syncthreads();
+      if (pc != 0.0)
+        t += pc * b.O[9 * i + 6 + a1] * sv[a2][lane] - pc * b.O[9 * i + 6 + a2] * sv[a1][lane];
+    }
+    F += f;
+    T += t;
+  }
+  FF k[kKinCols];
+#pragma unroll
+  for (int c = 0; c < kKinCols; ++c) k[c] = ff_of(0.f);
+  k[4] = ff_from(ok ? uext : 0.0);
+  if (mode & kFlagMoveP) {
+    // moveP last half (v25/functions.cpp:2150-2173), with xi after moveTher
+    // 0 and 1 (xi_mid_kernel)
+    const double h = 0.5 * P.dt;
+    const double p = b.p[3 * i + a] * (1. - h * S.xi_mid[0]) + h * F;
+    const double l = b.l[3 * i + a] * (1. - h * S.xi_mid[1]) + h * T;
+    const double im = b.invm[i];
+    sl[a][lane] = l;
+    sp[a][lane] = soft_d2f_rn(p);
+    __syncthreads();
+    if (ok) {
+      b.p[3 * i + a] = p;
+      b.l[3 * i + a] = l;
+      const double* O = b.O + 9 * i + 3 * a;
+      const double lb = O[0] * sl[0][lane] + O[1] * sl[1][lane] + O[2] * sl[2][lane];
+      k[0] = ff_from(p * p * im);
+      k[1] = ff_from(lb * lb * b.invI[3 * i + a]);
+      // kinetic pressure tensor p_a p_b / m: FP32 products, float-float sums
+      const float imf = soft_d2f_rn(im), pf = sp[a][lane];
+      k[2] = ff_of(pf * pf * imf);
+      k[3] = ff_of(pf * sp[a1][lane] * imf);
+    }
+  }
+  if (ok) {
+    b.F[3 * i + a] = F;
+    b.T[3 * i + a] = T;
+  }
+#pragma unroll
+  for (int c = 0; c < kKinCols; ++c) {
+    k[c] = ff_warp_sum(k[c]);
+    if (lane == 0) b.krow2[kKinCols * row + c] = make_float2(k[c].hi, k[c].lo);
   }
 }
 
@@ -508,62 +487,75 @@ __global__ void __launch_bounds__(kPartBlock) order_terms_kernel(Batch b) {
 
 // ---------------------------------------------------------------------
 // per-system sums and the thermostat's last update.  kRedGroups blocks per
-// system, one per group of sums (real-space tiles, k-vectors, WCA blocks,
+// system, one per group of sums (real-space tiles, k tiles, WCA pairs,
 // kinetic terms, order parameters), each in float-float with a fixed order;
-// the kinetic block also closes the step's thermostat and bookkeeping.
+// the kinetic block also closes the step's thermostat and bookkeeping.  The
+// warps' sums are added and converted one value per lane: an FP64 addition
+// per value in one thread would cost 64 cycles each.
 constexpr int kRedThreads = 128;
 __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mode) {
-  __shared__ double sh[12 * kRedThreads / 32];
+  constexpr int NV = 12;
+  __shared__ FF sh[NV][kRedThreads / 32];
   const int s = blockIdx.x / kRedGroups, grp = blockIdx.x % kRedGroups;
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   SysState& S = b.st[s];
   SysObs& ob = b.obs[s];
-  FF v[12];
+  FF v[NV];
 #pragma unroll
-  for (int c = 0; c < 12; ++c) v[c].hi = v[c].lo = 0.f;
-  {
+  for (int c = 0; c < NV; ++c) v[c] = ff_of(0.f);
+  if (grp == 2) {
+    // columns q of warp a of every row: term a + 3 q of U, W, PT
+    for (int t = threadIdx.x; t < P.nw; t += kRedThreads) {
+      const float2* w = b.wrow + (long long)(P.w_off + t) * 3 * kWcaCols;
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int q = 0; q < kWcaCols; ++q)
+          if (a + 3 * q < 11) v[a + 3 * q] = ff_add(v[a + 3 * q], FF{w[kWcaCols * a + q].x, w[kWcaCols * a + q].y});
+    }
+  } else if (grp == 3) {
+    // K_t, K_r, then (xx xy)(yy yz)(zz zx), U_ext
+    for (int t = threadIdx.x; t < P.nw; t += kRedThreads) {
+      const float2* k = b.krow2 + (long long)(P.w_off + t) * 3 * kKinCols;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const float2* q = k + kKinCols * a;
+        v[0] = ff_add(v[0], FF{q[0].x, q[0].y});
+        v[1] = ff_add(v[1], FF{q[1].x, q[1].y});
+        v[2 + 2 * a] = ff_add(v[2 + 2 * a], FF{q[2].x, q[2].y});
+        v[3 + 2 * a] = ff_add(v[3 + 2 * a], FF{q[3].x, q[3].y});
+        v[8] = ff_add(v[8], FF{q[4].x, q[4].y});
+      }
+    }
+  } else {
     // the rows of one per-system table, column by column: real-space tiles
-    // (U, PT; FP32) or, in large systems, strips (each strip's tiles summed
-    // in float-float by strip_energy), k tiles (U, PT), WCA blocks (U, W, PT), kinetic
-    // blocks (K_t, K_r, PT_kin, U_ext) or order-parameter blocks.  One code
-    // path for the five keeps the kernel small: its blocks are short, and a
-    // larger kernel waited on instruction fetch.
+    // (U, PT; FP32), in large systems strips (each strip's tiles summed by
+    // strip_energy) or the neighbour pass's blocks, k tiles (U, PT) or
+    // order-parameter blocks, through one code path
     const float* fsrc = nullptr;
     const double* dsrc = nullptr;
-    int nrow, ncol;
-    if (grp == 0 && P.rc_real > 0.0) {  // the neighbour pass's block sums (real_cut)
+    int nrow, ncol = 10;
+    if (grp == 0 && P.rc_real > 0.0) {
       dsrc = b.rlE + (long long)P.blk_off * 10;
       nrow = P.nblk;
-      ncol = 10;
-    } else if (grp == 0 && P.nstrip > kStripRows) {  // the strips' sums of their tiles (strip_energy)
+    } else if (grp == 0 && P.nstrip > kStripRows) {
       dsrc = b.stripE + (long long)P.strip_off * 10;
       nrow = P.nstrip;
-      ncol = 10;
-    } else if (grp == 0) {  // the tiles themselves
+    } else if (grp == 0) {
       fsrc = b.tileE + (long long)P.tile_off * 10;
       nrow = P.ntile;
-      ncol = 10;
     } else if (grp == 1) {
       dsrc = b.kE + (long long)P.kt_off * 10;
       nrow = P.nkt;
-      ncol = 10;
-    } else if (grp == 2) {
-      dsrc = b.wcaE + (long long)P.blk_off * 11;
-      nrow = P.nblk;
-      ncol = 11;
-    } else if (grp == 4) {
+    } else {
       dsrc = b.obk + (long long)P.blk_off * 12;
       nrow = P.nblk;
       ncol = 12;
-    } else {
-      dsrc = b.kin2 + (long long)P.blk_off * 9;
-      nrow = P.nblk;
-      ncol = 9;
     }
     for (int t = threadIdx.x; t < nrow; t += kRedThreads) {
 #pragma unroll
-      for (int c = 0; c < 12; ++c) {
+      for (int c = 0; c < NV; ++c) {
         if (c < ncol) {
           const long long e = (long long)t * ncol + c;
           v[c] = ff_add(v[c], fsrc ? ff_of(fsrc[e]) : ff_from(dsrc[e]));
@@ -571,75 +563,73 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
       }
     }
   }
-  double out[12];
-  block_sum<12, kRedThreads>(v, sh, out);
-  if (threadIdx.x != 0) return;
+#pragma unroll
+  for (int c = 0; c < NV; ++c) {
+    v[c] = ff_warp_sum(v[c]);
+    if ((threadIdx.x & 31) == 0) sh[c][threadIdx.x >> 5] = v[c];
+  }
+  __syncthreads();
+  const int c = threadIdx.x;
+  if (c >= 32) return;
+  double x = 0.0;
+  if (c < NV) {
+    const FF t = ff_add(ff_add(ff_add(sh[c][0], sh[c][1]), sh[c][2]), sh[c][3]);
+    x = soft_f2d(t.hi) + soft_f2d(t.lo);
+  }
   if (grp == 0) {
-    ob.U_dipR = out[0];
-    for (int c = 0; c < 9; ++c) ob.PT_dipR[c] = out[1 + c];
+    if (c == 0) ob.U_dipR = x;
+    else if (c < 10) ob.PT_dipR[c - 1] = x;
   } else if (grp == 1) {
-    ob.U_dipK = out[0];
-    for (int c = 0; c < 9; ++c) ob.PT_dipK[c] = out[1 + c];
+    if (c == 0) ob.U_dipK = x;
+    else if (c < 10) ob.PT_dipK[c - 1] = x;
   } else if (grp == 2) {
-    ob.U_ss = out[0];
-    ob.W_ss = out[1];
-    for (int c = 0; c < 9; ++c) ob.PT_ss[c] = out[2 + c];
+    if (c == 0) ob.U_ss = x;
+    else if (c == 1) ob.W_ss = x;
+    else if (c < 11) ob.PT_ss[c - 2] = x;
   } else if (grp == 4) {
-    for (int c = 0; c < 12; ++c) ob.osum[c] = out[c];
+    if (c < 12) ob.osum[c] = x;
   } else {
-    ob.U_ext = out[8];
-    ob.U_self = P.Uself;
-    if (mode & kRedStep) {
-      ob.K[0] = 0.5 * out[0];
-      ob.K[1] = 0.5 * out[1];
-      const double pt6[6] = {out[2], out[3], out[4], out[5], out[6], out[7]};
-      const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-      for (int c = 0; c < 9; ++c) ob.PT_kin[c] = pt6[map[c]];
-      // moveTher mode 2 (v25/functions.cpp:2207-2213) closes the step
-      const double* nz = b.noise + ((long long)S.iter * b.nsys + s) * 4;
-      S.xi[0] = P.ex1 * S.xi_mid[0] + P.cnoise * nz[1];
-      S.xi[1] = P.ex1 * S.xi_mid[1] + P.cnoise * nz[3];
-      S.strn[0] = nz[1];
-      S.strn[1] = nz[3];
-      S.step += 1;
-      S.iter += 1;
-      if (S.rebuild) S.list_builds += 1;
-      S.force_list = 0;
+    if (c == 8) {
+      ob.U_ext = x;
+      ob.U_self = P.Uself;
     }
-    ob.xi[0] = S.xi[0];
-    ob.xi[1] = S.xi[1];
-    ob.step = S.step;
-    ob.status = S.status;
-    ob.list_builds = S.list_builds;
+    if (mode & kRedStep) {
+      if (c < 2) {
+        ob.K[c] = 0.5 * x;
+        // moveTher mode 2 (v25/functions.cpp:2207-2213) closes the step
+        const double g = b.noise[((long long)S.iter * b.nsys + s) * 4 + 2 * c + 1];
+        const double xi = P.ex1 * S.xi_mid[c] + P.cnoise * g;
+        S.xi[c] = xi;
+        S.strn[c] = g;
+        ob.xi[c] = xi;
+      } else if (c < 8) {
+        // (xx xy)(yy yz)(zz zx) to their places and mirrors
+        const int a = (c - 2) >> 1, q = (c & 1) ? (a + 1) % 3 : a;
+        ob.PT_kin[3 * a + q] = x;
+        ob.PT_kin[3 * q + a] = x;
+      }
+      __syncwarp();
+      if (c == 0) {
+        S.step += 1;
+        S.iter += 1;
+        if (S.rebuild) S.list_builds += 1;
+        S.force_list = 0;
+      }
+      __syncwarp();
+    } else if (c < 2) {
+      ob.xi[c] = S.xi[c];
+    }
+    if (c == 0) {
+      ob.step = S.step;
+      ob.status = S.status;
+      ob.list_builds = S.list_builds;
+    }
   }
 }
 
 // ---------------------------------------------------------------------
 // function-level entry points
 // ---------------------------------------------------------------------
-__global__ void __launch_bounds__(kPartBlock) movex_kernel(Batch b) {
-  const int2 bk = b.blk[blockIdx.x];
-  const SysDev& P = b.sys[bk.x];
-  const int i = bk.y + threadIdx.x;
-  if (i >= P.part_off + P.n) return;
-  double r[3], p[3], l[3], O[9];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    r[a] = b.r[3 * i + a];
-    p[a] = b.p[3 * i + a];
-    l[a] = b.l[3 * i + a];
-  }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) O[k] = b.O[9 * i + k];
-  move_x(b, i, P.dt, r, p, O, l);
-#pragma unroll
-  for (int a = 0; a < 3; ++a) b.r[3 * i + a] = r[a];
-#pragma unroll
-  for (int k = 0; k < 9; ++k) b.O[9 * i + k] = O[k];
-  uint32_t u[3];
-  derive_particle(b, P, i, r, O, u);
-}
-
 __global__ void __launch_bounds__(kPartBlock) renorm_kernel(Batch b) {
   const int2 bk = b.blk[blockIdx.x];
   const SysDev& P = b.sys[bk.x];
@@ -719,13 +709,16 @@ void launch_reset_iter(const Batch& b, cudaStream_t s) {
   if (b.nsys) reset_iter_kernel<<<cdiv(b.nsys, 128), 128, 0, s>>>(b);
 }
 void launch_derive(const Batch& b, cudaStream_t s) {
-  if (b.nblk) derive_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
+  if (b.nwblk) particle_kernel<kPartDerive><<<b.nwblk, kRowBlock, 0, s>>>(b);
 }
 void launch_integrate_first(const Batch& b, cudaStream_t s) {
-  if (b.nblk) integrate_first_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
+  if (b.nwblk) particle_kernel<kPartStep><<<b.nwblk, kRowBlock, 0, s>>>(b);
+}
+void launch_xi_mid(const Batch& b, cudaStream_t s) {
+  if (b.nsys) xi_mid_kernel<<<b.nsys, 128, 0, s>>>(b);
 }
 void launch_finalize(const Batch& b, int mode, cudaStream_t s) {
-  if (b.nblk) finalize_kernel<<<b.nblk, kPartBlock, 0, s>>>(b, mode);
+  if (b.nwblk) finalize_kernel<<<b.nwblk, kRowBlock, 0, s>>>(b, mode);
 }
 void launch_order_terms(const Batch& b, cudaStream_t s) {
   if (b.nblk) order_terms_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
@@ -734,7 +727,7 @@ void launch_reduce_obs(const Batch& b, int mode, cudaStream_t s) {
   if (b.nsys) reduce_obs_kernel<<<kRedGroups * b.nsys, kRedThreads, 0, s>>>(b, mode);
 }
 void launch_movex(const Batch& b, cudaStream_t s) {
-  if (b.nblk) movex_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
+  if (b.nwblk) particle_kernel<kPartMoveX><<<b.nwblk, kRowBlock, 0, s>>>(b);
 }
 void launch_renorm(const Batch& b, cudaStream_t s) {
   if (b.nblk) renorm_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);

@@ -42,10 +42,11 @@ __global__ void __launch_bounds__(kPartBlock) list_prep_kernel(Batch b, int forc
   SysState& S = b.st[bk.x];
   bool need = (force_all || S.force_list) && !at_limit(b, bk.x);
   if (!need && !at_limit(b, bk.x)) {
-    double m = 0.0;
-    for (int k = 0; k < P.nblk; ++k) m = fmax(m, b.dmax[P.blk_off + k]);
-    need = 2.0 * m > P.skin;
+    float m = 0.f;
+    for (int k = threadIdx.x; k < P.nw; k += kPartBlock) m = fmaxf(m, b.dmax[P.w_off + k]);
+    need = 2.0 * soft_f2d(m) > P.skin;
   }
+  need = __syncthreads_or(need);
   const int j = blk_slot(P, bk) - P.blk_off;
   if (j == 0 && threadIdx.x == 0) {
     S.rebuild = need ? 1 : 0;

@@ -97,6 +97,7 @@ struct SysDev {
   int kt_off, nkt;          // k tiles: the system's energy rows
   int gch_off, pad_g;       // first chunk of the system in the G-tensor partials
   int blk_off, nblk;        // per-particle block range
+  int w_off, nw;            // rows of 32 particles: the per-particle kernels' partial sums
   int cl_fr;
   int cl_mode;     // cluster bonds: 0 the reference's geometric test, 1 pair energy
   // cell grid of the list build (set at upload from the shapes): ncell = 0
@@ -252,7 +253,6 @@ struct Batch {
   int* wlist_n;  // its length this step
   double* wown;  // n * kMaxC * 6: the lower index's force and torque of each candidate
   double* wev;   // n * kMaxC * 11: U, W, PT of each candidate
-  double* wcaE;  // per particle block: U, W, PT (11) of its own candidates
   int* wcand;    // n * kMaxC contact candidates (higher index) of each particle
   int* wcnt;     // n
   int* win;      // n * kMaxC: the candidate slots in which a lower-index particle holds this one
@@ -271,19 +271,22 @@ struct Batch {
   int2* ktile;   // (system, tile) of every k tile
   int nktile;
   double* kG;    // 6 per particle chunk: sum of m m^T (one dipole per particle)
-  int* icnt;     // per system: first-half blocks done this step (the last one sets xi_mid)
   int2* kgwork;  // (particle block, k tile or -1: all) of every k-space gather block
   int nkgwork;
   float* kgpart; // tile sums of split gathers: per (particle block, tile, dipole) 6 x kPartBlock
   int* kgdone;   // per particle block: tiles done this launch (the last one combines them)
   float2* Fk;    // 3 ndip: k-space force on each dipole, float-float (hi, lo)
   float2* Tk;    // 3 ndip: k-space torque m x G, float-float
-  // integrator partials, per block
-  double* kin1;  // 2 per block
-  double* kin2;  // 9 per block: K_t, K_r, PTkin xx xy xz yy yz zz, U_ext
-  double* dmax;  // 1 per block: largest displacement measure since the last list build
+  // integrator partials, float-float, per row of 32 particles and component
+  float2* krow;  // 2: K_t, K_r after the first half kick
+  float2* krow2; // 5: K_t, K_r, two kinetic pressure terms, U_ext (finalize_kernel)
+  float2* wrow;  // 4: WCA terms of the rods' own candidates (finalize_kernel)
+  float* dmax;   // 1 per row: largest displacement measure since the last list build
+  double* kin2;  // mdsc_moveP: 9 per particle block
   double* obk;   // 12 per block: the order-parameter terms of SysObs::osum
   int2* blk;     // (sys, first particle) per block
+  int2* wblk;    // (sys, first particle) per row of 32 particles
+  int nwblk;
   // cell bins of the list build: per cell its count, and kCellSlots slots
   // of (fixed-point position, batch index) and (axis, length), filled in
   // any order by the binning kernel

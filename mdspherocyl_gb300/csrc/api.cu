@@ -25,8 +25,7 @@ cudaError_t prepare_real_pairs();
 cudaError_t prepare_kspace();
 cudaError_t prepare_wca();
 void launch_real_sum(const Batch& b, cudaStream_t s);
-// the cutoff systems' neighbour pass: real space (1), WCA screen (2), both (3)
-void launch_near_pass(const Batch& b, int mode, cudaStream_t s);
+void launch_near_pass(const Batch& b, cudaStream_t s);  // the cutoff systems' real space
 void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, cudaStream_t s);
 void launch_derive(const Batch& b, cudaStream_t s);
 void launch_integrate_first(const Batch& b, cudaStream_t s);
@@ -38,9 +37,7 @@ void launch_movex(const Batch& b, cudaStream_t s);
 void launch_renorm(const Batch& b, cudaStream_t s);
 void launch_movep(const Batch& b, const double* xi, int last, cudaStream_t s);
 void launch_list_build(const Batch& b, int force_all, cudaStream_t s);
-// the WCA screens and FP64 evaluation; near_mode: what the cutoff systems'
-// neighbour pass runs besides its WCA screen (1: also their real space)
-void launch_wca(const Batch& b, int near_mode, cudaStream_t s);
+void launch_wca(const Batch& b, bool clear, cudaStream_t s);
 void launch_cluster_bonds(const Batch& b, cudaStream_t s);
 void launch_ebond(const Batch& b, cudaStream_t s);
 void launch_cluster_hook(const Batch& b, cudaStream_t s);
@@ -549,6 +546,7 @@ void carve(Arena& A, const Layout& Lo, int nsys, Batch& b, int4** kwork, int2** 
   b.cellblk = A.take<int2>(std::max<size_t>(Lo.cellblk.size(), 1));
   b.nb = A.take<int>(n * kMaxNb);
   b.nbc = A.take<int>(n);
+  b.nblo = A.take<int>(n);
   b.fsave = A.take<uint32_t>(3 * n);
   b.usave = A.take<float>(3 * n);
   b.comp = A.take<int>(n);
@@ -572,7 +570,7 @@ struct mdsc_batch {
   int nsys = 0;
   cudaStream_t st = nullptr, s2 = nullptr, s3 = nullptr, s4 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_j2 = nullptr, ev_j3 = nullptr, ev_j4 = nullptr, ev_k = nullptr,
-              ev_mid = nullptr;
+              ev_mid = nullptr, ev_list = nullptr;
   // mdsc_step_io: the stream that takes positions and orientations home
   // while a step's forces are computed, and the event its graph records
   // once they are final
@@ -647,7 +645,8 @@ mdsc_status eval_forces(mdsc_batch* B, int force_list, const int* skip = nullptr
   b.skip = skip;
   launch_derive(b, B->st);
   launch_list_build(b, force_list, B->st);
-  launch_wca(b, 1, B->st);  // with the cutoff systems' real space, in the same neighbour pass
+  launch_wca(b, false, B->st);
+  launch_near_pass(b, B->st);
   launch_real_pairs(b, B->lo.multi, B->st);
   launch_real_sum(b, B->st);
   launch_kspace(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, B->st);
@@ -724,7 +723,11 @@ mdsc_status autotune(mdsc_batch* B, int force, int reps) {
       const double t = time_launches(B, reps, launch);
       snprintf(line, sizeof line, "%s=%d %.4f ms; ", what, cand[k], t);
       B->tune_log += line;
-      if (t < tbest) {
+      // candidates ascend in what they hold of the SMs beside the step's other
+      // chains, which a kernel timed alone does not show (the WCA evaluation's
+      // grid on 608 blocks held every register of the GPU: 107 us per step of
+      // 4096 rods against 88 on 304): a larger one has to be clearly faster
+      if (t < (k ? 0.95 : 1.0) * tbest) {
         tbest = t;
         vbest = cand[k];
       }
@@ -735,7 +738,7 @@ mdsc_status autotune(mdsc_batch* B, int force, int reps) {
   {
     const int m = B->num_sms;
     const int cand[4] = {m * 2, m * 4, m * 8, m * 16};
-    pick("wca_blocks", cand, 4, b.tune.wca_blocks, [&] { launch_wca(b, 0, B->st); });
+    pick("wca_blocks", cand, 4, b.tune.wca_blocks, [&] { launch_wca(b, true, B->st); });
   }
   // real-space tiles per block, then the strip-sum block size
   if (b.ntiles > 0) {
@@ -781,12 +784,17 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   cudaStreamWaitEvent(B->s2, B->ev_fork, 0);
   cudaStreamWaitEvent(B->s3, B->ev_fork, 0);
   launch_list_build(b, 0, B->st);
-  launch_wca(b, 1, B->st);  // the cutoff systems' real space in their neighbour pass, after their list
-  // xi at mid-step, order terms, the list build's decision and scan (+ the cell
-  // binning), the WCA screen and evaluation (+ the cutoff pass)
-  launches += 6 + (b.cells && b.ncellblk ? 1 : 0) + (b.any_rc ? 1 : 0);
+  cudaEventRecord(B->ev_list, B->st);
+  launch_wca(b, false, B->st);
+  // xi at mid-step, order terms, the list build (+ the cell binning), the WCA
+  // screen and evaluation (+ the cutoff pass)
+  launches += 5 + (b.cells && b.ncellblk ? 1 : 0) + (b.any_rc ? 1 : 0);
   launch_real_pairs(b, B->lo.multi, B->s2);
   launch_real_sum(b, B->s2);
+  if (b.any_rc) {  // the cutoff systems' real space, once their lists stand
+    cudaStreamWaitEvent(B->s2, B->ev_list, 0);
+    launch_near_pass(b, B->s2);
+  }
   launches += b.ntiles > 0 ? 2 + (b.nbstrips > 0 ? 1 : 0) : 0;
   auto kpart = [&](int part, cudaStream_t s) {
     launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, part, s);
@@ -819,7 +827,7 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   e = cudaGraphInstantiate(io ? &B->graph_io[which] : &B->graph[which], g, cudaGraphInstantiateFlagUseNodePriority);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) return fail(B, MDSC_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-  if (!io) B->launches = launches;
+  B->launches = launches;
   return MDSC_OK;
 }
 
@@ -1258,6 +1266,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
       cudaEventCreateWithFlags(&B->ev_j4, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_k, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_mid, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&B->ev_list, cudaEventDisableTiming) != cudaSuccess ||
       cudaStreamCreateWithFlags(&B->sio, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_x, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_f, cudaEventDisableTiming) != cudaSuccess ||
@@ -1308,6 +1317,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   cudaMemsetAsync(b.fsave, 0, sizeof(uint32_t) * 3 * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(b.usave, 0, sizeof(float) * 3 * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(b.nbc, 0, sizeof(int) * std::max(lo.ntot, 1), B->st);
+  cudaMemsetAsync(b.nblo, 0, sizeof(int) * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(b.wcnt, 0, sizeof(int) * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(b.wincnt, 0, sizeof(int) * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(b.stripE, 0, sizeof(double) * 10 * std::max(lo.nstrips, 1), B->st);
@@ -1372,6 +1382,7 @@ mdsc_status mdsc_destroy(mdsc_batch* B) {
   if (B->ev_j4) cudaEventDestroy(B->ev_j4);
   if (B->ev_k) cudaEventDestroy(B->ev_k);
   if (B->ev_mid) cudaEventDestroy(B->ev_mid);
+  if (B->ev_list) cudaEventDestroy(B->ev_list);
   if (B->ev_x) cudaEventDestroy(B->ev_x);
   if (B->ev_f) cudaEventDestroy(B->ev_f);
   if (B->sio) cudaStreamDestroy(B->sio);
@@ -1651,7 +1662,7 @@ mdsc_status mdsc_force_sc(mdsc_batch* B, double* U, double* W, double* PT) {
   if (st) return st;
   launch_derive(B->b, B->st);
   launch_list_build(B->b, 0, B->st);
-  launch_wca(B->b, 0, B->st);
+  launch_wca(B->b, false, B->st);
   launch_finalize(B->b, kMaskWca | kFlagAccum, B->st);
   launch_order_terms(B->b, B->st);
   launch_reduce_obs(B->b, kRedEnergies, B->st);
@@ -1670,7 +1681,7 @@ mdsc_status mdsc_force_dipR(mdsc_batch* B, double* U, double* PT) {
   if (st) return st;
   launch_derive(B->b, B->st);
   if (B->b.any_rc) launch_list_build(B->b, 0, B->st);
-  launch_near_pass(B->b, 1, B->st);
+  launch_near_pass(B->b, B->st);
   launch_real_pairs(B->b, B->lo.multi, B->st);
   launch_real_sum(B->b, B->st);
   launch_finalize(B->b, kMaskReal | kFlagAccum, B->st);
@@ -2267,16 +2278,6 @@ static mdsc_status run_steps(mdsc_batch* B, int nsteps, mdsc_observables* trace,
       if (st) return st;
     }
   }
-  for (int w = 0; w < 2; ++w)
-    if (!B->graph[w]) {
-      st = capture_step(B, w);
-      if (st) return st;
-    }
-  for (int w = 0; out && w < 2; ++w)
-    if (!B->graph_io[w]) {
-      st = capture_step(B, w, true);
-      if (st) return st;
-    }
   if (trace && !B->h_trace) CU(cudaMallocHost(&B->h_trace, sizeof(SysObs) * kNoiseChunk * B->nsys));
   int which = 0;
   int done = 0;
@@ -2290,6 +2291,16 @@ static mdsc_status run_steps(mdsc_batch* B, int nsteps, mdsc_observables* trace,
       const long long k0 = B->step_h[s];
       const long long next = ((k0 + fr - 1) / fr) * fr;  // first k >= k0 with k % fr == 0
       chunk = (int)std::min<long long>(chunk, next - k0 + 1);
+    }
+    // the graphs this chunk runs (a call of one step needs one of the four)
+    const bool io_last = out && done + chunk == nsteps;
+    if (chunk > (io_last ? 1 : 0) && !B->graph[which]) {
+      st = capture_step(B, which);
+      if (st) return st;
+    }
+    if (io_last && !B->graph_io[which]) {
+      st = capture_step(B, which, true);
+      if (st) return st;
     }
     // noise for this chunk, into the host buffer of this noise buffer once
     // its last copy has gone (no wait for the GPU's other work: an upload or
@@ -2518,13 +2529,13 @@ mdsc_status mdsc_profile_steps(mdsc_batch* B, int nsteps, int max_kernels, char*
     cudaEventRecord(ev[2], B->st);
     launch_list_build(b, 0, B->st);
     cudaEventRecord(ev[3], B->st);
-    launch_wca(b, 0, B->st);
+    launch_wca(b, false, B->st);
     cudaEventRecord(ev[4], B->st);
     launch_real_pairs(b, B->lo.multi, B->st);
     cudaEventRecord(ev[5], B->st);
     launch_real_sum(b, B->st);
     cudaEventRecord(ev[6], B->st);
-    launch_near_pass(b, 1, B->st);
+    launch_near_pass(b, B->st);
     cudaEventRecord(ev[7], B->st);
     // the k-space kernels, timed one by one (the energies with the chunk sums)
     launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 0, B->st);

@@ -141,12 +141,16 @@ __device__ __forceinline__ float derive_comp(const Batch& b, const SysDev& P, Sh
   return disp;
 }
 
-// the block's largest displacement measure, from warp 2
-__device__ __forceinline__ void store_disp(const Batch& b, int row, int a, float disp) {
+// the block's largest displacement measure, from warp 2 (non-negative, so its
+// bits order as integers)
+__device__ __forceinline__ void store_disp(const Batch& b, SysState& S, int row, int a, float disp) {
   if (a != 2) return;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) disp = fmaxf(disp, __shfl_xor_sync(0xffffffffu, disp, off));
-  if ((threadIdx.x & 31) == 0) b.dmax[row] = disp;
+  if ((threadIdx.x & 31) == 0) {
+    b.dmax[row] = disp;
+    atomicMax(&S.dmax, __float_as_int(disp));
+  }
 }
 
 // the free-rotor move of the step (Spherocyl::rotate, v25/classes.cpp:240-304):
@@ -195,13 +199,22 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
   __shared__ double sfac[2];
   const int2 bk = b.wblk[blockIdx.x];
   const int s = bk.x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *b.wlist_n = 0;
   if (MODE == kPartStep && at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
-  const SysState& S = b.st[s];
+  SysState& S = b.st[s];
   const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool ok = bk.y + lane < P.part_off + P.n;
   const int i = ok ? bk.y + lane : bk.y;  // lanes past the end repeat the first rod and store nothing
   const int row = P.w_off + (bk.y - P.part_off) / kRows;
+  // what the lists and the WCA screen of the new configuration count up from:
+  // the partners' slots, and the cells (at most one per 8 rods)
+  if (a == 0 && ok) b.wincnt[i] = 0;
+  if (P.ncell > 0 && a == 1) {
+    const int c = (bk.y - P.part_off) / 8 + lane;
+    if (lane < kRows / 8 && c < P.ncell) b.ccnt[P.cell_off + c] = 0;
+    if (bk.y == P.part_off && lane == 0) S.cell_ovf = 0;
+  }
   double r = b.r[3 * i + a], O[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) O[c] = b.O[9 * i + 3 * a + c];
@@ -260,7 +273,7 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
     }
   }
   const float disp = derive_comp(b, P, sh, a, lane, i, ok, r, O);
-  if constexpr (MODE != kPartMoveX) store_disp(b, row, a, disp);
+  if constexpr (MODE != kPartMoveX) store_disp(b, S, row, a, disp);
 }
 
 // Thermostat coordinates of the second half kick, moveTher 0 then 1
@@ -311,8 +324,9 @@ __global__ void __launch_bounds__(kRowBlock) finalize_kernel(Batch b, int mode) 
   const int s = bk.x;
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
-  const SysState& S = b.st[s];
+  SysState& S = b.st[s];
   const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (bk.y == P.part_off && threadIdx.x == 0) S.dmax = 0;  // the lists of this configuration stand
   const bool ok = bk.y + lane < P.part_off + P.n;
   const int i = ok ? bk.y + lane : bk.y;
   const int row = 3 * (P.w_off + (bk.y - P.part_off) / kRows) + a;

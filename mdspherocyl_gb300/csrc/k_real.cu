@@ -57,7 +57,6 @@
 // reference's table is there to FP32 precision.
 #include "mdsc_dev.cuh"
 #include "reduce.cuh"
-#include "wca_screen.cuh"
 
 namespace mdsc {
 
@@ -635,11 +634,9 @@ __global__ void __launch_bounds__(32 * kSmemWarps, 1) real_pairs_smem_kernel(Bat
     tile_work<MULTI, kTabShared>(b, t, K, sj, smj, sa4, sa2);
 }
 
-// The neighbour pass of the systems with a real-space cutoff, over the two
-// lists one scan of list_build wrote for each rod.
-//
-// Real space (mode kNearReal): the reference's force_dipR with its table
-// zeroed beyond rc_real, where pairs
+// The neighbour pass of the systems with a real-space cutoff, over the
+// real-space list that list_build wrote for each rod: the reference's
+// force_dipR with its table zeroed beyond rc_real, where pairs
 // beyond rc_real + Lh add nothing, so only the rods on the system's
 // real-space list are visited -- those whose centres are within rc_real +
 // Lh + the dipoles' offsets + the skin (list_build).  A group of kCutLanes
@@ -652,28 +649,13 @@ __global__ void __launch_bounds__(32 * kSmemWarps, 1) real_pairs_smem_kernel(Bat
 // alone and in any batch.  Writes each dipole's force and torque where
 // real_sum writes them, and its block's energy and pressure tensor
 // (float-float block sums) for the per-system sum.
-//
-// WCA screen (mode kNearWca): in the same blocks, the first kPartBlock
-// threads, a particle each, screen its Verlet list as the WCA screen kernel
-// does for the other systems (wca_screen.cuh), feeding the same FP64
-// evaluation.
 constexpr int kCutLanes = 4;
-enum : int { kNearReal = 1, kNearWca = 2 };
 
-__global__ void __launch_bounds__(kPartBlock * kCutLanes) near_pass_kernel(Batch b, int mode) {
+__global__ void __launch_bounds__(kPartBlock * kCutLanes) near_pass_kernel(Batch b) {
   __shared__ double sh[10 * kPartBlock * kCutLanes / 32];
   const int2 bk = b.blk[blockIdx.x];
   const SysDev& P = b.sys[bk.x];
   if (P.rc_real <= 0.0 || at_limit(b, bk.x)) return;  // the same for the whole block
-  if ((mode & kNearWca) && threadIdx.x < kPartBlock) {  // whole warps
-    const int i = bk.y + threadIdx.x;
-    const bool ok = i < P.part_off + P.n;
-    const int nl = ok ? b.nbc[i] : 0;
-    const int* lst = b.nb + (long long)(ok ? i : bk.y) * kMaxNb;
-    int k = 0;
-    wca_screen_one(b, P, bk.x, i, ok, [&]() { return k < nl ? lst[k++] : -1; });
-  }
-  if (!(mode & kNearReal)) return;
   const int nd = P.nd;
   const int p0 = bk.y - P.part_off;
   const int np = min(kPartBlock, P.n - p0);
@@ -841,8 +823,8 @@ __global__ void __launch_bounds__(128) strip_energy_kernel(Batch b) {
   }
 }
 
-void launch_near_pass(const Batch& b, int mode, cudaStream_t s) {
-  if (b.any_rc && b.nblk && mode) near_pass_kernel<<<b.nblk, kPartBlock * kCutLanes, 0, s>>>(b, mode);
+void launch_near_pass(const Batch& b, cudaStream_t s) {
+  if (b.any_rc && b.nblk) near_pass_kernel<<<b.nblk, kPartBlock * kCutLanes, 0, s>>>(b);
 }
 
 void launch_real_sum(const Batch& b, cudaStream_t s) {

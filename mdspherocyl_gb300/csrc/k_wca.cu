@@ -30,30 +30,14 @@
 #include "mdsc_dev.cuh"
 #include "reduce.cuh"
 #include "seg_dist.cuh"
-#include "wca_screen.cuh"
 
 namespace mdsc {
 
-// Rebuild decision of every system (the same in every block of a system),
-// and, for a system that rebuilds on cells, its cell counts zeroed.
-__global__ void __launch_bounds__(kPartBlock) list_prep_kernel(Batch b, int force_all) {
-  const int2 bk = b.blk[blockIdx.x];
-  const SysDev& P = b.sys[bk.x];
-  SysState& S = b.st[bk.x];
-  bool need = (force_all || S.force_list) && !at_limit(b, bk.x);
-  if (!need && !at_limit(b, bk.x)) {
-    float m = 0.f;
-    for (int k = threadIdx.x; k < P.nw; k += kPartBlock) m = fmaxf(m, b.dmax[P.w_off + k]);
-    need = 2.0 * soft_f2d(m) > P.skin;
-  }
-  need = __syncthreads_or(need);
-  const int j = blk_slot(P, bk) - P.blk_off;
-  if (j == 0 && threadIdx.x == 0) {
-    S.rebuild = need ? 1 : 0;
-    S.cell_ovf = 0;
-  }
-  if (!need || P.ncell == 0) return;
-  for (int c = j * kPartBlock + threadIdx.x; c < P.ncell; c += P.nblk * kPartBlock) b.ccnt[P.cell_off + c] = 0;
+// Does the system build its list this step?  From the largest displacement
+// measure of the new configuration (particle_kernel), the same in every block.
+__device__ __forceinline__ bool list_due(const Batch& b, const SysDev& P, const SysState& S, int s, int force_all) {
+  if (at_limit(b, s)) return false;
+  return force_all || S.force_list || 2.0 * soft_f2d(__int_as_float(S.dmax)) > P.skin;
 }
 
 // cell of a fixed-point position: floor(fraction x cells), exact
@@ -64,12 +48,13 @@ __device__ __forceinline__ int cell_of(const SysDev& P, uint32_t ux, uint32_t uy
   return (cz * P.cny + cy) * P.cnx + cx;
 }
 
-// Each rod of a rebuilding cell system into a slot of its cell (any order).
-__global__ void __launch_bounds__(kPartBlock) cell_bin_kernel(Batch b) {
+// Each rod of a rebuilding cell system into a slot of its cell (any order; the
+// counts were cleared with the working copies).
+__global__ void __launch_bounds__(kPartBlock) cell_bin_kernel(Batch b, int force_all) {
   const int2 bk = b.blk[blockIdx.x];
   const SysDev& P = b.sys[bk.x];
   SysState& S = b.st[bk.x];
-  if (!S.rebuild || P.ncell == 0) return;
+  if (P.ncell == 0 || !list_due(b, P, S, bk.x, force_all)) return;
   const int i = bk.y + threadIdx.x;
   if (i >= P.part_off + P.n) return;
   const int N = b.ntot;
@@ -98,12 +83,17 @@ __device__ __forceinline__ void sort_small(A& v, int n) {
   }
 }
 
+// A fixed grid looks through the rows for those that are due: most steps
+// rebuild few systems, and a block per row held the registers of the SMs from
+// the tiles that start at the same time.
+constexpr int kListBlocks = 4 * 152;
+
 // The cell scan: blocks of two cells (two warps each), a thread per slot.
-__device__ void list_cells(const Batch& b) {
-  const int2 cb = b.cellblk[blockIdx.x - b.nblk];
+__device__ void list_cells(const Batch& b, int force_all) {
+  const int2 cb = b.cellblk[blockIdx.x - kListBlocks];
   const SysDev& P = b.sys[cb.x];
   SysState& S = b.st[cb.x];
-  if (!S.rebuild || P.ncell == 0 || S.cell_ovf) return;
+  if (P.ncell == 0 || S.cell_ovf || !list_due(b, P, S, cb.x, force_all)) return;
   const int c = cb.y + (threadIdx.x >> 6);
   if (c >= P.ncell) return;
   const int t = threadIdx.x & 63;
@@ -162,8 +152,13 @@ __device__ void list_cells(const Batch& b) {
   cnt = min(cnt, kMaxNb);
   sort_small(lst, cnt);
   int* out = b.nb + (long long)i * kMaxNb;
-  for (int k = 0; k < cnt; ++k) out[k] = lst[k];
+  int lower = 0;
+  for (int k = 0; k < cnt; ++k) {
+    out[k] = lst[k];
+    lower += lst[k] < i ? 1 : 0;
+  }
   b.nbc[i] = cnt;
+  b.nblo[i] = lower;
   if (rcut) {
     rcnt = min(rcnt, kMaxR);
     sort_small(rout, rcnt);
@@ -178,22 +173,21 @@ __device__ void list_cells(const Batch& b) {
   }
 }
 
-// The list build: blocks below nblk scan all pairs of their particle block
-// (systems without cells, or whose cells overflowed this build); the rest
-// scan cells.
-__global__ void __launch_bounds__(kPartBlock) list_build_kernel(Batch b) {
+// The list build: blocks below nwblk scan all pairs for 32 rods (systems
+// without cells, or whose cells overflowed this build); the rest scan cells.
+// A few systems rebuild at a time, so the scan is a latency: the four warps
+// of a block hold the same 32 rods and take a quarter each of every chunk of
+// 128 candidates, whose hits they place in ascending order.
+// Averaged over the steps of 64 systems of 128 to 2048 rods: 35 us a launch with
+// a lane per rod over whole chunks (and its decision kernel), 19 this way.
+__device__ void list_row(const Batch& b, int2 bk) {
   __shared__ uint32_t sx[kPartBlock], sy[kPartBlock], sz[kPartBlock];
   __shared__ float4 sa[kPartBlock];
-  if ((int)blockIdx.x >= b.nblk) {
-    list_cells(b);
-    return;
-  }
-  const int2 bk = b.blk[blockIdx.x];
-  const int s = bk.x;
-  const SysDev& P = b.sys[s];
-  SysState& S = b.st[s];
-  if (!S.rebuild || (b.cells && P.ncell > 0 && !S.cell_ovf)) return;
-  const int i = bk.y + threadIdx.x;
+  __shared__ uint32_t sm[2][4][32], sr[2][4][32];  // hits per (buffer, warp, rod): Verlet and real-space lists
+  const SysDev& P = b.sys[bk.x];
+  SysState& S = b.st[bk.x];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = bk.y + lane;
   const bool ok = i < P.part_off + P.n;
   const int N = b.ntot;
   uint32_t ux = 0, uy = 0, uz = 0;
@@ -215,7 +209,8 @@ __global__ void __launch_bounds__(kPartBlock) list_build_kernel(Batch b) {
   const bool rcut = P.rc_real > 0.0;
   int rcnt = 0;
   int* rout = b.rnb + (long long)i * kMaxR;
-  for (int q0 = 0; q0 < n; q0 += kPartBlock) {
+  int buf = 0, lower = 0;
+  for (int q0 = 0; q0 < n; q0 += kPartBlock, buf ^= 1) {
     const int nq = min(kPartBlock, n - q0);
     __syncthreads();
     if (threadIdx.x < nq) {
@@ -226,67 +221,92 @@ __global__ void __launch_bounds__(kPartBlock) list_build_kernel(Batch b) {
       sa[threadIdx.x] = b.pax[q];
     }
     __syncthreads();
-    if (!ok) continue;
-    if (rcut) {
-      for (int k = 0; k < nq; ++k) {
-        const float dx = fix_diff(ux, sx[k], Lx);
-        const float dy = fix_diff(uy, sy[k], Ly);
-        const float dz = fix_diff(uz, sz[k], Lz);
-        if (dx * dx + dy * dy + dz * dz < P.rl_r2 && first + q0 + k != i) {
-          if (rcnt < kMaxR) rout[rcnt] = first + q0 + k;
-          ++rcnt;
-        }
-      }
-    }
     // 1. centre distance against the reach of the two rods, branch-free,
-    //    into a mask of the chunk's 128 candidates: nearly every warp has a
+    //    into a mask of the warp's 32 candidates: nearly every warp has a
     //    lane with some candidate in reach, so testing the segments inside
     //    this loop would run the segment routine for every candidate
-    uint32_t m[4];
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      uint32_t bits = 0u;
+    uint32_t bits = 0u, rbits = 0u;
 #pragma unroll 8
-      for (int kk = 0; kk < 32; ++kk) {
-        const int k = 32 * w + kk;
-        const float dx = fix_diff(ux, sx[k], Lx);
-        const float dy = fix_diff(uy, sy[k], Ly);
-        const float dz = fix_diff(uz, sz[k], Lz);
-        const float reach = rl + 0.5f * (ai.w + sa[k].w);
-        const float r2 = dx * dx + dy * dy + dz * dz;
-        const bool in = k < nq && r2 < reach * reach && first + q0 + k != i;
-        bits |= (uint32_t)in << kk;
-      }
-      m[w] = bits;
+    for (int kk = 0; kk < 32; ++kk) {
+      const int k = 32 * w + kk;
+      const float dx = fix_diff(ux, sx[k], Lx);
+      const float dy = fix_diff(uy, sy[k], Ly);
+      const float dz = fix_diff(uz, sz[k], Lz);
+      const float reach = rl + 0.5f * (ai.w + sa[k].w);
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      const bool other = ok && k < nq && first + q0 + k != i;
+      bits |= (uint32_t)(other && r2 < reach * reach) << kk;
+      if (rcut) rbits |= (uint32_t)(other && r2 < P.rl_r2) << kk;
     }
-    // 2. segment distance of the candidates in reach, in ascending order
+    // 2. segment distance of the candidates in reach
+    uint32_t hits = 0u;
+    for (uint32_t m = bits; m; m &= m - 1u) {
+      const int kk = __ffs(m) - 1, k = 32 * w + kk;
+      const float dx = fix_diff(ux, sx[k], Lx);
+      const float dy = fix_diff(uy, sy[k], Ly);
+      const float dz = fix_diff(uz, sz[k], Lz);
+      const float4 aj = sa[k];
+      const float d2 = seg_dist_fast(dx, dy, dz, ai.x, ai.y, ai.z, ai.w, aj.x, aj.y, aj.z, aj.w);
+      if (d2 < rl2) hits |= 1u << kk;
+    }
+    // 3. into the lists, after the lower warps' hits
+    sm[buf][w][lane] = hits;
+    if (rcut) sr[buf][w][lane] = rbits;
+    __syncthreads();
+    int at = cnt, rat = rcnt;
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      for (uint32_t bits = m[w]; bits; bits &= bits - 1u) {
-        const int k = 32 * w + __ffs(bits) - 1;
-        const float dx = fix_diff(ux, sx[k], Lx);
-        const float dy = fix_diff(uy, sy[k], Ly);
-        const float dz = fix_diff(uz, sz[k], Lz);
-        const float4 aj = sa[k];
-        const float d2 = seg_dist_fast(dx, dy, dz, ai.x, ai.y, ai.z, ai.w, aj.x, aj.y, aj.z, aj.w);
-        if (d2 < rl2) {
-          if (cnt < kMaxNb) out[cnt] = first + q0 + k;
-          ++cnt;
-        }
+    for (int v = 0; v < 4; ++v) {
+      const uint32_t h = sm[buf][v][lane];
+      const int c = __popc(h), below = i - (first + q0 + 32 * v);  // candidates of lower index
+      at += v < w ? c : 0;
+      cnt += c;
+      lower += __popc(below >= 32 ? h : (below > 0 ? h & ((1u << below) - 1u) : 0u));
+      if (rcut) {
+        const int rc = __popc(sr[buf][v][lane]);
+        rat += v < w ? rc : 0;
+        rcnt += rc;
       }
     }
+    for (uint32_t m = hits; m; m &= m - 1u, ++at)
+      if (at < kMaxNb) out[at] = first + q0 + 32 * w + __ffs(m) - 1;
+    for (uint32_t m = rbits; m; m &= m - 1u, ++rat)
+      if (rat < kMaxR) rout[rat] = first + q0 + 32 * w + __ffs(m) - 1;
   }
-  if (!ok) return;
+  if (!ok || w > 0) return;
   int err = (cnt > kMaxNb || rcnt > kMaxR) ? kErrListOverflow : 0;
   b.nbc[i] = min(cnt, kMaxNb);
-  if (rcut) {
-    b.rnbc[i] = min(rcnt, kMaxR);
-  }
+  b.nblo[i] = min(lower, kMaxNb);
+  if (rcut) b.rnbc[i] = min(rcnt, kMaxR);
   if (err) atomicOr(&S.status, err);
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     b.fsave[3 * i + a] = b.pfx[a * N + i];
     b.usave[3 * i + a] = a == 0 ? ai.x : (a == 1 ? ai.y : ai.z);
+  }
+}
+
+__global__ void __launch_bounds__(kPartBlock) list_build_kernel(Batch b, int force_all) {
+  __shared__ int due_rows[kPartBlock], ndue;
+  if ((int)blockIdx.x >= kListBlocks) {
+    list_cells(b, force_all);
+    return;
+  }
+  for (int r0 = blockIdx.x; r0 < b.nwblk; r0 += kListBlocks * kPartBlock) {
+    if (threadIdx.x == 0) ndue = 0;
+    __syncthreads();
+    const int r = r0 + threadIdx.x * kListBlocks;
+    if (r < b.nwblk) {
+      const int2 bk = b.wblk[r];
+      const SysDev& P = b.sys[bk.x];
+      SysState& S = b.st[bk.x];
+      const bool due = list_due(b, P, S, bk.x, force_all);
+      if (bk.y == P.part_off) S.rebuild = due ? 1 : 0;
+      if (due && !(b.cells && P.ncell > 0 && !S.cell_ovf)) due_rows[atomicAdd(&ndue, 1)] = r;
+    }
+    __syncthreads();
+    const int nd = ndue;
+    for (int k = 0; k < nd; ++k) list_row(b, b.wblk[due_rows[k]]);
+    __syncthreads();
   }
 }
 
@@ -374,10 +394,10 @@ __device__ bool wca_pair(const Batch& b, const SysDev& P, int A, int B, double* 
   return true;
 }
 
-// WCA in two kernels.  (1) wca_screen: each thread screens its particle's
-// partners of higher index (each pair once) in FP32, keeps the candidates in
-// ascending index in its slots (wcand) and appends (slot, system) items to
-// a work list, one atomic per warp.  (2) wca_eval: every thread of a fixed
+// WCA in two kernels.  (1) wca_screen: each particle's partners of higher
+// index (each pair once) are screened in FP32 against 2^(1/3) sigma^2 with a
+// margin; the candidates go to the particle's slots (wcand) in ascending
+// index and (slot, system) items to a work list, one atomic per warp.  (2) wca_eval: every thread of a fixed
 // grid takes list items and evaluates them in FP64 -- only pairs that can
 // touch reach the FP64 unit (1/64 of the FP32 rate on this GPU), densely
 // packed, with no block-wide synchronisation.  Each item writes its own
@@ -387,17 +407,83 @@ __device__ bool wca_pair(const Batch& b, const SysDev& P, int A, int B, double* 
 // order, and the per-system reduction adds the slots' energies in particle
 // and slot order, so the list order (which depends on warp timing) does not
 // reach any result.
-__global__ void __launch_bounds__(kPartBlock) wca_screen_kernel(Batch b) {
-  const int2 bk = b.blk[blockIdx.x];
+//
+// The screen takes LANES lanes per rod: the lanes test LANES list entries of
+// higher index at a time (each a chain of gathers, so one
+// lane per rod waited for its whole list), a ballot puts the entries that
+// pass into the rod's slots in list order -- ascending partners -- and each
+// partner learns where its share of the pair will be (win, wincnt).
+template <int LANES>
+__global__ void __launch_bounds__(128) wca_screen_kernel(Batch b) {
+  constexpr int kPer = 32 * LANES / 128;  // blocks per row of 32 rods
+  const int2 bk = b.wblk[blockIdx.x / kPer];
   const int s = bk.x;
+  if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
-  if (P.rc_real > 0.0 || at_limit(b, s)) return;  // cutoff systems: screened in their neighbour pass
-  const int i = bk.y + threadIdx.x;
+  const int lane = threadIdx.x & 31, sub = lane % LANES, grp = lane / LANES;
+  const int i = bk.y + (blockIdx.x % kPer * 128 + threadIdx.x) / LANES;
   const bool ok = i < P.part_off + P.n;
-  const int nl = ok ? b.nbc[i] : 0;
+  const int N = b.ntot;
+  int nl = 0, lo = 0, nc = 0, err = 0;
+  uint32_t ux = 0, uy = 0, uz = 0;
+  float4 ai = make_float4(0.f, 0.f, 1.f, 0.f);
+  float di = 0.f;
+  if (ok) {
+    nl = b.nbc[i];
+    lo = b.nblo[i];  // the list ascends: entries from here on are above i
+    ux = b.pfx[i];
+    uy = b.pfx[N + i];
+    uz = b.pfx[2 * N + i];
+    ai = b.pax[i];
+    di = b.pdia[i];
+  }
   const int* lst = b.nb + (long long)i * kMaxNb;
-  int k = 0;
-  wca_screen_one(b, P, s, i, ok, [&]() { return k < nl ? lst[k++] : -1; });
+  for (int k = lo + sub; __any_sync(0xffffffffu, k < nl); k += LANES) {
+    bool cand = false;
+    int q = -1;
+    if (k < nl) {
+      q = lst[k];
+      const float dx = fix_diff(ux, b.pfx[q], P.Lfix[0]);
+      const float dy = fix_diff(uy, b.pfx[N + q], P.Lfix[1]);
+      const float dz = fix_diff(uz, b.pfx[2 * N + q], P.Lfix[2]);
+      const float4 aj = b.pax[q];
+      const float sg = 0.5f * (di + b.pdia[q]);
+      const float d2 = seg_dist_fast(dx, dy, dz, ai.x, ai.y, ai.z, ai.w, aj.x, aj.y, aj.z, aj.w);
+      // 2^(1/3) sigma^2, with a margin for the FP32 screen
+      cand = d2 < 1.2599211f * sg * sg * 1.002f;
+    }
+    const uint32_t mask = (__ballot_sync(0xffffffffu, cand) >> (grp * LANES)) & ((1u << LANES) - 1u);
+    if (cand) {
+      const int slot = nc + __popc(mask & ((1u << sub) - 1u));
+      if (slot < kMaxC) {
+        b.wcand[(long long)i * kMaxC + slot] = q;
+        const int t = atomicAdd(&b.wincnt[q], 1);
+        if (t < kMaxC)
+          b.win[(long long)q * kMaxC + t] = i * kMaxC + slot;
+        else
+          err |= kErrListOverflow;
+      }
+    }
+    nc += __popc(mask);
+  }
+  if (nc > kMaxC) {
+    err |= kErrListOverflow;
+    nc = kMaxC;
+  }
+  if (ok && sub == 0) b.wcnt[i] = nc;
+  // room on the work list for the warp's candidates: one atomic per warp
+  int at = 0, tot = 0;
+#pragma unroll
+  for (int g = 0; g < 32 / LANES; ++g) {
+    const int c = __shfl_sync(0xffffffffu, nc, g * LANES);
+    at += g < grp ? c : 0;
+    tot += c;
+  }
+  int base = 0;
+  if (lane == 0 && tot > 0) base = atomicAdd(b.wlist_n, tot);
+  at += __shfl_sync(0xffffffffu, base, 0);
+  for (int k = sub; k < nc; k += LANES) b.wlist[at + k] = make_int2(i * kMaxC + k, s);
+  if (err) atomicOr(&b.st[s].status, err);
 }
 
 __global__ void __launch_bounds__(128) wca_eval_kernel(Batch b) {
@@ -668,27 +754,33 @@ __global__ void __launch_bounds__(kPartBlock) cluster_compress_kernel(Batch b) {
 }
 
 void launch_list_build(const Batch& b, int force_all, cudaStream_t s) {
-  if (!b.nblk) return;
-  list_prep_kernel<<<b.nblk, kPartBlock, 0, s>>>(b, force_all);
+  if (!b.nwblk) return;
   const int ncb = b.cells ? b.ncellblk : 0;
-  if (ncb) cell_bin_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
-  list_build_kernel<<<b.nblk + ncb, kPartBlock, 0, s>>>(b);
+  if (ncb) cell_bin_kernel<<<b.nblk, kPartBlock, 0, s>>>(b, force_all);
+  list_build_kernel<<<kListBlocks + ncb, kPartBlock, 0, s>>>(b, force_all);
 }
 // once per device: the step's memory split
 cudaError_t prepare_wca() {
-  return set_carveout(list_prep_kernel, cell_bin_kernel, list_build_kernel, wca_screen_kernel, wca_eval_kernel);
+  return set_carveout(cell_bin_kernel, list_build_kernel, wca_screen_kernel<4>, wca_screen_kernel<8>,
+                      wca_eval_kernel);
 }
-void launch_near_pass(const Batch& b, int mode, cudaStream_t s);  // k_real.cu
 
-void launch_wca(const Batch& b, int near_mode, cudaStream_t s) {
-  if (!b.nblk) return;
-  cudaMemsetAsync(b.wlist_n, 0, sizeof(int), s);
-  cudaMemsetAsync(b.wincnt, 0, sizeof(int) * b.ntot, s);
-  // cutoff systems: the WCA screen over their Verlet list in their
-  // neighbour pass (with their real space when near_mode says so); the
-  // others: in the screen kernel
-  launch_near_pass(b, 2 | near_mode, s);
-  wca_screen_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
+// rows of 32 rods up to which the screen takes 8 lanes per rod
+constexpr int kScreenWideMax = 1200;
+
+// The WCA screen and evaluation.  The work list's length and the partners'
+// slot counts are cleared with the working copies of every new configuration
+// (particle_kernel); clear: here, for a screen that runs again without one.
+void launch_wca(const Batch& b, bool clear, cudaStream_t s) {
+  if (!b.nwblk) return;
+  if (clear) {
+    cudaMemsetAsync(b.wlist_n, 0, sizeof(int), s);
+    cudaMemsetAsync(b.wincnt, 0, sizeof(int) * b.ntot, s);
+  }
+  if (b.nwblk <= kScreenWideMax)
+    wca_screen_kernel<8><<<2 * b.nwblk, 128, 0, s>>>(b);
+  else
+    wca_screen_kernel<4><<<b.nwblk, 128, 0, s>>>(b);
   // a fixed grid (chosen by the autotuner); each thread loops over the list
   wca_eval_kernel<<<b.tune.wca_blocks, 128, 0, s>>>(b);
 }

@@ -172,6 +172,7 @@ struct SysState {
   int iter;          // step index within the current mdsc_step call (noise row)
   int force_list;    // rebuild the Verlet list at the next check regardless of the skin
   int cell_ovf;      // this build: a cell held more than kCellSlots rods (all-pairs scan instead)
+  int dmax;          // largest displacement measure of the configuration (FP32 bits; cleared by finalize_kernel)
   long long stop;    // the step count at which the system stops taking steps (mdsc_set_step_limit)
   double K_first[2]; // kinetic energies after the first half kick
   double xi_mid[2];  // xi used by the second half kick
@@ -256,7 +257,7 @@ struct Batch {
   int* wcand;    // n * kMaxC contact candidates (higher index) of each particle
   int* wcnt;     // n
   int* win;      // n * kMaxC: the candidate slots in which a lower-index particle holds this one
-  int* wincnt;   // n: their number (zeroed before each screen)
+  int* wincnt;   // n: their number (zeroed by particle_kernel)
   double* wrec;  // n * kMaxC * 6: the partner's force and torque of each candidate
   // k-space
   int4* kn;      // (nx, ny, nz, 0) per k
@@ -302,6 +303,7 @@ struct Batch {
   // neighbour list
   int* nb;       // n * kMaxNb
   int* nbc;      // n
+  int* nblo;     // n: how many of them have a lower index (the list ascends)
   uint32_t* fsave; // 3n fixed-point positions at the last build
   float* usave;     // 3n axes at the last build
   // clusters

@@ -551,7 +551,6 @@ void carve(Arena& A, const Layout& Lo, int nsys, Batch& b, int4** kwork, int2** 
   b.usave = A.take<float>(3 * n);
   b.comp = A.take<int>(n);
   b.eflag = A.take<unsigned char>(n * kMaxNb);
-  b.flag = A.take<int>(1);
   b.ebond = A.take<int>(n * kMaxC);
   b.ebcnt = A.take<int>(n);
   b.eovf = A.take<int>(std::max(nsys, 1));
@@ -868,42 +867,41 @@ mdsc_status run_clusters(mdsc_batch* B, const std::vector<int>& systems) {
   launch_cluster_bonds(b, B->st);
   bool energy = false;
   for (int s = 0; s < B->nsys; ++s) energy |= B->lo.sys[s].cl_mode == 1;
+  std::vector<int> ovf(energy ? B->nsys : 0);
   if (energy) {
     CU(cudaMemsetAsync(b.eovf, 0, sizeof(int) * B->nsys, B->st));
     launch_ebond(b, B->st);
-    std::vector<int> ovf(B->nsys);
     CU(cudaMemcpyAsync(ovf.data(), b.eovf, sizeof(int) * B->nsys, cudaMemcpyDeviceToHost, B->st));
-    CU(cudaStreamSynchronize(B->st));
+  }
+  launch_cluster_hook(b, B->st);
+  launch_cluster_compress(b, B->st);
+  std::vector<std::vector<int>> comps(systems.size());
+  for (size_t k = 0; k < systems.size(); ++k) {
+    const SysDev& P = B->lo.sys[systems[k]];
+    comps[k].resize(P.n);
+    if (P.n)
+      CU(cudaMemcpyAsync(comps[k].data(), b.comp + P.part_off, sizeof(int) * P.n, cudaMemcpyDeviceToHost, B->st));
+  }
+  CU(cudaStreamSynchronize(B->st));
+  CU(cudaGetLastError());
+  if (energy)
     for (int s : systems)
       if (ovf[s])
         return fail(B, MDSC_ERR_LIST_OVERFLOW,
                     "system " + std::to_string(s) + ": a particle has more than " + std::to_string(kMaxC) +
                         " energy bonds (or " + std::to_string(kMaxE) + " candidates) to higher indices");
-  }
-  for (int it = 0; it < 64; ++it) {
-    CU(cudaMemsetAsync(b.flag, 0, sizeof(int), B->st));
-    launch_cluster_hook(b, B->st);
-    launch_cluster_compress(b, B->st);
-    int flag = 0;
-    CU(cudaMemcpyAsync(&flag, b.flag, sizeof(int), cudaMemcpyDeviceToHost, B->st));
-    CU(cudaStreamSynchronize(B->st));
-    if (!flag) break;
-  }
-  CU(cudaGetLastError());
-  for (int s : systems) {
+  for (size_t k = 0; k < systems.size(); ++k) {
+    const int s = systems[k];
     const SysDev& P = B->lo.sys[s];
-    std::vector<int> comp(P.n);
-    if (P.n)
-      CU(cudaMemcpy(comp.data(), b.comp + P.part_off, sizeof(int) * P.n, cudaMemcpyDeviceToHost));
-    // members of each component, in index order
-    std::vector<int> head(P.n, -1), next(P.n, -1), tail(P.n, -1);
+    const std::vector<int>& comp = comps[k];
+    // members of each component, in index order; its root is its lowest index
+    std::vector<int> next(P.n, -1), tail(P.n);
     for (int i = 0; i < P.n; ++i) {
       const int r = comp[i] - P.part_off;
-      if (head[r] < 0) head[r] = i;
-      else next[tail[r]] = i;
+      if (r != i) next[tail[r]] = i;
       tail[r] = i;
     }
-    Fenwick fw(P.n);
+    RankSet left(P.n);
     std::vector<int>& lab = B->labels[s];
     lab.assign(P.n, -1);
     int remaining = P.n, nc = 0;
@@ -911,11 +909,10 @@ mdsc_status run_clusters(mdsc_batch* B, const std::vector<int>& systems) {
     while (remaining > 0) {
       const double u = g.uniform();
       const int ip = (int)std::floor(u * remaining);
-      const int seed = fw.kth(ip);
-      const int r = comp[seed] - P.part_off;
-      for (int m = head[r]; m >= 0; m = next[m]) {
+      const int seed = left.kth(ip);
+      for (int m = comp[seed] - P.part_off; m >= 0; m = next[m]) {
         lab[m] = nc;
-        fw.remove(m);
+        left.remove(m);
         --remaining;
       }
       ++nc;
@@ -1243,6 +1240,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   b.nblk = (int)lo.blk.size();
   b.nwblk = (int)lo.wblk.size();
   b.ncellblk = (int)lo.cellblk.size();
+  b.ncellcap = lo.ncellcap;
   b.nrpwork = (int)lo.rpwork.size();
   b.ngtile = (int)lo.gtile.size();
   b.smem_tn = lo.smem_tn;
@@ -1440,6 +1438,16 @@ static void set_cell_grid(SysDev& P, const double* len) {
   P.ncell = c[0] * c[1] * c[2];
 }
 
+// the system's list no longer stands: the next list build makes one
+static cudaError_t ask_for_list(mdsc_batch* B, int s) {
+  static const int zero = 0, one = 1;
+  char* st = (char*)(B->b.st + s);
+  cudaError_t e = cudaMemcpyAsync(st + offsetof(SysState, force_list), &one, sizeof(int), cudaMemcpyHostToDevice, B->st);
+  for (size_t f : {offsetof(SysState, list_ok), offsetof(SysState, rebuild)})
+    if (e == cudaSuccess) e = cudaMemcpyAsync(st + f, &zero, sizeof(int), cudaMemcpyHostToDevice, B->st);
+  return e;
+}
+
 static mdsc_status upload_one(mdsc_batch* B, int s, const mdsc_host_state* h, bool sync) {
   const SysDev& P = B->lo.sys[s];
   const int n = P.n;
@@ -1506,12 +1514,24 @@ static mdsc_status upload_one(mdsc_batch* B, int s, const mdsc_host_state* h, bo
       Pm.rl_r2 = (float)(rr * rr);
     }
     set_cell_grid(Pm, h->len);
+    // bounds of the energy criterion's screen (ebond_prep_kernel forms each rod's in FP32)
+    double mm = 0, em = 0;
+    for (int i = 0; i < n; ++i) {
+      double m = 0;
+      for (int w = 0; w < P.nd; ++w) {
+        const double* o = &dob[3 * ((size_t)i * P.nd + w)];
+        m += std::fabs(dmu[(size_t)i * P.nd + w]) * std::sqrt(o[0] * o[0] + o[1] * o[1] + o[2] * o[2]);
+        em = std::max(em, std::fabs(dpc[(size_t)i * P.nd + w]));
+      }
+      mm = std::max(mm, m);
+    }
+    Pm.cl_mmax = (float)(1.001 * mm);
+    Pm.cl_emax = (float)(1.001 * em);
     Pm.Uself = Uself;
     CU(up((void*)(b.sys + s), &Pm, sizeof(SysDev)));
     if (B->uploaded[s]) {
       // new shapes: the list must be rebuilt
-      const int one = 1;
-      CU(up((char*)(b.st + s) + offsetof(SysState, force_list), &one, sizeof(int)));
+      CU(ask_for_list(B, s));
     }
   }
   B->uploaded[s] = 1;
@@ -2021,9 +2041,7 @@ mdsc_status mdsc_lattice(mdsc_batch* B, int sys, int nspecies, const int* counts
   launch_overlap_count(b, sys, P.n, d_cnt, B->st);
   CU(cudaMemcpyAsync(&cnt, d_cnt, sizeof(int), cudaMemcpyDeviceToHost, B->st));
   CU(cudaFreeAsync(d_cnt, B->st));
-  const int one = 1;
-  CU(cudaMemcpyAsync((char*)(b.st + sys) + offsetof(SysState, force_list), &one, sizeof(int), cudaMemcpyHostToDevice,
-                     B->st));
+  CU(ask_for_list(B, sys));
   CU(cudaStreamSynchronize(B->st));
   B->have_forces[sys] = 0;
   if (n_overlaps) *n_overlaps = cnt;
@@ -2156,6 +2174,8 @@ mdsc_status mdsc_transfer(mdsc_batch* D, int dsys, mdsc_batch* S, int ssys) {
   Pd.skin = Ps.skin;
   Pd.r_list = Ps.r_list;
   Pd.Uself = Ps.Uself;
+  Pd.cl_mmax = Ps.cl_mmax;
+  Pd.cl_emax = Ps.cl_emax;
   Pd.cl_mode = Ps.cl_mode;
   Pd.rl_r2 = Ps.rl_r2;
   Pd.ncell = Ps.ncell;
@@ -2171,6 +2191,7 @@ mdsc_status mdsc_transfer(mdsc_batch* D, int dsys, mdsc_batch* S, int ssys) {
   SysState st;
   CU(cudaMemcpy(&st, a.st + ssys, sizeof st, cudaMemcpyDeviceToHost));
   st.force_list = 1;
+  st.list_ok = 0;
   st.rebuild = 0;
   st.iter = 0;
   CU(cudaMemcpyAsync(b.st + dsys, &st, sizeof st, cudaMemcpyHostToDevice, D->st));
@@ -2221,6 +2242,8 @@ mdsc_status mdsc_transfer_many(mdsc_batch* D, mdsc_batch* S, const int* dsys, co
     Pd.skin = Ps.skin;
     Pd.r_list = Ps.r_list;
     Pd.Uself = Ps.Uself;
+    Pd.cl_mmax = Ps.cl_mmax;
+    Pd.cl_emax = Ps.cl_emax;
     Pd.cl_mode = Ps.cl_mode;
     Pd.rl_r2 = Ps.rl_r2;
     Pd.ncell = Ps.ncell;

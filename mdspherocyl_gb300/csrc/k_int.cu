@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
   // what the lists and the WCA screen of the new configuration count up from:
   // the partners' slots, and the cells (at most one per 8 rods)
   if (a == 0 && ok) b.wincnt[i] = 0;
+  if (a == 1 && bk.y == P.part_off && lane == 0 && S.rebuild) S.list_ok = 1;
   if (P.ncell > 0 && a == 1) {
     const int c = (bk.y - P.part_off) / 8 + lane;
     if (lane < kRows / 8 && c < P.ncell) b.ccnt[P.cell_off + c] = 0;
@@ -626,7 +627,9 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
       if (c == 0) {
         S.step += 1;
         S.iter += 1;
-        if (S.rebuild) S.list_builds += 1;
+        // a list asked for counts with the step that would have built it, also
+        // where a force evaluation of the same state had built it already
+        if (S.rebuild || S.force_list) S.list_builds += 1;
         S.force_list = 0;
       }
       __syncwarp();
@@ -803,6 +806,7 @@ __global__ void transfer_kernel(Batch dst, Batch src, TransferPairs tp) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     SysState st = src.st[q];
     st.force_list = 1;
+    st.list_ok = 0;
     st.rebuild = 0;
     st.iter = 0;
     dst.st[d] = st;

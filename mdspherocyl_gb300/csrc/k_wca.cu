@@ -37,7 +37,7 @@ namespace mdsc {
 // measure of the new configuration (particle_kernel), the same in every block.
 __device__ __forceinline__ bool list_due(const Batch& b, const SysDev& P, const SysState& S, int s, int force_all) {
   if (at_limit(b, s)) return false;
-  return force_all || S.force_list || 2.0 * soft_f2d(__int_as_float(S.dmax)) > P.skin;
+  return force_all || (S.force_list && !S.list_ok) || 2.0 * soft_f2d(__int_as_float(S.dmax)) > P.skin;
 }
 
 // cell of a fixed-point position: floor(fraction x cells), exact
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(128) wca_screen_kernel(Batch b) {
       const float sg = 0.5f * (di + b.pdia[q]);
       const float d2 = seg_dist_fast(dx, dy, dz, ai.x, ai.y, ai.z, ai.w, aj.x, aj.y, aj.z, aj.w);
       // 2^(1/3) sigma^2, with a margin for the FP32 screen
-      cand = d2 < 1.2599211f * sg * sg * 1.002f;
+      cand = !(d2 >= 1.2599211f * sg * sg * 1.002f);  // NaN (no length) is left to the FP64 evaluation
     }
     const uint32_t mask = (__ballot_sync(0xffffffffu, cand) >> (grp * LANES)) & ((1u << LANES) - 1u);
     if (cand) {
@@ -519,37 +519,58 @@ __global__ void __launch_bounds__(128) wca_eval_kernel(Batch b) {
 }
 
 // ---- clusters (v25/functions.cpp:2987-3016,3282-3324) ----------------
-// bond flags for list entries q > i: segment distance < (D_i + D_j)/2 + min_s,
-// evaluated in FP64 with the reference's routine (lower index first)
-__global__ void __launch_bounds__(kPartBlock) cluster_bonds_kernel(Batch b) {
-  const int2 bk = b.blk[blockIdx.x];
+// Bond flags for list entries q > i: segment distance < (D_i + D_j)/2 + min_s
+// in FP64 with the reference's routine (lower index first).  An FP32 distance
+// decides first: it is a distance between two points of the segments, so
+// below the threshold (by more than its rounding) the rods are bonded, and
+// where the axes are not nearly parallel it is the smallest one to ~1e-6, so
+// above the threshold they are not.  What is left -- within half a percent of
+// the threshold, or axes within 0.01 of parallel, where the closest points are
+// ill-determined -- takes the FP64 routine (~20,000 cycles of a warp).  Eight
+// lanes per rod: 32,768 rods 237 us a launch with one lane and FP64 for every
+// entry, 18 this way.
+__device__ __forceinline__ bool bonded_ref(const Batch& b, const SysDev& P, int i, int q) {
+  RodD ri, rq;
+  load_rod(b, i, ri);
+  load_rod(b, q, rq);
+  const double sigma = (b.dia[i] + b.dia[q]) / 2 + P.min_s;
+  double rij[3], dij[3], st[2];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    rij[a] = ri.r[a] - rq.r[a];
+    rij[a] -= P.L[a] * floor(rij[a] / P.L[a] + 0.5);
+  }
+  return seg_dist_ref<true>(ri, rq, P.L, rij, dij, st) < sigma * sigma;
+}
+
+constexpr int kBondLanes = 8;
+__global__ void __launch_bounds__(128) cluster_bonds_kernel(Batch b) {
+  constexpr int kPer = 32 * kBondLanes / 128;  // blocks per row of 32 rods
+  const int2 bk = b.wblk[blockIdx.x / kPer];
   const SysDev& P = b.sys[bk.x];
-  const int i = bk.y + threadIdx.x;
+  const int i = bk.y + (blockIdx.x % kPer * 128 + threadIdx.x) / kBondLanes, sub = threadIdx.x % kBondLanes;
   if (i >= P.part_off + P.n) return;
-  b.comp[i] = i;
-  if (P.cl_mode) return;  // energy criterion: ebond_kernel
+  if (sub == 0) b.comp[i] = i;
+  if (sub == 0 && i == P.part_off) b.st[bk.x].dmax = 0;  // the list of this configuration stands
+  if (P.cl_mode) return;  // energy criterion: ebond_eval_kernel
   const int nc = b.nbc[i];
   const int* lst = b.nb + (long long)i * kMaxNb;
   unsigned char* fl = b.eflag + (long long)i * kMaxNb;
-  RodD ri;
-  load_rod(b, i, ri);
-  for (int k = 0; k < nc; ++k) {
+  const int N = b.ntot;
+  const uint32_t ux = b.pfx[i], uy = b.pfx[N + i], uz = b.pfx[2 * N + i];
+  const float4 ai = b.pax[i];
+  const float di = b.pdia[i], ms = (float)P.min_s;
+  for (int k = b.nblo[i] + sub; k < nc; k += kBondLanes) {
     const int q = lst[k];
-    unsigned char bond = 0;
-    if (q > i) {
-      RodD rq;
-      load_rod(b, q, rq);
-      const double sigma = (b.dia[i] + b.dia[q]) / 2 + P.min_s;
-      double rij[3], dij[3], st[2];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        rij[a] = ri.r[a] - rq.r[a];
-        rij[a] -= P.L[a] * floor(rij[a] / P.L[a] + 0.5);
-      }
-      const double dsq = seg_dist_ref<true>(ri, rq, P.L, rij, dij, st);
-      bond = dsq < sigma * sigma ? 1 : 0;
-    }
-    fl[k] = bond;
+    const float4 aj = b.pax[q];
+    const float d2 = seg_dist_fast(fix_diff(ux, b.pfx[q], P.Lfix[0]), fix_diff(uy, b.pfx[N + q], P.Lfix[1]),
+                                   fix_diff(uz, b.pfx[2 * N + q], P.Lfix[2]), ai.x, ai.y, ai.z, ai.w, aj.x, aj.y, aj.z,
+                                   aj.w);
+    const float sg = 0.5f * (di + b.pdia[q]) + ms, thr = sg * sg;
+    const float dot = ai.x * aj.x + ai.y * aj.y + ai.z * aj.z;
+    bool bond = d2 < 0.995f * thr;
+    if (!bond && !(d2 > 1.005f * thr && dot * dot < 0.9999f)) bond = bonded_ref(b, P, i, q);
+    fl[k] = bond ? 1 : 0;
   }
 }
 
@@ -622,40 +643,135 @@ __device__ double pair_energy_ref(const Batch& b, const SysDev& P, int A, int B)
 // system: an FP32 screen on the centres (fixed-point minimum image) keeps
 // the pairs that can bond, |U_dd| <= 2 M_i M_j / (r - e_i - e_j)^3 with M
 // the sum of a rod's moments and e its largest dipole offset, U_WCA >= 0.
-// Ascending order; ebond_eval_kernel evaluates them exactly.
+// ebond_eval_kernel evaluates them exactly; their order reaches no result.
+//
+// That bound is a distance, so a system with a cell grid (systems of
+// kCellMinRods rods or more) bins its rods and screens the 27 cells around
+// each, where the bound of its largest M and e fits a cell; the others, and
+// systems with an overfull cell, screen all pairs.  32,768 rods, screen and
+// evaluation: 3470 us over all pairs with the bounds formed anew for every
+// pair of blocks and one lane per rod evaluating, 128 this way; 3000 rods
+// (all pairs) 356 and 83.
+__device__ __forceinline__ bool ebond_near(float2 mi, float2 mj, float dx, float dy, float dz, float thr,
+                                           float reach2) {
+  const float r2 = dx * dx + dy * dy + dz * dz;
+  if (r2 > reach2) return false;
+  const float gap = sqrtf(r2) * 0.9999f - mi.y - mj.y;
+  return mj.x != 0.f && (gap <= 0.f || 2.f * mi.x * mj.x >= thr * gap * gap * gap);
+}
+// no pair of the system passes that test beyond this distance
+__device__ __forceinline__ float ebond_reach(const SysDev& P) {
+  return (cbrtf(2.f * P.cl_mmax * P.cl_mmax / ((float)P.cl_ubond * 0.999f)) + 2.f * P.cl_emax) * 1.001f;
+}
+__device__ __forceinline__ bool ebond_on_cells(const Batch& b, const SysDev& P) {
+  return b.cells && P.ncell > 0 &&
+         ebond_reach(P) <= fminf(P.Lf[0] / P.cnx, fminf(P.Lf[1] / P.cny, P.Lf[2] / P.cnz));
+}
+
+// (M, e) of every rod, to scratch (the WCA terms' slots, read by the force
+// assembly only), the bond counts cleared, and the rods into their cells
+__global__ void __launch_bounds__(kPartBlock) ebond_prep_kernel(Batch b) {
+  const int2 bk = b.blk[blockIdx.x];
+  const SysDev& P = b.sys[bk.x];
+  const int i = bk.y + threadIdx.x;
+  if (P.cl_mode != 1 || i >= P.part_off + P.n) return;
+  float m = 0.f, e = 0.f;
+  for (int w = 0; w < P.nd; ++w) {
+    const int g = P.dip_off + (i - P.part_off) * P.nd + w;
+    const float ob = (float)sqrt(b.dob[3 * g] * b.dob[3 * g] + b.dob[3 * g + 1] * b.dob[3 * g + 1] +
+                                 b.dob[3 * g + 2] * b.dob[3 * g + 2]);
+    m += fabsf((float)b.dmu[g]) * ob;
+    e = fmaxf(e, fabsf((float)b.dpc[g]));
+  }
+  const float2 me = make_float2(m * 1.0001f, e * 1.0001f);
+  reinterpret_cast<float2*>(b.wev)[i] = me;
+  b.ecnt[i] = 0;
+  b.ebcnt[i] = 0;
+  if (!ebond_on_cells(b, P)) return;
+  const int N = b.ntot;
+  const uint32_t ux = b.pfx[i], uy = b.pfx[N + i], uz = b.pfx[2 * N + i];
+  const int c = P.cell_off + cell_of(P, ux, uy, uz);
+  const int slot = atomicAdd(&b.ccnt[c], 1);
+  if (slot < kCellSlots) {
+    b.cpos[(long long)c * kCellSlots + slot] = make_uint4(ux, uy, uz, (uint32_t)i);
+    b.cax[(long long)c * kCellSlots + slot] = make_float4(me.x, me.y, 0.f, 0.f);
+  } else {
+    atomicExch(&b.st[bk.x].cell_ovf, 1);
+  }
+}
+
+__device__ void ebond_cells(const Batch& b) {
+  const int2 cb = b.cellblk[blockIdx.x - b.nwblk];
+  const SysDev& P = b.sys[cb.x];
+  if (P.cl_mode != 1 || b.st[cb.x].cell_ovf || !ebond_on_cells(b, P)) return;
+  const int c = cb.y + (threadIdx.x >> 6);
+  if (c >= P.ncell) return;
+  const int t = threadIdx.x & 63;
+  const bool ok = t < b.ccnt[P.cell_off + c];
+  uint4 me = make_uint4(0u, 0u, 0u, 0u);
+  float4 mi = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (ok) {
+    me = b.cpos[(long long)(P.cell_off + c) * kCellSlots + t];
+    mi = b.cax[(long long)(P.cell_off + c) * kCellSlots + t];
+  }
+  const float thr = (float)P.cl_ubond * 0.999f, reach = ebond_reach(P), reach2 = reach * reach;
+  const float Lx = P.Lfix[0], Ly = P.Lfix[1], Lz = P.Lfix[2];
+  int* out = b.ecand + (long long)me.w * kMaxE;
+  int cnt = 0;
+  const int cx = c % P.cnx, cy = (c / P.cnx) % P.cny, cz = c / (P.cnx * P.cny);
+  for (int n = 0; n < 27; ++n) {
+    const int qx = (cx + n % 3 - 1 + P.cnx) % P.cnx, qy = (cy + n / 3 % 3 - 1 + P.cny) % P.cny,
+              qz = (cz + n / 9 - 1 + P.cnz) % P.cnz;
+    const long long q = P.cell_off + (qz * P.cny + qy) * P.cnx + qx;
+    const int m = b.ccnt[q];
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) {
+      const uint4 pj = b.cpos[q * kCellSlots + k];
+      const float4 mj = b.cax[q * kCellSlots + k];
+      if (ok && pj.w > me.w && mi.x != 0.f &&
+          ebond_near(make_float2(mi.x, mi.y), make_float2(mj.x, mj.y), fix_diff(me.x, pj.x, Lx),
+                     fix_diff(me.y, pj.y, Ly), fix_diff(me.z, pj.z, Lz), thr, reach2)) {
+        if (cnt < kMaxE) out[cnt] = (int)pj.w;
+        ++cnt;
+      }
+    }
+  }
+  if (!ok) return;
+  b.ecnt[me.w] = min(cnt, kMaxE);
+  if (cnt > kMaxE) atomicOr(&b.eovf[cb.x], 1);
+}
+
+// blocks below nwblk: 32 rods against all higher indices of their system, the
+// four warps a quarter each of every 128; the rest: cells
 __global__ void __launch_bounds__(kPartBlock) ebond_screen_kernel(Batch b) {
   __shared__ uint32_t sx[kPartBlock], sy[kPartBlock], sz[kPartBlock];
   __shared__ float2 sme[kPartBlock];
-  const int2 bk = b.blk[blockIdx.x];
+  __shared__ int cnt[32];
+  if ((int)blockIdx.x >= b.nwblk) {
+    ebond_cells(b);
+    return;
+  }
+  const int2 bk = b.wblk[blockIdx.x];
   const int s = bk.x;
   const SysDev& P = b.sys[s];
-  if (P.cl_mode != 1) return;  // the same for the whole block
+  if (P.cl_mode != 1 || (ebond_on_cells(b, P) && !b.st[s].cell_ovf)) return;  // the same for the whole block
   const int first = P.part_off, n = P.n, N = b.ntot;
-  const int i = bk.y + threadIdx.x;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = bk.y + lane;
   const bool ok = i < first + n;
-  auto bound = [&](int q) {
-    float m = 0.f, e = 0.f;
-    for (int w = 0; w < P.nd; ++w) {
-      const int g = P.dip_off + (q - first) * P.nd + w;
-      const float ob = (float)sqrt(b.dob[3 * g] * b.dob[3 * g] + b.dob[3 * g + 1] * b.dob[3 * g + 1] +
-                                   b.dob[3 * g + 2] * b.dob[3 * g + 2]);
-      m += fabsf((float)b.dmu[g]) * ob;
-      e = fmaxf(e, fabsf((float)b.dpc[g]));
-    }
-    return make_float2(m * 1.0001f, e * 1.0001f);
-  };
+  const float2* scr = reinterpret_cast<const float2*>(b.wev);
   uint32_t ux = 0, uy = 0, uz = 0;
   float2 mi = make_float2(0.f, 0.f);
   if (ok) {
     ux = b.pfx[i];
     uy = b.pfx[N + i];
     uz = b.pfx[2 * N + i];
-    mi = bound(i);
+    mi = scr[i];
   }
+  if (w == 0) cnt[lane] = 0;
   const float Lx = P.Lfix[0], Ly = P.Lfix[1], Lz = P.Lfix[2];
-  const float thr = (float)P.cl_ubond * 0.999f;
+  const float thr = (float)P.cl_ubond * 0.999f, reach = ebond_reach(P), reach2 = reach * reach;
   int* out = b.ecand + (long long)i * kMaxE;
-  int cnt = 0;
   for (int q0 = (bk.y - first) / kPartBlock * kPartBlock; q0 < n; q0 += kPartBlock) {
     __syncthreads();
     if (q0 + (int)threadIdx.x < n) {
@@ -663,82 +779,98 @@ __global__ void __launch_bounds__(kPartBlock) ebond_screen_kernel(Batch b) {
       sx[threadIdx.x] = b.pfx[q];
       sy[threadIdx.x] = b.pfx[N + q];
       sz[threadIdx.x] = b.pfx[2 * N + q];
-      sme[threadIdx.x] = bound(q);
+      sme[threadIdx.x] = scr[q];
     }
     __syncthreads();
     if (!ok || mi.x == 0.f) continue;
-    const int nq = min(kPartBlock, n - q0);
-    for (int t = 0; t < nq; ++t) {
+    const int k1 = min(32 * w + 32, n - q0);
+#pragma unroll 4
+    for (int t = 32 * w; t < k1; ++t) {
       const int j = first + q0 + t;
-      const float2 mj = sme[t];
-      const float dx = fix_diff(ux, sx[t], Lx), dy = fix_diff(uy, sy[t], Ly), dz = fix_diff(uz, sz[t], Lz);
-      const float gap = sqrtf(dx * dx + dy * dy + dz * dz) * 0.9999f - mi.y - mj.y;
-      const bool cand = j > i && mj.x != 0.f && (gap <= 0.f || 2.f * mi.x * mj.x >= thr * gap * gap * gap);
-      if (cand) {
-        if (cnt < kMaxE) out[cnt] = j;
-        ++cnt;
+      if (j > i && ebond_near(mi, sme[t], fix_diff(ux, sx[t], Lx), fix_diff(uy, sy[t], Ly), fix_diff(uz, sz[t], Lz),
+                              thr, reach2)) {
+        const int k = atomicAdd(&cnt[lane], 1);
+        if (k < kMaxE) out[k] = j;
       }
     }
   }
-  if (ok) {
-    b.ecnt[i] = min(cnt, kMaxE);
-    if (cnt > kMaxE) atomicOr(&b.eovf[s], 1);
+  __syncthreads();
+  if (ok && w == 0) {
+    b.ecnt[i] = min(cnt[lane], kMaxE);
+    if (cnt[lane] > kMaxE) atomicOr(&b.eovf[s], 1);
   }
 }
 
-// the screened candidates of each rod, exactly: a bond where the FP64 pair
-// energy (pair_energy_ref, lower index first) is below -cl_ubond
+// The screened candidates, exactly: a bond where the FP64 pair energy
+// (pair_energy_ref, lower index first) is below -cl_ubond.  A block packs the
+// candidates of its rods one per thread (few rods have any, and a pair is
+// ~400 FP64 instructions of a warp however many of its lanes take part).
 __global__ void __launch_bounds__(kPartBlock) ebond_eval_kernel(Batch b) {
+  __shared__ int pre[kPartBlock + 1];
+  __shared__ int wsum[kPartBlock / 32];
   const int2 bk = b.blk[blockIdx.x];
   const int s = bk.x;
   const SysDev& P = b.sys[s];
   if (P.cl_mode != 1) return;
-  const int i = bk.y + threadIdx.x;
-  if (i >= P.part_off + P.n) return;
-  const int nc = b.ecnt[i];
-  const int* cand = b.ecand + (long long)i * kMaxE;
-  int* out = b.ebond + (long long)i * kMaxC;
-  int cnt = 0;
-  for (int k = 0; k < nc; ++k) {
-    const int j = cand[k];
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const int nc = bk.y + t < P.part_off + P.n ? b.ecnt[bk.y + t] : 0;
+  int inc = nc;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= d) inc += v;
+  }
+  if (lane == 31) wsum[w] = inc;
+  __syncthreads();
+  for (int v = 0; v < w; ++v) inc += wsum[v];
+  pre[t + 1] = inc;
+  if (t == 0) pre[0] = 0;
+  __syncthreads();
+  const int tot = pre[kPartBlock];
+  for (int e = t; e < tot; e += kPartBlock) {
+    int lo = 0;  // the rod of item e: the last with pre <= e
+#pragma unroll
+    for (int d = kPartBlock / 2; d; d >>= 1)
+      if (pre[lo + d] <= e) lo += d;
+    const int i = bk.y + lo, j = b.ecand[(long long)i * kMaxE + (e - pre[lo])];
     if (pair_energy_ref(b, P, i, j) < -P.cl_ubond) {
-      if (cnt < kMaxC) out[cnt] = j;
-      ++cnt;
+      const int k = atomicAdd(&b.ebcnt[i], 1);
+      if (k < kMaxC) b.ebond[(long long)i * kMaxC + k] = j;
+      else atomicOr(&b.eovf[s], 1);
     }
   }
-  b.ebcnt[i] = min(cnt, kMaxC);
-  if (cnt > kMaxC) atomicOr(&b.eovf[s], 1);
 }
 
 __device__ __forceinline__ int find_root(const int* comp, int x) {
-  int p = comp[x];
+  int p = __ldcg(comp + x);
   while (p != x) {
     x = p;
-    p = comp[x];
+    p = __ldcg(comp + x);
   }
   return x;
 }
 
-// hook: for every bond, attach the larger root to the smaller one
+// Hook: for every bond, attach the larger root to the smaller one.  A bond
+// retries until its ends share a root: where another bond took the larger
+// root first, atomicMin leaves it at the smaller of the two new parents and
+// the loop goes on to join the other, so one pass over the bonds joins them
+// all and a component's root is its smallest index.
 __global__ void __launch_bounds__(kPartBlock) cluster_hook_kernel(Batch b) {
   const int2 bk = b.blk[blockIdx.x];
   const SysDev& P = b.sys[bk.x];
   const int i = bk.y + threadIdx.x;
   if (i >= P.part_off + P.n) return;
   const bool en = P.cl_mode == 1;
-  const int nc = en ? b.ebcnt[i] : b.nbc[i];
+  const int nc = en ? min(b.ebcnt[i], kMaxC) : b.nbc[i];
   const int* lst = en ? b.ebond + (long long)i * kMaxC : b.nb + (long long)i * kMaxNb;
   const unsigned char* fl = en ? nullptr : b.eflag + (long long)i * kMaxNb;
-  for (int k = 0; k < nc; ++k) {
+  for (int k = en ? 0 : b.nblo[i]; k < nc; ++k) {
     if (fl && !fl[k]) continue;
     int ra = find_root(b.comp, i), rb = find_root(b.comp, lst[k]);
     while (ra != rb) {
       const int hi = max(ra, rb), lo = min(ra, rb);
       const int old = atomicMin(&b.comp[hi], lo);
-      if (old == hi) {
-        *b.flag = 1;
-        break;
-      }
+      if (old == hi) break;
       ra = find_root(b.comp, old);
       rb = find_root(b.comp, lo);
     }
@@ -785,11 +917,14 @@ void launch_wca(const Batch& b, bool clear, cudaStream_t s) {
   wca_eval_kernel<<<b.tune.wca_blocks, 128, 0, s>>>(b);
 }
 void launch_cluster_bonds(const Batch& b, cudaStream_t s) {
-  if (b.nblk) cluster_bonds_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
+  if (b.nwblk) cluster_bonds_kernel<<<b.nwblk * (32 * kBondLanes / 128), 128, 0, s>>>(b);
 }
 void launch_ebond(const Batch& b, cudaStream_t s) {
   if (!b.nblk || !b.ecand) return;
-  ebond_screen_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
+  const int ncb = b.cells ? b.ncellblk : 0;
+  if (ncb) cudaMemsetAsync(b.ccnt, 0, sizeof(int) * b.ncellcap, s);
+  ebond_prep_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
+  ebond_screen_kernel<<<b.nwblk + ncb, kPartBlock, 0, s>>>(b);
   ebond_eval_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
 }
 void launch_cluster_hook(const Batch& b, cudaStream_t s) {

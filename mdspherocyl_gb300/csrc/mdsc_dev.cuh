@@ -108,6 +108,7 @@ struct SysDev {
   int cell_off, cell_cap;
   float rl_r2;     // rc_real > 0: squared centre-distance radius of the real-space neighbour list
   double rc_real;  // real-space cutoff (0: all minimum-image pairs, the tiles)
+  float cl_mmax, cl_emax;  // largest sum of a rod's moments and dipole offset (bounds of mode 1's screen)
   double cl_ubond; // mode 1: a bond is U_pair < -cl_ubond (the threshold times T)
   double L[3];
   double invL[3];
@@ -171,8 +172,9 @@ struct SysState {
   int list_builds;
   int iter;          // step index within the current mdsc_step call (noise row)
   int force_list;    // rebuild the Verlet list at the next check regardless of the skin
+  int list_ok;       // a list was built since force_list was last set
   int cell_ovf;      // this build: a cell held more than kCellSlots rods (all-pairs scan instead)
-  int dmax;          // largest displacement measure of the configuration (FP32 bits; cleared by finalize_kernel)
+  int dmax;          // largest displacement measure of the configuration (FP32 bits; cleared by what reads the lists: finalize_kernel, cluster_bonds_kernel)
   long long stop;    // the step count at which the system stops taking steps (mdsc_set_step_limit)
   double K_first[2]; // kinetic energies after the first half kick
   double xi_mid[2];  // xi used by the second half kick
@@ -295,7 +297,7 @@ struct Batch {
   uint4* cpos;   // ncellcap * kCellSlots
   float4* cax;   // ncellcap * kCellSlots
   int2* cellblk; // per pair of cells of capacity: (system, first cell)
-  int ncellblk;
+  int ncellblk, ncellcap;
   int cells;     // 1: systems with a cell grid build their lists on it; 0: every system scans all pairs
   int honor_stop; // the step graph: kernels skip the systems at their step limit
   const int* skip; // per system, or null: kernels skip the flagged systems (a force evaluation
@@ -309,7 +311,6 @@ struct Batch {
   // clusters
   int* comp;     // n component representative
   unsigned char* eflag;  // n * kMaxNb: list entry is a cluster bond
-  int* flag;     // 1 changed flag
   int* ebond;    // n * kMaxC: energy-criterion bonds to higher indices
   int* ebcnt;    // n: their number
   int* eovf;     // nsys: a particle had more than kMaxC energy bonds (or kMaxE candidates)

@@ -135,7 +135,9 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
 mdsc_status mdsc_destroy(mdsc_batch* b);
 int mdsc_num_systems(const mdsc_batch* b);
 /* bytes of GPU memory the batch holds (with the energy criterion's
-   candidate lists once a system of it takes that criterion) */
+   candidate lists once a system of it takes that criterion, and what the
+   calls for correlations, order parameters and pictures keep: the largest
+   they asked for up to 64 MB) */
 size_t mdsc_device_bytes(const mdsc_batch* b);
 /* GPU memory a batch of these systems would need, without creating it.
    mdsc_set_cluster_energy later adds 260 bytes per particle of the batch. */

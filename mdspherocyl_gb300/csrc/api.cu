@@ -47,15 +47,15 @@ void launch_reset_iter(const Batch& b, cudaStream_t s);
 cudaError_t launch_transfer(const Batch& dst, const Batch& src, const std::vector<int2>& pairs, cudaStream_t s);
 void launch_kspace_parts(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, int part,
                          cudaStream_t s);
-void launch_correlations(const Batch& b, const CorrSys* cs, const unsigned char* species, double bar_w,
-                         int max_bins, unsigned long long* hist, cudaStream_t s);
+cudaError_t launch_correlations(const Batch& b, const CorrSys* c, const unsigned char* species, double bar_w,
+                                int ntiles, int max_bins, unsigned long long* hist, cudaStream_t s);
 void launch_order_sums(const Batch& b, double* out, cudaStream_t s);
 size_t render_scratch_bytes(int n, int nd, int images);
 void launch_lattice_sites(const Batch& b, int sys, double len, double dia, int num1, int num2, int nsites,
                           int prev_first, int prev_n, double* site_r, int* ok, cudaStream_t s);
 void launch_overlap_count(const Batch& b, int sys, int n, int* count, cudaStream_t s);
 void launch_thermalize(const Batch& b, int sys, int n, double temp, unsigned long long seed, cudaStream_t s);
-void launch_render(const Batch& b, int sys, int n, const unsigned char* species, const int* keep, int images,
+void launch_render(const Batch& b, int sys, int n, int nd, const unsigned char* species, const int* keep, int images,
                    int dipoles, int draw_box, float seg_rad, float box_rad, const float* eye, const float* fwd,
                    const float* right, const float* up, const float* light, float tan_half, int width,
                    int height, void* scratch, unsigned char* rgb, cudaStream_t s);
@@ -590,6 +590,8 @@ struct mdsc_batch {
   SysObs* h_trace = nullptr;  // pinned, kNoiseChunk x nsys: per-step observables of mdsc_step_trace
   char* arena = nullptr;
   size_t arena_bytes = 0;
+  char* scratch = nullptr;    // device memory of the observables' and pictures' calls, kept between them
+  size_t scratch_bytes = 0;
   std::vector<Mt19937> thermo_rng;  // 2 per system
   std::vector<Mt19937> clus_rng;    // 1 per system
   std::vector<long long> step_h;
@@ -857,6 +859,28 @@ void draw_noise(mdsc_batch* B, int steps, double* h) {
       }
     }
 }
+
+// Device memory for one call on the batch's stream (calls on a batch are not
+// concurrent): the batch keeps up to kScratchKeep bytes from call to call --
+// the stream-ordered allocator returned its memory at every synchronization
+// and took it from the system again on the next call -- and more than that is
+// allocated and freed by the call.  mdsc_destroy frees what is kept.
+constexpr size_t kScratchKeep = size_t(64) << 20;
+cudaError_t take_scratch(mdsc_batch* B, size_t bytes, char** out) {
+  if (bytes > kScratchKeep) return cudaMallocAsync((void**)out, bytes, B->st);
+  if (bytes > B->scratch_bytes) {
+    // the last call that used it has synchronized
+    if (B->scratch) cudaFree(B->scratch);
+    B->scratch = nullptr;
+    B->scratch_bytes = 0;
+    const cudaError_t e = cudaMalloc((void**)&B->scratch, bytes);
+    if (e != cudaSuccess) return e;
+    B->scratch_bytes = bytes;
+  }
+  *out = B->scratch;
+  return cudaSuccess;
+}
+cudaError_t give_scratch(mdsc_batch* B, char* d) { return d == B->scratch ? cudaSuccess : cudaFreeAsync(d, B->st); }
 
 // connected components on the GPU, then the reference's labelling order on
 // the host: repeatedly draw u, take the floor(u * remaining)-th remaining
@@ -1366,6 +1390,7 @@ mdsc_status mdsc_destroy(mdsc_batch* B) {
   for (auto& g : B->graph_io)
     if (g) cudaGraphExecDestroy(g);
   if (B->arena) cudaFree(B->arena);
+  if (B->scratch) cudaFree(B->scratch);
   if (B->b.ecand) cudaFree(B->b.ecand);
   if (B->b.ecnt) cudaFree(B->b.ecnt);
   if (B->h_noise) cudaFreeHost(B->h_noise);
@@ -1399,7 +1424,7 @@ size_t mdsc_device_bytes(const mdsc_batch* B) {
   if (!B) return 0;
   // + the energy criterion's candidate lists, allocated on first use
   const size_t n = (size_t)std::max(B->lo.ntot, 1);
-  return B->arena_bytes + (B->b.ecand ? sizeof(int) * n * (kMaxE + 1) : 0);
+  return B->arena_bytes + B->scratch_bytes + (B->b.ecand ? sizeof(int) * n * (kMaxE + 1) : 0);
 }
 int mdsc_launches_per_step(const mdsc_batch* B) { return B ? B->launches : 0; }
 void* mdsc_stream(const mdsc_batch* B) { return B ? (void*)B->st : nullptr; }
@@ -1913,12 +1938,14 @@ mdsc_status mdsc_correlations(mdsc_batch* B, double bar_w, double* hist) {
   if (!(bar_w > 0.0) || !hist) return fail(B, MDSC_ERR_BAD_ARG, "mdsc_correlations: bar_w > 0 and hist required");
   std::vector<CorrSys> cs(B->nsys);
   std::vector<unsigned char> sp(std::max(B->lo.ntot, 1), 0);
-  int tot = 0, max_bins = 0;
+  int tot = 0, max_bins = 0, ntiles = 0;
   for (int s = 0; s < B->nsys; ++s) {
     const int nb = std::max(0, corr_bins(B->lo.sys[s], bar_w));
     const int nc = (int)B->species[s].size();
     const int nblocks = nc + nc * (nc - 1) / 2;
-    cs[s] = CorrSys{nb, tot, nc, 0};
+    const int strips = cdiv(B->lo.sys[s].n, kPartBlock), tiles = nb ? strips * (strips + 1) / 2 : 0;
+    cs[s] = CorrSys{nb, tot, nc, ntiles, tiles};
+    ntiles += tiles;
     tot += nblocks * 4 * nb;
     max_bins = std::max(max_bins, nblocks * nb);
     int i = B->lo.sys[s].part_off;
@@ -1928,7 +1955,7 @@ mdsc_status mdsc_correlations(mdsc_batch* B, double bar_w, double* hist) {
   if (tot == 0) return MDSC_OK;
   char* d = nullptr;
   const size_t hbytes = sizeof(unsigned long long) * tot, cbytes = sizeof(CorrSys) * B->nsys;
-  CU(cudaMallocAsync((void**)&d, hbytes + cbytes + sp.size(), B->st));
+  CU(take_scratch(B, hbytes + cbytes + sp.size(), &d));
   unsigned long long* dh = reinterpret_cast<unsigned long long*>(d);
   CorrSys* dcs = reinterpret_cast<CorrSys*>(d + hbytes);
   unsigned char* dsp = reinterpret_cast<unsigned char*>(d + hbytes + cbytes);
@@ -1937,10 +1964,9 @@ mdsc_status mdsc_correlations(mdsc_batch* B, double bar_w, double* hist) {
   CU(cudaMemcpyAsync(dsp, sp.data(), sp.size(), cudaMemcpyHostToDevice, B->st));
   CU(cudaMemsetAsync(dh, 0, hbytes, B->st));
   launch_derive(B->b, B->st);
-  launch_correlations(B->b, dcs, dsp, bar_w, max_bins, dh, B->st);
-  CU(cudaGetLastError());
+  CU(launch_correlations(B->b, dcs, dsp, bar_w, ntiles, max_bins, dh, B->st));
   CU(cudaMemcpyAsync(h.data(), dh, hbytes, cudaMemcpyDeviceToHost, B->st));
-  CU(cudaFreeAsync(d, B->st));
+  CU(give_scratch(B, d));
   CU(cudaStreamSynchronize(B->st));
   // counts are exact integers; the other three are fixed point in 2^-24 units
   for (int s = 0; s < B->nsys; ++s) {
@@ -1959,13 +1985,13 @@ mdsc_status mdsc_order_params(mdsc_batch* B, double* G1, double* G2, double* M) 
   if (st) return st;
   const int nblk = B->b.nblk;
   std::vector<double> part(12 * (size_t)nblk);
-  double* d = nullptr;
-  CU(cudaMallocAsync((void**)&d, sizeof(double) * part.size(), B->st));
+  char* d = nullptr;
+  CU(take_scratch(B, sizeof(double) * part.size(), &d));
   launch_derive(B->b, B->st);
-  launch_order_sums(B->b, d, B->st);
+  launch_order_sums(B->b, reinterpret_cast<double*>(d), B->st);
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(part.data(), d, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, B->st));
-  CU(cudaFreeAsync(d, B->st));
+  CU(give_scratch(B, d));
   CU(cudaStreamSynchronize(B->st));
   for (int s = 0; s < B->nsys; ++s) {
     const SysDev& P = B->lo.sys[s];
@@ -2118,17 +2144,17 @@ mdsc_status mdsc_render(mdsc_batch* B, int sys, const mdsc_view* v, unsigned cha
   const size_t scratch = render_scratch_bytes(P.n, P.nd, v->images);
   char* d = nullptr;
   const size_t spb = (sp.size() + 255) / 256 * 256, kb = (keep.size() * sizeof(int) + 255) / 256 * 256;
-  CU(cudaMallocAsync((void**)&d, scratch + spb + kb + img, B->st));
+  CU(take_scratch(B, scratch + spb + kb + img, &d));
   unsigned char* dsp = reinterpret_cast<unsigned char*>(d + scratch);
   int* dkeep = keep.empty() ? nullptr : reinterpret_cast<int*>(d + scratch + spb);
   unsigned char* dimg = reinterpret_cast<unsigned char*>(d + scratch + spb + kb);
   CU(cudaMemcpyAsync(dsp, sp.data(), sp.size(), cudaMemcpyHostToDevice, B->st));
   if (dkeep) CU(cudaMemcpyAsync(dkeep, keep.data(), sizeof(int) * keep.size(), cudaMemcpyHostToDevice, B->st));
-  launch_render(B->b, sys, P.n, dsp, dkeep, v->images, v->dipoles, v->box, (float)pix, (float)(0.5 * pix), e, f, r,
+  launch_render(B->b, sys, P.n, P.nd, dsp, dkeep, v->images, v->dipoles, v->box, (float)pix, (float)(0.5 * pix), e, f, r,
                 u, l, (float)tan_half, v->width, v->height, d, dimg, B->st);
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(rgb, dimg, img, cudaMemcpyDeviceToHost, B->st));
-  CU(cudaFreeAsync(d, B->st));
+  CU(give_scratch(B, d));
   CU(cudaStreamSynchronize(B->st));
   return MDSC_OK;
 }

@@ -11,74 +11,120 @@
 // numbers them (calc_II / rev_II); a system's histograms are its nc species
 // blocks, then the nc (nc - 1) / 2 pair blocks in the order (0,1), (0,2), ...,
 // (1,2), ..., each 4 x nbins.
-// One block per particle block of 128: each thread holds one particle i and
-// meets every j > i of its system, 128 at a time from shared memory.  The
-// sums are integers -- the counts exactly, the three others in fixed point
-// with 2^24 units -- so they are the same whatever order the atomics land
-// in.  The bins live in shared memory when they fit (kCorrSmemBins per
-// block), else directly in global memory.
+//
+// Work: the pair triangle of a system in tiles of 128 x 128 particles (I <= J).
+// A fixed grid of blocks takes runs of tiles; a thread holds one particle of
+// the I strip and meets half of the J strip from shared memory.  The sums are
+// integers -- the counts exactly, the three others in fixed point with 2^24
+// units -- so they are the same whatever order the atomics land in.  A block
+// keeps its histogram in shared memory as 32-bit words, the fixed-point terms
+// split in two (v = hi 2^16 + lo): native shared atomics, where 64-bit ones
+// are loops, and no sum can leave its word within kCorrFlush tiles, after
+// which the block adds its words to the global 64-bit histogram.  Histograms
+// that do not fit (kCorrSmemBins) add to global memory directly.
+//
+// 4096 particles of two species at 0.1 (3 x 330 bins): one block per 128
+// particles with a 64-bit histogram took 1650 us (32 blocks, most atomics in
+// global memory), this 69.
 //
 #include "mdsc_dev.cuh"
 #include "reduce.cuh"
 
 namespace mdsc {
 
-constexpr int kCorrSmemBins = 1024;  // histogram bins (x 4 functions x 8 B = 32 KB) in shared memory
+constexpr int kCorrWords = 7;        // 32-bit words per bin: count, then (lo, hi) of the three sums
+constexpr int kCorrSmemBins = 7000;  // most bins of a histogram in shared memory (196 KB)
+constexpr int kCorrFlush = 4;        // tiles between flushes: 2^16 pairs of a block at most
+constexpr int kCorrThreads = 256;
 constexpr float kCorrScale = 16777216.f;  // 2^24: fixed-point unit of the non-count sums
 
+// a block's shared histogram into the system's global one, and cleared
+__device__ void corr_flush(uint32_t* sh, int nblocks, int nbins, unsigned long long* __restrict__ gh) {
+  __syncthreads();
+  const int bins = nblocks * nbins;
+  for (int k = threadIdx.x; k < bins; k += kCorrThreads) {
+    const uint32_t c = sh[k];
+    if (c == 0u) continue;
+    unsigned long long* g = gh + (size_t)(k / nbins) * 4 * nbins + k % nbins;
+    atomicAdd(g, (unsigned long long)c);
+    sh[k] = 0u;
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      const long long v = ((long long)(int32_t)sh[(2 * f + 2) * bins + k] << 16) + sh[(2 * f + 1) * bins + k];
+      atomicAdd(g + (f + 1) * nbins, (unsigned long long)v);
+      sh[(2 * f + 1) * bins + k] = sh[(2 * f + 2) * bins + k] = 0u;
+    }
+  }
+  __syncthreads();
+}
+
 template <bool SMEM>
-__global__ void __launch_bounds__(kPartBlock) corr_kernel(Batch b, const CorrSys* __restrict__ cs,
-                                                          const unsigned char* __restrict__ species, double bar_w,
-                                                          unsigned long long* __restrict__ hist) {
-  extern __shared__ unsigned long long shist[];
+__global__ void __launch_bounds__(kCorrThreads) corr_kernel(Batch b, const CorrSys* __restrict__ cs,
+                                                            const unsigned char* __restrict__ species, double bar_w,
+                                                            int ntiles, unsigned long long* __restrict__ hist) {
+  extern __shared__ uint32_t shist[];
   __shared__ uint32_t sx[kPartBlock], sy[kPartBlock], sz[kPartBlock];
   __shared__ float4 sa[kPartBlock];
   __shared__ unsigned char ssp[kPartBlock];
-  const int2 bk = b.blk[blockIdx.x];
-  const int s = bk.x;
-  const SysDev& P = b.sys[s];
-  const CorrSys C = cs[s];
-  const int nbins = C.nbins, nc = C.nsp;
-  const int nwords = (nc + nc * (nc - 1) / 2) * 4 * nbins;
-  unsigned long long* gh = hist + C.off;
-  unsigned long long* h = SMEM ? shist : gh;
+  const int per = cdiv(ntiles, gridDim.x);
+  const int t0 = blockIdx.x * per, t1 = min(ntiles, t0 + per);
+  if (t0 >= t1) return;
+  int s = 0;
+  while (t0 >= cs[s].tile_off + cs[s].ntiles) ++s;
+  CorrSys C = cs[s];
+  int nblocks = C.nsp + C.nsp * (C.nsp - 1) / 2, bins = nblocks * C.nbins;
   if (SMEM) {
-    for (int k = threadIdx.x; k < nwords; k += blockDim.x) shist[k] = 0ull;
-    __syncthreads();
+    for (int k = threadIdx.x; k < kCorrWords * bins; k += kCorrThreads) shist[k] = 0u;
   }
   const int N = b.ntot;
-  const int i = bk.y + threadIdx.x;
-  const int iend = P.part_off + P.n;
-  const bool ok = i < iend;
-  uint32_t ux = 0, uy = 0, uz = 0;
-  float4 ai = make_float4(0.f, 0.f, 1.f, 0.f);
-  int spi = 0;
-  if (ok) {
-    ux = b.pfx[i];
-    uy = b.pfx[N + i];
-    uz = b.pfx[2 * N + i];
-    ai = b.pax[i];
-    spi = species[i];
-  }
   const float ibw = (float)(1.0 / bar_w);
-  // how far the FP32 t = r / bar_w may be from the reference's: ~8 roundings
-  // relative (bounded by 1e-6 t) plus the fixed-point quantum of each
-  // coordinate difference (L / 2^32 per axis, doubled)
-  const float q0 = (float)(4.0 * fmax(P.L[0], fmax(P.L[1], P.L[2])) / 4294967296.0 / bar_w) + 1e-6f;
-  for (int j0 = bk.y; j0 < iend; j0 += kPartBlock) {
+  int since = 0;
+  for (int tile = t0; tile < t1; ++tile) {
+    if (tile >= C.tile_off + C.ntiles || since == kCorrFlush) {
+      if (SMEM) corr_flush(shist, nblocks, C.nbins, hist + C.off);
+      since = 0;
+      if (tile >= C.tile_off + C.ntiles) {
+        while (tile >= cs[s].tile_off + cs[s].ntiles) ++s;
+        C = cs[s];
+        nblocks = C.nsp + C.nsp * (C.nsp - 1) / 2;
+        bins = nblocks * C.nbins;
+        if (SMEM)
+          for (int k = threadIdx.x; k < kCorrWords * bins; k += kCorrThreads) shist[k] = 0u;
+      }
+    }
+    ++since;
+    const SysDev& P = b.sys[s];
+    const int nbins = C.nbins, nc = C.nsp;
+    // tile -> strips (I, J), I <= J, row by row of the upper triangle
+    const int ns = cdiv(P.n, kPartBlock);
+    int I = 0, q = tile - C.tile_off;
+    while (q >= ns - I) q -= ns - I++;
+    const int J = I + q;
+    const int iend = P.part_off + P.n;
+    const int i = P.part_off + I * kPartBlock + (threadIdx.x & (kPartBlock - 1));
+    const int j0 = P.part_off + J * kPartBlock;
     const int nj = min(kPartBlock, iend - j0);
+    const bool ok = i < iend;
+    // how far the FP32 t = r / bar_w may be from the reference's: ~8 roundings
+    // relative (bounded by 1e-6 t) plus the fixed-point quantum of each
+    // coordinate difference (L / 2^32 per axis, doubled)
+    const float q0 = (float)(4.0 * fmax(P.L[0], fmax(P.L[1], P.L[2])) / 4294967296.0 / bar_w) + 1e-6f;
     __syncthreads();
     if (threadIdx.x < nj) {
-      const int q = j0 + threadIdx.x;
-      sx[threadIdx.x] = b.pfx[q];
-      sy[threadIdx.x] = b.pfx[N + q];
-      sz[threadIdx.x] = b.pfx[2 * N + q];
-      sa[threadIdx.x] = b.pax[q];
-      ssp[threadIdx.x] = species[q];
+      const int p = j0 + threadIdx.x;
+      sx[threadIdx.x] = b.pfx[p];
+      sy[threadIdx.x] = b.pfx[N + p];
+      sz[threadIdx.x] = b.pfx[2 * N + p];
+      sa[threadIdx.x] = b.pax[p];
+      ssp[threadIdx.x] = species[p];
     }
     __syncthreads();
     if (!ok) continue;
-    for (int k = 0; k < nj; ++k) {
+    const uint32_t ux = b.pfx[i], uy = b.pfx[N + i], uz = b.pfx[2 * N + i];
+    const float4 ai = b.pax[i];
+    const int spi = species[i];
+    const int k1 = min(nj, (threadIdx.x >> 7) * 64 + 64);
+    for (int k = (threadIdx.x >> 7) * 64; k < k1; ++k) {
       const int j = j0 + k;
       if (j <= i) continue;
       const float dx = fix_diff(ux, sx[k], P.Lfix[0]);
@@ -117,18 +163,25 @@ __global__ void __launch_bounds__(kPartBlock) corr_kernel(Batch b, const CorrSys
       const int v110 = __float2int_rn(w * dot * kCorrScale);
       const int v112 = __float2int_rn(w * (3.f * doti * dotj - dot) * kCorrScale);
       const int v220 = __float2int_rn(0.5f * w * (3.f * dot * dot - 1.f) * kCorrScale);
-      unsigned long long* hb = h + (size_t)blkno * 4 * nbins;
-      atomicAdd(&hb[0 * nbins + bin], intra ? 2ull : 1ull);
-      atomicAdd(&hb[1 * nbins + bin], (unsigned long long)(long long)v110);
-      atomicAdd(&hb[2 * nbins + bin], (unsigned long long)(long long)v112);
-      atomicAdd(&hb[3 * nbins + bin], (unsigned long long)(long long)v220);
+      if (SMEM) {
+        uint32_t* h = shist + blkno * nbins + bin;
+        atomicAdd(h, intra ? 2u : 1u);
+        atomicAdd(h + 1 * bins, (uint32_t)v110 & 0xffffu);
+        atomicAdd(h + 2 * bins, (uint32_t)(v110 >> 16));
+        atomicAdd(h + 3 * bins, (uint32_t)v112 & 0xffffu);
+        atomicAdd(h + 4 * bins, (uint32_t)(v112 >> 16));
+        atomicAdd(h + 5 * bins, (uint32_t)v220 & 0xffffu);
+        atomicAdd(h + 6 * bins, (uint32_t)(v220 >> 16));
+      } else {
+        unsigned long long* hb = hist + C.off + (size_t)blkno * 4 * nbins;
+        atomicAdd(&hb[0 * nbins + bin], intra ? 2ull : 1ull);
+        atomicAdd(&hb[1 * nbins + bin], (unsigned long long)(long long)v110);
+        atomicAdd(&hb[2 * nbins + bin], (unsigned long long)(long long)v112);
+        atomicAdd(&hb[3 * nbins + bin], (unsigned long long)(long long)v220);
+      }
     }
   }
-  if (SMEM) {
-    __syncthreads();
-    for (int k = threadIdx.x; k < nwords; k += blockDim.x)
-      if (shist[k] != 0ull) atomicAdd(&gh[k], shist[k]);
-  }
+  if (SMEM) corr_flush(shist, nblocks, C.nbins, hist + C.off);
 }
 
 // Per particle block: sum of the rod axes (3), of their outer products (6,
@@ -171,15 +224,23 @@ __global__ void __launch_bounds__(kPartBlock) order_sums_kernel(Batch b, double*
   }
 }
 
-// max_bins: the largest (species blocks + pair blocks) x nbins of any system
-void launch_correlations(const Batch& b, const CorrSys* c, const unsigned char* species, double bar_w,
-                         int max_bins, unsigned long long* hist, cudaStream_t s) {
-  if (!b.nblk) return;
-  if (max_bins <= kCorrSmemBins)
-    corr_kernel<true><<<b.nblk, kPartBlock, 4 * max_bins * sizeof(unsigned long long), s>>>(b, c, species, bar_w,
-                                                                                             hist);
-  else
-    corr_kernel<false><<<b.nblk, kPartBlock, 0, s>>>(b, c, species, bar_w, hist);
+// ntiles: 128 x 128 tiles over all systems (CorrSys); max_bins: the largest
+// (species blocks + pair blocks) x nbins of any system
+cudaError_t launch_correlations(const Batch& b, const CorrSys* c, const unsigned char* species, double bar_w,
+                                int ntiles, int max_bins, unsigned long long* hist, cudaStream_t s) {
+  if (ntiles <= 0) return cudaSuccess;
+  // two blocks per SM: a run of tiles pays for a block's clearing and flush
+  const int grid = ntiles < 2 * 152 ? ntiles : 2 * 152;
+  if (max_bins <= kCorrSmemBins) {
+    const int bytes = kCorrWords * max_bins * (int)sizeof(uint32_t);
+    const cudaError_t e = cudaFuncSetAttribute(corr_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               kCorrWords * kCorrSmemBins * (int)sizeof(uint32_t));
+    if (e != cudaSuccess) return e;
+    corr_kernel<true><<<grid, kCorrThreads, bytes, s>>>(b, c, species, bar_w, ntiles, hist);
+  } else {
+    corr_kernel<false><<<grid, kCorrThreads, 0, s>>>(b, c, species, bar_w, ntiles, hist);
+  }
+  return cudaGetLastError();
 }
 
 void launch_order_sums(const Batch& b, double* out, cudaStream_t s) {

@@ -321,9 +321,9 @@ struct Batch {
 };
 
 // Per system, for the pair-correlation histograms: bins, first histogram
-// word, number of species.
+// word, number of species, its tiles of 128 x 128 particles.
 struct CorrSys {
-  int nbins, off, nsp, pad;
+  int nbins, off, nsp, tile_off, ntiles;
 };
 
 // ---- small helpers ----------------------------------------------------

@@ -1,7 +1,10 @@
-"""The splits of a step's work that a small batch runs on (one k tile per
-gather block, one k-vector per structure-factor thread) and those of a batch
-that fills the GPU give a system the same bits, at the edges of their blocks
-and tiles; and both agree with the oracle."""
+"""How work is split over the GPU, at the edges of the splits.
+
+The splits of a step that a small batch runs on (one k tile per gather block,
+one k-vector per structure-factor thread) and those of a batch that fills the
+GPU give a system the same bits, and both agree with the oracle; so do the
+clusters, histograms and pictures.
+"""
 import math
 
 import numpy as np
@@ -78,3 +81,70 @@ def test_forces_against_the_oracle(systems, k):
             assert rms_rel(d["T"], o.T) <= TOL_F, name
             assert rms_rel(PT[0], PTo) <= TOL_F, name
             assert abs(U[0] - Uo) <= TOL_F * max(abs(Uo), np.abs(PTo).max()), name
+
+
+# ---- clusters, histograms and pictures at the edges of their splits --------
+def _plain(n, seed, phi=0.1, mu=2.2):
+    rng = np.random.default_rng(seed)
+    st, box = S.make_system(n=n, phi=phi, lengths=rng.uniform(2.0, 4.0, n), mu=np.full(n, mu), seed=seed)
+    spec = S.SystemSpec(n=n, box=box, alpha=6.0 / float(box[0]), K_max=2, ksq_max=1)
+    return spec, st
+
+
+def _osys(spec, st):
+    return oracle.System(st.r, st.p, st.O, st.l, st.length, st.dia, st.mass, st.dip, spec.box)
+
+
+@pytest.mark.parametrize("n,u_bond", [(2, 1.0), (32, 0.0), (129, 0.8), (700, 0.0), (700, 0.8), (4095, 0.8),
+                                      (4500, 0.0), (4500, 0.8)])
+def test_cluster_labels_equal_the_oracle(n, u_bond):
+    """Geometric and energy bonds; systems below 4096 rods screen all pairs,
+    the others the cells around each rod; three calls, the second and third
+    on the list the first one built."""
+    spec, st = _plain(n, 60 + n, phi=0.2)
+    spec.min_s, spec.cl_energy = 0.25, u_bond
+    orc = oracle.Oracle()
+    skip = 0
+    with L.Batch([spec], [st]) as bt:
+        for _ in range(3):
+            lab, nc = bt.clust_conf(0)
+            o = _osys(spec, st)
+            want, nw, _ = (orc.clust_energy(o, u_bond * spec.temp, skip=skip) if u_bond
+                           else orc.clust_conf(o, spec.min_s, skip=skip))
+            assert nc == nw
+            assert np.array_equal(lab, want)
+            skip += nw  # one draw per cluster
+
+
+@pytest.mark.parametrize("n,counts,bar_w", [(1, [1], 0.2), (128, [128], 0.1), (129, [1, 128], 0.1),
+                                            (700, [128, 256, 316], 0.05), (1300, [650, 650], 0.002),
+                                            (1300, [1300], 0.1)])
+def test_histograms_equal_the_oracle(n, counts, bar_w):
+    """Tile edges, several tiles between flushes, and (bar_w = 0.002) more bins
+    than shared memory holds: counts equal, the others to the FP32 of a pair's
+    term, as in the observables' tests."""
+    spec, st = _plain(n, 90 + n)
+    orc = oracle.Oracle()
+    with L.Batch([spec], [st]) as bt:
+        bt.set_species(0, counts)
+        got = bt.correlations(bar_w)[0]
+    want = orc.acc_correl_species(_osys(spec, st), counts, bar_w, got.shape[2])
+    for q in range(want.shape[0]):
+        assert np.array_equal(got[q][0], want[q][0]), q
+        pairs = want[q][0] / (2.0 if q < len(counts) else 1.0)
+        assert np.all(np.abs(got[q][1:] - want[q][1:]) <= 5e-6 * pairs + 1e-7), q
+
+
+@pytest.mark.parametrize("n,width,height,dist", [(3, 16, 8, 8.0), (60, 77, 41, 14.0), (300, 96, 65, 3.0)])
+def test_picture_close_to_the_restatement(n, width, height, dist):
+    """Sizes that are no multiple of a block of pixels, and a camera inside the
+    box: as the picture's tests, all but 2% of the pixels within 3 levels."""
+    from oracle import render_np
+
+    spec, st = _plain(n, 30 + n, phi=0.05)
+    with L.Batch([spec], [st]) as bt:
+        img = bt.render(0, width=width, height=height, theta=0.8, phi=0.3, dist=dist)
+    want = render_np.render(width, height, st.r, st.O, st.length, st.dia, np.zeros(n, int), st.dip, spec.box,
+                            theta=0.8, phi=0.3, dist=dist)
+    off = np.abs(img.astype(int) - want.astype(int)).max(axis=-1) > 3
+    assert off.mean() <= 0.02, off.mean()

@@ -29,12 +29,15 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <mutex>
 
 #include "mdsc.h"
 #include "mdsc_dev.cuh"
+#include "reduce.cuh"
 
 namespace mdsc {
 void launch_real_pairs(const Batch& b, bool multi, cudaStream_t s);
@@ -65,38 +68,21 @@ static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
 constexpr double kLh = 0.5 * (200 * 1.001) / 32768;  // the reference's table spacing
 
-// copies of the inputs the tile kernel reads, its constants and its tile list
-__global__ void noalloc_prep_kernel(unsigned char* scr, int ndip, const double* __restrict__ pos,
-                                    const double* __restrict__ mom, double bx, double by, double bz,
-                                    double alpha) {
-  SysDev* P = reinterpret_cast<SysDev*>(scr + kOffSys);
+// Copies of the inputs the tile kernel reads, its constants (formed on the
+// host: one thread's FP64 divisions took longer than the rest of the kernel)
+// and its tile list.
+__global__ void noalloc_prep_kernel(unsigned char* scr, SysDev sys, const double* __restrict__ pos,
+                                    const double* __restrict__ mom) {
+  uint32_t* P = reinterpret_cast<uint32_t*>(scr + kOffSys);
   int4* tiles = reinterpret_cast<int4*>(scr + kOffTiles);
   uint32_t* fx = reinterpret_cast<uint32_t*>(scr + kOffFix);
   float* m = reinterpret_cast<float*>(scr + kOffMom);
   int* own = reinterpret_cast<int*>(scr + kOffOwner);
-  const int ns = cdiv(ndip, kTile);
-  const int ntile = ns * (ns + 1) / 2;
+  static_assert(sizeof(SysDev) % 4 == 0, "copied by words");
+  const int ndip = sys.ndip, ns = sys.nstrip;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const double L[3] = {bx, by, bz};
-  if (t == 0) {
-    SysDev d;
-    memset(&d, 0, sizeof d);
-    d.n = d.ndip = ndip;
-    d.nd = 1;
-    d.nstrip = ns;
-    d.ntile = ntile;
-    for (int a = 0; a < 3; ++a) {
-      d.L[a] = L[a];
-      d.invL[a] = 1.0 / L[a];
-      d.invL32[a] = d.invL[a] * 4294967296.0;
-      d.Lfix[a] = (float)(L[a] / 4294967296.0);
-      d.Lf[a] = (float)L[a];
-    }
-    d.alpha = alpha;
-    set_real_consts(d, kLh);
-    *P = d;
-  }
-  if (t < ntile) {
+  if (t < (int)(sizeof(SysDev) / 4)) P[t] = reinterpret_cast<const uint32_t*>(&sys)[t];
+  if (t < sys.ntile) {
     // row-major upper triangle: tile t -> strips (I, J), I <= J
     int I = 0, start = 0;
     while (start + (ns - I) <= t) {
@@ -106,47 +92,57 @@ __global__ void noalloc_prep_kernel(unsigned char* scr, int ndip, const double* 
     tiles[t] = make_int4(0, I, I + (t - start), 0);
   }
   if (t < ndip) {
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      fx[a * ndip + t] = to_fix(pos[3 * t + a], 4294967296.0 / L[a]);
+      fx[a * ndip + t] = to_fix(pos[3 * t + a], sys.invL32[a]);
       m[a * ndip + t] = (float)mom[3 * t + a];
     }
     own[t] = t;
   }
 }
 
-// per dipole: the tile partials over all partner strips -> F and torque
-// (FP64 outputs); one extra block sums the tiles' energy and pressure tensor
-__global__ void noalloc_reduce_kernel(const unsigned char* scr, int ndip, double* __restrict__ F,
-                                      double* __restrict__ T, double* __restrict__ UPT) {
+// Blocks of 256: the tile partials of a dipole's component over all partner
+// strips, a thread each, in float-float (48 bits; FP64 additions and
+// conversions hold a warp 64 cycles each: 3001 dipoles took 42 us in FP64 with
+// a thread per dipole, 6 this way) -> F and T in FP64; the last block sums the
+// tiles' energy and pressure tensor the same way.
+__global__ void __launch_bounds__(256) noalloc_reduce_kernel(const unsigned char* scr, int ndip,
+                                                             double* __restrict__ F, double* __restrict__ T,
+                                                             double* __restrict__ UPT) {
+  __shared__ FF sh[10][8];
   const float* part = reinterpret_cast<const float*>(scr + kOffPart);
   const float* tE = reinterpret_cast<const float*>(scr + kOffTileE);
   const int ns = cdiv(ndip, kTile);
-  const int nblk_d = cdiv(ndip, blockDim.x);
-  if ((int)blockIdx.x < nblk_d) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ndip) return;
-    const int X = g / kTile, lx = g % kTile;
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int Y = 0; Y < ns; ++Y)
-      for (int c = 0; c < 6; ++c) acc[c] += (double)part[((size_t)(X * ns + Y) * 6 + c) * kTile + lx];
-    for (int a = 0; a < 3; ++a) {
-      F[3 * g + a] = acc[a];
-      T[3 * g + a] = acc[3 + a];
-    }
+  if (blockIdx.x + 1 < gridDim.x) {
+    const int k = blockIdx.x * 256 + threadIdx.x;
+    if (k >= 6 * ndip) return;
+    const int c = k / ndip, g = k - c * ndip;  // component-major: a warp reads consecutive dipoles
+    const float* p = part + ((size_t)(g / kTile) * ns * 6 + c) * kTile + g % kTile;
+    FF acc = ff_of(0.f);
+#pragma unroll 8
+    for (int Y = 0; Y < ns; ++Y) acc = ff_add(acc, ff_of(p[(size_t)Y * 6 * kTile]));
+    const double v = soft_f2d(acc.hi) + soft_f2d(acc.lo);
+    if (c < 3) F[3 * g + c] = v;
+    else T[3 * g + c - 3] = v;
     return;
   }
-  // energy and pressure tensor: one block, fixed order
-  __shared__ double sh[10][256];
-  const int ntile = ns * (ns + 1) / 2;
-  double v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-  for (int t = threadIdx.x; t < ntile; t += blockDim.x)
-    for (int c = 0; c < 10; ++c) v[c] += (double)tE[(size_t)t * 10 + c];
-  for (int c = 0; c < 10; ++c) sh[c][threadIdx.x] = v[c];
+  const int ntile = ns * (ns + 1) / 2, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  FF v[10];
+#pragma unroll
+  for (int c = 0; c < 10; ++c) v[c] = ff_of(0.f);
+  for (int t = threadIdx.x; t < ntile; t += 256)
+#pragma unroll
+    for (int c = 0; c < 10; ++c) v[c] = ff_add(v[c], ff_of(tE[(size_t)t * 10 + c]));
+#pragma unroll
+  for (int c = 0; c < 10; ++c) {
+    v[c] = ff_warp_sum(v[c]);
+    if (lane == 0) sh[c][w] = v[c];
+  }
   __syncthreads();
   if (threadIdx.x < 10) {
-    double s = 0.0;
-    for (int k = 0; k < (int)blockDim.x; ++k) s += sh[threadIdx.x][k];
-    UPT[threadIdx.x] = s;
+    FF t = sh[threadIdx.x][0];
+    for (int q = 1; q < 8; ++q) t = ff_add(t, sh[threadIdx.x][q]);
+    UPT[threadIdx.x] = soft_f2d(t.hi) + soft_f2d(t.lo);
   }
 }
 
@@ -206,9 +202,23 @@ extern "C" mdsc_status mdsc_force_dipR_noalloc(int ndip, const double* d_pos, co
   unsigned char* base = (unsigned char*)scr;
   const int ns = cdiv(ndip, kTile);
   const int ntile = ns * (ns + 1) / 2;
-  const int nthr = ndip > ntile ? ndip : ntile;
-  noalloc_prep_kernel<<<cdiv(nthr, 256), 256, 0, st>>>(base, ndip, d_pos, d_mom, box[0], box[1], box[2],
-                                                        alpha);
+  const int nthr = std::max(std::max(ndip, ntile), (int)(sizeof(SysDev) / 4));
+  SysDev sys;
+  memset(&sys, 0, sizeof sys);
+  sys.n = sys.ndip = ndip;
+  sys.nd = 1;
+  sys.nstrip = ns;
+  sys.ntile = ntile;
+  for (int a = 0; a < 3; ++a) {
+    sys.L[a] = box[a];
+    sys.invL[a] = 1.0 / box[a];
+    sys.invL32[a] = 4294967296.0 / box[a];
+    sys.Lfix[a] = (float)(box[a] / 4294967296.0);
+    sys.Lf[a] = (float)box[a];
+  }
+  sys.alpha = alpha;
+  set_real_consts(sys, kLh);
+  noalloc_prep_kernel<<<cdiv(nthr, 256), 256, 0, st>>>(base, sys, d_pos, d_mom);
   if (cudaGetLastError() != cudaSuccess) return MDSC_ERR_CUDA;
   Batch b{};
   b.nsys = 1;
@@ -224,6 +234,6 @@ extern "C" mdsc_status mdsc_force_dipR_noalloc(int ndip, const double* d_pos, co
   b.tileE = reinterpret_cast<float*>(base + kOffTileE);
   launch_real_pairs(b, false, st);
   if (cudaGetLastError() != cudaSuccess) return MDSC_ERR_CUDA;
-  noalloc_reduce_kernel<<<cdiv(ndip, 256) + 1, 256, 0, st>>>(base, ndip, d_F, d_T, d_UPT);
+  noalloc_reduce_kernel<<<cdiv(6 * ndip, 256) + 1, 256, 0, st>>>(base, ndip, d_F, d_T, d_UPT);
   return cudaGetLastError() == cudaSuccess ? MDSC_OK : MDSC_ERR_CUDA;
 }

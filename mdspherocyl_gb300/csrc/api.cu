@@ -25,6 +25,7 @@ cudaError_t prepare_real_pairs();
 cudaError_t prepare_kspace();
 cudaError_t prepare_wca();
 void launch_real_sum(const Batch& b, cudaStream_t s);
+void launch_strip_energy(const Batch& b, cudaStream_t s);
 void launch_near_pass(const Batch& b, cudaStream_t s);  // the cutoff systems' real space
 void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, cudaStream_t s);
 void launch_derive(const Batch& b, cudaStream_t s);
@@ -66,6 +67,12 @@ using namespace mdsc;
 namespace {
 
 constexpr int kNoiseChunk = 256;  // steps of thermostat noise per upload
+// Batches of more tiles than this (4 per SM, one per scheduler) start them
+// behind a short kernel.  4096 rods (2080 tiles): 100 us per step where the
+// tiles came first and the other chains waited for them to end (its step ran
+// in 84 or in 100 us, by which was first), 89 behind it; 64 systems 195 and
+// 190; 2048 rods (528 tiles), where the tiles are the longest chain, 52 and 56.
+constexpr int kTilesAfter = 4 * 152;
 // Batches of at most this many particle blocks (2 per SM) gather one k tile
 // per block: 2048 rods (16 blocks) 85 us per step with whole walks and 80
 // split, 24 systems of 128 to 2048 rods (140 blocks) 144 and 135; 64 systems
@@ -339,8 +346,9 @@ void make_layout(const mdsc_system_desc* descs, int nsys, Layout& Lo) {
     kp += (long long)P.nkchunk * P.nk;
     P.gch_off = Lo.nchunks;
     Lo.nchunks += P.nkchunk;
+    // the chunk's k tiles, and (-1) the moment tensor of a single-dipole system
     for (int ch = 0; ch < P.nkchunk; ++ch)
-      for (int kt = 0; kt < cdiv(P.nk, kKBlock); ++kt) Lo.kwork.push_back(make_int4(s, ch, kt, 0));
+      for (int kt = d.nd == 1 ? -1 : 0; kt < cdiv(P.nk, kKBlock); ++kt) Lo.kwork.push_back(make_int4(s, ch, kt, 0));
     // cell capacity of the list build: at most one cell per 8 rods (the
     // grid is chosen at upload, when the shapes are known)
     P.cell_off = Lo.ncellcap;
@@ -532,8 +540,8 @@ void carve(Arena& A, const Layout& Lo, int nsys, Batch& b, int4** kwork, int2** 
   b.Fk = A.take<float2>(3 * nd);
   b.Tk = A.take<float2>(3 * nd);
   const size_t nw = 3 * std::max<size_t>(Lo.wblk.size(), 1);
-  b.krow = A.take<float2>(2 * nw);
-  b.krow2 = A.take<float2>(5 * nw);
+  b.krow = A.take<float2>(2 * nw / 3);
+  b.krow2 = A.take<float2>(4 * nw);
   b.wrow = A.take<float2>(4 * nw);
   b.dmax = A.take<float>(nw / 3);
   b.wblk = A.take<int2>(nw / 3);
@@ -569,7 +577,7 @@ struct mdsc_batch {
   int nsys = 0;
   cudaStream_t st = nullptr, s2 = nullptr, s3 = nullptr, s4 = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_j2 = nullptr, ev_j3 = nullptr, ev_j4 = nullptr, ev_k = nullptr,
-              ev_mid = nullptr, ev_list = nullptr;
+              ev_mid = nullptr, ev_list = nullptr, ev_tile = nullptr;
   // mdsc_step_io: the stream that takes positions and orientations home
   // while a step's forces are computed, and the event its graph records
   // once they are final
@@ -650,6 +658,7 @@ mdsc_status eval_forces(mdsc_batch* B, int force_list, const int* skip = nullptr
   launch_near_pass(b, B->st);
   launch_real_pairs(b, B->lo.multi, B->st);
   launch_real_sum(b, B->st);
+  launch_strip_energy(b, B->st);
   launch_kspace(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, B->st);
   launch_finalize(b, kMaskAll, B->st);
   launch_order_terms(b, B->st);
@@ -790,13 +799,23 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   // xi at mid-step, order terms, the list build (+ the cell binning), the WCA
   // screen and evaluation (+ the cutoff pass)
   launches += 5 + (b.cells && b.ncellblk ? 1 : 0) + (b.any_rc ? 1 : 0);
+  // the mid-step thermostat: ahead of the tiles where those fill the GPU
+  // (kTilesAfter), so that the first kernels of the other chains have their
+  // blocks placed first -- the stream priority orders blocks that wait, it
+  // does not move the tiles aside once they hold an SM's registers
+  const bool mid_first = b.ntiles > kTilesAfter;
+  if (mid_first) {
+    launch_xi_mid(b, B->s2);
+    cudaEventRecord(B->ev_mid, B->s2);
+  }
   launch_real_pairs(b, B->lo.multi, B->s2);
+  cudaEventRecord(B->ev_tile, B->s2);
   launch_real_sum(b, B->s2);
   if (b.any_rc) {  // the cutoff systems' real space, once their lists stand
     cudaStreamWaitEvent(B->s2, B->ev_list, 0);
     launch_near_pass(b, B->s2);
   }
-  launches += b.ntiles > 0 ? 2 + (b.nbstrips > 0 ? 1 : 0) : 0;
+  launches += b.ntiles > 0 ? 1 + (b.nbstrips > 0 ? 2 : 0) : 0;
   auto kpart = [&](int part, cudaStream_t s) {
     launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, part, s);
   };
@@ -806,13 +825,18 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   kpart(2, B->s3);
   // what only the second half kick and the per-system sums read
   cudaStreamWaitEvent(B->s4, B->ev_fork, 0);
-  launch_xi_mid(b, B->s4);
-  cudaEventRecord(B->ev_mid, B->s4);
+  if (!mid_first) {
+    launch_xi_mid(b, B->s4);
+    cudaEventRecord(B->ev_mid, B->s4);
+  }
   launch_order_terms(b, B->s4);
   cudaStreamWaitEvent(B->s4, B->ev_k, 0);
   kpart(3, B->s4);
+  cudaStreamWaitEvent(B->s4, B->ev_tile, 0);
+  launch_strip_energy(b, B->s4);
   cudaEventRecord(B->ev_j4, B->s4);
-  launches += b.nktot > 0 ? (B->lo.maxnd > 1 ? 6 : 4) : 0;  // multi-dipole batches: both ksum and kgather forms
+  // the chunk sums and energies, and the structure-factor and gather forms that have systems
+  launches += b.nktot > 0 ? 2 + (b.ones ? 2 : 0) + (B->lo.maxnd > 1 ? 2 : 0) : 0;
   cudaEventRecord(B->ev_j2, B->s2);
   cudaEventRecord(B->ev_j3, B->s3);
   cudaStreamWaitEvent(B->st, B->ev_j2, 0);
@@ -1260,6 +1284,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   b.nbstrips = (int)lo.bstrips.size();
   b.any_rc = lo.any_rc ? 1 : 0;
   b.nkgwork = (int)lo.kgwork.size();
+  for (int s = 0; s < nsys; ++s) b.ones += descs[s].nd == 1;
   b.nktile = (int)lo.ktile.size();
   b.nblk = (int)lo.blk.size();
   b.nwblk = (int)lo.wblk.size();
@@ -1289,6 +1314,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
       cudaEventCreateWithFlags(&B->ev_k, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_mid, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_list, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&B->ev_tile, cudaEventDisableTiming) != cudaSuccess ||
       cudaStreamCreateWithFlags(&B->sio, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_x, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&B->ev_f, cudaEventDisableTiming) != cudaSuccess ||
@@ -1406,6 +1432,7 @@ mdsc_status mdsc_destroy(mdsc_batch* B) {
   if (B->ev_k) cudaEventDestroy(B->ev_k);
   if (B->ev_mid) cudaEventDestroy(B->ev_mid);
   if (B->ev_list) cudaEventDestroy(B->ev_list);
+  if (B->ev_tile) cudaEventDestroy(B->ev_tile);
   if (B->ev_x) cudaEventDestroy(B->ev_x);
   if (B->ev_f) cudaEventDestroy(B->ev_f);
   if (B->sio) cudaStreamDestroy(B->sio);
@@ -1729,6 +1756,7 @@ mdsc_status mdsc_force_dipR(mdsc_batch* B, double* U, double* PT) {
   launch_near_pass(B->b, B->st);
   launch_real_pairs(B->b, B->lo.multi, B->st);
   launch_real_sum(B->b, B->st);
+  launch_strip_energy(B->b, B->st);
   launch_finalize(B->b, kMaskReal | kFlagAccum, B->st);
   launch_order_terms(B->b, B->st);
   launch_reduce_obs(B->b, kRedEnergies, B->st);
@@ -2583,6 +2611,7 @@ mdsc_status mdsc_profile_steps(mdsc_batch* B, int nsteps, int max_kernels, char*
     launch_real_pairs(b, B->lo.multi, B->st);
     cudaEventRecord(ev[5], B->st);
     launch_real_sum(b, B->st);
+    launch_strip_energy(b, B->st);
     cudaEventRecord(ev[6], B->st);
     launch_near_pass(b, B->st);
     cudaEventRecord(ev[7], B->st);

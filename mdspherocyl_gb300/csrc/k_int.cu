@@ -83,6 +83,8 @@ constexpr int kRowBlock = 3 * kRows;
 struct Shared3 {
   double l[3][kRows];
   double ax[3][kRows];
+  double p[3][kRows];
+  double lb2[3][kRows];
   float O[9][kRows];   // orientation before the move
   float O2[9][kRows];  // and after it
   float d2[3][kRows];
@@ -93,9 +95,11 @@ struct Shared3 {
 // length; sh.O2 and sh.ax hold the new orientation.  Returns, in warp 2, how
 // far the rod's ends may have moved since the last list build: the centre's
 // move from the fixed-point coordinates (exact minimum image) plus half the
-// length times the axis change.
+// length times the axis change (u_built, ax_built: its position component and
+// axis at that build, loaded with the rest of the state).
 __device__ __forceinline__ float derive_comp(const Batch& b, const SysDev& P, Shared3& sh, int a, int lane, int i,
-                                             bool ok, double r, const double* O) {
+                                             bool ok, double r, const double* O, uint32_t u_built,
+                                             const float* ax_built) {
   const int N = b.ntot, ND = b.ndtot;
   const uint32_t u = to_fix(r, P.invL32[a]);
 #pragma unroll
@@ -105,7 +109,7 @@ __device__ __forceinline__ float derive_comp(const Batch& b, const SysDev& P, Sh
     for (int c = 0; c < 3; ++c) sh.ax[c][lane] = O[c];
   }
   {
-    const float d = fix_diff(u, b.fsave[3 * i + a], P.Lfix[a]);
+    const float d = fix_diff(u, u_built, P.Lfix[a]);
     sh.d2[a][lane] = d * d;
   }
   __syncthreads();
@@ -132,7 +136,7 @@ __device__ __forceinline__ float derive_comp(const Batch& b, const SysDev& P, Sh
       float du2 = 0.f;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const float q = x[c] - b.usave[3 * i + c];
+        const float q = x[c] - ax_built[c];
         du2 += q * q;
       }
       disp = sqrtf(sh.d2[0][lane] + sh.d2[1][lane] + sh.d2[2][lane]) + 0.5f * ln * sqrtf(du2);
@@ -151,6 +155,32 @@ __device__ __forceinline__ void store_disp(const Batch& b, SysState& S, int row,
     b.dmax[row] = disp;
     atomicMax(&S.dmax, __float_as_int(disp));
   }
+}
+
+// A particle's kinetic energies, doubled: translational from its momentum,
+// rotational, sum_a (O l)_a^2 / I_a (v25/functions.cpp:2123-2148), from the
+// squares; each by one warp, in the order of the components.
+__device__ __forceinline__ double kin_t(const double (&p)[3][kRows], int lane, double invm) {
+  double psq = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) psq += p[c][lane] * p[c][lane];
+  return psq * invm;
+}
+__device__ __forceinline__ double kin_r(const Batch& b, const double (&lb2)[3][kRows], int lane, int i) {
+  double k = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) k += lb2[c][lane] * b.invI[3 * i + c];
+  return k;
+}
+
+// The row's kinetic energies, translational by warp 0 and rotational by warp
+// 1, after the rest of the kernel: nothing before the second half kick reads
+// them.
+__device__ __forceinline__ void store_kin(const Batch& b, const Shared3& sh, int row, int a, int lane, int i, bool ok) {
+  if (a == 2) return;
+  const double v = !ok ? 0.0 : a == 0 ? kin_t(sh.p, lane, b.invm[i]) : kin_r(b, sh.lb2, lane, i);
+  const FF k = ff_warp_sum(ff_from(v));
+  if (lane == 0) b.krow[2 * row + a] = make_float2(k.hi, k.lo);
 }
 
 // the free-rotor move of the step (Spherocyl::rotate, v25/classes.cpp:240-304):
@@ -219,6 +249,12 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
   double r = b.r[3 * i + a], O[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) O[c] = b.O[9 * i + 3 * a + c];
+  const uint32_t u_built = b.fsave[3 * i + a];
+  float ax_built[3] = {0.f, 0.f, 0.f};
+  if (a == 2) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) ax_built[c] = b.usave[3 * i + c];
+  }
   if constexpr (MODE != kPartDerive) {
     double p = b.p[3 * i + a], l = b.l[3 * i + a];
     const double im = b.invm[i];
@@ -248,14 +284,10 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
     for (int c = 0; c < 3; ++c) sh.O[3 * a + c][lane] = soft_d2f_rn(O[c]);
     __syncthreads();
     if constexpr (MODE == kPartStep) {
-      // the kinetic energies of this component, before the move
+      // the kinetic energies before the move, in store_kin
       const double lb = O[0] * sh.l[0][lane] + O[1] * sh.l[1][lane] + O[2] * sh.l[2][lane];
-      FF k[2] = {ff_from(ok ? p * p * im : 0.0), ff_from(ok ? lb * lb * b.invI[3 * i + a] : 0.0)};
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        k[c] = ff_warp_sum(k[c]);
-        if (lane == 0) b.krow[2 * (3 * row + a) + c] = make_float2(k[c].hi, k[c].lo);
-      }
+      sh.p[a][lane] = p;
+      sh.lb2[a][lane] = lb * lb;
       if (ok) {
         b.p[3 * i + a] = p;
         b.l[3 * i + a] = l;
@@ -273,35 +305,49 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
       for (int c = 0; c < 3; ++c) b.O[9 * i + 3 * a + c] = O[c];
     }
   }
-  const float disp = derive_comp(b, P, sh, a, lane, i, ok, r, O);
+  const float disp = derive_comp(b, P, sh, a, lane, i, ok, r, O, u_built, ax_built);
   if constexpr (MODE != kPartMoveX) store_disp(b, S, row, a, disp);
+  if constexpr (MODE == kPartStep) store_kin(b, sh, row, a, lane, i, ok);
 }
 
 // Thermostat coordinates of the second half kick, moveTher 0 then 1
 // (v25/functions.cpp:2193-2206), from the first-half kinetic energies: a
 // block per system, beside the force chains (only the second kick reads them).
+// The rows of 128 particles are added in float-float and those sums in FP64,
+// in order: the thermostat feeds back on every momentum, so its last bits stay
+// what they were when a block of 128 threads summed its particles.
 __global__ void __launch_bounds__(128) xi_mid_kernel(Batch b) {
-  __shared__ FF sh[2][4];
+  __shared__ double sh[2][128];
   const int s = blockIdx.x;
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   SysState& S = b.st[s];
-  FF v[2] = {ff_of(0.f), ff_of(0.f)};
-  for (int t = threadIdx.x; t < 3 * P.nw; t += 128) {
-    const float4 q = reinterpret_cast<const float4*>(b.krow)[3 * P.w_off + t];
-    v[0] = ff_add(v[0], FF{q.x, q.y});
-    v[1] = ff_add(v[1], FF{q.z, q.w});
-  }
+  const int nb = cdiv(P.nw, 4);
+  double K = 0.0;
+  for (int b0 = 0; b0 < nb; b0 += 128) {
+    const int blk = b0 + threadIdx.x;
+    if (blk < nb) {
+      const float4* in = reinterpret_cast<const float4*>(b.krow) + P.w_off + 4 * blk;
+      float4 x[4];
 #pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    v[c] = ff_warp_sum(v[c]);
-    if ((threadIdx.x & 31) == 0) sh[c][threadIdx.x >> 5] = v[c];
+      for (int q = 0; q < 4; ++q) x[q] = 4 * blk + q < P.nw ? in[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+      FF t{x[0].x, x[0].y}, r{x[0].z, x[0].w};
+#pragma unroll
+      for (int q = 1; q < 4; ++q) {
+        t = ff_add(t, FF{x[q].x, x[q].y});
+        r = ff_add(r, FF{x[q].z, x[q].w});
+      }
+      sh[0][threadIdx.x] = soft_f2d(t.hi) + soft_f2d(t.lo);
+      sh[1][threadIdx.x] = soft_f2d(r.hi) + soft_f2d(r.lo);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2)
+      for (int k = 0; k < min(128, nb - b0); ++k) K += sh[threadIdx.x][k];
+    __syncthreads();
   }
-  __syncthreads();
   const int c = threadIdx.x;
   if (c >= 2) return;
-  const FF t = ff_add(ff_add(ff_add(sh[c][0], sh[c][1]), sh[c][2]), sh[c][3]);
-  const double Kf = 0.5 * (soft_f2d(t.hi) + soft_f2d(t.lo));
+  const double Kf = 0.5 * K;
   const double* nz = b.noise + ((long long)S.iter * b.nsys + s) * 4;
   const double x1 = P.ex1 * S.xi[c] + P.cnoise * nz[2 * c];
   S.K_first[c] = Kf;
@@ -311,16 +357,17 @@ __global__ void __launch_bounds__(128) xi_mid_kernel(Batch b) {
 // ---------------------------------------------------------------------
 // force assembly (+ ext_field) and optionally moveP(last): three lanes per
 // rod as above.  Each warp leaves its sums for the per-system reduction as
-// float-float rows: krow2 (K_t, K_r, two kinetic pressure terms, U_ext) and
+// float-float rows: krow2 (K_t or K_r, two kinetic pressure terms, U_ext) and
 // wrow (the WCA terms a, a + 3, ... of U, W, PT of the rods' own pairs).
 // ---------------------------------------------------------------------
-constexpr int kKinCols = 5, kWcaCols = 4;
+constexpr int kKinCols = 4, kWcaCols = 4;
 // kinetic pressure terms of warp a: (xx, xy), (yy, yz), (zz, zx)
 
 __global__ void __launch_bounds__(kRowBlock) finalize_kernel(Batch b, int mode) {
   __shared__ double sl[3][kRows];
   __shared__ double sv[3][kRows];
   __shared__ float sp[3][kRows];
+  __shared__ double sk[2][3][kRows];  // p; (O l)_a^2
   const int2 bk = b.wblk[blockIdx.x];
   const int s = bk.x;
   if (at_limit(b, s)) return;
@@ -394,10 +441,18 @@ __global__ void __launch_bounds__(kRowBlock) finalize_kernel(Batch b, int mode) 
     // float-float (FP32 instructions), one conversion to FP64 at the end
     FF qf = ff_of(0.f), qt = ff_of(0.f);
     if (mode & kMaskReal) {
-      // this dipole's tile partials summed over all partner strips (real_sum_kernel)
-      const float2 x = b.rsum[(long long)a * b.ndtot + g], y = b.rsum[(long long)(3 + a) * b.ndtot + g];
-      qf = FF{x.x, x.y};
-      qt = FF{y.x, y.y};
+      // this dipole's tile partials summed over all partner strips: here, or
+      // by real_sum_kernel (or near_pass_kernel) before
+      if (P.rc_real <= 0.0 && P.nstrip <= kStripRows) {
+        const int loc = g - P.dip_off;
+        const float* part = b.rpart + P.pp_off + ((long long)(loc / kTile) * P.nstrip * 6 + a) * kTile + loc % kTile;
+        qf = strip_sum<8>(part, P.nstrip, 6 * kTile);
+        qt = strip_sum<8>(part + 3 * kTile, P.nstrip, 6 * kTile);
+      } else {
+        const float2 x = b.rsum[(long long)a * b.ndtot + g], y = b.rsum[(long long)(3 + a) * b.ndtot + g];
+        qf = FF{x.x, x.y};
+        qt = FF{y.x, y.y};
+      }
     }
     if (mode & kMaskK) {
       const float2 x = b.Fk[3 * g + a], y = b.Tk[3 * g + a];
@@ -428,31 +483,36 @@ __global__ void __launch_bounds__(kRowBlock) finalize_kernel(Batch b, int mode) 
     F += f;
     T += t;
   }
+  // warp 0: K_t, warp 1: K_r; then two terms of the pressure tensor, U_ext
   FF k[kKinCols];
 #pragma unroll
   for (int c = 0; c < kKinCols; ++c) k[c] = ff_of(0.f);
-  k[4] = ff_from(ok ? uext : 0.0);
+  k[3] = ff_from(ok ? uext : 0.0);
   if (mode & kFlagMoveP) {
     // moveP last half (v25/functions.cpp:2150-2173), with xi after moveTher
     // 0 and 1 (xi_mid_kernel)
     const double h = 0.5 * P.dt;
-    const double p = b.p[3 * i + a] * (1. - h * S.xi_mid[0]) + h * F;
-    const double l = b.l[3 * i + a] * (1. - h * S.xi_mid[1]) + h * T;
+    // (the products' roundings written out: both kicks keep their last bits)
+    const double p = __fma_rn(b.p[3 * i + a], 1. - h * S.xi_mid[0], h * F);
+    const double l = __fma_rn(b.l[3 * i + a], 1. - h * S.xi_mid[1], h * T);
     const double im = b.invm[i];
     sl[a][lane] = l;
     sp[a][lane] = soft_d2f_rn(p);
     __syncthreads();
+    const double* O = b.O + 9 * i + 3 * a;
+    const double lb = O[0] * sl[0][lane] + O[1] * sl[1][lane] + O[2] * sl[2][lane];
+    sk[0][a][lane] = p;
+    sk[1][a][lane] = lb * lb;
+    __syncthreads();
     if (ok) {
       b.p[3 * i + a] = p;
       b.l[3 * i + a] = l;
-      const double* O = b.O + 9 * i + 3 * a;
-      const double lb = O[0] * sl[0][lane] + O[1] * sl[1][lane] + O[2] * sl[2][lane];
-      k[0] = ff_from(p * p * im);
-      k[1] = ff_from(lb * lb * b.invI[3 * i + a]);
+      if (a == 0) k[0] = ff_from(kin_t(sk[0], lane, im));
+      if (a == 1) k[0] = ff_from(kin_r(b, sk[1], lane, i));
       // kinetic pressure tensor p_a p_b / m: FP32 products, float-float sums
       const float imf = soft_d2f_rn(im), pf = sp[a][lane];
-      k[2] = ff_of(pf * pf * imf);
-      k[3] = ff_of(pf * sp[a1][lane] * imf);
+      k[1] = ff_of(pf * pf * imf);
+      k[2] = ff_of(pf * sp[a1][lane] * imf);
     }
   }
   if (ok) {
@@ -530,17 +590,32 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
           if (a + 3 * q < 11) v[a + 3 * q] = ff_add(v[a + 3 * q], FF{w[kWcaCols * a + q].x, w[kWcaCols * a + q].y});
     }
   } else if (grp == 3) {
-    // K_t, K_r, then (xx xy)(yy yz)(zz zx), U_ext
-    for (int t = threadIdx.x; t < P.nw; t += kRedThreads) {
-      const float2* k = b.krow2 + (long long)(P.w_off + t) * 3 * kKinCols;
+    // K_t, K_r, then (xx xy)(yy yz)(zz zx), U_ext.  K_t and K_r by blocks of
+    // 128 particles, as in xi_mid_kernel
+    const float2* k = b.krow2 + (long long)P.w_off * 3 * kKinCols;
+    for (int t = threadIdx.x; t < cdiv(P.nw, 4); t += kRedThreads) {
+      float2 x[4][2];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          x[q][c] = 4 * t + q < P.nw ? k[((4 * t + q) * 3 + c) * kKinCols] : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        FF y{x[0][c].x, x[0][c].y};
+#pragma unroll
+        for (int q = 1; q < 4; ++q) y = ff_add(y, FF{x[q][c].x, x[q][c].y});
+        v[c] = ff_add(v[c], ff_from(soft_f2d(y.hi) + soft_f2d(y.lo)));
+      }
+    }
+    // from the last thread down: in small systems beside the sums above
+    for (int t = kRedThreads - 1 - threadIdx.x; t < P.nw; t += kRedThreads) {
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        const float2* q = k + kKinCols * a;
-        v[0] = ff_add(v[0], FF{q[0].x, q[0].y});
-        v[1] = ff_add(v[1], FF{q[1].x, q[1].y});
-        v[2 + 2 * a] = ff_add(v[2 + 2 * a], FF{q[2].x, q[2].y});
-        v[3 + 2 * a] = ff_add(v[3 + 2 * a], FF{q[3].x, q[3].y});
-        v[8] = ff_add(v[8], FF{q[4].x, q[4].y});
+        const float2* q = k + (3 * t + a) * kKinCols;
+        v[2 + 2 * a] = ff_add(v[2 + 2 * a], FF{q[1].x, q[1].y});
+        v[3 + 2 * a] = ff_add(v[3 + 2 * a], FF{q[2].x, q[2].y});
+        v[8] = ff_add(v[8], FF{q[3].x, q[3].y});
       }
     }
   } else {

@@ -35,12 +35,10 @@ namespace mdsc {
 // and 226, 256 systems 693 and 696.
 constexpr int kKsumScalarMax = 4 * 152;
 
-__device__ __forceinline__ void phase_cs(uint32_t ph, float& c, float& s) {
-  // (int)ph * 2^-31 * pi: the phase, already reduced to [-pi, pi); the
-  // hardware sine/cosine is accurate to ~4e-7 absolute on that range
-  const float x = (float)(int32_t)ph * 1.4629180792671596e-09f;
-  __sincosf(x, &s, &c);
-}
+// (int)ph * 2^-31 * pi: the phase, already reduced to [-pi, pi); the
+// hardware sine/cosine is accurate to ~4e-7 absolute on that range
+__device__ __forceinline__ float phase_rad(uint32_t ph) { return (float)(int32_t)ph * 1.4629180792671596e-09f; }
+__device__ __forceinline__ void phase_cs(uint32_t ph, float& c, float& s) { __sincosf(phase_rad(ph), &s, &c); }
 __device__ __forceinline__ uint32_t phase_of(uint32_t ux, uint32_t uy, uint32_t uz, int4 n) {
   return (uint32_t)n.x * ux + (uint32_t)n.y * uy + (uint32_t)n.z * uz;
 }
@@ -57,40 +55,34 @@ __device__ __forceinline__ uint32_t phase_next(uint32_t ph, bool have, uint32_t 
 }
 
 // The moment tensor of one particle chunk, sum of m m^T (one dipole per
-// particle), for the self terms of kenergy.  Float-float: the products exact
-// (one FMA each for the low half), 48-bit sums -- in FP64 the six sums cost
-// 64 cycles an instruction and a warp (the FP64 unit's issue rate on this GPU,
-// whatever the number of independent chains).
-// The block's first two warps take the chunk, whatever the block's size: one
-// order of the sums for both forms of the kernel.
-template <class M>
-__device__ __forceinline__ void chunk_tensor(const Batch& b, long long row, int np, FF (*sh)[6], M&& moment) {
-  const int w = threadIdx.x >> 5;
-  if (w < 2) {
-    FF g[6];
+// particle), for the self terms of kenergy, by a warp of its own block (work
+// items of k tile -1).  Float-float: the products exact (one FMA each for the
+// low half), 48-bit sums -- in FP64 the six sums cost 64 cycles an instruction
+// and a warp (the FP64 unit's issue rate on this GPU, whatever the number of
+// independent chains).
+__device__ __forceinline__ void chunk_tensor(const Batch& b, const SysDev& P, int chunk) {
+  if (threadIdx.x >= 32) return;
+  const int N = b.ndtot, p0 = chunk * kKChunk, np = min(kKChunk, P.n - p0);
+  FF g[6];
 #pragma unroll
-    for (int c = 0; c < 6; ++c) g[c] = ff_of(0.f);
-    for (int q = threadIdx.x; q < np; q += 64) {
-      const float4 m = moment(q);
-      const float u[6] = {m.x, m.x, m.x, m.y, m.y, m.z}, v[6] = {m.x, m.y, m.z, m.y, m.z, m.z};
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        FF t;
-        t.hi = __fmul_rn(u[c], v[c]);
-        t.lo = __fmaf_rn(u[c], v[c], -t.hi);
-        g[c] = ff_add(g[c], t);
-      }
-    }
+  for (int c = 0; c < 6; ++c) g[c] = ff_of(0.f);
+#pragma unroll 4
+  for (int q = threadIdx.x; q < np; q += 32) {
+    const int d = P.dip_off + p0 + q;
+    const float x = b.dm[d], y = b.dm[N + d], z = b.dm[2 * N + d];
+    const float u[6] = {x, x, x, y, y, z}, v[6] = {x, y, z, y, z, z};
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      g[c] = ff_warp_sum(g[c]);
-      if ((threadIdx.x & 31) == 0) sh[w][c] = g[c];
+      FF t;
+      t.hi = __fmul_rn(u[c], v[c]);
+      t.lo = __fmaf_rn(u[c], v[c], -t.hi);
+      g[c] = ff_add(g[c], t);
     }
   }
-  __syncthreads();
-  if (threadIdx.x < 6) {
-    const FF g = ff_add(sh[0][threadIdx.x], sh[1][threadIdx.x]);
-    b.kG[row * 6 + threadIdx.x] = soft_f2d(g.hi) + soft_f2d(g.lo);
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    g[c] = ff_warp_sum(g[c]);
+    if (threadIdx.x == c) b.kG[((long long)P.gch_off + chunk) * 6 + c] = soft_f2d(g[c].hi) + soft_f2d(g[c].lo);
   }
 }
 
@@ -165,20 +157,21 @@ __global__ void __launch_bounds__(kKBlock) ksum_kernel(Batch b, const int4* __re
 // Single-dipole systems.  The particle's own terms need no per-k work:
 // |S_i(k)|^2 = (m_i.k)^2 and Re(conj(S_i) U_ic) = (m_i.k) m_ic, so
 // self(k) = k^T G k and uvslf(k) = G k with G = sum_i m_i m_i^T
-// (chunk_tensor, by the first k tile of every chunk).
+// (chunk_tensor).
 //
 // Two forms, the same IEEE operations in the same order per (particle, k)
 // and so the same bits.  ksum1: two k-vectors per thread (kl and kl + 64 of
 // the block's k tile) in the halves of float2 values, so every particle
 // read from shared memory serves two k's and the six multiply-adds of U(k)
 // issue once for both -- for batches that fill the GPU.  ksum1s: one k per
-// thread, twice the warps -- for the others, where one warp's chain of
-// sines and cosines over the chunk (the special-function unit takes a warp
-// 16 cycles per particle and k) is the time.
+// thread, the cosine sums and the sine sums on different warps -- for the
+// others, where one warp's walk over the chunk is the time (the special-
+// function unit takes a warp 8 cycles per sine or cosine): 256 rods 10.7 us a
+// launch with both sums on one warp, 7.9 this way.
+constexpr int kAhead = 8;  // waves formed ahead of their sums
 struct KChunk {
   uint4 u[kKChunk];   // fixed-point x, y, z
   float4 m[kKChunk];  // moment
-  FF sh[2][6];
 };
 
 template <int NT>
@@ -191,8 +184,6 @@ __device__ __forceinline__ int stage_chunk(const Batch& b, const SysDev& P, int4
     c.m[q] = make_float4(b.dm[g], b.dm[N + g], b.dm[2 * N + g], 0.f);
   }
   __syncthreads();
-  if (w.z == 0)
-    chunk_tensor(b, (long long)P.gch_off + w.y, np, c.sh, [&](int q) { return c.m[q]; });
   return np;
 }
 
@@ -201,6 +192,10 @@ __global__ void __launch_bounds__(kKBlock / 2) ksum1_kernel(Batch b, const int4*
   const int4 w = kwork[blockIdx.x];
   const SysDev& P = b.sys[w.x];
   if (P.nd != 1 || at_limit(b, w.x)) return;  // other systems: ksum_kernel<ND>
+  if (w.z < 0) {
+    chunk_tensor(b, P, w.y);
+    return;
+  }
   const int np = stage_chunk<kKBlock / 2>(b, P, w, ck);
   const int kl0 = w.z * kKBlock + threadIdx.x, kl1 = kl0 + kKBlock / 2;
   const bool v0 = kl0 < P.nk, v1 = kl1 < P.nk;
@@ -234,52 +229,76 @@ __global__ void __launch_bounds__(kKBlock / 2) ksum1_kernel(Batch b, const int4*
   }
 }
 
-__global__ void __launch_bounds__(kKBlock) ksum1s_kernel(Batch b, const int4* __restrict__ kwork) {
+__global__ void __launch_bounds__(2 * kKBlock) ksum1s_kernel(Batch b, const int4* __restrict__ kwork) {
   __shared__ KChunk ck;
   const int4 w = kwork[blockIdx.x];
   const SysDev& P = b.sys[w.x];
   if (P.nd != 1 || at_limit(b, w.x)) return;  // other systems: ksum_kernel<ND>
-  const int np = stage_chunk<kKBlock>(b, P, w, ck);
-  const int kl = w.z * kKBlock + threadIdx.x;
+  if (w.z < 0) {
+    chunk_tensor(b, P, w.y);
+    return;
+  }
+  const int np = stage_chunk<2 * kKBlock>(b, P, w, ck);
+  const bool sine = threadIdx.x >= kKBlock;  // the same for a warp
+  const int kl = w.z * kKBlock + (threadIdx.x & (kKBlock - 1));
   if (kl >= P.nk) return;
   const int4 n = b.kn[P.k_off + kl];
-  float acc[6];
+  float acc[3] = {0.f, 0.f, 0.f};
+  auto walk = [&](auto&& wave) {
+    int p = 0;
+#pragma unroll 1
+    for (; p + kAhead <= np; p += kAhead) {
+      float v[kAhead];
 #pragma unroll
-  for (int c = 0; c < 6; ++c) acc[c] = 0.f;
-#pragma unroll 8
-  for (int p = 0; p < np; ++p) {
-    float c, s;
-    const uint4 u = ck.u[p];
-    phase_exp(u.x, u.y, u.z, n, c, s);
-    const float4 m = ck.m[p];
-    acc[0] = __fmaf_rn(m.x, c, acc[0]);
-    acc[1] = __fmaf_rn(m.x, -s, acc[1]);
-    acc[2] = __fmaf_rn(m.y, c, acc[2]);
-    acc[3] = __fmaf_rn(m.y, -s, acc[3]);
-    acc[4] = __fmaf_rn(m.z, c, acc[4]);
-    acc[5] = __fmaf_rn(m.z, -s, acc[5]);
-  }
-  float* out = ksum_part(b, P, w.y, 6) + kl;
+      for (int q = 0; q < kAhead; ++q) v[q] = wave(p + q);
 #pragma unroll
-  for (int c = 0; c < 6; ++c) out[(long long)c * P.nk] = acc[c];
+      for (int q = 0; q < kAhead; ++q) {
+        const float4 m = ck.m[p + q];
+        acc[0] = __fmaf_rn(m.x, v[q], acc[0]);
+        acc[1] = __fmaf_rn(m.y, v[q], acc[1]);
+        acc[2] = __fmaf_rn(m.z, v[q], acc[2]);
+      }
+    }
+#pragma unroll 1
+    for (; p < np; ++p) {
+      const float v = wave(p);
+      const float4 m = ck.m[p];
+      acc[0] = __fmaf_rn(m.x, v, acc[0]);
+      acc[1] = __fmaf_rn(m.y, v, acc[1]);
+      acc[2] = __fmaf_rn(m.z, v, acc[2]);
+    }
+  };
+  // E = exp(-i k.r) = (c, -s); U_c += m_c E
+  if (sine)
+    walk([&](int p) { return -__sinf(phase_rad(phase_of(ck.u[p].x, ck.u[p].y, ck.u[p].z, n))); });
+  else
+    walk([&](int p) { return __cosf(phase_rad(phase_of(ck.u[p].x, ck.u[p].y, ck.u[p].z, n))); });
+  float* out = ksum_part(b, P, w.y, 6) + (sine ? P.nk : 0) + kl;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) out[(long long)2 * c * P.nk] = acc[c];
 }
 
 template <int ND>
 static void launch_ksum(const Batch& b, const int4* kwork, int nkwork, cudaStream_t s) {
   // every single-dipole system through a single-dipole kernel, in any
   // batch, so that it gives the same bits alone and beside multi-dipole ones
-  if (nkwork <= kKsumScalarMax)
-    ksum1s_kernel<<<nkwork, kKBlock, 0, s>>>(b, kwork);
+  if (!b.ones)
+    ;
+  else if (nkwork <= kKsumScalarMax)
+    ksum1s_kernel<<<nkwork, 2 * kKBlock, 0, s>>>(b, kwork);
   else
     ksum1_kernel<<<nkwork, kKBlock / 2, 0, s>>>(b, kwork);
   if constexpr (ND > 1) ksum_kernel<ND><<<nkwork, kKBlock, 0, s>>>(b, kwork);
 }
 
-// Chunk sums per k and val S(k): all the gather needs, nothing more.  A
-// block takes 32 consecutive k-vectors of the batch, its four warps the
-// chunks w, w + 4, ... of each (float-float); warp 0 adds the four in order.
-__global__ void __launch_bounds__(128) kstruct_kernel(Batch b, const int2* __restrict__ kowner) {
-  __shared__ FF sh[3][10][32];
+// Chunk sums per k and val S(k): all the gather needs, nothing more.  A block
+// takes 32 consecutive k-vectors of the batch; warp w sums components w, w +
+// kStructWarps, ... over the chunks, in chunk order (float-float; sixteen
+// loads in flight), and warp 0 forms val S(k): the gathers' input keeps one
+// order of its sums.
+constexpr int kStructWarps = 6;
+__global__ void __launch_bounds__(32 * kStructWarps) kstruct_kernel(Batch b, const int2* __restrict__ kowner) {
+  __shared__ double sh[6][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
   bool on = k < b.nktot;
@@ -287,41 +306,34 @@ __global__ void __launch_bounds__(128) kstruct_kernel(Batch b, const int2* __res
   on = on && !at_limit(b, ow.x);
   const SysDev& P = b.sys[ow.x];
   const int nv = P.nd == 1 ? 6 : 10;
-  FF sf[10];
-#pragma unroll
-  for (int c = 0; c < 10; ++c) sf[c] = ff_of(0.f);
   if (on) {
-    for (int ch = w; ch < P.nkchunk; ch += 4) {
-      const float* in = ksum_part(b, P, ch, nv) + ow.y;
+    for (int c = w; c < nv; c += kStructWarps) {
+      const float* in = ksum_part(b, P, 0, nv) + (long long)c * P.nk + ow.y;
+      const long long stride = (long long)nv * P.nk;
+      FF sf = ff_of(0.f);
+      for (int ch = 0; ch < P.nkchunk; ch += 16) {
+        float x[16];
 #pragma unroll
-      for (int c = 0; c < 10; ++c)
-        if (c < nv) sf[c] = ff_add(sf[c], ff_of(in[(long long)c * P.nk]));
+        for (int q = 0; q < 16; ++q) x[q] = ch + q < P.nkchunk ? in[(ch + q) * stride] : 0.f;
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+          if (ch + q < P.nkchunk) sf = ff_add(sf, ff_of(x[q]));
+      }
+      const double s = soft_f2d(sf.hi) + soft_f2d(sf.lo);
+      b.ksum[(long long)k * 10 + c] = s;
+      if (c < 6) sh[c][lane] = s;
     }
-  }
-  if (w > 0) {
-#pragma unroll
-    for (int c = 0; c < 10; ++c) sh[w - 1][c][lane] = sf[c];
   }
   __syncthreads();
   if (w > 0 || !on) return;
-  double s[10];
+  double s[6];
 #pragma unroll
-  for (int c = 0; c < 10; ++c) {
-    if (c < nv) {
-#pragma unroll
-      for (int q = 0; q < 3; ++q) sf[c] = ff_add(sf[c], sh[q][c][lane]);
-      s[c] = soft_f2d(sf[c].hi) + soft_f2d(sf[c].lo);
-    }
-  }
+  for (int c = 0; c < 6; ++c) s[c] = sh[c][lane];
   const double kx = b.kvec[3 * k], ky = b.kvec[3 * k + 1], kz = b.kvec[3 * k + 2];
   const double val = b.kval[k];
   const double Sr = kx * s[0] + ky * s[2] + kz * s[4];
   const double Si = kx * s[1] + ky * s[3] + kz * s[5];
   b.kS[k] = make_float2(soft_d2f_rn(val * Sr), soft_d2f_rn(val * Si));
-  double* ks = b.ksum + (long long)k * 10;
-#pragma unroll
-  for (int c = 0; c < 10; ++c)
-    if (c < nv) ks[c] = s[c];
 }
 
 // Energy and pressure tensor of one k tile (v25/functions.cpp:1839-1952),
@@ -787,7 +799,9 @@ __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
 
 template <int ND>
 static void launch_kgather(const Batch& b, cudaStream_t s) {
-  if (b.tune.kg_scalar)
+  if (!b.ones)
+    ;
+  else if (b.tune.kg_scalar)
     kgather1s_kernel<<<b.nkgwork, kPartBlock, 0, s>>>(b);
   else
     kgather1_kernel<<<b.nkgwork, kPartBlock / 2, 0, s>>>(b);
@@ -799,7 +813,7 @@ static void kspace_part_nd(const Batch& b, const int4* kwork, int nkwork, const 
                            cudaStream_t s) {
   if (b.nktot == 0) return;
   if (part == 0 && nkwork > 0) launch_ksum<ND>(b, kwork, nkwork, s);
-  if (part == 1) kstruct_kernel<<<cdiv(b.nktot, 32), 128, 0, s>>>(b, kowner);
+  if (part == 1) kstruct_kernel<<<cdiv(b.nktot, 32), 32 * kStructWarps, 0, s>>>(b, kowner);
   if (part == 2) launch_kgather<ND>(b, s);
   if (part == 3) kenergy_kernel<<<b.nktile, kKBlock, 0, s>>>(b);
 }

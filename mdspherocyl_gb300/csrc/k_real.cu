@@ -759,37 +759,24 @@ __global__ void __launch_bounds__(kPartBlock * kCutLanes) near_pass_kernel(Batch
   }
 }
 
-// Each dipole's real-space force and torque: the sum of its tile partials
-// over all partner strips, in strip order, in float-float.  One thread per
-// (dipole, component) of a particle block, component-major so that a warp
-// reads 32 consecutive dipoles of one component (coalesced) and the block
-// has six times as many independent load streams as dipoles.
+// Each dipole's real-space force and torque in a system of more than
+// kStripRows strips: the sum of its tile partials over all partner strips,
+// in strip order, in float-float.  A block per strip, a thread per (component,
+// dipole) so that a warp reads 32 consecutive dipoles of one component.  Bound
+// by the partials' bytes (32,768 rods: 403 MB); sixteen loads in flight per
+// thread, and strips rather than particle blocks to even out the SMs: 108 us a
+// launch with eight loads over particle blocks, 86 this way.
 __global__ void __launch_bounds__(512) real_sum_kernel(Batch b) {
-  const int2 bk = b.blk[blockIdx.x];
-  const SysDev& P = b.sys[bk.x];
-  if (P.rc_real > 0.0 || at_limit(b, bk.x)) return;  // cutoff systems: summed by their neighbour pass
-  const int nd = P.nd;
-  const int p0 = bk.y - P.part_off;
-  const int np = min(kPartBlock, P.n - p0);
-  const int nloc = np * nd, loc0 = p0 * nd;
-  const int ns = P.nstrip;
-  const int ND = b.ndtot;
-  for (int it = threadIdx.x; it < 6 * nloc; it += blockDim.x) {
-    const int c = it / nloc, loc = loc0 + (it - c * nloc);
-    const int X = loc / kTile, lx = loc % kTile;
-    const float* base = b.rpart + P.pp_off + (long long)X * ns * 6 * kTile + c * kTile + lx;
-    float hi = 0.f, lo = 0.f;
-#pragma unroll 8
-    for (int Y = 0; Y < ns; ++Y) {
-      // float-float accumulation (TwoSum)
-      const float v = base[(long long)Y * 6 * kTile];
-      const float sum = hi + v;
-      const float bb = sum - hi;
-      lo += (hi - (sum - bb)) + (v - bb);
-      hi = sum;
-    }
-    const float r = hi + lo;
-    b.rsum[(long long)c * ND + P.dip_off + loc] = make_float2(r, lo - (r - hi));
+  const int2 sx = b.bstrips[blockIdx.x];
+  if (at_limit(b, sx.x)) return;
+  const SysDev& P = b.sys[sx.x];
+  const int X = sx.y, ns = P.nstrip;
+  const float* base = b.rpart + P.pp_off + (long long)X * ns * 6 * kTile;
+  for (int it = threadIdx.x; it < 6 * kTile; it += blockDim.x) {
+    const int c = it / kTile, loc = X * kTile + it % kTile;
+    if (loc >= P.ndip) continue;
+    const FF t = strip_sum<16>(base + it, ns, 6 * kTile);
+    b.rsum[(long long)c * b.ndtot + P.dip_off + loc] = make_float2(t.hi, t.lo);
   }
 }
 
@@ -828,8 +815,9 @@ void launch_near_pass(const Batch& b, cudaStream_t s) {
 }
 
 void launch_real_sum(const Batch& b, cudaStream_t s) {
-  if (b.ntiles == 0 || b.nblk == 0) return;
-  real_sum_kernel<<<b.nblk, b.tune.rsum_threads, 0, s>>>(b);
+  if (b.nbstrips) real_sum_kernel<<<b.nbstrips, b.tune.rsum_threads, 0, s>>>(b);
+}
+void launch_strip_energy(const Batch& b, cudaStream_t s) {
   if (b.nbstrips) strip_energy_kernel<<<cdiv(b.nbstrips, 4), 128, 0, s>>>(b);
 }
 

@@ -35,9 +35,11 @@ namespace mdsc {
 
 // Does the system build its list this step?  From the largest displacement
 // measure of the new configuration (particle_kernel), the same in every block.
+// A list asked for is built unless one was built at this very configuration:
+// the neighbour pass's lists also fix the order of its FP32 sums.
 __device__ __forceinline__ bool list_due(const Batch& b, const SysDev& P, const SysState& S, int s, int force_all) {
   if (at_limit(b, s)) return false;
-  return force_all || (S.force_list && !S.list_ok) || 2.0 * soft_f2d(__int_as_float(S.dmax)) > P.skin;
+  return force_all || (S.force_list && (!S.list_ok || S.dmax != 0)) || 2.0 * soft_f2d(__int_as_float(S.dmax)) > P.skin;
 }
 
 // cell of a fixed-point position: floor(fraction x cells), exact

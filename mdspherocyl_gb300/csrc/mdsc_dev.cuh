@@ -23,8 +23,12 @@ constexpr int kMaxD = 4;         // dipoles per particle (MDSC_MAX_DIPOLES)
 constexpr int kPartBlock = 128;  // threads per block of the per-particle kernels
 constexpr int kKBlock = 128;     // k-vectors per block of the k-space kernels
 constexpr int kKChunk = 256;     // particles per block of the structure-factor kernel
-// systems of more strips than this sum their real-space tile energies per
-// strip first (real_sum); smaller ones are summed tile by tile
+// Systems of more strips than this sum their tiles' partials and energies per
+// strip first (real_sum, strip_energy); in the others the force assembly adds
+// a dipole's partials and the per-system sums the tiles' energies.  With the
+// partials in a kernel of their own as well, one system of 256 rods took 45.8
+// us per step, without 43.5; 64 systems of 128 to 2048 rods 196 and 189, 192
+// systems 519 and 509; 4096 rods (64 strips) 102 and, in the assembly, 108.
 constexpr int kStripRows = 32;
 constexpr int kMaxR = 256;       // neighbour-pass list entries per rod (systems with a real-space cutoff)
 constexpr int kMaxE = 64;        // energy-criterion candidates (higher index) per rod
@@ -274,15 +278,16 @@ struct Batch {
   int2* ktile;   // (system, tile) of every k tile
   int nktile;
   double* kG;    // 6 per particle chunk: sum of m m^T (one dipole per particle)
+  int ones;      // systems of one dipole per particle
   int2* kgwork;  // (particle block, k tile or -1: all) of every k-space gather block
   int nkgwork;
   float* kgpart; // tile sums of split gathers: per (particle block, tile, dipole) 6 x kPartBlock
   int* kgdone;   // per particle block: tiles done this launch (the last one combines them)
   float2* Fk;    // 3 ndip: k-space force on each dipole, float-float (hi, lo)
   float2* Tk;    // 3 ndip: k-space torque m x G, float-float
-  // integrator partials, float-float, per row of 32 particles and component
-  float2* krow;  // 2: K_t, K_r after the first half kick
-  float2* krow2; // 5: K_t, K_r, two kinetic pressure terms, U_ext (finalize_kernel)
+  // integrator partials, float-float, per row of 32 particles (and component)
+  float2* krow;  // 2 per row: K_t, K_r after the first half kick
+  float2* krow2; // 4: K_t or K_r, two kinetic pressure terms, U_ext (finalize_kernel)
   float2* wrow;  // 4: WCA terms of the rods' own candidates (finalize_kernel)
   float* dmax;   // 1 per row: largest displacement measure since the last list build
   double* kin2;  // mdsc_moveP: 9 per particle block

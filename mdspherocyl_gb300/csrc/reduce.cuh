@@ -86,6 +86,30 @@ __device__ __forceinline__ FF ff_of(float x) {
   return r;
 }
 
+// The sum of n floats `stride` apart, in order, in float-float (a dipole's
+// real-space tile partials over its partner strips): hi + lo.  W loads at a
+// time; the ones past the end are zeros, which change nothing.
+template <int W>
+__device__ __forceinline__ FF strip_sum(const float* v, int n, long long stride) {
+  float hi = 0.f, lo = 0.f;
+  for (int k = 0; k < n; k += W) {
+    float x[W];
+#pragma unroll
+    for (int q = 0; q < W; ++q) x[q] = k + q < n ? v[(k + q) * stride] : 0.f;
+#pragma unroll
+    for (int q = 0; q < W; ++q) {
+      const float sum = hi + x[q];
+      const float bb = sum - hi;
+      lo += (hi - (sum - bb)) + (x[q] - bb);
+      hi = sum;
+    }
+  }
+  FF r;
+  r.hi = hi + lo;
+  r.lo = lo - (r.hi - hi);
+  return r;
+}
+
 // Per-block maximum of non-negative values.
 template <int NT>
 __device__ __forceinline__ float block_max(float v, float* sh) {

@@ -5,6 +5,7 @@ one k-vector per structure-factor thread) and those of a batch that fills the
 GPU give a system the same bits, and both agree with the oracle; so do the
 clusters, histograms and pictures.
 """
+import ctypes
 import math
 
 import numpy as np
@@ -81,6 +82,38 @@ def test_forces_against_the_oracle(systems, k):
             assert rms_rel(d["T"], o.T) <= TOL_F, name
             assert rms_rel(PT[0], PTo) <= TOL_F, name
             assert abs(U[0] - Uo) <= TOL_F * max(abs(Uo), np.abs(PTo).max()), name
+
+
+# ---- strips of 64 dipoles: a lone one, one dipole in the last, as many as the
+# force assembly adds by itself (32) and one more -----------------------------
+@pytest.mark.parametrize("n", [2, 64, 65, 2048, 2049])
+def test_real_space_strips_against_the_oracle(n):
+    """The batch's own sums over the strips and those of the call that holds no
+    GPU memory of its own."""
+    import torch
+
+    spec, st = _plain(n, 300 + n)
+    o = _osys(spec, st)
+    Uo, PTo = oracle.Oracle().force_dipR(o, spec.alpha)
+    with L.Batch([spec], [st]) as bt:
+        bt.zero_forces()
+        U, PT = bt.force_dipR()
+        d = bt.download(0)
+    pos, mom = (torch.tensor(x, dtype=torch.float64, device="cuda:0")
+                for x in (st.r, st.dip[:, 0, 4:5] * st.O[:, 2, :]))
+    F, T, UPT = (torch.zeros(k, dtype=torch.float64, device="cuda:0") for k in ((n, 3), (n, 3), (10,)))
+    box = (ctypes.c_double * 3)(*[float(x) for x in spec.box])
+    code = L.load().mdsc_force_dipR_noalloc(
+        n, *(ctypes.c_void_p(x.data_ptr()) for x in (pos, mom)), ctypes.cast(box, ctypes.POINTER(ctypes.c_double)),
+        float(spec.alpha), *(ctypes.c_void_p(x.data_ptr()) for x in (F, T, UPT)),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert code == 0
+    upt = UPT.cpu().numpy()
+    for f, t, u, pt in ((d["F"], d["T"], U[0], PT[0]), (F.cpu().numpy(), T.cpu().numpy(), upt[0], upt[1:].reshape(3, 3))):
+        assert rms_rel(f, o.F) <= TOL_F
+        assert rms_rel(t, o.T) <= TOL_F
+        assert rms_rel(pt, PTo) <= TOL_F
+        assert abs(u - Uo) <= TOL_F * max(abs(Uo), np.abs(PTo).max())
 
 
 # ---- clusters, histograms and pictures at the edges of their splits --------

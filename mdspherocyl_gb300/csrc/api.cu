@@ -78,7 +78,15 @@ constexpr int kTilesAfter = 4 * 152;
 // split, 24 systems of 128 to 2048 rods (140 blocks) 144 and 135; 64 systems
 // (400 blocks) 226 and 231, 256 systems 693 and 701 (the tiles' sums through
 // memory then cost more than the added blocks gain).
+// They also take the gather with one rod per thread until the autotuner has
+// chosen.
 constexpr int kGatherSplitMax = 300;
+// Where those batches have no system of more structure-factor chunks (256 rods
+// each) than this, the gathers total the chunks and form val S(k) as they
+// stage a k tile, and the kernel that does it for the energies runs beside
+// them: 256 rods 41.4 us per step with the kernel between, 39.5 without; 24
+// systems of up to 2048 rods (8 chunks) 95.7 with it and 100.
+constexpr int kStageChunks = 4;
 // the reference's table covers r <= 0.5 * 200.2 (v25/functions.cpp:1563,1681)
 constexpr double kTableRmax = 0.5 * 200 * 1.001;
 constexpr double kLh = 0.5 * (200 * 1.001) / 32768;
@@ -100,6 +108,7 @@ struct Layout {
   int smem_tn = 0;
   bool rp_table = false;      // the tiles interpolate in the table (MDSC_REAL_FORM=table)
   int ncellcap = 0;           // cells of capacity over all systems
+  int maxchunk = 0;           // structure-factor chunks of the largest system
   long long kgsets = 0;       // partial sets of the split gathers
   int ntot = 0, ndtot = 0, nktot = 0, maxnd = 0, nchunks = 0, nstrips = 0;
   bool any_rc = false;  // some system sums its real space over a neighbour list
@@ -342,6 +351,7 @@ void make_layout(const mdsc_system_desc* descs, int nsys, Layout& Lo) {
     }
     P.nk = (int)kn.size();
     P.nkchunk = P.nk > 0 ? cdiv(d.n, kKChunk) : 0;
+    Lo.maxchunk = std::max(Lo.maxchunk, P.nkchunk);
     P.kchunk_off = (int)kp;
     kp += (long long)P.nkchunk * P.nk;
     P.gch_off = Lo.nchunks;
@@ -509,7 +519,6 @@ void carve(Arena& A, const Layout& Lo, int nsys, Batch& b, int4** kwork, int2** 
   b.bstrips = A.take<int2>(std::max<size_t>(Lo.bstrips.size(), 1));
   b.kgwork = A.take<int2>(std::max<size_t>(Lo.kgwork.size(), 1));
   b.kgpart = A.take<float>(std::max<long long>(Lo.kgsets, 1) * kPartBlock * 6);
-  b.kgdone = A.take<int>(nb);
   b.rnb = A.take<int>(Lo.any_rc ? n * kMaxR : 1);
   b.rnbc = A.take<int>(n);
   b.rlE = A.take<double>(10 * nb);
@@ -820,7 +829,7 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
     launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, part, s);
   };
   kpart(0, B->s3);
-  kpart(1, B->s3);
+  if (!b.stage_k) kpart(1, B->s3);
   cudaEventRecord(B->ev_k, B->s3);
   kpart(2, B->s3);
   // what only the second half kick and the per-system sums read
@@ -831,6 +840,7 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   }
   launch_order_terms(b, B->s4);
   cudaStreamWaitEvent(B->s4, B->ev_k, 0);
+  if (b.stage_k) kpart(1, B->s4);
   kpart(3, B->s4);
   cudaStreamWaitEvent(B->s4, B->ev_tile, 0);
   launch_strip_energy(b, B->s4);
@@ -1267,6 +1277,8 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   carve(A, lo, nsys, B->b, &B->kwork, &B->kowner, B->noise, &B->d_skip);
   B->arena_bytes = A.off;
   B->b.tune.wca_blocks = 8 * B->num_sms;
+  B->b.tune.kg_scalar = (int)lo.blk.size() <= kGatherSplitMax;
+  B->b.stage_k = (int)lo.blk.size() <= kGatherSplitMax && lo.maxchunk <= kStageChunks;
   cudaError_t e = cudaMalloc(&B->arena, B->arena_bytes);
   if (e != cudaSuccess) {
     delete B;
@@ -1371,7 +1383,6 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   cudaMemsetAsync(b.stripE, 0, sizeof(double) * 10 * std::max(lo.nstrips, 1), B->st);
   cudaMemsetAsync(b.rnbc, 0, sizeof(int) * std::max(lo.ntot, 1), B->st);
   cudaMemsetAsync(b.ccnt, 0, sizeof(int) * std::max(lo.ncellcap, 1), B->st);
-  cudaMemsetAsync(b.kgdone, 0, sizeof(int) * std::max<size_t>(lo.blk.size(), 1), B->st);
   cudaMemsetAsync(b.rlE, 0, sizeof(double) * 10 * std::max<size_t>(lo.blk.size(), 1), B->st);
   cudaMemsetAsync(b.wrow, 0, sizeof(float2) * 12 * std::max<size_t>(lo.wblk.size(), 1), B->st);
   cudaMemsetAsync(b.F, 0, sizeof(double) * 3 * std::max(lo.ntot, 1), B->st);

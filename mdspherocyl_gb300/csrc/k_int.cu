@@ -322,8 +322,9 @@ __global__ void __launch_bounds__(128) xi_mid_kernel(Batch b) {
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   SysState& S = b.st[s];
-  const int nb = cdiv(P.nw, 4);
-  double K = 0.0;
+  const int nb = cdiv(P.nw, 4), c = threadIdx.x;
+  double K = 0.0, x1 = 0.0;
+  if (c < 2) x1 = P.ex1 * S.xi[c] + P.cnoise * b.noise[((long long)S.iter * b.nsys + s) * 4 + 2 * c];
   for (int b0 = 0; b0 < nb; b0 += 128) {
     const int blk = b0 + threadIdx.x;
     if (blk < nb) {
@@ -341,54 +342,90 @@ __global__ void __launch_bounds__(128) xi_mid_kernel(Batch b) {
       sh[1][threadIdx.x] = soft_f2d(r.hi) + soft_f2d(r.lo);
     }
     __syncthreads();
-    if (threadIdx.x < 2)
-      for (int k = 0; k < min(128, nb - b0); ++k) K += sh[threadIdx.x][k];
+    if (c < 2) {
+#pragma unroll 8
+      for (int k = 0; k < min(128, nb - b0); ++k) K += sh[c][k];
+    }
     __syncthreads();
   }
-  const int c = threadIdx.x;
   if (c >= 2) return;
   const double Kf = 0.5 * K;
-  const double* nz = b.noise + ((long long)S.iter * b.nsys + s) * 4;
-  const double x1 = P.ex1 * S.xi[c] + P.cnoise * nz[2 * c];
   S.K_first[c] = Kf;
   S.xi_mid[c] = x1 + P.dt * (2. * Kf - P.ntemp3) / P.Q;
 }
 
 // ---------------------------------------------------------------------
 // force assembly (+ ext_field) and optionally moveP(last): three lanes per
-// rod as above.  Each warp leaves its sums for the per-system reduction as
-// float-float rows: krow2 (K_t or K_r, two kinetic pressure terms, U_ext) and
-// wrow (the WCA terms a, a + 3, ... of U, W, PT of the rods' own pairs).
+// rod as above, twice.  Warps 3 to 5 add the WCA pairs' shares while warps 0
+// to 2 add the dipoles' real- and reciprocal-space parts and then, from both,
+// make the kick: a chain of dependent reads each (records by slot; partials by
+// tile), one behind the other 10.0 us a launch for 256 rods, side by side 6.9.
+// Each warp leaves its sums for the per-system reduction as float-float rows:
+// krow2 (K_t or K_r, two kinetic pressure terms, U_ext) and wrow (the WCA terms
+// a, a + 3, ... of U, W, PT of the rods' own pairs).
 // ---------------------------------------------------------------------
 constexpr int kKinCols = 4, kWcaCols = 4;
 // kinetic pressure terms of warp a: (xx, xy), (yy, yz), (zz, zx)
 
-__global__ void __launch_bounds__(kRowBlock) finalize_kernel(Batch b, int mode) {
-  __shared__ double sl[3][kRows];
-  __shared__ double sv[3][kRows];
+// warps 0 to 2 only
+__device__ __forceinline__ void sync_rows() { asm volatile("bar.sync 1, %0;" ::"n"(kRowBlock) : "memory"); }
+
+// k-space force and torque of dipole w (g) of rod i, component a, from the k
+// tiles' sums: the force, and the torque m x G of the second triple with the
+// FP32 moment, as the gather forms them where it walks all tiles.  Called by
+// all of warps 0 to 2.
+__device__ __forceinline__ void ktile_force(const Batch& b, const SysDev& P, FF (&sg)[3][kRows], int i, int g, int w,
+                                            int a, int lane, FF& kf, FF& kt) {
+  const int a1 = a == 2 ? 0 : a + 1, a2 = a == 0 ? 2 : a - 1;
+  const float* set = ktile_set(b, P, i, 0) + (w * 6 + a) * kPartBlock;
+  FF q[2];
+  ktile_sums<6>(set, P.nkt, P.nd * kSet, 3 * kPartBlock, P.kgs, q);
+  kf = q[0];
+  const float m1 = b.dm[a1 * b.ndtot + g], m2 = b.dm[a2 * b.ndtot + g];
+  sync_rows();
+  sg[a][lane] = q[1];
+  sync_rows();
+  kt = ff_cross(m1, sg[a2][lane], m2, sg[a1][lane]);
+}
+
+__global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int mode) {
+  __shared__ double sw[2][3][kRows];  // F, T with the WCA pairs' shares
+  __shared__ double sl[3][kRows], sv[3][kRows], sf[3][kRows];
   __shared__ float sp[3][kRows];
   __shared__ double sk[2][3][kRows];  // p; (O l)_a^2
+  __shared__ FF sg[3][kRows];
   const int2 bk = b.wblk[blockIdx.x];
   const int s = bk.x;
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   SysState& S = b.st[s];
-  const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (bk.y == P.part_off && threadIdx.x == 0) S.dmax = 0;  // the lists of this configuration stand
+  const bool pairs = threadIdx.x >= kRowBlock;  // the same for a warp
+  const int a = (threadIdx.x >> 5) - (pairs ? 3 : 0), lane = threadIdx.x & 31;
   const bool ok = bk.y + lane < P.part_off + P.n;
   const int i = ok ? bk.y + lane : bk.y;
   const int row = 3 * (P.w_off + (bk.y - P.part_off) / kRows) + a;
-  const int a1 = a == 2 ? 0 : a + 1, a2 = a == 0 ? 2 : a - 1;  // the cyclic next and previous component
-  double F = (mode & kFlagAccum) ? b.F[3 * i + a] : 0.0;
-  double T = (mode & kFlagAccum) ? b.T[3 * i + a] : 0.0;
-  if (mode & kMaskWca) {
+  if (pairs) {
+    if (bk.y == P.part_off && threadIdx.x == kRowBlock) S.dmax = 0;  // the lists of this configuration stand
+    double F = (mode & kFlagAccum) ? b.F[3 * i + a] : 0.0;
+    double T = (mode & kFlagAccum) ? b.T[3 * i + a] : 0.0;
     FF w[kWcaCols];
 #pragma unroll
     for (int c = 0; c < kWcaCols; ++c) w[c] = ff_of(0.f);
-    if (ok) {
+    if ((mode & kMaskWca) && ok) {
+      const int nc = b.wcnt[i];
+      const int nin = min(b.wincnt[i], kMaxC);
+      const int4* win = reinterpret_cast<const int4*>(b.win + (long long)i * kMaxC);
+      int v[kMaxC];
+#pragma unroll
+      for (int q = 0; q < kMaxC / 4; ++q) {
+        const int4 x = 4 * q < nin ? win[q] : make_int4(0, 0, 0, 0);
+        v[4 * q] = 4 * q < nin ? x.x : INT_MAX;
+        v[4 * q + 1] = 4 * q + 1 < nin ? x.y : INT_MAX;
+        v[4 * q + 2] = 4 * q + 2 < nin ? x.z : INT_MAX;
+        v[4 * q + 3] = 4 * q + 3 < nin ? x.w : INT_MAX;
+      }
       // its own shares of its candidate pairs (higher-index partners), in
       // slot order, as force_sc adds them
-      const int nc = b.wcnt[i];
       const double* own = b.wown + (long long)i * kMaxC * 6;
       const double* ev = b.wev + (long long)i * kMaxC * 11;
       for (int c = 0; c < nc; ++c) {
@@ -403,17 +440,6 @@ __global__ void __launch_bounds__(kRowBlock) finalize_kernel(Batch b, int mode) 
       // their slots here in arrival order; taken in ascending order the slots
       // ascend with the partner (slot = partner * kMaxC + c), the order
       // force_sc adds them.
-      const int nin = min(b.wincnt[i], kMaxC);
-      const int4* win = reinterpret_cast<const int4*>(b.win + (long long)i * kMaxC);
-      int v[kMaxC];
-#pragma unroll
-      for (int q = 0; q < kMaxC / 4; ++q) {
-        const int4 x = 4 * q < nin ? win[q] : make_int4(0, 0, 0, 0);
-        v[4 * q] = 4 * q < nin ? x.x : INT_MAX;
-        v[4 * q + 1] = 4 * q + 1 < nin ? x.y : INT_MAX;
-        v[4 * q + 2] = 4 * q + 2 < nin ? x.z : INT_MAX;
-        v[4 * q + 3] = 4 * q + 3 < nin ? x.w : INT_MAX;
-      }
       int last = -1;
       for (int k = 0; k < nin; ++k) {
         int m = INT_MAX;
@@ -425,99 +451,130 @@ __global__ void __launch_bounds__(kRowBlock) finalize_kernel(Batch b, int mode) 
         last = m;
       }
     }
+    sw[0][a][lane] = F;
+    sw[1][a][lane] = T;
+    __syncthreads();
+    if (mode & kMaskWca) {
 #pragma unroll
-    for (int c = 0; c < kWcaCols; ++c) {
-      w[c] = ff_warp_sum(w[c]);
-      if (lane == 0) b.wrow[kWcaCols * row + c] = make_float2(w[c].hi, w[c].lo);
+      for (int c = 0; c < kWcaCols; ++c) {
+        w[c] = ff_warp_sum(w[c]);
+        if (lane == 0) b.wrow[kWcaCols * row + c] = make_float2(w[c].hi, w[c].lo);
+      }
     }
+    return;
+  }
+  const int a1 = a == 2 ? 0 : a + 1, a2 = a == 0 ? 2 : a - 1;  // the cyclic next and previous component
+  const bool kick = mode & kFlagMoveP;
+  double p = 0.0, l = 0.0, im = 0.0, O[3] = {0.0, 0.0, 0.0};
+  if (kick) {  // asked for ahead of the forces
+    p = b.p[3 * i + a];
+    l = b.l[3 * i + a];
+    im = b.invm[i];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) O[c] = b.O[9 * i + 3 * a + c];
   }
   const int nd = P.nd;
   // the field term needs the FP64 moment; without a field it adds nothing
   const bool ext = (mode & kMaskExt) && (P.B[0] != 0.0 || P.B[1] != 0.0 || P.B[2] != 0.0);
-  double uext = 0.0;
-  for (int w = 0; w < nd; ++w) {
-    const int g = P.dip_off + (i - P.part_off) * nd + w;
-    // real- and reciprocal-space force and torque of this dipole in
-    // float-float (FP32 instructions), one conversion to FP64 at the end
-    FF qf = ff_of(0.f), qt = ff_of(0.f);
-    if (mode & kMaskReal) {
-      // this dipole's tile partials summed over all partner strips: here, or
-      // by real_sum_kernel (or near_pass_kernel) before
-      if (P.rc_real <= 0.0 && P.nstrip <= kStripRows) {
-        const int loc = g - P.dip_off;
-        const float* part = b.rpart + P.pp_off + ((long long)(loc / kTile) * P.nstrip * 6 + a) * kTile + loc % kTile;
-        qf = strip_sum<8>(part, P.nstrip, 6 * kTile);
-        qt = strip_sum<8>(part + 3 * kTile, P.nstrip, 6 * kTile);
-      } else {
-        const float2 x = b.rsum[(long long)a * b.ndtot + g], y = b.rsum[(long long)(3 + a) * b.ndtot + g];
-        qf = FF{x.x, x.y};
-        qt = FF{y.x, y.y};
+  double F = 0.0, T = 0.0, uext = 0.0;
+  for (int w = 0; w < max(nd, 1); ++w) {
+    double f = 0.0, t = 0.0;
+    if (w < nd) {
+      const int g = P.dip_off + (i - P.part_off) * nd + w;
+      const double pc = b.dpc[g];
+      // real- and reciprocal-space force and torque of this dipole in
+      // float-float (FP32 instructions), one conversion to FP64 at the end
+      FF qf = ff_of(0.f), qt = ff_of(0.f);
+      if (mode & kMaskReal) {
+        // this dipole's tile partials summed over all partner strips: here, or
+        // by real_sum_kernel (or near_pass_kernel) before
+        if (P.rc_real <= 0.0 && P.nstrip <= kStripRows) {
+          const int loc = g - P.dip_off;
+          const float* part = b.rpart + P.pp_off + ((long long)(loc / kTile) * P.nstrip * 6 + a) * kTile + loc % kTile;
+          FF q[2];
+          strip_sums<8>(part, P.nstrip, 6 * kTile, 3 * kTile, q);
+          qf = q[0];
+          qt = q[1];
+        } else {
+          const float2 x = b.rsum[(long long)a * b.ndtot + g], y = b.rsum[(long long)(3 + a) * b.ndtot + g];
+          qf = FF{x.x, x.y};
+          qt = FF{y.x, y.y};
+        }
       }
+      if (mode & kMaskK) {
+        FF kf, kt;
+        if (P.kgt > 1) {
+          ktile_force(b, P, sg, i, g, w, a, lane, kf, kt);
+        } else {
+          const float2 x = b.Fk[3 * g + a], y = b.Tk[3 * g + a];
+          kf = FF{x.x, x.y};
+          kt = FF{y.x, y.y};
+        }
+        qf = ff_add(qf, kf);
+        qt = ff_add(qt, kt);
+      }
+      f = soft_f2d(qf.hi) + soft_f2d(qf.lo);
+      t = soft_f2d(qt.hi) + soft_f2d(qt.lo);
+      if (ext) {
+        // ext_field: torque mu o x B, energy -mu o.B (v25/functions.cpp:2014-2020),
+        // with the dipole vector mu O^T o_body in FP64
+        const double* Oi = b.O + 9 * i;
+        const double m = b.dmu[g] * (Oi[a] * b.dob[3 * g] + Oi[3 + a] * b.dob[3 * g + 1] + Oi[6 + a] * b.dob[3 * g + 2]);
+        sync_rows();
+        sv[a][lane] = m;
+        sync_rows();
+        t += sv[a1][lane] * P.B[a2] - sv[a2][lane] * P.B[a1];
+        uext -= m * P.B[a];
+      }
+      // lever arm of an off-centre dipole: d x f (v25/classes.hpp:135-136)
+      sync_rows();
+      sf[a][lane] = f;
+      sync_rows();
+      if (pc != 0.0) t += pc * b.O[9 * i + 6 + a1] * sf[a2][lane] - pc * b.O[9 * i + 6 + a2] * sf[a1][lane];
     }
-    if (mode & kMaskK) {
-      const float2 x = b.Fk[3 * g + a], y = b.Tk[3 * g + a];
-      qf = ff_add(qf, FF{x.x, x.y});
-      qt = ff_add(qt, FF{y.x, y.y});
+    if (w == 0) {
+      __syncthreads();  // the pairs' shares come first
+      F = sw[0][a][lane];
+      T = sw[1][a][lane];
     }
-    const double f = soft_f2d(qf.hi) + soft_f2d(qf.lo);
-    double t = soft_f2d(qt.hi) + soft_f2d(qt.lo);
-    if (ext) {
-      // ext_field: torque mu o x B, energy -mu o.B (v25/functions.cpp:2014-2020),
-      // with the dipole vector mu O^T o_body in FP64
-      const double* O = b.O + 9 * i;
-      const double m = b.dmu[g] * (O[a] * b.dob[3 * g] + O[3 + a] * b.dob[3 * g + 1] + O[6 + a] * b.dob[3 * g + 2]);
-      __syncthreads();
-      sv[a][lane] = m;
-      __syncthreads();
-      t += sv[a1][lane] * P.B[a2] - sv[a2][lane] * P.B[a1];
-      uext -= m * P.B[a];
+    if (w < nd) {
+      F += f;
+      T += t;
     }
-    // lever arm of an off-centre dipole: d x f (v25/classes.hpp:135-136)
-    const double pc = b.dpc[g];
-    if (__syncthreads_or(pc != 0.0)) {
-      sv[a][lane] = f;
-      __syncthreads();
-      if (pc != 0.0)
-        t += pc * b.O[9 * i + 6 + a1] * sv[a2][lane] - pc * b.O[9 * i + 6 + a2] * sv[a1][lane];
-    }
-    F += f;
-    T += t;
   }
   // warp 0: K_t, warp 1: K_r; then two terms of the pressure tensor, U_ext
   FF k[kKinCols];
 #pragma unroll
   for (int c = 0; c < kKinCols; ++c) k[c] = ff_of(0.f);
   k[3] = ff_from(ok ? uext : 0.0);
-  if (mode & kFlagMoveP) {
+  if (ok) {
+    b.F[3 * i + a] = F;
+    b.T[3 * i + a] = T;
+  }
+  if (kick) {
     // moveP last half (v25/functions.cpp:2150-2173), with xi after moveTher
     // 0 and 1 (xi_mid_kernel)
     const double h = 0.5 * P.dt;
     // (the products' roundings written out: both kicks keep their last bits)
-    const double p = __fma_rn(b.p[3 * i + a], 1. - h * S.xi_mid[0], h * F);
-    const double l = __fma_rn(b.l[3 * i + a], 1. - h * S.xi_mid[1], h * T);
-    const double im = b.invm[i];
+    p = __fma_rn(p, 1. - h * S.xi_mid[0], h * F);
+    l = __fma_rn(l, 1. - h * S.xi_mid[1], h * T);
     sl[a][lane] = l;
     sp[a][lane] = soft_d2f_rn(p);
-    __syncthreads();
-    const double* O = b.O + 9 * i + 3 * a;
-    const double lb = O[0] * sl[0][lane] + O[1] * sl[1][lane] + O[2] * sl[2][lane];
     sk[0][a][lane] = p;
+    sync_rows();
+    const double lb = O[0] * sl[0][lane] + O[1] * sl[1][lane] + O[2] * sl[2][lane];
     sk[1][a][lane] = lb * lb;
-    __syncthreads();
     if (ok) {
       b.p[3 * i + a] = p;
       b.l[3 * i + a] = l;
       if (a == 0) k[0] = ff_from(kin_t(sk[0], lane, im));
-      if (a == 1) k[0] = ff_from(kin_r(b, sk[1], lane, i));
       // kinetic pressure tensor p_a p_b / m: FP32 products, float-float sums
       const float imf = soft_d2f_rn(im), pf = sp[a][lane];
       k[1] = ff_of(pf * pf * imf);
       k[2] = ff_of(pf * sp[a1][lane] * imf);
     }
-  }
-  if (ok) {
-    b.F[3 * i + a] = F;
-    b.T[3 * i + a] = T;
+    sync_rows();
+    if (ok && a == 1) k[0] = ff_from(kin_r(b, sk[1], lane, i));
   }
 #pragma unroll
   for (int c = 0; c < kKinCols; ++c) {
@@ -810,7 +867,7 @@ void launch_xi_mid(const Batch& b, cudaStream_t s) {
   if (b.nsys) xi_mid_kernel<<<b.nsys, 128, 0, s>>>(b);
 }
 void launch_finalize(const Batch& b, int mode, cudaStream_t s) {
-  if (b.nwblk) finalize_kernel<<<b.nwblk, kRowBlock, 0, s>>>(b, mode);
+  if (b.nwblk) finalize_kernel<<<b.nwblk, 2 * kRowBlock, 0, s>>>(b, mode);
 }
 void launch_order_terms(const Batch& b, cudaStream_t s) {
   if (b.nblk) order_terms_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);

@@ -291,13 +291,48 @@ static void launch_ksum(const Batch& b, const int4* kwork, int nkwork, cudaStrea
   if constexpr (ND > 1) ksum_kernel<ND><<<nkwork, kKBlock, 0, s>>>(b, kwork);
 }
 
+// The totals of NC components of a system's k-vector, c0, c0 + 1, ..., over the
+// chunks, in chunk order (float-float; W loads of each in flight): the gathers'
+// input keeps one order of its sums.
+template <int W, int NC>
+__device__ __forceinline__ void ksum_totals(const Batch& b, const SysDev& P, int kl, int c0, int nv, double (&s)[NC]) {
+  const float* in = ksum_part(b, P, 0, nv) + (long long)c0 * P.nk + kl;
+  FF sf[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) sf[c] = ff_of(0.f);
+  for (int ch = 0; ch < P.nkchunk; ch += W) {
+    float x[W][NC];
+#pragma unroll
+    for (int q = 0; q < W; ++q)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) x[q][c] = ch + q < P.nkchunk ? in[((long long)(ch + q) * nv + c) * P.nk] : 0.f;
+#pragma unroll
+    for (int q = 0; q < W; ++q)
+      if (ch + q < P.nkchunk) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) sf[c] = ff_add(sf[c], ff_of(x[q][c]));
+      }
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) s[c] = soft_f2d(sf[c].hi) + soft_f2d(sf[c].lo);
+}
+
+// val S(k) from the six totals (the roundings written out: two kernels form it)
+__device__ __forceinline__ float2 val_S(const Batch& b, long long k, const double (&s)[6]) {
+  const double kx = b.kvec[3 * k], ky = b.kvec[3 * k + 1], kz = b.kvec[3 * k + 2];
+  const double val = b.kval[k];
+  const double Sr = __fma_rn(kz, s[4], __fma_rn(kx, s[0], __dmul_rn(ky, s[2])));
+  const double Si = __fma_rn(kz, s[5], __fma_rn(kx, s[1], __dmul_rn(ky, s[3])));
+  return make_float2(soft_d2f_rn(val * Sr), soft_d2f_rn(val * Si));
+}
+
 // Chunk sums per k and val S(k): all the gather needs, nothing more.  A block
-// takes 32 consecutive k-vectors of the batch; warp w sums components w, w +
-// kStructWarps, ... over the chunks, in chunk order (float-float; sixteen
-// loads in flight), and warp 0 forms val S(k): the gathers' input keeps one
-// order of its sums.
+// takes 32 consecutive k-vectors of the batch; warp w totals components w, w +
+// kStructWarps, ..., and warp 0 forms val S(k).  Five blocks an SM: with 128
+// registers a thread its blocks waited for the tiles of 4096 rods to leave, 15
+// us of the 82 of a step.
 constexpr int kStructWarps = 6;
-__global__ void __launch_bounds__(32 * kStructWarps) kstruct_kernel(Batch b, const int2* __restrict__ kowner) {
+__global__ void __launch_bounds__(32 * kStructWarps, 5) kstruct_kernel(Batch b, const int2* __restrict__ kowner) {
   __shared__ double sh[6][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
@@ -308,20 +343,10 @@ __global__ void __launch_bounds__(32 * kStructWarps) kstruct_kernel(Batch b, con
   const int nv = P.nd == 1 ? 6 : 10;
   if (on) {
     for (int c = w; c < nv; c += kStructWarps) {
-      const float* in = ksum_part(b, P, 0, nv) + (long long)c * P.nk + ow.y;
-      const long long stride = (long long)nv * P.nk;
-      FF sf = ff_of(0.f);
-      for (int ch = 0; ch < P.nkchunk; ch += 16) {
-        float x[16];
-#pragma unroll
-        for (int q = 0; q < 16; ++q) x[q] = ch + q < P.nkchunk ? in[(ch + q) * stride] : 0.f;
-#pragma unroll
-        for (int q = 0; q < 16; ++q)
-          if (ch + q < P.nkchunk) sf = ff_add(sf, ff_of(x[q]));
-      }
-      const double s = soft_f2d(sf.hi) + soft_f2d(sf.lo);
-      b.ksum[(long long)k * 10 + c] = s;
-      if (c < 6) sh[c][lane] = s;
+      double s[1];
+      ksum_totals<8>(b, P, ow.y, c, nv, s);
+      b.ksum[(long long)k * 10 + c] = s[0];
+      if (c < 6) sh[c][lane] = s[0];
     }
   }
   __syncthreads();
@@ -329,11 +354,7 @@ __global__ void __launch_bounds__(32 * kStructWarps) kstruct_kernel(Batch b, con
   double s[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) s[c] = sh[c][lane];
-  const double kx = b.kvec[3 * k], ky = b.kvec[3 * k + 1], kz = b.kvec[3 * k + 2];
-  const double val = b.kval[k];
-  const double Sr = kx * s[0] + ky * s[2] + kz * s[4];
-  const double Si = kx * s[1] + ky * s[3] + kz * s[5];
-  b.kS[k] = make_float2(soft_d2f_rn(val * Sr), soft_d2f_rn(val * Si));
+  b.kS[k] = val_S(b, k, s);
 }
 
 // Energy and pressure tensor of one k tile (v25/functions.cpp:1839-1952),
@@ -415,11 +436,13 @@ __device__ __forceinline__ void store_kout(const Batch& b, int g, const float* f
                                            float mx, float my, float mz) {
 #pragma unroll
   for (int c = 0; c < 3; ++c) b.Fk[3 * g + c] = make_float2(fo[c], -fc[c]);
-  const float gx = fo[3], gy = fo[4], gz = fo[5];
-  const float lx = -fc[3], ly = -fc[4], lz = -fc[5];
-  b.Tk[3 * g + 0] = make_float2(my * gz - mz * gy, my * lz - mz * ly);
-  b.Tk[3 * g + 1] = make_float2(mz * gx - mx * gz, mz * lx - mx * lz);
-  b.Tk[3 * g + 2] = make_float2(mx * gy - my * gx, mx * ly - my * lx);
+  const FF G[3] = {{fo[3], -fc[3]}, {fo[4], -fc[4]}, {fo[5], -fc[5]}};
+  const float m[3] = {mx, my, mz};
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const FF t = ff_cross(m[(c + 1) % 3], G[(c + 2) % 3], m[(c + 2) % 3], G[(c + 1) % 3]);
+    b.Tk[3 * g + c] = make_float2(t.hi, t.lo);
+  }
 }
 
 // The gathers: per particle over all k of its system, force and torque
@@ -427,77 +450,14 @@ __device__ __forceinline__ void store_kout(const Batch& b, int g, const float* f
 // order (Kahan), and a system of SysDev::kgs > 1 parts adds its parts'
 // sums the same way -- the order of every addition is the system's own.
 //
-// The work of one particle block goes to one block (it walks every tile) or
-// to one block per tile (SysDev::kgt > 1): each leaves its tile's sums in the
-// partial set of (particle block, tile) and the block that finishes last
-// adds the tiles, in the same order, so the bits are the same either way and
-// whichever block ends last.
-constexpr int kSet = kPartBlock * 6;  // floats of a partial set per dipole: 6 components x kPartBlock particles
-__device__ __forceinline__ float* ktile_set(const Batch& b, const SysDev& P, int slot, int tile) {
-  const long long tiles = cdiv(P.nk, kKBlock);
-  return b.kgpart + ((long long)P.kgp_off + ((slot - P.blk_off) * tiles + tile) * P.nd) * kSet;
-}
-
-// one Kahan addition: (fo, fc) += v
-__device__ __forceinline__ void kahan(float& fo, float& fc, float v) {
-  const float y = __fadd_rn(v, -fc);
-  const float t = __fadd_rn(fo, y);
-  fc = __fadd_rn(__fadd_rn(t, -fo), -y);
-  fo = t;
-}
-
-// the tile sums of local particle p, dipole d, in the order described above
-__device__ __forceinline__ void ktile_combine(const Batch& b, const SysDev& P, int slot, int p, int d, float* fo,
-                                              float* fc) {
-  const int tiles = cdiv(P.nk, kKBlock), tpk = cdiv(tiles, P.kgs);
-  float cs[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) fo[c] = fc[c] = cs[c] = 0.f;
-  for (int q = 0; q < P.kgs; ++q) {
-    float po[6], pc[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) po[c] = pc[c] = 0.f;
-    const int t1 = min(tiles, (q + 1) * tpk);
-#pragma unroll 4
-    for (int t = q * tpk; t < t1; ++t) {
-      const float* set = ktile_set(b, P, slot, t) + d * kSet + p;
-#pragma unroll
-      for (int c = 0; c < 6; ++c) kahan(po[c], pc[c], __ldcg(set + c * kPartBlock));
-    }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      if (P.kgs == 1) {
-        fo[c] = po[c];
-        fc[c] = pc[c];
-      } else {
-        kahan(fo[c], fc[c], po[c]);
-        cs[c] = __fadd_rn(cs[c], pc[c]);
-      }
-    }
-  }
-  if (P.kgs > 1) {
-#pragma unroll
-    for (int c = 0; c < 6; ++c) fc[c] = __fadd_rn(fc[c], cs[c]);
-  }
-}
-
-// Counts a tile of a particle block done; true for every thread of the block
-// that finishes last, which then sees every other block's sums (each thread
-// fences its own before the count, and again after it).
-__device__ __forceinline__ bool ktile_last(const Batch& b, const SysDev& P, int slot, int* last) {
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int tiles = cdiv(P.nk, kKBlock);
-    *last = atomicAdd(&b.kgdone[slot], 1) == tiles - 1;
-    if (*last) b.kgdone[slot] = 0;
-  }
-  __syncthreads();
-  if (!*last) return false;
-  __threadfence();
-  return true;
-}
-
+// The work of one particle block goes to one block (it walks every tile and
+// leaves force and torque, store_kout) or to one block per tile (SysDev::kgt >
+// 1): each leaves its tile's sums in the partial set of (particle block, tile)
+// and the force assembly adds the tiles, in the same order (ktile_sums).  The
+// block that finished last added them before: with the fences, the count and
+// one thread per rod for all six sums, 14.5 us a launch for 256 rods in the
+// step and 23 for 4096 with 9 tiles; one thread per rod and waves ahead as well
+// as this, 6.3 and 9.5.
 // the k-vectors of a work item: tile wk.y, or all of them (wk.y < 0)
 __device__ __forceinline__ void ktile_range(const SysDev& P, int2 wk, int& kb, int& ke) {
   kb = wk.y < 0 ? 0 : wk.y * kKBlock;
@@ -508,7 +468,6 @@ struct KTile {
   int4 n[kKBlock];
   float4 v[kKBlock];  // kx, ky, kz, val
   float2 S[kKBlock];  // val * S(k)
-  int last;
 };
 template <int NT>
 __device__ __forceinline__ int stage_ktile(const Batch& b, const SysDev& P, int k0, int ke, KTile& kt) {
@@ -517,7 +476,13 @@ __device__ __forceinline__ int stage_ktile(const Batch& b, const SysDev& P, int 
   for (int q = threadIdx.x; q < nk; q += NT) {
     kt.n[q] = b.kn[P.k_off + k0 + q];
     kt.v[q] = b.kv[P.k_off + k0 + q];
-    kt.S[q] = b.kS[P.k_off + k0 + q];
+    if (b.stage_k) {
+      double s[6];
+      ksum_totals<4>(b, P, k0 + q, 0, P.nd == 1 ? 6 : 10, s);
+      kt.S[q] = val_S(b, P.k_off + k0 + q, s);
+    } else {
+      kt.S[q] = b.kS[P.k_off + k0 + q];
+    }
   }
   __syncthreads();
   return nk;
@@ -609,21 +574,17 @@ __global__ void __launch_bounds__(kPartBlock) kgather_kernel(Batch b) {
 #pragma unroll
       for (int c = 0; c < 6; ++c) kahan(fo[d][c], fc[d][c], ft[d][c]);
   }
-  if (wk.y >= 0) {  // one tile: leave its sums, the last block combines
-    const int slot = blk_slot(P, bk);
-    float* mine = ktile_set(b, P, slot, wk.y) + threadIdx.x;
+  if (!ok) return;
+  if (wk.y >= 0) {  // one tile: leave its sums
+    float* mine = ktile_set(b, P, i, wk.y);
 #pragma unroll
     for (int d = 0; d < ND; ++d)
       if (d < nd) {
 #pragma unroll
         for (int c = 0; c < 6; ++c) mine[d * kSet + c * kPartBlock] = ft[d][c];
       }
-    if (!ktile_last(b, P, slot, &kt.last)) return;
-#pragma unroll
-    for (int d = 0; d < ND; ++d)
-      if (d < nd) ktile_combine(b, P, slot, threadIdx.x, d, fo[d], fc[d]);
+    return;
   }
-  if (!ok) return;
 #pragma unroll
   for (int d = 0; d < ND; ++d)
     if (d < nd) store_kout(b, gd0 + d, fo[d], fc[d], mx[d], my[d], mz[d]);
@@ -706,26 +667,22 @@ __global__ void __launch_bounds__(kPartBlock / 2) kgather1_kernel(Batch b) {
       fo[c] = tt;
     }
   }
+  if (wk.y >= 0) {  // one tile: leave its sums
+    float *s0 = ktile_set(b, P, i0, wk.y), *s1 = s0 + kPartBlock / 2;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+      if (ok0) s0[c * kPartBlock] = ft[c].x;
+      if (ok1) s1[c * kPartBlock] = ft[c].y;
+    }
+    return;
+  }
   float a0[6], c0[6], a1[6], c1[6];
-  if (wk.y >= 0) {  // one tile: leave its sums, the last block combines
-    const int slot = blk_slot(P, bk);
-    float* mine = ktile_set(b, P, slot, wk.y) + t;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      mine[c * kPartBlock] = ft[c].x;
-      mine[c * kPartBlock + kPartBlock / 2] = ft[c].y;
-    }
-    if (!ktile_last(b, P, slot, &kt.last)) return;
-    ktile_combine(b, P, slot, t, 0, a0, c0);
-    ktile_combine(b, P, slot, t + kPartBlock / 2, 0, a1, c1);
-  } else {
-#pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      a0[c] = fo[c].x;
-      c0[c] = fc[c].x;
-      a1[c] = fo[c].y;
-      c1[c] = fc[c].y;
-    }
+  for (int c = 0; c < 6; ++c) {
+    a0[c] = fo[c].x;
+    c0[c] = fc[c].x;
+    a1[c] = fo[c].y;
+    c1[c] = fc[c].y;
   }
   if (ok0) store_kout(b, g0, a0, c0, mx.x, my.x, mz.x);
   if (ok1) store_kout(b, g1, a1, c1, mx.y, my.y, mz.y);
@@ -735,7 +692,11 @@ __global__ void __launch_bounds__(kPartBlock / 2) kgather1_kernel(Batch b) {
 // twice the warps of the packed form and no paired instructions.  Every
 // particle goes through the same IEEE operations in the same order as in
 // the packed kernel (explicit _rn intrinsics, no contraction), so the two
-// forms give identical bits and the autotuner may pick either.
+// forms give identical bits and the autotuner may pick either.  kWavesAhead
+// waves are formed before their sums: in the small batches this form is for, a
+// warp often has its scheduler to itself and a k-vector's chain (phase, sine,
+// four dependent multiply-adds) would be the time.
+constexpr int kWavesAhead = 8;
 __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
   __shared__ KTile kt;
   const int2 wk = b.kgwork[blockIdx.x];  // (particle block, tile)
@@ -755,21 +716,13 @@ __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
   float fo[6], fc[6], ft[6];
 #pragma unroll
   for (int c = 0; c < 6; ++c) fo[c] = fc[c] = ft[c] = 0.f;
-  uint32_t ph = 0u;
-  bool have = false;
   for (int k0 = kb; k0 < ke; k0 += kKBlock) {
     const int nk = stage_ktile<kPartBlock>(b, P, k0, ke, kt);
 #pragma unroll
     for (int c = 0; c < 6; ++c) ft[c] = 0.f;
-#pragma unroll 4
-    for (int q = 0; q < nk; ++q) {
-      const int4 n = kt.n[q];
+    auto add = [&](int q, float c, float sn) {
       const float4 kv = kt.v[q];
       const float2 vS = kt.S[q];
-      float c, sn;
-      ph = phase_next(ph, have, ux0, uy0, uz0, n);
-      have = true;
-      phase_cs(ph, c, sn);
       const float a = __fmaf_rn(mz, kv.z, __fmaf_rn(my, kv.y, __fmul_rn(mx, kv.x)));
       const float va = __fmul_rn(kv.w, a);
       const float Dr = __fmaf_rn(-va, c, vS.x);
@@ -782,19 +735,33 @@ __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
       ft[3] = __fmaf_rn(fT, kv.x, ft[3]);
       ft[4] = __fmaf_rn(fT, kv.y, ft[4]);
       ft[5] = __fmaf_rn(fT, kv.z, ft[5]);
+    };
+    int q0 = 0;
+#pragma unroll 1
+    for (; q0 + kWavesAhead <= nk; q0 += kWavesAhead) {
+      float c[kWavesAhead], sn[kWavesAhead];
+#pragma unroll
+      for (int q = 0; q < kWavesAhead; ++q) phase_exp(ux0, uy0, uz0, kt.n[q0 + q], c[q], sn[q]);
+#pragma unroll
+      for (int q = 0; q < kWavesAhead; ++q) add(q0 + q, c[q], sn[q]);
+    }
+#pragma unroll 1
+    for (; q0 < nk; ++q0) {
+      float c, sn;
+      phase_exp(ux0, uy0, uz0, kt.n[q0], c, sn);
+      add(q0, c, sn);
     }
 #pragma unroll
     for (int c = 0; c < 6; ++c) kahan(fo[c], fc[c], ft[c]);
   }
-  if (wk.y >= 0) {  // one tile: leave its sums, the last block combines
-    const int slot = blk_slot(P, bk);
-    float* mine = ktile_set(b, P, slot, wk.y) + t;
+  if (!ok0) return;
+  if (wk.y >= 0) {  // one tile: leave its sums
+    float* mine = ktile_set(b, P, i0, wk.y);
 #pragma unroll
     for (int c = 0; c < 6; ++c) mine[c * kPartBlock] = ft[c];
-    if (!ktile_last(b, P, slot, &kt.last)) return;
-    ktile_combine(b, P, slot, t, 0, fo, fc);
+    return;
   }
-  if (ok0) store_kout(b, g0, fo, fc, mx, my, mz);
+  store_kout(b, g0, fo, fc, mx, my, mz);
 }
 
 template <int ND>

@@ -775,8 +775,9 @@ __global__ void __launch_bounds__(512) real_sum_kernel(Batch b) {
   for (int it = threadIdx.x; it < 6 * kTile; it += blockDim.x) {
     const int c = it / kTile, loc = X * kTile + it % kTile;
     if (loc >= P.ndip) continue;
-    const FF t = strip_sum<16>(base + it, ns, 6 * kTile);
-    b.rsum[(long long)c * b.ndtot + P.dip_off + loc] = make_float2(t.hi, t.lo);
+    FF t[1];
+    strip_sums<16>(base + it, ns, 6 * kTile, 0, t);
+    b.rsum[(long long)c * b.ndtot + P.dip_off + loc] = make_float2(t[0].hi, t[0].lo);
   }
 }
 

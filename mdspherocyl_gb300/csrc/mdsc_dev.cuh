@@ -28,7 +28,8 @@ constexpr int kKChunk = 256;     // particles per block of the structure-factor 
 // a dipole's partials and the per-system sums the tiles' energies.  With the
 // partials in a kernel of their own as well, one system of 256 rods took 45.8
 // us per step, without 43.5; 64 systems of 128 to 2048 rods 196 and 189, 192
-// systems 519 and 509; 4096 rods (64 strips) 102 and, in the assembly, 108.
+// systems 519 and 509; 1500 rods of two dipoles (47 strips) 80.4 and, in the
+// assembly, 82.0; 4096 rods (64 strips) 81 either way.
 constexpr int kStripRows = 32;
 constexpr int kMaxR = 256;       // neighbour-pass list entries per rod (systems with a real-space cutoff)
 constexpr int kMaxE = 64;        // energy-criterion candidates (higher index) per rod
@@ -281,8 +282,8 @@ struct Batch {
   int ones;      // systems of one dipole per particle
   int2* kgwork;  // (particle block, k tile or -1: all) of every k-space gather block
   int nkgwork;
-  float* kgpart; // tile sums of split gathers: per (particle block, tile, dipole) 6 x kPartBlock
-  int* kgdone;   // per particle block: tiles done this launch (the last one combines them)
+  int stage_k;   // the gathers form val S(k) themselves (kStageChunks)
+  float* kgpart; // tile sums of split gathers: per (particle block, tile, dipole) 6 x kPartBlock (ktile_set)
   float2* Fk;    // 3 ndip: k-space force on each dipole, float-float (hi, lo)
   float2* Tk;    // 3 ndip: k-space torque m x G, float-float
   // integrator partials, float-float, per row of 32 particles (and component)
@@ -353,6 +354,15 @@ __device__ inline uint32_t to_fix(double x, double invL32) {
 // at blk_off .. blk_off + nblk - 1
 __device__ __forceinline__ int blk_slot(const SysDev& P, int2 bk) {
   return P.blk_off + (bk.y - P.part_off) / kPartBlock;
+}
+
+// k-space sums of particle i over one k tile, its first dipole's: 6 components
+// kPartBlock apart, dipoles kSet apart, the next tile's nd * kSet on
+constexpr int kSet = kPartBlock * 6;
+__device__ __forceinline__ float* ktile_set(const Batch& b, const SysDev& P, int i, int tile) {
+  const int loc = i - P.part_off;
+  return b.kgpart + ((long long)P.kgp_off + ((long long)(loc / kPartBlock) * P.nkt + tile) * P.nd) * kSet +
+         loc % kPartBlock;
 }
 
 // minimum-image difference of two fixed-point coordinates, in length units

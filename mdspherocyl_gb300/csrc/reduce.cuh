@@ -86,28 +86,92 @@ __device__ __forceinline__ FF ff_of(float x) {
   return r;
 }
 
-// The sum of n floats `stride` apart, in order, in float-float (a dipole's
-// real-space tile partials over its partner strips): hi + lo.  W loads at a
-// time; the ones past the end are zeros, which change nothing.
-template <int W>
-__device__ __forceinline__ FF strip_sum(const float* v, int n, long long stride) {
-  float hi = 0.f, lo = 0.f;
+// NS sums of n floats `stride` apart, in order, in float-float (a dipole's
+// real-space tile partials over its partner strips): hi + lo; the sums' floats
+// are `next` apart.  W loads of each at a time; the ones past the end are zeros,
+// which change nothing.
+template <int W, int NS>
+__device__ __forceinline__ void strip_sums(const float* v, int n, long long stride, int next, FF (&out)[NS]) {
+  float hi[NS], lo[NS];
+#pragma unroll
+  for (int c = 0; c < NS; ++c) hi[c] = lo[c] = 0.f;
   for (int k = 0; k < n; k += W) {
-    float x[W];
+    float x[W][NS];
 #pragma unroll
-    for (int q = 0; q < W; ++q) x[q] = k + q < n ? v[(k + q) * stride] : 0.f;
+    for (int q = 0; q < W; ++q)
 #pragma unroll
-    for (int q = 0; q < W; ++q) {
-      const float sum = hi + x[q];
-      const float bb = sum - hi;
-      lo += (hi - (sum - bb)) + (x[q] - bb);
-      hi = sum;
-    }
+      for (int c = 0; c < NS; ++c) x[q][c] = k + q < n ? v[(k + q) * stride + c * next] : 0.f;
+#pragma unroll
+    for (int q = 0; q < W; ++q)
+#pragma unroll
+      for (int c = 0; c < NS; ++c) {
+        const float sum = hi[c] + x[q][c];
+        const float bb = sum - hi[c];
+        lo[c] += (hi[c] - (sum - bb)) + (x[q][c] - bb);
+        hi[c] = sum;
+      }
   }
-  FF r;
-  r.hi = hi + lo;
-  r.lo = lo - (r.hi - hi);
-  return r;
+#pragma unroll
+  for (int c = 0; c < NS; ++c) {
+    out[c].hi = hi[c] + lo[c];
+    out[c].lo = lo[c] - (out[c].hi - hi[c]);
+  }
+}
+
+// m1 g2 - m2 g1, one component of a cross product with FP32 factors, high and
+// low parts (the roundings written out: two kernels form it)
+__device__ __forceinline__ FF ff_cross(float m1, FF g2, float m2, FF g1) {
+  return FF{__fmaf_rn(m1, g2.hi, -__fmul_rn(m2, g1.hi)), __fmaf_rn(-m2, g1.lo, __fmul_rn(m1, g2.lo))};
+}
+
+// one Kahan addition: (fo, fc) += v
+__device__ __forceinline__ void kahan(float& fo, float& fc, float v) {
+  const float y = __fadd_rn(v, -fc);
+  const float t = __fadd_rn(fo, y);
+  fc = __fadd_rn(__fadd_rn(t, -fo), -y);
+  fo = t;
+}
+
+// NS sums of n k tiles' sums `stride` apart in order, added in `parts` parts and
+// the parts the same way: fo - fc; the sums' floats are `next` apart.  W loads of
+// each at a time in flight.
+template <int W, int NS>
+__device__ __forceinline__ void ktile_sums(const float* in, int n, int stride, int next, int parts, FF (&out)[NS]) {
+  const int per = parts == 1 ? n : (n + parts - 1) / parts;
+  float po[NS], pc[NS], fo[NS], fc[NS], cs[NS];
+#pragma unroll
+  for (int c = 0; c < NS; ++c) po[c] = pc[c] = fo[c] = fc[c] = cs[c] = 0.f;
+  auto close = [&] {  // a part ends
+#pragma unroll
+    for (int c = 0; c < NS; ++c) {
+      kahan(fo[c], fc[c], po[c]);
+      cs[c] = __fadd_rn(cs[c], pc[c]);
+      po[c] = pc[c] = 0.f;
+    }
+  };
+  int in_part = 0, done = 0;
+  for (int t0 = 0; t0 < n; t0 += W) {
+    float v[W][NS];
+#pragma unroll
+    for (int q = 0; q < W; ++q)
+#pragma unroll
+      for (int c = 0; c < NS; ++c) v[q][c] = t0 + q < n ? in[(long long)(t0 + q) * stride + c * next] : 0.f;
+#pragma unroll
+    for (int q = 0; q < W; ++q)
+      if (t0 + q < n) {
+#pragma unroll
+        for (int c = 0; c < NS; ++c) kahan(po[c], pc[c], v[q][c]);
+        if (parts > 1 && ++in_part == per) {
+          close();
+          in_part = 0;
+          ++done;
+        }
+      }
+  }
+  if (parts > 1)
+    for (; done < parts; ++done) close();  // the last part if it is not full, and empty ones
+#pragma unroll
+  for (int c = 0; c < NS; ++c) out[c] = parts == 1 ? FF{po[c], -pc[c]} : FF{fo[c], -__fadd_rn(fc[c], cs[c])};
 }
 
 // Per-block maximum of non-negative values.

@@ -81,6 +81,14 @@ constexpr int kTilesAfter = 4 * 152;
 // They also take the gather with one rod per thread until the autotuner has
 // chosen.
 constexpr int kGatherSplitMax = 300;
+// Batches of at most this many particle blocks form the sums (ksum_split) and
+// the gather (kgather_split) of systems of several dipoles per rod by several
+// warps per walk, which costs the tiles' kernel what it gains where the tiles
+// are the longer chain.  Two dipoles per rod, us per step with neither, the
+// sums and both: 700 rods (6 blocks) 68.1, 53.8, 49.7; 1500 (12) 78.4, 65.2,
+// 66.1; 2048 (16) 85.2, 84.6, 86.3; 4096 (32) 186, 190, 191; 8 systems (64) 131,
+// 135, 136.
+constexpr int kSumSplitMax = 15, kGatherNdSplitMax = 8;
 // Where those batches have no system of more structure-factor chunks (256 rods
 // each) than this, the gathers total the chunks and form val S(k) as they
 // stage a k tile, and the kernel that does it for the energies runs beside
@@ -1278,6 +1286,8 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   B->arena_bytes = A.off;
   B->b.tune.wca_blocks = 8 * B->num_sms;
   B->b.tune.kg_scalar = (int)lo.blk.size() <= kGatherSplitMax;
+  B->b.sum_split = (int)lo.blk.size() <= kSumSplitMax;
+  B->b.gather_split = (int)lo.blk.size() <= kGatherNdSplitMax;
   B->b.stage_k = (int)lo.blk.size() <= kGatherSplitMax && lo.maxchunk <= kStageChunks;
   cudaError_t e = cudaMalloc(&B->arena, B->arena_bytes);
   if (e != cudaSuccess) {

@@ -154,6 +154,87 @@ __global__ void __launch_bounds__(kKBlock) ksum_kernel(Batch b, const int4* __re
   for (int c = 0; c < 10; ++c) out[(long long)c * P.nk] = acc[c];
 }
 
+// The same sums for batches that leave SMs idle: a block takes 32 k-vectors of
+// a work item, its ten warps the particles in turn -- each forms one particle's
+// sums over its dipoles and leaves them in shared memory -- and then each warp
+// adds one of the ten components over those particles, in particle order, so
+// every sum keeps its order.  One thread's walk over the chunk was the time:
+// 1500 rods of two dipoles (24 work items) 39 us a launch beside the tiles, 13
+// this way.
+constexpr int kSumWarps = 10;
+constexpr int kSumTerms = 8;  // U (3 real and imaginary pairs), S
+template <int ND>
+__global__ void __launch_bounds__(32 * kSumWarps) ksum_split_kernel(Batch b, const int4* __restrict__ kwork) {
+  __shared__ uint32_t sx[kKChunk * ND], sy[kKChunk * ND], sz[kKChunk * ND];
+  __shared__ float smx[kKChunk * ND], smy[kKChunk * ND], smz[kKChunk * ND];
+  __shared__ float term[2][kSumWarps][kSumTerms][32];
+  const int4 wk = kwork[blockIdx.x / (kKBlock / 32)];
+  const SysDev& P = b.sys[wk.x];
+  if (P.nd <= 1 || at_limit(b, wk.x)) return;  // single-dipole systems: ksum1_kernel, ksum1s_kernel
+  const int k0 = wk.z * kKBlock + (blockIdx.x % (kKBlock / 32)) * 32;
+  if (k0 >= P.nk) return;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kl = min(k0 + lane, P.nk - 1);
+  const int N = b.ndtot, nd = P.nd;
+  const int p0 = wk.y * kKChunk, np = min(kKChunk, P.n - p0);
+  for (int q = threadIdx.x; q < np * nd; q += 32 * kSumWarps) {
+    const int g = P.dip_off + p0 * nd + q;
+    sx[q] = b.dfx[g];
+    sy[q] = b.dfx[N + g];
+    sz[q] = b.dfx[2 * N + g];
+    smx[q] = b.dm[g];
+    smy[q] = b.dm[N + g];
+    smz[q] = b.dm[2 * N + g];
+  }
+  const int4 n = b.kn[P.k_off + kl];
+  const float4 kv = b.kv[P.k_off + kl];
+  float acc = 0.f;
+  __syncthreads();
+  for (int r = 0, buf = 0; r < np; r += kSumWarps, buf ^= 1) {
+    if (r + w < np) {
+      float S[2] = {0.f, 0.f}, U[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int d = 0; d < ND; ++d) {
+        if (d < nd) {
+          const int q = (r + w) * nd + d;
+          float c, s;
+          phase_exp(sx[q], sy[q], sz[q], n, c, s);
+          const float m[3] = {smx[q], smy[q], smz[q]};
+          const float a = m[0] * kv.x + m[1] * kv.y + m[2] * kv.z;
+          S[0] += a * c;
+          S[1] -= a * s;
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            U[2 * e] += m[e] * c;
+            U[2 * e + 1] -= m[e] * s;
+          }
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 6; ++e) term[buf][w][e][lane] = U[e];
+      term[buf][w][6][lane] = S[0];
+      term[buf][w][7][lane] = S[1];
+    }
+    // one barrier a round: a buffer is written again only after the next one,
+    // which every warp reaches with its reads of this one done
+    __syncthreads();
+    const int cnt = min(kSumWarps, np - r);
+    const float(*t)[kSumTerms][32] = term[buf];
+    if (w < 6) {
+#pragma unroll
+      for (int q = 0; q < kSumWarps; ++q)
+        if (q < cnt) acc = __fadd_rn(acc, t[q][w][lane]);
+    } else {
+      // w = 6: |S_i|^2; 7 to 9: Re(conj(S_i) U_i)
+      const int ur = w == 6 ? 6 : 2 * (w - 7), ui = ur + 1;
+#pragma unroll
+      for (int q = 0; q < kSumWarps; ++q)
+        if (q < cnt) acc = __fadd_rn(acc, __fmaf_rn(t[q][6][lane], t[q][ur][lane], __fmul_rn(t[q][7][lane], t[q][ui][lane])));
+    }
+  }
+  if (k0 + lane < P.nk) ksum_part(b, P, wk.y, 10)[(long long)w * P.nk + kl] = acc;
+}
+
 // Single-dipole systems.  The particle's own terms need no per-k work:
 // |S_i(k)|^2 = (m_i.k)^2 and Re(conj(S_i) U_ic) = (m_i.k) m_ic, so
 // self(k) = k^T G k and uvslf(k) = G k with G = sum_i m_i m_i^T
@@ -288,7 +369,12 @@ static void launch_ksum(const Batch& b, const int4* kwork, int nkwork, cudaStrea
     ksum1s_kernel<<<nkwork, 2 * kKBlock, 0, s>>>(b, kwork);
   else
     ksum1_kernel<<<nkwork, kKBlock / 2, 0, s>>>(b, kwork);
-  if constexpr (ND > 1) ksum_kernel<ND><<<nkwork, kKBlock, 0, s>>>(b, kwork);
+  if constexpr (ND > 1) {
+    if (b.sum_split)
+      ksum_split_kernel<ND><<<nkwork * (kKBlock / 32), 32 * kSumWarps, 0, s>>>(b, kwork);
+    else
+      ksum_kernel<ND><<<nkwork, kKBlock, 0, s>>>(b, kwork);
+  }
 }
 
 // The totals of NC components of a system's k-vector, c0, c0 + 1, ..., over the
@@ -432,17 +518,21 @@ __global__ void __launch_bounds__(kKBlock) kenergy_kernel(Batch b) {
 // k-space results of one dipole from its Kahan sums (sum = fo - fc): the
 // force as float-float, and the torque m x G (G the second triple) with the
 // FP32 moment -- as accurate as the FP32 sums it is built from
-__device__ __forceinline__ void store_kout(const Batch& b, int g, const float* fo, const float* fc,
-                                           float mx, float my, float mz) {
-#pragma unroll
-  for (int c = 0; c < 3; ++c) b.Fk[3 * g + c] = make_float2(fo[c], -fc[c]);
-  const FF G[3] = {{fo[3], -fc[3]}, {fo[4], -fc[4]}, {fo[5], -fc[5]}};
+__device__ __forceinline__ void store_tk(const Batch& b, int g, const float* go, const float* gc, float mx, float my,
+                                         float mz) {
+  const FF G[3] = {{go[0], -gc[0]}, {go[1], -gc[1]}, {go[2], -gc[2]}};
   const float m[3] = {mx, my, mz};
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const FF t = ff_cross(m[(c + 1) % 3], G[(c + 2) % 3], m[(c + 2) % 3], G[(c + 1) % 3]);
     b.Tk[3 * g + c] = make_float2(t.hi, t.lo);
   }
+}
+__device__ __forceinline__ void store_kout(const Batch& b, int g, const float* fo, const float* fc,
+                                           float mx, float my, float mz) {
+#pragma unroll
+  for (int c = 0; c < 3; ++c) b.Fk[3 * g + c] = make_float2(fo[c], -fc[c]);
+  store_tk(b, g, fo + 3, fc + 3, mx, my, mz);
 }
 
 // The gathers: per particle over all k of its system, force and torque
@@ -588,6 +678,131 @@ __global__ void __launch_bounds__(kPartBlock) kgather_kernel(Batch b) {
 #pragma unroll
   for (int d = 0; d < ND; ++d)
     if (d < nd) store_kout(b, gd0 + d, fo[d], fc[d], mx[d], my[d], mz[d]);
+}
+
+// The same for batches that leave SMs idle: a block takes 32 particles of the
+// work item, a lane each; its four warps form the terms of the k-vectors in
+// turn (force and torque factor of each dipole) and leave them in shared
+// memory, and each then adds its dipoles' force or torque sums over those
+// k-vectors, in order: a thread's walk over a k tile was the time (700 rods of
+// two dipoles 53.8 us per step, 49.7 this way).
+constexpr int kGatherWarps = 4, kGatherTurn = 4;  // k-vectors a warp forms per round
+template <int ND>
+__global__ void __launch_bounds__(32 * kGatherWarps) kgather_split_kernel(Batch b) {
+  constexpr int kRound = kGatherWarps * kGatherTurn;
+  constexpr int kMine = (2 * ND + kGatherWarps - 1) / kGatherWarps;  // sums (dipole; force or torque) of a warp
+  __shared__ KTile kt;
+  __shared__ float term[2][kRound][2 * ND][32];
+  const int2 wk = b.kgwork[blockIdx.x / (kPartBlock / 32)];  // (particle block, tile)
+  const int2 bk = b.blk[wk.x];
+  const SysDev& P = b.sys[bk.x];
+  if (P.nd <= 1 || at_limit(b, bk.x)) return;  // single-dipole systems: kgather1 / kgather1s
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int r0 = bk.y + (blockIdx.x % (kPartBlock / 32)) * 32, end = P.part_off + P.n;
+  if (r0 >= end) return;
+  const bool ok = r0 + lane < end;
+  const int i = ok ? r0 + lane : r0;
+  const int nd = P.nd, N = b.ndtot;
+  const int g0 = P.dip_off + (i - P.part_off) * nd;
+  uint32_t ux[ND], uy[ND], uz[ND];
+  float mx[ND], my[ND], mz[ND];
+#pragma unroll
+  for (int d = 0; d < ND; ++d) {
+    const int g = d < nd ? g0 + d : g0;
+    ux[d] = b.dfx[g];
+    uy[d] = b.dfx[N + g];
+    uz[d] = b.dfx[2 * N + g];
+    mx[d] = b.dm[g];
+    my[d] = b.dm[N + g];
+    mz[d] = b.dm[2 * N + g];
+  }
+  float fo[kMine][3], fc[kMine][3], ft[kMine][3];
+#pragma unroll
+  for (int m = 0; m < kMine; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) fo[m][c] = fc[m][c] = 0.f;
+  int kb, ke, buf = 0;
+  ktile_range(P, wk, kb, ke);
+  for (int k0 = kb; k0 < ke; k0 += kKBlock) {
+    const int nk = stage_ktile<32 * kGatherWarps>(b, P, k0, ke, kt);
+#pragma unroll
+    for (int m = 0; m < kMine; ++m)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) ft[m][c] = 0.f;
+    for (int q0 = 0; q0 < nk; q0 += kRound, buf ^= 1) {
+#pragma unroll
+      for (int u = 0; u < kGatherTurn; ++u) {
+        const int q = q0 + u * kGatherWarps + w;
+        if (q < nk) {
+          const int4 n = kt.n[q];
+          const float4 kv = kt.v[q];
+          const float2 vS = kt.S[q];
+          float Ec[ND], Es[ND], a[ND];
+          float Sr = 0.f, Si = 0.f;
+#pragma unroll
+          for (int d = 0; d < ND; ++d) {
+            if (d < nd) {
+              phase_exp(ux[d], uy[d], uz[d], n, Ec[d], Es[d]);
+              a[d] = mx[d] * kv.x + my[d] * kv.y + mz[d] * kv.z;
+              Sr += a[d] * Ec[d];
+              Si -= a[d] * Es[d];
+            }
+          }
+          // D = conj(val S) - val conj(S_i)
+          const float Dr = vS.x - kv.w * Sr;
+          const float Di = -vS.y + kv.w * Si;
+#pragma unroll
+          for (int d = 0; d < ND; ++d) {
+            if (d < nd) {
+              // Z = E D with E = (c, -s)
+              const float Zr = Ec[d] * Dr + Es[d] * Di;
+              const float Zi = Ec[d] * Di - Es[d] * Dr;
+              term[buf][q - q0][2 * d][lane] = -a[d] * Zi;
+              term[buf][q - q0][2 * d + 1][lane] = -Zr;
+            }
+          }
+        }
+      }
+      // one barrier a round, as in ksum_split_kernel
+      __syncthreads();
+      const int cnt = min(kRound, nk - q0);
+#pragma unroll
+      for (int m = 0; m < kMine; ++m) {
+        const int j = w + m * kGatherWarps;
+        if (j < 2 * nd) {
+#pragma unroll
+          for (int q = 0; q < kRound; ++q)
+            if (q < cnt) {
+              const float4 kv = kt.v[q0 + q];
+              const float f = term[buf][q][j][lane];
+              ft[m][0] = __fmaf_rn(f, kv.x, ft[m][0]);
+              ft[m][1] = __fmaf_rn(f, kv.y, ft[m][1]);
+              ft[m][2] = __fmaf_rn(f, kv.z, ft[m][2]);
+            }
+        }
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < kMine; ++m)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) kahan(fo[m][c], fc[m][c], ft[m][c]);
+  }
+  if (!ok) return;
+#pragma unroll
+  for (int m = 0; m < kMine; ++m) {
+    const int j = w + m * kGatherWarps, d = j >> 1, g = g0 + d;
+    if (j >= 2 * nd) continue;
+    if (wk.y >= 0) {  // one tile: leave its sums
+      float* mine = ktile_set(b, P, i, wk.y) + d * kSet + (j & 1) * 3 * kPartBlock;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) mine[c * kPartBlock] = ft[m][c];
+    } else if (j & 1) {
+      store_tk(b, g, fo[m], fc[m], b.dm[g], b.dm[N + g], b.dm[2 * N + g]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) b.Fk[3 * g + c] = make_float2(fo[m][c], -fc[m][c]);
+    }
+  }
 }
 
 // Single-dipole systems: a thread takes two particles, i and i + 64 of its
@@ -772,7 +987,12 @@ static void launch_kgather(const Batch& b, cudaStream_t s) {
     kgather1s_kernel<<<b.nkgwork, kPartBlock, 0, s>>>(b);
   else
     kgather1_kernel<<<b.nkgwork, kPartBlock / 2, 0, s>>>(b);
-  if constexpr (ND > 1) kgather_kernel<ND><<<b.nkgwork, kPartBlock, 0, s>>>(b);
+  if constexpr (ND > 1) {
+    if (b.gather_split)
+      kgather_split_kernel<ND><<<b.nkgwork * (kPartBlock / 32), 32 * kGatherWarps, 0, s>>>(b);
+    else
+      kgather_kernel<ND><<<b.nkgwork, kPartBlock, 0, s>>>(b);
+  }
 }
 
 template <int ND>
@@ -800,7 +1020,8 @@ void launch_kspace_parts(const Batch& b, int maxnd, const int4* kwork, int nkwor
 // once per device: the step's memory split
 cudaError_t prepare_kspace() {
   return set_carveout(ksum1_kernel, ksum1s_kernel, ksum_kernel<2>, ksum_kernel<4>, kstruct_kernel, kenergy_kernel,
-                      kgather1_kernel, kgather1s_kernel, kgather_kernel<2>, kgather_kernel<4>);
+                      kgather1_kernel, kgather1s_kernel, kgather_kernel<2>, kgather_kernel<4>, ksum_split_kernel<2>,
+                      ksum_split_kernel<4>, kgather_split_kernel<2>, kgather_split_kernel<4>);
 }
 
 void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, cudaStream_t s) {

@@ -23,7 +23,7 @@ TOL_F = 1e-5  # the bar of the Ewald forces
 # rods, dipoles per rod, |n|^2 limit: one particle block and its edges, one
 # k tile (13, 62 and 128 k-vectors) and several, chunks of 256 rods and one more
 SIZES = [(2, 1, 3), (64, 1, 9), (128, 1, 16), (129, 1, 36), (257, 1, 64), (700, 1, 27), (65, 2, 27), (257, 2, 36),
-         (130, 4, 9)]
+         (130, 4, 9), (1030, 3, 27)]
 
 
 def _system(n, nd, ksq, seed):

@@ -73,6 +73,12 @@ constexpr int kNoiseChunk = 256;  // steps of thermostat noise per upload
 // in 84 or in 100 us, by which was first), 89 behind it; 64 systems 195 and
 // 190; 2048 rods (528 tiles), where the tiles are the longest chain, 52 and 56.
 constexpr int kTilesAfter = 4 * 152;
+// Batches of at most this many tiles run each on four warps.  us per step on one
+// warp and on four: 256 rods (10 tiles) 39.4 and 33.4, 333 (21) 41.4 and 36.3,
+// 1000 (136) 43.9 and 39.3, 1200 (190) 43.2 and 39.9, 700 rods of two dipoles
+// (253) 49.5 and 49.6, 1500 (300) 43.5 and 44.8, 2048 (528) 47.6 and 49.8: there
+// the tiles have a scheduler's time to share and the exchange costs instructions.
+constexpr int kSplitTilesMax = 210;
 // Batches of at most this many particle blocks (2 per SM) gather one k tile
 // per block: 2048 rods (16 blocks) 85 us per step with whole walks and 80
 // split, 24 systems of 128 to 2048 rods (140 blocks) 144 and 135; 64 systems
@@ -1286,6 +1292,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   B->arena_bytes = A.off;
   B->b.tune.wca_blocks = 8 * B->num_sms;
   B->b.tune.kg_scalar = (int)lo.blk.size() <= kGatherSplitMax;
+  B->b.split_tiles = (int)lo.tiles.size() <= kSplitTilesMax;
   B->b.sum_split = (int)lo.blk.size() <= kSumSplitMax;
   B->b.gather_split = (int)lo.blk.size() <= kGatherNdSplitMax;
   B->b.stage_k = (int)lo.blk.size() <= kGatherSplitMax && lo.maxchunk <= kStageChunks;

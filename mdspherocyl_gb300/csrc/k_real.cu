@@ -165,12 +165,17 @@ struct JOut {
   f2 fx, fy, fz, ex, ey, ez;
 };
 
-// one step of a tile loop: the lane's two i-dipoles against j0 (half 0)
-// and j1 (half 1) -- the same j in off-diagonal tiles.  Pairs masked off
-// (a0, a1 false) contribute exactly zero: both moments are scaled by 0.
+// a pair's separation, energy and the factors of its forces and fields
+struct Pair2 {
+  f2 dx, dy, dz, u, Ac, fact, mirB, mjrB, mix, miy, miz, mjx, mjy, mjz;
+};
+
+// the pair terms of one step of a tile loop: the lane's two i-dipoles against
+// j0 (half 0) and j1 (half 1) -- the same j in off-diagonal tiles.  Pairs masked
+// off (a0, a1 false) contribute exactly zero: both moments are scaled by 0.
 template <bool MASKED, int MODE>
-__device__ __forceinline__ void tile_step(const PairConst& K, Lane2& s, const uint4 jp0, const float4 jm0,
-                                          const uint4 jp1, const float4 jm1, bool a0, bool a1, JOut& o) {
+__device__ __forceinline__ void pair_step(const PairConst& K, const Lane2& s, const uint4 jp0, const float4 jm0,
+                                          const uint4 jp1, const float4 jm1, bool a0, bool a1, Pair2& o) {
   f2 mix = s.mx, miy = s.my, miz = s.mz;
   f2 mjx = make_float2(jm0.x, jm1.x), mjy = make_float2(jm0.y, jm1.y), mjz = make_float2(jm0.z, jm1.z);
   if (MASKED) {
@@ -297,38 +302,63 @@ __device__ __forceinline__ void tile_step(const PairConst& K, Lane2& s, const ui
   const f2 qq = mul2(pr, rinv2);
   const f2 fact = fma2(neg2(qq), Cc, mul2(fma2(b2(-5.f), qq, mimj), Bc));
   const f2 mirB = mul2(mir, Bc), mjrB = mul2(mjr, Bc);
-  const f2 fx = fma2(fact, dx, fma2(mirB, mjx, mul2(mjrB, mix)));
-  const f2 fy = fma2(fact, dy, fma2(mirB, mjy, mul2(mjrB, miy)));
-  const f2 fz = fma2(fact, dz, fma2(mirB, mjz, mul2(mjrB, miz)));
-  // field of j at i, (mj.r) B r - A mj, into the lane's sums; field of i at j
-  const f2 nA = neg2(Ac);
-  s.E[0] = fma2(nA, mjx, fma2(mjrB, dx, s.E[0]));
-  s.E[1] = fma2(nA, mjy, fma2(mjrB, dy, s.E[1]));
-  s.E[2] = fma2(nA, mjz, fma2(mjrB, dz, s.E[2]));
-  o.ex = fma2(mirB, dx, mul2(nA, mix));
-  o.ey = fma2(mirB, dy, mul2(nA, miy));
-  o.ez = fma2(mirB, dz, mul2(nA, miz));
+  o = Pair2{dx, dy, dz, u, Ac, fact, mirB, mjrB, mix, miy, miz, mjx, mjy, mjz};
+}
 
+// the force on i; the field of i at j (nA is -A); the field of j at i, (mj.r) B
+// r - A mj, into the sums E
+__device__ __forceinline__ void pair_force(const Pair2& p, f2& fx, f2& fy, f2& fz) {
+  fx = fma2(p.fact, p.dx, fma2(p.mirB, p.mjx, mul2(p.mjrB, p.mix)));
+  fy = fma2(p.fact, p.dy, fma2(p.mirB, p.mjy, mul2(p.mjrB, p.miy)));
+  fz = fma2(p.fact, p.dz, fma2(p.mirB, p.mjz, mul2(p.mjrB, p.miz)));
+}
+__device__ __forceinline__ void pair_field(const Pair2& p, f2 nA, f2& ex, f2& ey, f2& ez) {
+  ex = fma2(p.mirB, p.dx, mul2(nA, p.mix));
+  ey = fma2(p.mirB, p.dy, mul2(nA, p.miy));
+  ez = fma2(p.mirB, p.dz, mul2(nA, p.miz));
+}
+__device__ __forceinline__ void add_field(f2 (&E)[3], f2 nA, f2 mjrB, f2 mjx, f2 mjy, f2 mjz, f2 dx, f2 dy, f2 dz) {
+  E[0] = fma2(nA, mjx, fma2(mjrB, dx, E[0]));
+  E[1] = fma2(nA, mjy, fma2(mjrB, dy, E[1]));
+  E[2] = fma2(nA, mjz, fma2(mjrB, dz, E[2]));
+}
+__device__ __forceinline__ void add_energy(f2& U, f2& Uc, f2 u) {  // Kahan: U += u
+  const f2 yk = sub2(u, Uc);
+  const f2 tk = add2(U, yk);
+  Uc = sub2(sub2(tk, U), yk);
+  U = tk;
+}
+__device__ __forceinline__ void add_tensor(f2 (&pt)[9], f2 dx, f2 dy, f2 dz, f2 fx, f2 fy, f2 fz) {
+  pt[0] = fma2(dx, fx, pt[0]);
+  pt[1] = fma2(dx, fy, pt[1]);
+  pt[2] = fma2(dx, fz, pt[2]);
+  pt[3] = fma2(dy, fx, pt[3]);
+  pt[4] = fma2(dy, fy, pt[4]);
+  pt[5] = fma2(dy, fz, pt[5]);
+  pt[6] = fma2(dz, fx, pt[6]);
+  pt[7] = fma2(dz, fy, pt[7]);
+  pt[8] = fma2(dz, fz, pt[8]);
+}
+
+// one step of a tile loop
+template <bool MASKED, int MODE>
+__device__ __forceinline__ void tile_step(const PairConst& K, Lane2& s, const uint4 jp0, const float4 jm0,
+                                          const uint4 jp1, const float4 jm1, bool a0, bool a1, JOut& o) {
+  Pair2 q;
+  pair_step<MASKED, MODE>(K, s, jp0, jm0, jp1, jm1, a0, a1, q);
+  f2 fx, fy, fz;
+  pair_force(q, fx, fy, fz);
+  const f2 nA = neg2(q.Ac);
+  add_field(s.E, nA, q.mjrB, q.mjx, q.mjy, q.mjz, q.dx, q.dy, q.dz);
+  pair_field(q, nA, o.ex, o.ey, o.ez);
   s.F[0] = add2(s.F[0], fx);
   s.F[1] = add2(s.F[1], fy);
   s.F[2] = add2(s.F[2], fz);
   o.fx = fx;
   o.fy = fy;
   o.fz = fz;
-  // Kahan: U += u
-  const f2 yk = sub2(u, s.Uc);
-  const f2 tk = add2(s.U, yk);
-  s.Uc = sub2(sub2(tk, s.U), yk);
-  s.U = tk;
-  s.pt[0] = fma2(dx, fx, s.pt[0]);
-  s.pt[1] = fma2(dx, fy, s.pt[1]);
-  s.pt[2] = fma2(dx, fz, s.pt[2]);
-  s.pt[3] = fma2(dy, fx, s.pt[3]);
-  s.pt[4] = fma2(dy, fy, s.pt[4]);
-  s.pt[5] = fma2(dy, fz, s.pt[5]);
-  s.pt[6] = fma2(dz, fx, s.pt[6]);
-  s.pt[7] = fma2(dz, fy, s.pt[7]);
-  s.pt[8] = fma2(dz, fz, s.pt[8]);
+  add_energy(s.U, s.Uc, q.u);
+  add_tensor(s.pt, q.dx, q.dy, q.dz, fx, fy, fz);
 }
 
 // Off-diagonal tile (strips I < J): 64 steps, at step t lane l pairs both
@@ -448,6 +478,27 @@ __device__ __forceinline__ float to_len(float v, const float* sc) {
   return fmaf(v, sc[0], v * sc[1]);
 }
 
+// the lane's two i-dipoles of strip I
+__device__ __forceinline__ void load_lane(const Batch& b, const SysDev& P, int I, int lane, Lane2& s) {
+  const int ND = b.ndtot;
+  const int i0 = I * kTile + lane, i1 = i0 + 32;
+  s.ok0 = i0 < P.ndip;
+  s.ok1 = i1 < P.ndip;
+  const int g0 = P.dip_off + (s.ok0 ? i0 : 0), g1 = P.dip_off + (s.ok1 ? i1 : 0);
+  s.x0 = b.dfx[g0];
+  s.y0 = b.dfx[ND + g0];
+  s.z0 = b.dfx[2 * ND + g0];
+  s.x1 = b.dfx[g1];
+  s.y1 = b.dfx[ND + g1];
+  s.z1 = b.dfx[2 * ND + g1];
+  const float z0 = s.ok0 ? 1.f : 0.f, z1 = s.ok1 ? 1.f : 0.f;
+  s.mx = make_float2(z0 * b.dm[g0], z1 * b.dm[g1]);
+  s.my = make_float2(z0 * b.dm[ND + g0], z1 * b.dm[ND + g1]);
+  s.mz = make_float2(z0 * b.dm[2 * ND + g0], z1 * b.dm[2 * ND + g1]);
+  s.own0 = b.downer[g0];
+  s.own1 = b.downer[g1];
+}
+
 // One tile (strips I <= J of one system) by one warp: the j-strip staged in
 // the warp's shared arrays, the i-strip in registers, the pair loop, the
 // partial slots and the tile's energy and pressure tensor.
@@ -473,29 +524,12 @@ __device__ __forceinline__ void tile_work(const Batch& b, int tile, const PairCo
   }
 
   Lane2 s;
-  {
-    const int i0 = I * kTile + lane, i1 = i0 + 32;
-    s.ok0 = i0 < ndip;
-    s.ok1 = i1 < ndip;
-    const int g0 = P.dip_off + (s.ok0 ? i0 : 0), g1 = P.dip_off + (s.ok1 ? i1 : 0);
-    s.x0 = b.dfx[g0];
-    s.y0 = b.dfx[ND + g0];
-    s.z0 = b.dfx[2 * ND + g0];
-    s.x1 = b.dfx[g1];
-    s.y1 = b.dfx[ND + g1];
-    s.z1 = b.dfx[2 * ND + g1];
-    const float z0 = s.ok0 ? 1.f : 0.f, z1 = s.ok1 ? 1.f : 0.f;
-    s.mx = make_float2(z0 * b.dm[g0], z1 * b.dm[g1]);
-    s.my = make_float2(z0 * b.dm[ND + g0], z1 * b.dm[ND + g1]);
-    s.mz = make_float2(z0 * b.dm[2 * ND + g0], z1 * b.dm[2 * ND + g1]);
-    s.own0 = b.downer[g0];
-    s.own1 = b.downer[g1];
+  load_lane(b, P, I, lane, s);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) s.F[c] = s.E[c] = b2(0.f);
+  for (int c = 0; c < 3; ++c) s.F[c] = s.E[c] = b2(0.f);
 #pragma unroll
-    for (int c = 0; c < 9; ++c) s.pt[c] = b2(0.f);
-    s.U = s.Uc = b2(0.f);
-  }
+  for (int c = 0; c < 9; ++c) s.pt[c] = b2(0.f);
+  s.U = s.Uc = b2(0.f);
   __syncwarp();
 
   const int jvalid = min(kTile, ndip - J * kTile);
@@ -596,6 +630,214 @@ __global__ void __launch_bounds__(32 * W, 20 / W) real_pairs_kernel(Batch b, con
   const SysDev& P = b.sys[b.tiles[tile].x];
   const PairConst K = pair_consts(b, P, MODE, nullptr);
   tile_work<MULTI, MODE>(b, tile, K, sj_all[wid], smj_all[wid], sa4_all[wid], sa2_all[wid]);
+}
+
+// A tile by four warps, for batches that leave SM schedulers idle: a warp's walk
+// over the 64 steps is one long chain (460 cycles a step where it has its
+// scheduler to itself, of which its instructions take 230).  The warps form the
+// pair terms of the steps in turn -- eight steps a round -- and leave them in
+// shared memory; then each adds one part of the sums over those steps, in step
+// order: forces and energy, fields at the i-dipoles, pressure tensor, and the
+// j-side sums, whose lane L keeps j-dipoles L and L + 32.  The same operations
+// in the same order as tile_work, and so the same bits.  1000 rods (136 tiles)
+// 20.5 us a launch on one warp each, 10.2 this way.
+constexpr int kSplitWarps = 4, kSplitRound = 8;
+enum : int { kTdx, kTdy, kTdz, kTu, kTfx, kTfy, kTfz, kTex, kTey, kTez, kTmjrB, kTnA, kTerms };
+struct SplitTile {
+  uint4 sj[kTile];
+  float4 smj[kTile];
+  f2 term[kTerms][kSplitRound][32];
+};
+
+template <bool MASKED, bool MULTI, bool DIAG, int MODE>
+__device__ __forceinline__ void split_loop(const PairConst& K, const Lane2& s, SplitTile& sh, int w, int lane,
+                                           int jvalid, f2 (&acc)[9]) {
+  constexpr int steps = DIAG ? kTile / 2 : kTile, t_first = DIAG ? 1 : 0;
+#pragma unroll 1
+  for (int r = 0; r < steps; r += kSplitRound) {
+#pragma unroll
+    for (int v = 0; v < kSplitRound / kSplitWarps; ++v) {
+      const int q = v * kSplitWarps + w, t = r + q + t_first;
+      const int j0 = (lane + t) & (kTile - 1), j1 = DIAG ? (j0 ^ 32) : j0;
+      const uint4 jp0 = sh.sj[j0], jp1 = DIAG ? sh.sj[j1] : jp0;
+      const float4 jm0 = sh.smj[j0], jm1 = DIAG ? sh.smj[j1] : jm0;
+      bool a0 = true, a1 = true;
+      if (MASKED) {
+        a0 = s.ok0 && j0 < jvalid;
+        a1 = s.ok1 && j1 < jvalid && !(DIAG && t == kTile / 2);
+        if (MULTI) {
+          a0 = a0 && (s.own0 != (int)jp0.w);
+          a1 = a1 && (s.own1 != (int)jp1.w);
+        }
+      }
+      Pair2 o;
+      pair_step<MASKED, MODE>(K, s, jp0, jm0, jp1, jm1, a0, a1, o);
+      f2 nA = neg2(o.Ac), f[3], e[3];
+      pair_force(o, f[0], f[1], f[2]);
+      pair_field(o, nA, e[0], e[1], e[2]);
+      // (mj.r) B of a pair masked off is zero already
+      if (MASKED) nA = make_float2(a0 ? nA.x : 0.f, a1 ? nA.y : 0.f);
+      sh.term[kTdx][q][lane] = o.dx;
+      sh.term[kTdy][q][lane] = o.dy;
+      sh.term[kTdz][q][lane] = o.dz;
+      sh.term[kTu][q][lane] = o.u;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        sh.term[kTfx + c][q][lane] = f[c];
+        sh.term[kTex + c][q][lane] = e[c];
+      }
+      sh.term[kTmjrB][q][lane] = o.mjrB;
+      sh.term[kTnA][q][lane] = nA;
+    }
+    __syncthreads();
+    if (w == 0) {  // force, energy
+#pragma unroll
+      for (int q = 0; q < kSplitRound; ++q) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] = add2(acc[c], sh.term[kTfx + c][q][lane]);
+        add_energy(acc[3], acc[4], sh.term[kTu][q][lane]);
+      }
+    } else if (w == 1) {  // field
+      f2 E[3] = {acc[0], acc[1], acc[2]};
+#pragma unroll
+      for (int q = 0; q < kSplitRound; ++q) {
+        const int j0 = (lane + r + q + t_first) & (kTile - 1);
+        const float4 m0 = sh.smj[j0], m1 = DIAG ? sh.smj[j0 ^ 32] : m0;
+        add_field(E, sh.term[kTnA][q][lane], sh.term[kTmjrB][q][lane], make_float2(m0.x, m1.x),
+                  make_float2(m0.y, m1.y), make_float2(m0.z, m1.z), sh.term[kTdx][q][lane], sh.term[kTdy][q][lane],
+                  sh.term[kTdz][q][lane]);
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) acc[c] = E[c];
+    } else if (w == 2) {
+#pragma unroll
+      for (int q = 0; q < kSplitRound; ++q)
+        add_tensor(acc, sh.term[kTdx][q][lane], sh.term[kTdy][q][lane], sh.term[kTdz][q][lane],
+                   sh.term[kTfx][q][lane], sh.term[kTfy][q][lane], sh.term[kTfz][q][lane]);
+    } else {
+      // j = L meets lane (L - t) mod 64 where that is an i-dipole of half 0
+      // (and, in a diagonal tile, L + 32 then meets half 1 of the same lane);
+      // otherwise it is L + 32 that meets half 0, of lane (L - t) mod 32
+#pragma unroll
+      for (int q = 0; q < kSplitRound; ++q) {
+        const int d = lane - (r + q + t_first), from = d & 31;
+        const bool low = (d & 32) == 0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const f2 f = sh.term[kTfx + c][q][from], e = sh.term[kTex + c][q][from];
+          if (DIAG) {
+            acc[c].x -= low ? f.x : f.y;
+            acc[c].y -= low ? f.y : f.x;
+            acc[3 + c].x += low ? e.x : e.y;
+            acc[3 + c].y += low ? e.y : e.x;
+          } else if (low) {
+            acc[c].x -= f.x + f.y;
+            acc[3 + c].x += e.x + e.y;
+          } else {
+            acc[c].y -= f.x + f.y;
+            acc[3 + c].y += e.x + e.y;
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <bool MULTI, int MODE>
+__global__ void __launch_bounds__(32 * kSplitWarps, 4) real_pairs_split_kernel(Batch b, const int* gtile) {
+  __shared__ SplitTile sh;
+  const int tile = gtile ? gtile[blockIdx.x] : blockIdx.x;
+  const int4 tl = b.tiles[tile];
+  if (at_limit(b, tl.x)) return;
+  const SysDev& P = b.sys[tl.x];
+  const PairConst K = pair_consts(b, P, MODE, nullptr);
+  const int I = tl.y, J = tl.z, ndip = P.ndip, ND = b.ndtot;
+  const bool diag = I == J;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x < kTile) {
+    const int k = threadIdx.x, jj = J * kTile + k;
+    const bool v = jj < ndip;
+    const int g = P.dip_off + (v ? jj : 0);
+    sh.sj[k] = make_uint4(b.dfx[g], b.dfx[ND + g], b.dfx[2 * ND + g], v ? (uint32_t)b.downer[g] : 0xffffffffu);
+    sh.smj[k] = v ? make_float4(b.dm[g], b.dm[ND + g], b.dm[2 * ND + g], 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  Lane2 s;
+  load_lane(b, P, I, lane, s);
+  f2 acc[9];
+#pragma unroll
+  for (int c = 0; c < 9; ++c) acc[c] = b2(0.f);
+  __syncthreads();
+  const int jvalid = min(kTile, ndip - J * kTile);
+  if (diag)
+    split_loop<true, MULTI, true, MODE>(K, s, sh, w, lane, jvalid, acc);
+  else if (!MULTI && jvalid == kTile)
+    split_loop<false, MULTI, false, MODE>(K, s, sh, w, lane, jvalid, acc);
+  else
+    split_loop<true, MULTI, false, MODE>(K, s, sh, w, lane, jvalid, acc);
+  // a diagonal tile's j-side sums belong to its i-dipoles
+  f2(*js)[32] = sh.term[0];
+  if (diag) {
+    if (w == 3) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) js[c][lane] = acc[c];
+    }
+    __syncthreads();
+    if (w < 2) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) acc[c] = add2(acc[c], js[3 * w + c][lane]);
+    }
+  }
+  // partial slots: (strip X, strip Y, component c, local index)
+  const int ns = P.nstrip;
+  float* base_ij = b.rpart + P.pp_off + ((long long)(I * ns + J) * 6) * kTile;
+  float* base_ji = b.rpart + P.pp_off + ((long long)(J * ns + I) * 6) * kTile;
+  float red[9];
+  int nred = 0;
+  if (w == 0) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      base_ij[c * kTile + lane] = to_len<MODE>(acc[c].x, P.sc4);
+      base_ij[c * kTile + lane + 32] = to_len<MODE>(acc[c].y, P.sc4);
+    }
+    red[0] = (acc[3].x + (-acc[4].x)) + (acc[3].y + (-acc[4].y));
+    nred = 1;
+  } else if (w == 1) {
+    // torque without lever arm: moment x field
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float mx = h ? s.mx.y : s.mx.x, my = h ? s.my.y : s.my.x, mz = h ? s.mz.y : s.mz.x;
+      const float ex = h ? acc[0].y : acc[0].x, ey = h ? acc[1].y : acc[1].x, ez = h ? acc[2].y : acc[2].x;
+      float* t = base_ij + 3 * kTile + lane + 32 * h;
+      t[0 * kTile] = to_len<MODE>(my * ez - mz * ey, P.sc3);
+      t[1 * kTile] = to_len<MODE>(mz * ex - mx * ez, P.sc3);
+      t[2 * kTile] = to_len<MODE>(mx * ey - my * ex, P.sc3);
+    }
+  } else if (w == 2) {
+#pragma unroll
+    for (int c = 0; c < 9; ++c) red[c] = acc[c].x + acc[c].y;
+    nred = 9;
+  } else if (!diag) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = lane + 32 * h;
+      const float4 mj = sh.smj[k];
+      const float ex = h ? acc[3].y : acc[3].x, ey = h ? acc[4].y : acc[4].x, ez = h ? acc[5].y : acc[5].x;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) base_ji[c * kTile + k] = to_len<MODE>(h ? acc[c].y : acc[c].x, P.sc4);
+      base_ji[3 * kTile + k] = to_len<MODE>(mj.y * ez - mj.z * ey, P.sc3);
+      base_ji[4 * kTile + k] = to_len<MODE>(mj.z * ex - mj.x * ez, P.sc3);
+      base_ji[5 * kTile + k] = to_len<MODE>(mj.x * ey - mj.y * ex, P.sc3);
+    }
+  }
+  // tile energy and pressure tensor
+#pragma unroll
+  for (int c = 0; c < 9; ++c) {
+    if (c >= nred) break;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) red[c] += __shfl_xor_sync(0xffffffffu, red[c], off);
+    if (lane == 0) b.tileE[(long long)tile * 10 + c + (w == 2)] = to_len<MODE>(red[c], P.sc3);
+  }
 }
 
 // Tiles of systems whose table fits a block's shared memory: a block takes
@@ -838,7 +1080,8 @@ cudaError_t prepare_real_pairs() {
     e = set_carveout(real_sum_kernel, strip_energy_kernel, real_pairs_kernel<true, 1, kAnalytic>,
                      real_pairs_kernel<false, 1, kAnalytic>, real_pairs_kernel<true, 2, kAnalytic>,
                      real_pairs_kernel<false, 2, kAnalytic>, real_pairs_kernel<true, 4, kAnalytic>,
-                     real_pairs_kernel<false, 4, kAnalytic>);
+                     real_pairs_kernel<false, 4, kAnalytic>, real_pairs_split_kernel<true, kAnalytic>,
+                     real_pairs_split_kernel<false, kAnalytic>);
   return e;
 }
 
@@ -846,7 +1089,10 @@ cudaError_t prepare_real_pairs() {
 template <int MODE>
 void launch_tiles(const Batch& b, bool multi, int W, const int* list, int n, cudaStream_t s) {
   const int grid = cdiv(n, W);
-  if (W == 4) {
+  if (b.split_tiles) {
+    if (multi) real_pairs_split_kernel<true, MODE><<<n, 32 * kSplitWarps, 0, s>>>(b, list);
+    else real_pairs_split_kernel<false, MODE><<<n, 32 * kSplitWarps, 0, s>>>(b, list);
+  } else if (W == 4) {
     if (multi) real_pairs_kernel<true, 4, MODE><<<grid, 128, 0, s>>>(b, list, n);
     else real_pairs_kernel<false, 4, MODE><<<grid, 128, 0, s>>>(b, list, n);
   } else if (W == 2) {

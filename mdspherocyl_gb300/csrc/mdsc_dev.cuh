@@ -282,6 +282,7 @@ struct Batch {
   int ones;      // systems of one dipole per particle
   int2* kgwork;  // (particle block, k tile or -1: all) of every k-space gather block
   int nkgwork;
+  int split_tiles;  // real-space tiles by four warps each (real_pairs_split_kernel)
   int sum_split, gather_split;  // systems of several dipoles per rod through ksum_split, kgather_split
   int stage_k;   // the gathers form val S(k) themselves (kStageChunks)
   float* kgpart; // tile sums of split gathers: per (particle block, tile, dipole) 6 x kPartBlock (ktile_set)

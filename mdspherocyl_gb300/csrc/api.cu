@@ -43,7 +43,8 @@ void launch_cluster_bonds(const Batch& b, cudaStream_t s);
 void launch_ebond(const Batch& b, cudaStream_t s);
 void launch_cluster_hook(const Batch& b, cudaStream_t s);
 void launch_cluster_compress(const Batch& b, cudaStream_t s);
-void launch_reset_iter(const Batch& b, cudaStream_t s);
+void launch_reset_iter(const Batch& b, double* noise, const NoiseArgs& a, cudaStream_t s);
+void launch_copy_arrays(const ArrayCopies& c, cudaStream_t s);
 // copies systems (dst slot, src slot) between batches on the destination's stream
 cudaError_t launch_transfer(const Batch& dst, const Batch& src, const std::vector<int2>& pairs, cudaStream_t s);
 void launch_kspace_parts(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, int part,
@@ -812,7 +813,6 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   int launches = 0;
   launch_integrate_first(b, B->st);
   ++launches;
-  if (io) cudaEventRecordWithFlags(B->ev_x, B->st, cudaEventRecordExternal);
   cudaEventRecord(B->ev_fork, B->st);
   cudaStreamWaitEvent(B->s2, B->ev_fork, 0);
   cudaStreamWaitEvent(B->s3, B->ev_fork, 0);
@@ -848,6 +848,7 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   kpart(2, B->s3);
   // what only the second half kick and the per-system sums read
   cudaStreamWaitEvent(B->s4, B->ev_fork, 0);
+  if (io) cudaEventRecordWithFlags(B->ev_x, B->s4, cudaEventRecordExternal);
   if (!mid_first) {
     launch_xi_mid(b, B->s4);
     cudaEventRecord(B->ev_mid, B->s4);
@@ -867,9 +868,15 @@ mdsc_status capture_step(mdsc_batch* B, int which, bool io = false) {
   cudaStreamWaitEvent(B->st, B->ev_j3, 0);
   cudaStreamWaitEvent(B->st, B->ev_mid, 0);
   launch_finalize(b, kMaskAll | kFlagMoveP, B->st);
-  if (io) cudaEventRecordWithFlags(B->ev_f, B->st, cudaEventRecordExternal);
+  if (io) {  // beside the chain, as ev_x: a record between two kernels delays the second
+    cudaEventRecord(B->ev_k, B->st);
+    cudaStreamWaitEvent(B->s2, B->ev_k, 0);
+    cudaEventRecordWithFlags(B->ev_f, B->s2, cudaEventRecordExternal);
+    cudaEventRecord(B->ev_j2, B->s2);
+  }
   cudaStreamWaitEvent(B->st, B->ev_j4, 0);
   launch_reduce_obs(b, kRedStep, B->st);
+  if (io) cudaStreamWaitEvent(B->st, B->ev_j2, 0);
   launches += 2;
   cudaError_t e = cudaStreamEndCapture(B->st, &g);
   if (e != cudaSuccess) return fail(B, MDSC_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -1626,6 +1633,47 @@ mdsc_status mdsc_upload(mdsc_batch* B, int sys, const mdsc_host_state* h) {
   return upload_one(B, sys, h, true);
 }
 
+// The device's address of n doubles of pinned host memory; null for any other
+// memory (both ends are looked at: a registered range may end before the array).
+static double* pinned(const double* p, long long n) {
+  cudaPointerAttributes a, z;
+  if (n < 1 || cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&z, p + n - 1) != cudaSuccess ||
+      a.type != cudaMemoryTypeHost || z.type != cudaMemoryTypeHost)
+    return nullptr;
+  double* d = (double*)a.devicePointer;
+  return (double*)z.devicePointer == d + (n - 1) ? d : nullptr;
+}
+
+// Copies of state arrays (host -> device, or device -> host) on stream s: in
+// one launch where the batch is small and every host array is pinned, else a
+// copy each.  Null host arrays are left out.
+constexpr int kCopyKernelRods = 8192;
+static cudaError_t copy_state(mdsc_batch* B, bool to_device, int k, double* const* host, double* const* dev,
+                              const int* width, cudaStream_t s) {
+  const long long n = B->lo.ntot;
+  ArrayCopies c;
+  c.k = 0;
+  bool one = n <= kCopyKernelRods;
+  for (int q = 0; q < k && one; ++q) {
+    if (!host[q]) continue;
+    double* h = pinned(host[q], width[q] * n);
+    one = h != nullptr;
+    c.dst[c.k] = to_device ? dev[q] : h;
+    c.src[c.k] = to_device ? h : dev[q];
+    c.n[c.k++] = width[q] * n;
+  }
+  if (one) {
+    launch_copy_arrays(c, s);
+    return cudaGetLastError();
+  }
+  cudaError_t e = cudaSuccess;
+  for (int q = 0; q < k && e == cudaSuccess; ++q)
+    if (host[q])
+      e = cudaMemcpyAsync(to_device ? dev[q] : host[q], to_device ? host[q] : dev[q], sizeof(double) * width[q] * n,
+                          to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, s);
+  return e;
+}
+
 mdsc_status mdsc_upload_all(mdsc_batch* B, const mdsc_host_state* h) {
   if (!B || !h) return MDSC_ERR_BAD_ARG;
   cudaSetDevice(B->device);
@@ -1653,22 +1701,17 @@ mdsc_status mdsc_upload_all(mdsc_batch* B, const mdsc_host_state* h) {
     CU(cudaStreamSynchronize(B->st));
     return MDSC_OK;
   }
-  // state only: one copy per array for the whole batch, one after another on
-  // the main stream.  Each copy runs at the host link's rate (~205 GB/s to
-  // the device on this GB300); spreading the arrays over several streams
-  // made the copies share the link and the whole no faster (the same e2e
-  // within 1%, 175 GB/s for 4 concurrent copies against 207 for one)
-  const size_t n = B->lo.ntot;
+  // state only, one after another on the main stream.  Each copy runs at the
+  // host link's rate (~205 GB/s to the device on this GB300); spreading the
+  // arrays over several streams made the copies share the link and the whole no
+  // faster (the same e2e within 1%, 175 GB/s for 4 concurrent copies against
+  // 207 for one)
   Batch& b = B->b;
   const bool forces = h->F && h->T;
-  CU(cudaMemcpyAsync(b.O, h->O, sizeof(double) * 9 * n, cudaMemcpyHostToDevice, B->st));
-  CU(cudaMemcpyAsync(b.r, h->r, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, B->st));
-  CU(cudaMemcpyAsync(b.p, h->p, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, B->st));
-  CU(cudaMemcpyAsync(b.l, h->l, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, B->st));
-  if (forces) {
-    CU(cudaMemcpyAsync(b.F, h->F, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, B->st));
-    CU(cudaMemcpyAsync(b.T, h->T, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, B->st));
-  }
+  double* const host[6] = {(double*)h->O, (double*)h->r, (double*)h->p, (double*)h->l, (double*)h->F, (double*)h->T};
+  double* const dev[6] = {b.O, b.r, b.p, b.l, b.F, b.T};
+  const int width[6] = {9, 3, 3, 3, 3, 3};
+  CU(copy_state(B, true, forces ? 6 : 4, host, dev, width, B->st));
   for (int s = 0; s < B->nsys; ++s) B->have_forces[s] = forces ? 1 : 0;
   return MDSC_OK;
 }
@@ -2414,9 +2457,16 @@ static mdsc_status run_steps(mdsc_batch* B, int nsteps, mdsc_observables* trace,
     CU(cudaEventSynchronize(B->ev_noise[which]));
     draw_noise(B, chunk, hn);
     CU(cudaEventRecord(B->t_beg, B->st));
-    CU(cudaMemcpyAsync(B->noise[which], hn, sizeof(double) * chunk * B->nsys * 4, cudaMemcpyHostToDevice, B->st));
-    CU(cudaEventRecord(B->ev_noise[which], B->st));
-    launch_reset_iter(B->b, B->st);
+    NoiseArgs args;
+    args.n = 0;
+    if (4LL * chunk * B->nsys <= kNoiseArgs) {
+      args.n = 4 * chunk * B->nsys;
+      std::copy(hn, hn + args.n, args.v);
+    } else {
+      CU(cudaMemcpyAsync(B->noise[which], hn, sizeof(double) * chunk * B->nsys * 4, cudaMemcpyHostToDevice, B->st));
+      CU(cudaEventRecord(B->ev_noise[which], B->st));
+    }
+    launch_reset_iter(B->b, B->noise[which], args, B->st);
     for (int k = 0; k < chunk; ++k) {
       const bool io = out && done + k == nsteps - 1;
       CU(cudaGraphLaunch(io ? B->graph_io[which] : B->graph[which], B->st));
@@ -2425,26 +2475,29 @@ static mdsc_status run_steps(mdsc_batch* B, int nsteps, mdsc_observables* trace,
         // 100 steps before it): they go home while the forces are computed;
         // p, l, F, T once the force assembly has written them, beside the
         // per-system sums
-        const size_t n = B->lo.ntot;
-        auto dn = [&](double* dst, const double* src, size_t w) -> cudaError_t {
-          return dst ? cudaMemcpyAsync(dst, src, sizeof(double) * w * n, cudaMemcpyDeviceToHost, B->sio) : cudaSuccess;
-        };
+        const Batch& b = B->b;
+        double* const pos[2] = {out->r, out->O};
+        double* const pos_d[2] = {b.r, b.O};
+        double* const mom[4] = {out->p, out->l, out->F, out->T};
+        double* const mom_d[4] = {b.p, b.l, b.F, b.T};
+        const int width[4] = {3, 9, 3, 3}, width3[4] = {3, 3, 3, 3};
         CU(cudaStreamWaitEvent(B->sio, B->ev_x, 0));
-        CU(dn(out->r, B->b.r, 3));
-        CU(dn(out->O, B->b.O, 9));
+        CU(copy_state(B, false, 2, pos, pos_d, width, B->sio));
         CU(cudaStreamWaitEvent(B->sio, B->ev_f, 0));
-        CU(dn(out->p, B->b.p, 3));
-        CU(dn(out->l, B->b.l, 3));
-        CU(dn(out->F, B->b.F, 3));
-        CU(dn(out->T, B->b.T, 3));
+        CU(copy_state(B, false, 4, mom, mom_d, width3, B->sio));
       }
       if (trace)
         CU(cudaMemcpyAsync(B->h_trace + (size_t)k * B->nsys, B->b.obs, sizeof(SysObs) * B->nsys,
                            cudaMemcpyDeviceToHost, B->st));
     }
     CU(cudaEventRecord(B->t_end, B->st));
+    // mdsc_step_io: the observables behind the last step, one wait for both
+    if (io_last) CU(cudaMemcpyAsync(B->h_obs, B->b.obs, sizeof(SysObs) * B->nsys, cudaMemcpyDeviceToHost, B->st));
     {
-      CU(cudaEventSynchronize(B->t_end));
+      if (io_last)
+        CU(cudaStreamSynchronize(B->st));
+      else
+        CU(cudaEventSynchronize(B->t_end));
       float t = 0.f;
       CU(cudaEventElapsedTime(&t, B->t_beg, B->t_end));
       dev_ms += t;
@@ -2497,9 +2550,13 @@ mdsc_status mdsc_step_io(mdsc_batch* B, const mdsc_host_state* in, int nsteps, m
     return st ? st : read_obs(B, obs);
   }
   st = run_steps(B, nsteps, nullptr, out);
-  if (st) return st;
-  // the observables behind the state on the same stream, one wait for both
-  CU(cudaMemcpyAsync(B->h_obs, B->b.obs, sizeof(SysObs) * B->nsys, cudaMemcpyDeviceToHost, B->st));
+  if (st) {
+    // nothing of the call reads or writes the caller's arrays after it
+    cudaStreamSynchronize(B->sio);
+    cudaStreamSynchronize(B->st);
+    return st;
+  }
+  if (!out) CU(cudaMemcpyAsync(B->h_obs, B->b.obs, sizeof(SysObs) * B->nsys, cudaMemcpyDeviceToHost, B->st));
   CU(cudaStreamSynchronize(B->sio));
   CU(cudaStreamSynchronize(B->st));
   if (out) {
@@ -2625,7 +2682,7 @@ mdsc_status mdsc_profile_steps(mdsc_batch* B, int nsteps, int max_kernels, char*
   Batch b = batch_with_noise(B, 0);
   for (int it = 0; it < nsteps; ++it) {
     CU(cudaMemcpyAsync(B->noise[0], B->h_noise, sizeof(double) * B->nsys * 4, cudaMemcpyHostToDevice, B->st));
-    launch_reset_iter(b, B->st);
+    launch_reset_iter(b, nullptr, NoiseArgs{}, B->st);
     cudaEventRecord(ev[0], B->st);
     launch_integrate_first(b, B->st);
     launch_xi_mid(b, B->st);

@@ -846,16 +846,35 @@ __global__ void __launch_bounds__(kPartBlock) movep_kernel(Batch b, const double
   }
 }
 
-__global__ void reset_iter_kernel(Batch b) {
+// Opens a run of steps; a short run's noise comes with the launch (a copy of it
+// took 2 us of the stream and as much of the host) into `noise`.
+__global__ void reset_iter_kernel(Batch b, double* noise, NoiseArgs a) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s < b.nsys) b.st[s].iter = 0;
+  if (s < a.n) noise[s] = a.v[s];
+}
+
+// The arrays of a small batch's state, to or from the host in one launch: six
+// copies of 333 rods' arrays take 12.5 us of the stream, one launch 4.2 (2048
+// rods 15 and 6.2, 8192 15 and 11.7; above, the copy engine's 205 GB/s against
+// 150 here decide).
+__global__ void __launch_bounds__(256) copy_arrays_kernel(ArrayCopies c) {
+  const int q = blockIdx.y;
+  const double* src = c.src[q];
+  double* dst = c.dst[q];
+  for (long long i = blockIdx.x * 256 + threadIdx.x; i < c.n[q]; i += (long long)gridDim.x * 256) dst[i] = src[i];
 }
 
 // ---------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------
-void launch_reset_iter(const Batch& b, cudaStream_t s) {
-  if (b.nsys) reset_iter_kernel<<<cdiv(b.nsys, 128), 128, 0, s>>>(b);
+void launch_reset_iter(const Batch& b, double* noise, const NoiseArgs& a, cudaStream_t s) {
+  if (b.nsys) reset_iter_kernel<<<cdiv(std::max(b.nsys, a.n), 128), 128, 0, s>>>(b, noise, a);
+}
+void launch_copy_arrays(const ArrayCopies& c, cudaStream_t s) {
+  long long most = 0;
+  for (int q = 0; q < c.k; ++q) most = std::max(most, c.n[q]);
+  if (most) copy_arrays_kernel<<<dim3((unsigned)std::min<long long>((most + 255) / 256, 152), c.k), 256, 0, s>>>(c);
 }
 void launch_derive(const Batch& b, cudaStream_t s) {
   if (b.nwblk) particle_kernel<kPartDerive><<<b.nwblk, kRowBlock, 0, s>>>(b);

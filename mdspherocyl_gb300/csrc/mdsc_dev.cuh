@@ -351,6 +351,22 @@ __device__ inline uint32_t to_fix(double x, double invL32) {
   return soft_floor_u32(x * invL32);
 }
 
+// Arrays copied by one kernel (copy_arrays): between device memory and pinned
+// host memory, which the device addresses directly.
+struct ArrayCopies {
+  double* dst[6];
+  const double* src[6];
+  long long n[6];
+  int k;
+};
+
+// Thermostat noise of one run of steps as a kernel argument.
+constexpr int kNoiseArgs = 64;
+struct NoiseArgs {
+  double v[kNoiseArgs];
+  int n;
+};
+
 // slot of a particle block in the per-block partial arrays: blocks are
 // launched largest system first, but each system's partials sit in order
 // at blk_off .. blk_off + nblk - 1

@@ -181,3 +181,32 @@ def test_picture_close_to_the_restatement(n, width, height, dist):
                             theta=0.8, phi=0.3, dist=dist)
     off = np.abs(img.astype(int) - want.astype(int)).max(axis=-1) > 3
     assert off.mean() <= 0.02, off.mean()
+
+
+@pytest.mark.parametrize("n,steps", [(2, 1), (129, 16), (129, 17), (8192, 1), (8193, 1)])
+def test_step_io_from_pinned_and_pageable_arrays(n, steps):
+    """State arrays the device reads and writes by itself (pinned, up to 8192
+    rods) and by copies, noise with the launch (up to 16 steps) and by a copy:
+    the same bits as a call on pageable arrays and as steps without them."""
+    import torch
+
+    spec, st = _plain(n, 700 + n)
+    width = {"r": 3, "p": 3, "O": 9, "l": 3, "F": 3, "T": 3}
+    with L.Batch([spec], [st]) as bt:
+        bt.step(1)
+        first = bt.download(0)
+        bt.step(steps)
+        bt.step(steps)
+        want = bt.download(0)
+    for pin in (True, False):
+        host = {k: (torch.empty(n, w, dtype=torch.float64, pin_memory=pin).numpy()) for k, w in width.items()}
+        with L.Batch([spec], [st]) as bt:
+            bt.step(1)
+            for k in host:
+                host[k][...] = np.asarray(first[k]).reshape(n, width[k])
+            obs = (L.Observables * 1)()
+            for _ in range(2):
+                bt.step_io(host, steps, host, obs)
+            assert obs[0].step == 1 + 2 * steps
+        for k in host:
+            assert np.array_equal(host[k], np.asarray(want[k]).reshape(n, width[k])), (pin, k)

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <unistd.h>
 #include <map>
 #include <atomic>
 #include <mutex>
@@ -32,6 +33,7 @@ void launch_derive(const Batch& b, cudaStream_t s);
 void launch_integrate_first(const Batch& b, cudaStream_t s);
 void launch_xi_mid(const Batch& b, cudaStream_t s);
 void launch_finalize(const Batch& b, int mode, cudaStream_t s);
+void launch_finalize_order(const Batch& b, int mode, cudaStream_t s);
 void launch_reduce_obs(const Batch& b, int mode, cudaStream_t s);
 void launch_order_terms(const Batch& b, cudaStream_t s);
 void launch_movex(const Batch& b, cudaStream_t s);
@@ -615,6 +617,8 @@ struct mdsc_batch {
   int2* kowner = nullptr;
   double* noise[2] = {nullptr, nullptr};
   int* d_skip = nullptr;      // per system: skipped by a force evaluation of the others
+  double* stage = nullptr;    // pinned, state on its way home (state_home): at most kStageRods rods
+  long long stage_n = 0;
   double* h_noise = nullptr;  // pinned, the draws of a run of steps (noise buffer 0)
   double* h_noise2 = nullptr; // the same for noise buffer 1: the host draws a run while the last one's copy runs
   cudaEvent_t ev_noise[2] = {nullptr, nullptr};  // the last copy out of each
@@ -684,8 +688,7 @@ mdsc_status eval_forces(mdsc_batch* B, int force_list, const int* skip = nullptr
   launch_real_sum(b, B->st);
   launch_strip_energy(b, B->st);
   launch_kspace(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, B->st);
-  launch_finalize(b, kMaskAll, B->st);
-  launch_order_terms(b, B->st);
+  launch_finalize_order(b, kMaskAll, B->st);
   launch_reduce_obs(b, kRedEnergies, B->st);
   CU(cudaGetLastError());
   for (int s = 0; s < B->nsys; ++s) {
@@ -1041,6 +1044,18 @@ mdsc_status finish_obs(mdsc_batch* B, mdsc_observables* out) {
   return MDSC_OK;
 }
 
+// The sums of a function-level call, reduced into the host's observables as well
+// as the device's: no copy before the wait.  Only the fields of that call's
+// energies are the host's then.
+mdsc_status reduce_home(mdsc_batch* B) {
+  Batch b = B->b;
+  b.obs_host = B->h_obs;
+  launch_reduce_obs(b, kRedEnergies, B->st);
+  CU(cudaGetLastError());
+  CU(cudaStreamSynchronize(B->st));
+  return finish_obs(B, nullptr);
+}
+
 mdsc_status read_obs(mdsc_batch* B, mdsc_observables* out) {
   CU(cudaMemcpyAsync(B->h_obs, B->b.obs, sizeof(SysObs) * B->nsys, cudaMemcpyDeviceToHost, B->st));
   CU(cudaStreamSynchronize(B->st));
@@ -1299,6 +1314,7 @@ mdsc_status mdsc_create(const mdsc_system_desc* descs, int nsys, int device, mds
   B->arena_bytes = A.off;
   B->b.tune.wca_blocks = 8 * B->num_sms;
   B->b.tune.kg_scalar = (int)lo.blk.size() <= kGatherSplitMax;
+  B->b.obs_host = nullptr;
   B->b.split_tiles = (int)lo.tiles.size() <= kSplitTilesMax;
   B->b.sum_split = (int)lo.blk.size() <= kSumSplitMax;
   B->b.gather_split = (int)lo.blk.size() <= kGatherNdSplitMax;
@@ -1454,6 +1470,7 @@ mdsc_status mdsc_destroy(mdsc_batch* B) {
   if (B->scratch) cudaFree(B->scratch);
   if (B->b.ecand) cudaFree(B->b.ecand);
   if (B->b.ecnt) cudaFree(B->b.ecnt);
+  if (B->stage) cudaFreeHost(B->stage);
   if (B->h_noise) cudaFreeHost(B->h_noise);
   if (B->h_noise2) cudaFreeHost(B->h_noise2);
   for (cudaEvent_t e : B->ev_noise)
@@ -1644,13 +1661,12 @@ static double* pinned(const double* p, long long n) {
   return (double*)z.devicePointer == d + (n - 1) ? d : nullptr;
 }
 
-// Copies of state arrays (host -> device, or device -> host) on stream s: in
-// one launch where the batch is small and every host array is pinned, else a
+// Copies of state arrays of n rods (host -> device, or device -> host) on stream
+// s: in one launch where they are few and every host array is pinned, else a
 // copy each.  Null host arrays are left out.
 constexpr int kCopyKernelRods = 8192;
-static cudaError_t copy_state(mdsc_batch* B, bool to_device, int k, double* const* host, double* const* dev,
-                              const int* width, cudaStream_t s) {
-  const long long n = B->lo.ntot;
+static cudaError_t copy_state(bool to_device, int k, double* const* host, double* const* dev, const int* width,
+                              long long n, cudaStream_t s) {
   ArrayCopies c;
   c.k = 0;
   bool one = n <= kCopyKernelRods;
@@ -1668,10 +1684,66 @@ static cudaError_t copy_state(mdsc_batch* B, bool to_device, int k, double* cons
   }
   cudaError_t e = cudaSuccess;
   for (int q = 0; q < k && e == cudaSuccess; ++q)
-    if (host[q])
+    if (host[q] && n > 0)
       e = cudaMemcpyAsync(to_device ? dev[q] : host[q], to_device ? host[q] : dev[q], sizeof(double) * width[q] * n,
                           to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, s);
   return e;
+}
+
+// State arrays of n rods to the host, there on return.  Few rods into plain host
+// memory: one launch into pinned memory of the batch's own and from there by the
+// host (256 rods 81 us with a copy each, 41 this way; 1500 rods 83 and 54; 4096
+// 99 and 94, into arrays in use 68 and 76).  More: a copy each, into pages that
+// the host has touched first -- a copy into fresh pages takes a fault of the
+// device for each (32,768 rods into new arrays 4.4 ms, 0.51 this way).
+constexpr int kStageRods = 2048;
+static cudaError_t state_home(mdsc_batch* B, int k, double* const* host, double* const* dev, const int* width,
+                              long long n) {
+  cudaError_t e = cudaSuccess;
+  bool plain = false;  // an array of plain host memory, and none that the host cannot write
+  long long total = 0;
+  for (int q = 0; q < k && n > 0; ++q)
+    if (host[q]) {
+      total += width[q] * n;
+      cudaPointerAttributes a;
+      if (cudaPointerGetAttributes(&a, host[q]) != cudaSuccess || a.type == cudaMemoryTypeDevice) {
+        plain = false;
+        break;
+      }
+      plain = plain || a.type == cudaMemoryTypeUnregistered;
+    }
+  if (plain && n <= kStageRods) {
+    if (total > B->stage_n) {
+      if (B->stage) cudaFreeHost(B->stage);
+      B->stage = nullptr;
+      B->stage_n = 0;
+      e = cudaMallocHost((void**)&B->stage, sizeof(double) * total);
+      if (e != cudaSuccess) return e;
+      B->stage_n = total;
+    }
+    double* at[6];
+    long long off = 0;
+    for (int q = 0; q < k; ++q) {
+      at[q] = host[q] ? B->stage + off : nullptr;
+      if (host[q]) off += width[q] * n;
+    }
+    e = copy_state(false, k, at, dev, width, n, B->st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(B->st);
+    for (int q = 0; q < k && e == cudaSuccess; ++q)
+      if (host[q]) memcpy(host[q], at[q], sizeof(double) * width[q] * n);
+    return e;
+  }
+  if (plain) {
+    const long long page = sysconf(_SC_PAGESIZE) / (long long)sizeof(double);
+    for (int q = 0; q < k; ++q)
+      if (host[q]) {
+        volatile double* h = host[q];
+        for (long long i = 0; i < width[q] * n; i += page) h[i] = 0.0;
+        h[width[q] * n - 1] = 0.0;
+      }
+  }
+  e = copy_state(false, k, host, dev, width, n, B->st);
+  return e == cudaSuccess ? cudaStreamSynchronize(B->st) : e;
 }
 
 mdsc_status mdsc_upload_all(mdsc_batch* B, const mdsc_host_state* h) {
@@ -1711,7 +1783,7 @@ mdsc_status mdsc_upload_all(mdsc_batch* B, const mdsc_host_state* h) {
   double* const host[6] = {(double*)h->O, (double*)h->r, (double*)h->p, (double*)h->l, (double*)h->F, (double*)h->T};
   double* const dev[6] = {b.O, b.r, b.p, b.l, b.F, b.T};
   const int width[6] = {9, 3, 3, 3, 3, 3};
-  CU(copy_state(B, true, forces ? 6 : 4, host, dev, width, B->st));
+  CU(copy_state(true, forces ? 6 : 4, host, dev, width, B->lo.ntot, B->st));
   for (int s = 0; s < B->nsys; ++s) B->have_forces[s] = forces ? 1 : 0;
   return MDSC_OK;
 }
@@ -1719,18 +1791,12 @@ mdsc_status mdsc_upload_all(mdsc_batch* B, const mdsc_host_state* h) {
 static mdsc_status download_range(mdsc_batch* B, int i0, int n, int s_first, int s_last,
                                   mdsc_host_state* h) {
   Batch& b = B->b;
-  // after the main stream's work, one copy per array on that stream (as
-  // the uploads: concurrent copies share the host link)
-  auto dn = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
-    return (dst && bytes) ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, B->st) : cudaSuccess;
-  };
-  CU(dn(h->O, b.O + 9 * i0, sizeof(double) * 9 * n));
-  CU(dn(h->r, b.r + 3 * i0, sizeof(double) * 3 * n));
-  CU(dn(h->p, b.p + 3 * i0, sizeof(double) * 3 * n));
-  CU(dn(h->F, b.F + 3 * i0, sizeof(double) * 3 * n));
-  CU(dn(h->l, b.l + 3 * i0, sizeof(double) * 3 * n));
-  CU(dn(h->T, b.T + 3 * i0, sizeof(double) * 3 * n));
-  CU(cudaStreamSynchronize(B->st));
+  // after the main stream's work
+  double* const host[6] = {h->O, h->r, h->p, h->F, h->l, h->T};
+  double* const dev[6] = {b.O + 9 * (size_t)i0, b.r + 3 * (size_t)i0, b.p + 3 * (size_t)i0,
+                          b.F + 3 * (size_t)i0, b.l + 3 * (size_t)i0, b.T + 3 * (size_t)i0};
+  const int width[6] = {9, 3, 3, 3, 3, 3};
+  CU(state_home(B, 6, host, dev, width, n));
   if (h->clust) {
     int off = 0;
     for (int s = s_first; s <= s_last; ++s) {
@@ -1796,8 +1862,7 @@ mdsc_status mdsc_zero_forces(mdsc_batch* B) {
   if (st) return st;
   CU(cudaMemsetAsync(B->b.F, 0, sizeof(double) * 3 * B->lo.ntot, B->st));
   CU(cudaMemsetAsync(B->b.T, 0, sizeof(double) * 3 * B->lo.ntot, B->st));
-  CU(cudaStreamSynchronize(B->st));
-  return MDSC_OK;
+  return MDSC_OK;  // what reads the forces runs behind it on the stream
 }
 
 mdsc_status mdsc_force_sc(mdsc_batch* B, double* U, double* W, double* PT) {
@@ -1806,10 +1871,8 @@ mdsc_status mdsc_force_sc(mdsc_batch* B, double* U, double* W, double* PT) {
   launch_derive(B->b, B->st);
   launch_list_build(B->b, 0, B->st);
   launch_wca(B->b, false, B->st);
-  launch_finalize(B->b, kMaskWca | kFlagAccum, B->st);
-  launch_order_terms(B->b, B->st);
-  launch_reduce_obs(B->b, kRedEnergies, B->st);
-  st = read_obs(B, nullptr);
+  launch_finalize_order(B->b, kMaskWca | kFlagAccum, B->st);
+  st = reduce_home(B);
   for (int s = 0; s < B->nsys; ++s) {
     const SysObs& o = B->h_obs[s];
     if (U) U[s] = o.U_ss;
@@ -1828,10 +1891,8 @@ mdsc_status mdsc_force_dipR(mdsc_batch* B, double* U, double* PT) {
   launch_real_pairs(B->b, B->lo.multi, B->st);
   launch_real_sum(B->b, B->st);
   launch_strip_energy(B->b, B->st);
-  launch_finalize(B->b, kMaskReal | kFlagAccum, B->st);
-  launch_order_terms(B->b, B->st);
-  launch_reduce_obs(B->b, kRedEnergies, B->st);
-  st = read_obs(B, nullptr);
+  launch_finalize_order(B->b, kMaskReal | kFlagAccum, B->st);
+  st = reduce_home(B);
   for (int s = 0; s < B->nsys; ++s) {
     const SysObs& o = B->h_obs[s];
     if (U) U[s] = o.U_dipR;
@@ -1845,10 +1906,8 @@ mdsc_status mdsc_force_dipK(mdsc_batch* B, double* U, double* PT) {
   if (st) return st;
   launch_derive(B->b, B->st);
   launch_kspace(B->b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, B->st);
-  launch_finalize(B->b, kMaskK | kFlagAccum, B->st);
-  launch_order_terms(B->b, B->st);
-  launch_reduce_obs(B->b, kRedEnergies, B->st);
-  st = read_obs(B, nullptr);
+  launch_finalize_order(B->b, kMaskK | kFlagAccum, B->st);
+  st = reduce_home(B);
   for (int s = 0; s < B->nsys; ++s) {
     const SysObs& o = B->h_obs[s];
     if (U) U[s] = o.U_dipK;
@@ -1861,10 +1920,8 @@ mdsc_status mdsc_ext_field(mdsc_batch* B, double* U) {
   mdsc_status st = need_state(B);
   if (st) return st;
   launch_derive(B->b, B->st);
-  launch_finalize(B->b, kMaskExt | kFlagAccum, B->st);
-  launch_order_terms(B->b, B->st);
-  launch_reduce_obs(B->b, kRedEnergies, B->st);
-  st = read_obs(B, nullptr);
+  launch_finalize_order(B->b, kMaskExt | kFlagAccum, B->st);
+  st = reduce_home(B);
   for (int s = 0; s < B->nsys; ++s)
     if (U) U[s] = B->h_obs[s].U_ext;
   return st;
@@ -2482,9 +2539,9 @@ static mdsc_status run_steps(mdsc_batch* B, int nsteps, mdsc_observables* trace,
         double* const mom_d[4] = {b.p, b.l, b.F, b.T};
         const int width[4] = {3, 9, 3, 3}, width3[4] = {3, 3, 3, 3};
         CU(cudaStreamWaitEvent(B->sio, B->ev_x, 0));
-        CU(copy_state(B, false, 2, pos, pos_d, width, B->sio));
+        CU(copy_state(false, 2, pos, pos_d, width, B->lo.ntot, B->sio));
         CU(cudaStreamWaitEvent(B->sio, B->ev_f, 0));
-        CU(copy_state(B, false, 4, mom, mom_d, width3, B->sio));
+        CU(copy_state(false, 4, mom, mom_d, width3, B->lo.ntot, B->sio));
       }
       if (trace)
         CU(cudaMemcpyAsync(B->h_trace + (size_t)k * B->nsys, B->b.obs, sizeof(SysObs) * B->nsys,

@@ -13,6 +13,7 @@
 // scalars stay in FP64.
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 #include <vector>
 
 #include "mdsc_dev.cuh"
@@ -388,13 +389,13 @@ __device__ __forceinline__ void ktile_force(const Batch& b, const SysDev& P, FF 
   kt = ff_cross(m1, sg[a2][lane], m2, sg[a1][lane]);
 }
 
-__global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int mode) {
+__device__ __forceinline__ void finalize_row(const Batch& b, int mode, int block) {
   __shared__ double sw[2][3][kRows];  // F, T with the WCA pairs' shares
   __shared__ double sl[3][kRows], sv[3][kRows], sf[3][kRows];
   __shared__ float sp[3][kRows];
   __shared__ double sk[2][3][kRows];  // p; (O l)_a^2
   __shared__ FF sg[3][kRows];
-  const int2 bk = b.wblk[blockIdx.x];
+  const int2 bk = b.wblk[block];
   const int s = bk.x;
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
@@ -589,9 +590,9 @@ __global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int
 // the rod axis o, o o^T and the dipole vectors mu o_dipole, float-float
 // block sums.  Its own small kernel, early in the step on the WCA stream:
 // widening finalize's sums cost that kernel occupancy.
-__global__ void __launch_bounds__(kPartBlock) order_terms_kernel(Batch b) {
+__device__ __forceinline__ void order_terms_block(const Batch& b, int block) {
   __shared__ double sh[12 * kPartBlock / 32];
-  const int2 bk = b.blk[blockIdx.x];
+  const int2 bk = b.blk[block];
   if (at_limit(b, bk.x)) return;
   const SysDev& P = b.sys[bk.x];
   const int i = bk.y + threadIdx.x;
@@ -614,6 +615,23 @@ __global__ void __launch_bounds__(kPartBlock) order_terms_kernel(Batch b) {
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int c = 0; c < 12; ++c) b.obk[12 * blk_slot(P, bk) + c] = tot[c];
+  }
+}
+
+__global__ void __launch_bounds__(kPartBlock) order_terms_kernel(Batch b) { order_terms_block(b, blockIdx.x); }
+
+__global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int mode) {
+  finalize_row(b, mode, blockIdx.x);
+}
+
+// Both in one launch, the order-parameter blocks (their first kPartBlock
+// threads) behind the rows: the function-level calls run one kernel after
+// another, and a kernel for the order terms was 5.4 us of each of them.
+__global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_order_kernel(Batch b, int mode) {
+  if ((int)blockIdx.x < b.nwblk) {
+    finalize_row(b, mode, blockIdx.x);
+  } else if (threadIdx.x < kPartBlock) {
+    order_terms_block(b, blockIdx.x - b.nwblk);
   }
 }
 
@@ -723,37 +741,42 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
     const FF t = ff_add(ff_add(ff_add(sh[c][0], sh[c][1]), sh[c][2]), sh[c][3]);
     x = soft_f2d(t.hi) + soft_f2d(t.lo);
   }
+  const long long home = b.obs_host ? (char*)(b.obs_host + s) - (char*)&ob : 0;
+  auto put = [&](auto& field, auto v) {
+    field = v;
+    if (home) *reinterpret_cast<std::remove_reference_t<decltype(field)>*>((char*)&field + home) = field;
+  };
   if (grp == 0) {
-    if (c == 0) ob.U_dipR = x;
-    else if (c < 10) ob.PT_dipR[c - 1] = x;
+    if (c == 0) put(ob.U_dipR, x);
+    else if (c < 10) put(ob.PT_dipR[c - 1], x);
   } else if (grp == 1) {
-    if (c == 0) ob.U_dipK = x;
-    else if (c < 10) ob.PT_dipK[c - 1] = x;
+    if (c == 0) put(ob.U_dipK, x);
+    else if (c < 10) put(ob.PT_dipK[c - 1], x);
   } else if (grp == 2) {
-    if (c == 0) ob.U_ss = x;
-    else if (c == 1) ob.W_ss = x;
-    else if (c < 11) ob.PT_ss[c - 2] = x;
+    if (c == 0) put(ob.U_ss, x);
+    else if (c == 1) put(ob.W_ss, x);
+    else if (c < 11) put(ob.PT_ss[c - 2], x);
   } else if (grp == 4) {
-    if (c < 12) ob.osum[c] = x;
+    if (c < 12) put(ob.osum[c], x);
   } else {
     if (c == 8) {
-      ob.U_ext = x;
-      ob.U_self = P.Uself;
+      put(ob.U_ext, x);
+      put(ob.U_self, P.Uself);
     }
     if (mode & kRedStep) {
       if (c < 2) {
-        ob.K[c] = 0.5 * x;
+        put(ob.K[c], 0.5 * x);
         // moveTher mode 2 (v25/functions.cpp:2207-2213) closes the step
         const double g = b.noise[((long long)S.iter * b.nsys + s) * 4 + 2 * c + 1];
         const double xi = P.ex1 * S.xi_mid[c] + P.cnoise * g;
         S.xi[c] = xi;
         S.strn[c] = g;
-        ob.xi[c] = xi;
+        put(ob.xi[c], xi);
       } else if (c < 8) {
         // (xx xy)(yy yz)(zz zx) to their places and mirrors
         const int a = (c - 2) >> 1, q = (c & 1) ? (a + 1) % 3 : a;
-        ob.PT_kin[3 * a + q] = x;
-        ob.PT_kin[3 * q + a] = x;
+        put(ob.PT_kin[3 * a + q], x);
+        put(ob.PT_kin[3 * q + a], x);
       }
       __syncwarp();
       if (c == 0) {
@@ -766,12 +789,12 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
       }
       __syncwarp();
     } else if (c < 2) {
-      ob.xi[c] = S.xi[c];
+      put(ob.xi[c], S.xi[c]);
     }
     if (c == 0) {
-      ob.step = S.step;
-      ob.status = S.status;
-      ob.list_builds = S.list_builds;
+      put(ob.step, S.step);
+      put(ob.status, S.status);
+      put(ob.list_builds, S.list_builds);
     }
   }
 }
@@ -887,6 +910,9 @@ void launch_xi_mid(const Batch& b, cudaStream_t s) {
 }
 void launch_finalize(const Batch& b, int mode, cudaStream_t s) {
   if (b.nwblk) finalize_kernel<<<b.nwblk, 2 * kRowBlock, 0, s>>>(b, mode);
+}
+void launch_finalize_order(const Batch& b, int mode, cudaStream_t s) {
+  if (b.nwblk) finalize_order_kernel<<<b.nwblk + b.nblk, 2 * kRowBlock, 0, s>>>(b, mode);
 }
 void launch_order_terms(const Batch& b, cudaStream_t s) {
   if (b.nblk) order_terms_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);

@@ -213,6 +213,7 @@ struct Batch {
   const SysDev* sys;
   SysState* st;
   SysObs* obs;
+  SysObs* obs_host;  // the same for the host (pinned), null unless a call asks for it
   // FP64 master state, AoS per particle
   double* r;     // 3n
   double* p;     // 3n

@@ -210,3 +210,24 @@ def test_step_io_from_pinned_and_pageable_arrays(n, steps):
             assert obs[0].step == 1 + 2 * steps
         for k in host:
             assert np.array_equal(host[k], np.asarray(want[k]).reshape(n, width[k])), (pin, k)
+
+
+@pytest.mark.parametrize("n", [1, 2048, 2049, 9000])
+def test_downloads_into_any_host_memory(n):
+    """Through the batch's own pinned memory (up to 2048 rods) or straight into
+    plain arrays, new or in use, and into pinned ones: the same state."""
+    import torch
+
+    spec, st = _plain(n, 40 + n)
+    width = (3, 3, 9, 3, 3, 3)
+    with L.Batch([spec], [st]) as bt:
+        bt.observe()
+        d = bt.download(0)
+        want = [np.asarray(d[k]).reshape(n, w) for k, w in zip(("r", "p", "O", "l", "F", "T"), width)]
+        assert np.array_equal(want[0], st.r) and np.abs(want[4]).max() < np.inf
+        pinned = [torch.full((n, w), 7.0, dtype=torch.float64, pin_memory=True).numpy() for w in width]
+        mixed = [np.full((n, w), 7.0) if k % 2 else x.copy() * 0 for k, (w, x) in enumerate(zip(width, pinned))]
+        for arrays in (pinned, mixed, mixed, pinned[:2] + mixed[2:]):
+            bt.download_all(*arrays)
+            for got, x in zip(arrays, want):
+                assert np.array_equal(got, x)

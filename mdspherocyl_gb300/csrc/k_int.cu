@@ -356,6 +356,42 @@ __global__ void __launch_bounds__(128) xi_mid_kernel(Batch b) {
 }
 
 // ---------------------------------------------------------------------
+// oo_params' terms (v25/functions.cpp:2720-2760, Qmat_3d :3426-3445) per
+// particle block, from the FP32 working copies of this step's orientations:
+// the rod axis o, o o^T and the dipole vectors mu o_dipole, float-float
+// block sums.  Its own small kernel, early in the step on the WCA stream:
+// widening finalize's sums cost that kernel occupancy.
+__device__ __forceinline__ void order_terms_block(const Batch& b, int block) {
+  __shared__ double sh[12 * kPartBlock / 32];
+  const int2 bk = b.blk[block];
+  if (at_limit(b, bk.x)) return;
+  const SysDev& P = b.sys[bk.x];
+  const int i = bk.y + threadIdx.x;
+  FF v[12];
+#pragma unroll
+  for (int c = 0; c < 12; ++c) v[c].hi = v[c].lo = 0.f;
+  if (i < P.part_off + P.n) {
+    const float4 q = b.pax[i];
+    const float t[9] = {q.x, q.y, q.z, q.x * q.x, q.x * q.y, q.x * q.z, q.y * q.y, q.y * q.z, q.z * q.z};
+#pragma unroll
+    for (int c = 0; c < 9; ++c) v[c] = ff_of(t[c]);
+    const int ND = b.ndtot, g0 = P.dip_off + (i - P.part_off) * P.nd;
+    for (int w = 0; w < P.nd; ++w) {
+#pragma unroll
+      for (int a = 0; a < 3; ++a) v[9 + a] = ff_add(v[9 + a], ff_of(b.dm[a * ND + g0 + w]));
+    }
+  }
+  double tot[12];
+  block_sum<12, kPartBlock>(v, sh, tot);
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int c = 0; c < 12; ++c) b.obk[12 * blk_slot(P, bk) + c] = tot[c];
+  }
+}
+
+__global__ void __launch_bounds__(kPartBlock) order_terms_kernel(Batch b) { order_terms_block(b, blockIdx.x); }
+
+// ---------------------------------------------------------------------
 // force assembly (+ ext_field) and optionally moveP(last): three lanes per
 // rod as above, twice.  Warps 3 to 5 add the WCA pairs' shares while warps 0
 // to 2 add the dipoles' real- and reciprocal-space parts and then, from both,
@@ -389,13 +425,23 @@ __device__ __forceinline__ void ktile_force(const Batch& b, const SysDev& P, FF 
   kt = ff_cross(m1, sg[a2][lane], m2, sg[a1][lane]);
 }
 
-__device__ __forceinline__ void finalize_row(const Batch& b, int mode, int block) {
+// ORDER: the order-parameter blocks (their first kPartBlock threads) in the same
+// launch, behind the rows: the function-level calls run one kernel after
+// another, and a kernel for the order terms was 5.4 us of each of them.
+template <bool ORDER>
+__global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int mode) {
+  if constexpr (ORDER) {
+    if ((int)blockIdx.x >= b.nwblk) {
+      if (threadIdx.x < kPartBlock) order_terms_block(b, blockIdx.x - b.nwblk);
+      return;
+    }
+  }
   __shared__ double sw[2][3][kRows];  // F, T with the WCA pairs' shares
   __shared__ double sl[3][kRows], sv[3][kRows], sf[3][kRows];
   __shared__ float sp[3][kRows];
   __shared__ double sk[2][3][kRows];  // p; (O l)_a^2
   __shared__ FF sg[3][kRows];
-  const int2 bk = b.wblk[block];
+  const int2 bk = b.wblk[blockIdx.x];
   const int s = bk.x;
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
@@ -585,57 +631,6 @@ __device__ __forceinline__ void finalize_row(const Batch& b, int mode, int block
 }
 
 // ---------------------------------------------------------------------
-// oo_params' terms (v25/functions.cpp:2720-2760, Qmat_3d :3426-3445) per
-// particle block, from the FP32 working copies of this step's orientations:
-// the rod axis o, o o^T and the dipole vectors mu o_dipole, float-float
-// block sums.  Its own small kernel, early in the step on the WCA stream:
-// widening finalize's sums cost that kernel occupancy.
-__device__ __forceinline__ void order_terms_block(const Batch& b, int block) {
-  __shared__ double sh[12 * kPartBlock / 32];
-  const int2 bk = b.blk[block];
-  if (at_limit(b, bk.x)) return;
-  const SysDev& P = b.sys[bk.x];
-  const int i = bk.y + threadIdx.x;
-  FF v[12];
-#pragma unroll
-  for (int c = 0; c < 12; ++c) v[c].hi = v[c].lo = 0.f;
-  if (i < P.part_off + P.n) {
-    const float4 q = b.pax[i];
-    const float t[9] = {q.x, q.y, q.z, q.x * q.x, q.x * q.y, q.x * q.z, q.y * q.y, q.y * q.z, q.z * q.z};
-#pragma unroll
-    for (int c = 0; c < 9; ++c) v[c] = ff_of(t[c]);
-    const int ND = b.ndtot, g0 = P.dip_off + (i - P.part_off) * P.nd;
-    for (int w = 0; w < P.nd; ++w) {
-#pragma unroll
-      for (int a = 0; a < 3; ++a) v[9 + a] = ff_add(v[9 + a], ff_of(b.dm[a * ND + g0 + w]));
-    }
-  }
-  double tot[12];
-  block_sum<12, kPartBlock>(v, sh, tot);
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int c = 0; c < 12; ++c) b.obk[12 * blk_slot(P, bk) + c] = tot[c];
-  }
-}
-
-__global__ void __launch_bounds__(kPartBlock) order_terms_kernel(Batch b) { order_terms_block(b, blockIdx.x); }
-
-__global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int mode) {
-  finalize_row(b, mode, blockIdx.x);
-}
-
-// Both in one launch, the order-parameter blocks (their first kPartBlock
-// threads) behind the rows: the function-level calls run one kernel after
-// another, and a kernel for the order terms was 5.4 us of each of them.
-__global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_order_kernel(Batch b, int mode) {
-  if ((int)blockIdx.x < b.nwblk) {
-    finalize_row(b, mode, blockIdx.x);
-  } else if (threadIdx.x < kPartBlock) {
-    order_terms_block(b, blockIdx.x - b.nwblk);
-  }
-}
-
-// ---------------------------------------------------------------------
 // per-system sums and the thermostat's last update.  kRedGroups blocks per
 // system, one per group of sums (real-space tiles, k tiles, WCA pairs,
 // kinetic terms, order parameters), each in float-float with a fixed order;
@@ -643,6 +638,9 @@ __global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_order_kernel(Batch 
 // warps' sums are added and converted one value per lane: an FP64 addition
 // per value in one thread would cost 64 cycles each.
 constexpr int kRedThreads = 128;
+// HOME: into the host's observables as well (a step's kernel without it: 1 us
+// shorter).
+template <bool HOME>
 __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mode) {
   constexpr int NV = 12;
   __shared__ FF sh[NV][kRedThreads / 32];
@@ -741,10 +739,12 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
     const FF t = ff_add(ff_add(ff_add(sh[c][0], sh[c][1]), sh[c][2]), sh[c][3]);
     x = soft_f2d(t.hi) + soft_f2d(t.lo);
   }
-  const long long home = b.obs_host ? (char*)(b.obs_host + s) - (char*)&ob : 0;
   auto put = [&](auto& field, auto v) {
     field = v;
-    if (home) *reinterpret_cast<std::remove_reference_t<decltype(field)>*>((char*)&field + home) = field;
+    if constexpr (HOME) {
+      const long long home = (char*)(b.obs_host + s) - (char*)&ob;
+      *reinterpret_cast<std::remove_reference_t<decltype(field)>*>((char*)&field + home) = v;
+    }
   };
   if (grp == 0) {
     if (c == 0) put(ob.U_dipR, x);
@@ -909,16 +909,20 @@ void launch_xi_mid(const Batch& b, cudaStream_t s) {
   if (b.nsys) xi_mid_kernel<<<b.nsys, 128, 0, s>>>(b);
 }
 void launch_finalize(const Batch& b, int mode, cudaStream_t s) {
-  if (b.nwblk) finalize_kernel<<<b.nwblk, 2 * kRowBlock, 0, s>>>(b, mode);
+  if (b.nwblk) finalize_kernel<false><<<b.nwblk, 2 * kRowBlock, 0, s>>>(b, mode);
 }
 void launch_finalize_order(const Batch& b, int mode, cudaStream_t s) {
-  if (b.nwblk) finalize_order_kernel<<<b.nwblk + b.nblk, 2 * kRowBlock, 0, s>>>(b, mode);
+  if (b.nwblk) finalize_kernel<true><<<b.nwblk + b.nblk, 2 * kRowBlock, 0, s>>>(b, mode);
 }
 void launch_order_terms(const Batch& b, cudaStream_t s) {
   if (b.nblk) order_terms_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);
 }
 void launch_reduce_obs(const Batch& b, int mode, cudaStream_t s) {
-  if (b.nsys) reduce_obs_kernel<<<kRedGroups * b.nsys, kRedThreads, 0, s>>>(b, mode);
+  if (!b.nsys) return;
+  if (b.obs_host)
+    reduce_obs_kernel<true><<<kRedGroups * b.nsys, kRedThreads, 0, s>>>(b, mode);
+  else
+    reduce_obs_kernel<false><<<kRedGroups * b.nsys, kRedThreads, 0, s>>>(b, mode);
 }
 void launch_movex(const Batch& b, cudaStream_t s) {
   if (b.nwblk) particle_kernel<kPartMoveX><<<b.nwblk, kRowBlock, 0, s>>>(b);

@@ -231,3 +231,25 @@ def test_downloads_into_any_host_memory(n):
             bt.download_all(*arrays)
             for got, x in zip(arrays, want):
                 assert np.array_equal(got, x)
+
+
+@pytest.mark.parametrize("steps", [3, 4, 5, 8])
+def test_steps_in_pairs_and_one_by_one(steps):
+    """A call of several steps runs two to a graph; a step limit inside a pair and
+    a trace of every step (one to a graph) leave the same states."""
+    spec, st = _plain(130, 77)
+    with L.Batch([spec], [st]) as bt:
+        for _ in range(steps):
+            one = bt.step(1)[0]
+        want = bt.download(0)
+    with L.Batch([spec, spec], [st, st]) as bt:
+        bt.set_step_limit(1, steps - 2)
+        obs = bt.step(steps)
+        got, short = bt.download(0), bt.download(1)
+    with L.Batch([spec], [st]) as bt:
+        bt.step(steps - 2)
+        before = bt.download(0)
+    assert obs[0]["step"] == one["step"] == steps and obs[1]["step"] == steps - 2
+    for k in ("r", "p", "O", "l", "F", "T"):
+        assert np.array_equal(got[k], want[k]), k
+        assert np.array_equal(short[k], before[k]), k

@@ -520,6 +520,181 @@ __global__ void __launch_bounds__(128) wca_eval_kernel(Batch b) {
   }
 }
 
+// The same on four lanes per pair, for batches whose contacts leave the FP64
+// units idle: an FP64 instruction takes a warp 64 cycles whatever its lanes do,
+// and the pair's 210 of them are the time.  Lane 0 to 2 take the components of
+// vectors, or one of three values of the same form each (products, candidate
+// points, crosses), exchanged by shuffles: 100 instructions, the same operations
+// on the same values as wca_pair with seg_dist_wca, and so the same bits: 10.4 us
+// a launch in the step of 256 rods on one lane, 7.6 on four.
+__device__ __forceinline__ double quad(double v, int from) { return __shfl_sync(0xffffffffu, v, from, 4); }
+__device__ __forceinline__ double sel(const double (&v)[3], int k) { return k == 0 ? v[0] : (k == 1 ? v[1] : v[2]); }
+
+__global__ void __launch_bounds__(128) wca_eval4_kernel(Batch b) {
+  const int n = *(volatile const int*)b.wlist_n;
+  const int lane = threadIdx.x & 31, c = lane & 3, cc = min(c, 2);
+  for (int w0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * 8; w0 < n; w0 += gridDim.x * 32) {
+    const bool ok = w0 + (lane >> 2) < n;
+    const int2 it = b.wlist[ok ? w0 + (lane >> 2) : n - 1];  // spare lanes repeat the last pair and store nothing
+    const int slot = it.x, A = slot / kMaxC, B = b.wcand[slot];
+    const SysDev& P = b.sys[it.y];
+    double oA[3], oB[3], rij[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      oA[q] = b.O[9 * A + 6 + q];
+      oB[q] = b.O[9 * B + 6 + q];
+    }
+    const double lA = b.len[A], lB = b.len[B];
+    const double sigma = (b.dia[A] + b.dia[B]) / 2;
+    const double sig_sq = sigma * sigma;
+    double x = b.r[3 * A + cc] - b.r[3 * B + cc];
+    x = fma(-P.L[cc], floor(fma(x, P.invL[cc], 0.5)), x);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) rij[q] = quad(x, q);
+    // oA.oB, rij.oA, rij.oB, rij.rij
+    double u[3], v[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      u[q] = c == 0 ? oA[q] : rij[q];
+      v[q] = c == 1 ? oA[q] : (c == 3 ? rij[q] : oB[q]);
+    }
+    x = fma(u[2], v[2], fma(u[1], v[1], u[0] * v[0]));
+    const double doto = quad(x, 0), dotrA = quad(x, 1), dotrB = quad(x, 2), rsq = quad(x, 3);
+    // lA^2, lB^2, (oA.oB) lA
+    x = (c == 0 ? lA : (c == 1 ? lB : doto)) * (c == 1 ? lB : lA);
+    const double a2 = quad(x, 0), c2 = quad(x, 1), bb = quad(x, 2) * lB;
+    // d, e
+    const double hb = 0.5 * bb;
+    x = fma(c == 0 ? dotrA : dotrB, c == 0 ? lA : lB, (c == 0 ? -0.5 : 0.5) * (c == 0 ? a2 : c2));
+    x = x + (c == 0 ? hb : -hb);
+    const double d = quad(x, 0), e = quad(x, 1);
+    // s, t, det
+    x = fma(c == 0 ? bb : a2, c < 2 ? e : c2, -(c == 0 ? c2 : bb) * (c < 2 ? d : bb));
+    const double s = quad(x, 0), t = quad(x, 1), det = quad(x, 2);
+    const bool par = !(det > 1.e-12);
+    const double dets = par ? 1.0 : det;
+    const double ac = a2 * c2;
+    const double inv = 1.0 / (dets * ac);
+    // 1 / det, 1 / c, 1 / a: what the lane's candidate needs
+    const double scale = inv * (c == 0 ? ac : dets) * (c == 0 ? 1.0 : (c == 1 ? a2 : c2));
+    double laA[3], lbB[3];
+    x = lA * sel(oA, cc);
+    const double y = lB * sel(oB, cc);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      laA[q] = quad(x, q);
+      lbB[q] = quad(y, q);
+    }
+    const double lo = c == 0 ? det : (c == 1 ? det : (c == 2 ? s : t));
+    const double hi = c == 0 ? s : (c == 1 ? t : 0.0);
+    const unsigned f = (__ballot_sync(0xffffffffu, lo < hi) >> (lane & 28)) & 15u;
+    const bool sbig = f & 1, tbig = f & 2, sneg = f & 4, tneg = f & 8;
+    const double S = sbig ? 1.0 : 0.0, T = tbig ? 1.0 : 0.0;
+    // the candidates: lane 0 the interior point, 1 s held, 2 t held
+    x = (c == 0 ? s : fma(bb, c == 1 ? S : T, c == 1 ? e : -d)) * scale;
+    const double tI = t * scale;
+    const double xc = x > 1.0 ? 1.0 : (x < 0.0 ? 0.0 : x);
+    const double sv = c == 0 ? x : (c == 1 ? S : xc), tv = c == 0 ? tI : (c == 1 ? xc : T);
+    const double sm = sv - 0.5, tm = 0.5 - tv;
+    double o[3], dij[3], st[2];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) o[q] = fma(tm, lbB[q], fma(sm, laA[q], rij[q]));
+    x = fma(o[2], o[2], fma(o[1], o[1], o[0] * o[0]));
+    const double dI = quad(x, 0), dS = quad(x, 1), dT = quad(x, 2);
+    const bool sout = sneg || sbig, tout = tneg || tbig;
+    int pick;
+    if (!sout && !tout) pick = 0;
+    else if (!tout) pick = 1;
+    else if (!sout) pick = 2;
+    else if (sbig) pick = (dT < dS) ? 2 : 1;
+    else pick = (dS < dT) ? 1 : 2;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) dij[q] = quad(o[q], pick);
+    st[0] = quad(sv, pick);
+    st[1] = quad(tv, pick);
+    double dsq = quad(x, pick);
+    if (par || dI < 1.e-12) {  // parallel or intersecting axes: every lane of the pair alike
+      RodD ra, rb;
+      load_rod(b, A, ra);
+      load_rod(b, B, rb);
+      dsq = seg_dist_ref<false>(ra, rb, P.L, rij, dij, st);
+    }
+    __syncwarp();
+    const double srt = 1.122462048309373;  // 2^(1/6)
+    const double lim = (c == 0 ? 0.49 : (c == 1 ? srt * srt : 1.00001)) * (c < 2 ? sig_sq : rsq);
+    const unsigned g =
+        (__ballot_sync(0xffffffffu, c == 2 ? lim < dsq : dsq < lim) >> (lane & 28)) & 7u;
+    int err = (g & 5u) ? kErrOverlap : 0;
+    const bool in = g & 2u;
+    double fA = 0.0, tA = 0.0, tB = 0.0, row[3] = {0.0, 0.0, 0.0}, e0 = 0.0, e1 = 0.0;
+    if (__any_sync(0xffffffffu, in)) {
+      const double inv_dsq = 1.0 / dsq;
+      const double SR2s = sig_sq * inv_dsq;
+      const double SR6s = SR2s * SR2s * SR2s;
+      const double q4 = 4 * SR6s;
+      const double pot = fma(q4, SR6s, -q4);
+      const double ddr = fma(rij[2], dij[2], fma(rij[1], dij[1], rij[0] * dij[0]));
+      const double fw = 6 * fma(q4, SR6s, pot) * inv_dsq;
+      const double FIJ = (ddr != 0.0) ? fw : __longlong_as_double(0x7ff8000000000000LL);
+      if (in && !(fabs(FIJ) < 1e300)) err |= kErrNan;
+      const double fc = FIJ * sel(dij, cc);
+      const int k1 = cc == 2 ? 0 : cc + 1, k2 = cc == 0 ? 2 : cc - 1;
+      const double oi1 = sel(oA, k1), oi2 = sel(oA, k2), oj1 = sel(oB, k1), oj2 = sel(oB, k2);
+      const double r1 = sel(rij, k1), r2 = sel(rij, k2), rc = sel(rij, cc);
+      const double icroj = fma(oi1, oj2, -oi2 * oj1);
+      const double icror = fma(oi1, r2, -oi2 * r1);
+      const double jcror = fma(oj1, r2, -oj2 * r1);
+      x = (c == 0 ? st[0] : st[1]) - 0.5;
+      x = (c == 0 ? x : -x) * (c == 0 ? lA : lB);
+      double fact1 = quad(x, 0), fact2 = quad(x, 1);
+      if (st[0] < -1.e+5) {  // the sentinels, as wca_pair
+        if (st[0] == -1.e+6) fact1 = fact2 = 0.;
+        if (st[0] == -1.e+10) {
+          fact1 = 0.5 * lA;
+          fact2 = 0.5 * lB;
+        } else if (st[0] == -2.e+10) {
+          fact1 = -0.5 * lA;
+          fact2 = -0.5 * lB;
+        } else if (st[0] == -3.e+10) {
+          fact1 = 0.5 * lA;
+          fact2 = -0.5 * lB;
+        }
+      }
+      __syncwarp();
+      const double fmul = fact1 * fact2;
+      const double ta = FIJ * fma(fact1, icror, fmul * icroj), tb = FIJ * fma(fact2, jcror, -fmul * icroj);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const double fq = quad(fc, q);
+        if (in) row[q] = rc * fq;
+      }
+      if (in) {
+        fA = fc;
+        tA = ta;
+        tB = tb;
+        e0 = pot + 1.;
+        e1 = fw * ddr;
+      }
+    }
+    if (!ok) continue;
+    double* evo = b.wev + (long long)slot * 11;
+    if (c < 3) {
+      double* own = b.wown + (long long)slot * 6;
+      double* rec = b.wrec + (long long)slot * 6;
+      own[c] = fA;
+      own[3 + c] = tA;
+      rec[c] = -fA;
+      rec[3 + c] = tB;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) evo[2 + 3 * c + q] = row[q];
+    } else {
+      evo[0] = e0;
+      evo[1] = e1;
+      if (err) atomicOr(&b.st[it.y].status, err);
+    }
+  }
+}
+
 // ---- clusters (v25/functions.cpp:2987-3016,3282-3324) ----------------
 // Bond flags for list entries q > i: segment distance < (D_i + D_j)/2 + min_s
 // in FP64 with the reference's routine (lower index first).  An FP32 distance
@@ -896,11 +1071,17 @@ void launch_list_build(const Batch& b, int force_all, cudaStream_t s) {
 // once per device: the step's memory split
 cudaError_t prepare_wca() {
   return set_carveout(cell_bin_kernel, list_build_kernel, wca_screen_kernel<4>, wca_screen_kernel<8>,
-                      wca_eval_kernel);
+                      wca_eval_kernel, wca_eval4_kernel);
 }
 
 // rows of 32 rods up to which the screen takes 8 lanes per rod
 constexpr int kScreenWideMax = 1200;
+// Batches of at most this many rows evaluate a pair on four lanes.  us per step on
+// one lane and on four: 256 rods 34.4 and 33.2, 333 rods 35.8 and 33.5, 700 rods
+// 37.5 and 34.3, 1500 rods with a cutoff 37.5 and 36.3, 2048 and 32,768 rods (1024
+// rows) the same; 64 systems (1800 rows) 196.6 and 199, 192 systems 528 and 536,
+// whose contacts fill the FP64 units.
+constexpr int kEvalQuadMax = 1200;
 
 // The WCA screen and evaluation.  The work list's length and the partners'
 // slot counts are cleared with the working copies of every new configuration
@@ -916,7 +1097,10 @@ void launch_wca(const Batch& b, bool clear, cudaStream_t s) {
   else
     wca_screen_kernel<4><<<b.nwblk, 128, 0, s>>>(b);
   // a fixed grid (chosen by the autotuner); each thread loops over the list
-  wca_eval_kernel<<<b.tune.wca_blocks, 128, 0, s>>>(b);
+  if (b.nwblk <= kEvalQuadMax)
+    wca_eval4_kernel<<<b.tune.wca_blocks, 128, 0, s>>>(b);
+  else
+    wca_eval_kernel<<<b.tune.wca_blocks, 128, 0, s>>>(b);
 }
 void launch_cluster_bonds(const Batch& b, cudaStream_t s) {
   if (b.nwblk) cluster_bonds_kernel<<<b.nwblk * (32 * kBondLanes / 128), 128, 0, s>>>(b);

@@ -428,15 +428,17 @@ __device__ __forceinline__ void ktile_force(const Batch& b, const SysDev& P, FF 
 // ORDER: the order-parameter blocks (their first kPartBlock threads) in the same
 // launch, behind the rows: the function-level calls run one kernel after
 // another, and a kernel for the order terms was 5.4 us of each of them.
-template <bool ORDER>
-__global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int mode) {
+// TWO: the two halves side by side (warps 3 to 5 the pairs), else one behind the
+// other by three warps (kFinalizeTwoMax).
+template <bool ORDER, bool TWO>
+__global__ void __launch_bounds__((TWO ? 2 : 1) * kRowBlock, TWO ? 5 : 10) finalize_kernel(Batch b, int mode) {
   if constexpr (ORDER) {
     if ((int)blockIdx.x >= b.nwblk) {
       if (threadIdx.x < kPartBlock) order_terms_block(b, blockIdx.x - b.nwblk);
       return;
     }
   }
-  __shared__ double sw[2][3][kRows];  // F, T with the WCA pairs' shares
+  __shared__ double sw[2][3][TWO ? kRows : 1];  // F, T with the WCA pairs' shares
   __shared__ double sl[3][kRows], sv[3][kRows], sf[3][kRows];
   __shared__ float sp[3][kRows];
   __shared__ double sk[2][3][kRows];  // p; (O l)_a^2
@@ -446,15 +448,16 @@ __global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int
   if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   SysState& S = b.st[s];
-  const bool pairs = threadIdx.x >= kRowBlock;  // the same for a warp
+  const bool pairs = TWO && threadIdx.x >= kRowBlock;  // the same for a warp
   const int a = (threadIdx.x >> 5) - (pairs ? 3 : 0), lane = threadIdx.x & 31;
   const bool ok = bk.y + lane < P.part_off + P.n;
   const int i = ok ? bk.y + lane : bk.y;
   const int row = 3 * (P.w_off + (bk.y - P.part_off) / kRows) + a;
-  if (pairs) {
-    if (bk.y == P.part_off && threadIdx.x == kRowBlock) S.dmax = 0;  // the lists of this configuration stand
-    double F = (mode & kFlagAccum) ? b.F[3 * i + a] : 0.0;
-    double T = (mode & kFlagAccum) ? b.T[3 * i + a] : 0.0;
+  double F = 0.0, T = 0.0;
+  if (!TWO || pairs) {
+    if (bk.y == P.part_off && a == 0 && lane == 0) S.dmax = 0;  // the lists of this configuration stand
+    F = (mode & kFlagAccum) ? b.F[3 * i + a] : 0.0;
+    T = (mode & kFlagAccum) ? b.T[3 * i + a] : 0.0;
     FF w[kWcaCols];
 #pragma unroll
     for (int c = 0; c < kWcaCols; ++c) w[c] = ff_of(0.f);
@@ -498,9 +501,11 @@ __global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int
         last = m;
       }
     }
-    sw[0][a][lane] = F;
-    sw[1][a][lane] = T;
-    __syncthreads();
+    if constexpr (TWO) {
+      sw[0][a][lane] = F;
+      sw[1][a][lane] = T;
+      __syncthreads();
+    }
     if (mode & kMaskWca) {
 #pragma unroll
       for (int c = 0; c < kWcaCols; ++c) {
@@ -508,7 +513,7 @@ __global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int
         if (lane == 0) b.wrow[kWcaCols * row + c] = make_float2(w[c].hi, w[c].lo);
       }
     }
-    return;
+    if constexpr (TWO) return;
   }
   const int a1 = a == 2 ? 0 : a + 1, a2 = a == 0 ? 2 : a - 1;  // the cyclic next and previous component
   const bool kick = mode & kFlagMoveP;
@@ -523,7 +528,7 @@ __global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int
   const int nd = P.nd;
   // the field term needs the FP64 moment; without a field it adds nothing
   const bool ext = (mode & kMaskExt) && (P.B[0] != 0.0 || P.B[1] != 0.0 || P.B[2] != 0.0);
-  double F = 0.0, T = 0.0, uext = 0.0;
+  double uext = 0.0;
   for (int w = 0; w < max(nd, 1); ++w) {
     double f = 0.0, t = 0.0;
     if (w < nd) {
@@ -579,7 +584,7 @@ __global__ void __launch_bounds__(2 * kRowBlock, 5) finalize_kernel(Batch b, int
       sync_rows();
       if (pc != 0.0) t += pc * b.O[9 * i + 6 + a1] * sf[a2][lane] - pc * b.O[9 * i + 6 + a2] * sf[a1][lane];
     }
-    if (w == 0) {
+    if (TWO && w == 0) {
       __syncthreads();  // the pairs' shares come first
       F = sw[0][a][lane];
       T = sw[1][a][lane];
@@ -908,11 +913,21 @@ void launch_integrate_first(const Batch& b, cudaStream_t s) {
 void launch_xi_mid(const Batch& b, cudaStream_t s) {
   if (b.nsys) xi_mid_kernel<<<b.nsys, 128, 0, s>>>(b);
 }
+// Batches of at most this many rows of 32 rods run the force assembly's halves
+// side by side.  us per step one behind the other and side by side: 4096 rods (128
+// rows) 82.5 and 80.0, 24 systems (680) 97.4 and 95.4; 32,768 rods (1024) 2101 and
+// 2106, 64 systems (1800) 192 and 194.5, 192 systems 520 and 531, 256 systems (5700)
+// 682 and 698: twice the warps hold the registers of the next rows.
+constexpr int kFinalizeTwoMax = 1000;
 void launch_finalize(const Batch& b, int mode, cudaStream_t s) {
-  if (b.nwblk) finalize_kernel<false><<<b.nwblk, 2 * kRowBlock, 0, s>>>(b, mode);
+  if (!b.nwblk) return;
+  if (b.nwblk <= kFinalizeTwoMax)
+    finalize_kernel<false, true><<<b.nwblk, 2 * kRowBlock, 0, s>>>(b, mode);
+  else
+    finalize_kernel<false, false><<<b.nwblk, kRowBlock, 0, s>>>(b, mode);
 }
 void launch_finalize_order(const Batch& b, int mode, cudaStream_t s) {
-  if (b.nwblk) finalize_kernel<true><<<b.nwblk + b.nblk, 2 * kRowBlock, 0, s>>>(b, mode);
+  if (b.nwblk) finalize_kernel<true, true><<<b.nwblk + b.nblk, 2 * kRowBlock, 0, s>>>(b, mode);
 }
 void launch_order_terms(const Batch& b, cudaStream_t s) {
   if (b.nblk) order_terms_kernel<<<b.nblk, kPartBlock, 0, s>>>(b);

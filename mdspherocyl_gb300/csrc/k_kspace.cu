@@ -559,14 +559,16 @@ struct KTile {
   float4 v[kKBlock];  // kx, ky, kz, val
   float2 S[kKBlock];  // val * S(k)
 };
-template <int NT>
+// TOTALS (Batch::stage_k): val S(k) formed here; a template because its registers
+// (kgather1 80 -> 128) cost the large batches 8 us of the gather's 96
+template <int NT, bool TOTALS>
 __device__ __forceinline__ int stage_ktile(const Batch& b, const SysDev& P, int k0, int ke, KTile& kt) {
   const int nk = min(kKBlock, ke - k0);
   __syncthreads();
   for (int q = threadIdx.x; q < nk; q += NT) {
     kt.n[q] = b.kn[P.k_off + k0 + q];
     kt.v[q] = b.kv[P.k_off + k0 + q];
-    if (b.stage_k) {
+    if constexpr (TOTALS) {
       double s[6];
       ksum_totals<4>(b, P, k0 + q, 0, P.nd == 1 ? 6 : 10, s);
       kt.S[q] = val_S(b, P.k_off + k0 + q, s);
@@ -579,7 +581,7 @@ __device__ __forceinline__ int stage_ktile(const Batch& b, const SysDev& P, int 
 }
 
 // several dipoles per particle, one particle per thread
-template <int ND>
+template <int ND, bool TOTALS>
 __global__ void __launch_bounds__(kPartBlock) kgather_kernel(Batch b) {
   __shared__ KTile kt;
   const int2 wk = b.kgwork[blockIdx.x];  // (particle block, tile)
@@ -617,7 +619,7 @@ __global__ void __launch_bounds__(kPartBlock) kgather_kernel(Batch b) {
   int kb, ke;
   ktile_range(P, wk, kb, ke);
   for (int k0 = kb; k0 < ke; k0 += kKBlock) {
-    const int nk = stage_ktile<kPartBlock>(b, P, k0, ke, kt);
+    const int nk = stage_ktile<kPartBlock, TOTALS>(b, P, k0, ke, kt);
 #pragma unroll
     for (int d = 0; d < ND; ++d)
 #pragma unroll
@@ -687,7 +689,7 @@ __global__ void __launch_bounds__(kPartBlock) kgather_kernel(Batch b) {
 // k-vectors, in order: a thread's walk over a k tile was the time (700 rods of
 // two dipoles 53.8 us per step, 49.7 this way).
 constexpr int kGatherWarps = 4, kGatherTurn = 4;  // k-vectors a warp forms per round
-template <int ND>
+template <int ND, bool TOTALS>
 __global__ void __launch_bounds__(32 * kGatherWarps) kgather_split_kernel(Batch b) {
   constexpr int kRound = kGatherWarps * kGatherTurn;
   constexpr int kMine = (2 * ND + kGatherWarps - 1) / kGatherWarps;  // sums (dipole; force or torque) of a warp
@@ -724,7 +726,7 @@ __global__ void __launch_bounds__(32 * kGatherWarps) kgather_split_kernel(Batch 
   int kb, ke, buf = 0;
   ktile_range(P, wk, kb, ke);
   for (int k0 = kb; k0 < ke; k0 += kKBlock) {
-    const int nk = stage_ktile<32 * kGatherWarps>(b, P, k0, ke, kt);
+    const int nk = stage_ktile<32 * kGatherWarps, TOTALS>(b, P, k0, ke, kt);
 #pragma unroll
     for (int m = 0; m < kMine; ++m)
 #pragma unroll
@@ -846,7 +848,7 @@ __global__ void __launch_bounds__(kPartBlock / 2) kgather1_kernel(Batch b) {
   uint32_t ph0 = 0u, ph1 = 0u;
   bool have = false;  // a phase from the previous k-vector (the first of the range computes its own)
   for (int k0 = kb; k0 < ke; k0 += kKBlock) {
-    const int nk = stage_ktile<kPartBlock / 2>(b, P, k0, ke, kt);
+    const int nk = stage_ktile<kPartBlock / 2, false>(b, P, k0, ke, kt);
 #pragma unroll
     for (int c = 0; c < 6; ++c) ft[c] = bc(0.f);
 #pragma unroll 2
@@ -912,6 +914,7 @@ __global__ void __launch_bounds__(kPartBlock / 2) kgather1_kernel(Batch b) {
 // warp often has its scheduler to itself and a k-vector's chain (phase, sine,
 // four dependent multiply-adds) would be the time.
 constexpr int kWavesAhead = 8;
+template <bool TOTALS>
 __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
   __shared__ KTile kt;
   const int2 wk = b.kgwork[blockIdx.x];  // (particle block, tile)
@@ -932,7 +935,7 @@ __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
 #pragma unroll
   for (int c = 0; c < 6; ++c) fo[c] = fc[c] = ft[c] = 0.f;
   for (int k0 = kb; k0 < ke; k0 += kKBlock) {
-    const int nk = stage_ktile<kPartBlock>(b, P, k0, ke, kt);
+    const int nk = stage_ktile<kPartBlock, TOTALS>(b, P, k0, ke, kt);
 #pragma unroll
     for (int c = 0; c < 6; ++c) ft[c] = 0.f;
     auto add = [&](int q, float c, float sn) {
@@ -979,19 +982,19 @@ __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
   store_kout(b, g0, fo, fc, mx, my, mz);
 }
 
-template <int ND>
+template <int ND, bool TOTALS>
 static void launch_kgather(const Batch& b, cudaStream_t s) {
-  if (!b.ones)
-    ;
-  else if (b.tune.kg_scalar)
-    kgather1s_kernel<<<b.nkgwork, kPartBlock, 0, s>>>(b);
-  else
-    kgather1_kernel<<<b.nkgwork, kPartBlock / 2, 0, s>>>(b);
+  if (b.ones) {
+    if (b.tune.kg_scalar || TOTALS)  // the form that forms val S(k) itself is the one-rod one
+      kgather1s_kernel<TOTALS><<<b.nkgwork, kPartBlock, 0, s>>>(b);
+    else
+      kgather1_kernel<<<b.nkgwork, kPartBlock / 2, 0, s>>>(b);
+  }
   if constexpr (ND > 1) {
     if (b.gather_split)
-      kgather_split_kernel<ND><<<b.nkgwork * (kPartBlock / 32), 32 * kGatherWarps, 0, s>>>(b);
+      kgather_split_kernel<ND, TOTALS><<<b.nkgwork * (kPartBlock / 32), 32 * kGatherWarps, 0, s>>>(b);
     else
-      kgather_kernel<ND><<<b.nkgwork, kPartBlock, 0, s>>>(b);
+      kgather_kernel<ND, TOTALS><<<b.nkgwork, kPartBlock, 0, s>>>(b);
   }
 }
 
@@ -1001,7 +1004,8 @@ static void kspace_part_nd(const Batch& b, const int4* kwork, int nkwork, const 
   if (b.nktot == 0) return;
   if (part == 0 && nkwork > 0) launch_ksum<ND>(b, kwork, nkwork, s);
   if (part == 1) kstruct_kernel<<<cdiv(b.nktot, 32), 32 * kStructWarps, 0, s>>>(b, kowner);
-  if (part == 2) launch_kgather<ND>(b, s);
+  if (part == 2 && b.stage_k) launch_kgather<ND, true>(b, s);
+  if (part == 2 && !b.stage_k) launch_kgather<ND, false>(b, s);
   if (part == 3) kenergy_kernel<<<b.nktile, kKBlock, 0, s>>>(b);
 }
 
@@ -1019,9 +1023,11 @@ void launch_kspace_parts(const Batch& b, int maxnd, const int4* kwork, int nkwor
 
 // once per device: the step's memory split
 cudaError_t prepare_kspace() {
-  return set_carveout(ksum1_kernel, ksum1s_kernel, ksum_kernel<2>, ksum_kernel<4>, kstruct_kernel, kenergy_kernel,
-                      kgather1_kernel, kgather1s_kernel, kgather_kernel<2>, kgather_kernel<4>, ksum_split_kernel<2>,
-                      ksum_split_kernel<4>, kgather_split_kernel<2>, kgather_split_kernel<4>);
+  return set_carveout(ksum1_kernel, ksum1s_kernel, ksum_kernel<2>, ksum_kernel<4>, ksum_split_kernel<2>,
+                      ksum_split_kernel<4>, kstruct_kernel, kenergy_kernel, kgather1_kernel, kgather1s_kernel<false>,
+                      kgather1s_kernel<true>, kgather_kernel<2, false>, kgather_kernel<2, true>,
+                      kgather_kernel<4, false>, kgather_kernel<4, true>, kgather_split_kernel<2, false>,
+                      kgather_split_kernel<2, true>, kgather_split_kernel<4, false>, kgather_split_kernel<4, true>);
 }
 
 void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, cudaStream_t s) {

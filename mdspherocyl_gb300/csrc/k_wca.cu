@@ -697,15 +697,30 @@ __global__ void __launch_bounds__(128) wca_eval4_kernel(Batch b) {
 
 // ---- clusters (v25/functions.cpp:2987-3016,3282-3324) ----------------
 // Bond flags for list entries q > i: segment distance < (D_i + D_j)/2 + min_s
-// in FP64 with the reference's routine (lower index first).  An FP32 distance
-// decides first: it is a distance between two points of the segments, so
-// below the threshold (by more than its rounding) the rods are bonded, and
-// where the axes are not nearly parallel it is the smallest one to ~1e-6, so
-// above the threshold they are not.  What is left -- within half a percent of
-// the threshold, or axes within 0.01 of parallel, where the closest points are
-// ill-determined -- takes the FP64 routine (~20,000 cycles of a warp).  Eight
-// lanes per rod: 32,768 rods 237 us a launch with one lane and FP64 for every
-// entry, 18 this way.
+// in FP64 with the reference's routine (lower index first).  An FP32 distance,
+// the smallest one between the segments, decides first where it is the
+// routine's as well (bond_clear) and more than half a percent from the
+// threshold.  What is left takes the FP64 routine (~20,000 cycles of a warp).
+// Eight lanes per rod: 32,768 rods 237 us a launch with one lane and FP64 for
+// every entry, 17 this way.
+//
+// The routine's distance is the smallest one, to FP32 accuracy, unless the axes
+// are nearly parallel (it then takes the distance of the lines, or of the ends),
+// the axis lines meet (an end point's distance to the other segment, whichever
+// of the ends it tries first: coplanar rods within the threshold by their
+// smallest distance can be beyond it by the routine's), or a rod has hardly any
+// length (parallel to everything).  Bounds well inside its own (a^2 c^2 sin^2 <
+// 1e-12, lines within 1e-6): sin^2 above 1e-4, lengths' product above 1e-3 and
+// lines more than 0.001 apart; the distance of the lines in FP32 is good to ~5e-7
+// |r| / sin, which the last term covers.  And the axes of unit length, which the
+// routine takes for granted.  r: between the centres.
+__device__ __forceinline__ bool bond_clear(float rx, float ry, float rz, float4 ai, float4 aj) {
+  const float cx = ai.y * aj.z - ai.z * aj.y, cy = ai.z * aj.x - ai.x * aj.z, cz = ai.x * aj.y - ai.y * aj.x;
+  const float sin2 = cx * cx + cy * cy + cz * cz, h = rx * cx + ry * cy + rz * cz;
+  const float ni = ai.x * ai.x + ai.y * ai.y + ai.z * ai.z, nj = aj.x * aj.x + aj.y * aj.y + aj.z * aj.z;
+  return fmaxf(fabsf(ni - 1.f), fabsf(nj - 1.f)) < 1e-5f && sin2 > 1e-4f && ai.w * aj.w > 1e-3f &&
+         h * h > 1e-6f * sin2 + 1e-11f * (rx * rx + ry * ry + rz * rz);
+}
 __device__ __forceinline__ bool bonded_ref(const Batch& b, const SysDev& P, int i, int q) {
   RodD ri, rq;
   load_rod(b, i, ri);
@@ -740,13 +755,12 @@ __global__ void __launch_bounds__(128) cluster_bonds_kernel(Batch b) {
   for (int k = b.nblo[i] + sub; k < nc; k += kBondLanes) {
     const int q = lst[k];
     const float4 aj = b.pax[q];
-    const float d2 = seg_dist_fast(fix_diff(ux, b.pfx[q], P.Lfix[0]), fix_diff(uy, b.pfx[N + q], P.Lfix[1]),
-                                   fix_diff(uz, b.pfx[2 * N + q], P.Lfix[2]), ai.x, ai.y, ai.z, ai.w, aj.x, aj.y, aj.z,
-                                   aj.w);
+    const float dx = fix_diff(ux, b.pfx[q], P.Lfix[0]), dy = fix_diff(uy, b.pfx[N + q], P.Lfix[1]),
+                dz = fix_diff(uz, b.pfx[2 * N + q], P.Lfix[2]);
+    const float d2 = seg_dist_fast(dx, dy, dz, ai.x, ai.y, ai.z, ai.w, aj.x, aj.y, aj.z, aj.w);
     const float sg = 0.5f * (di + b.pdia[q]) + ms, thr = sg * sg;
-    const float dot = ai.x * aj.x + ai.y * aj.y + ai.z * aj.z;
     bool bond = d2 < 0.995f * thr;
-    if (!bond && !(d2 > 1.005f * thr && dot * dot < 0.9999f)) bond = bonded_ref(b, P, i, q);
+    if (!((bond || d2 > 1.005f * thr) && bond_clear(dx, dy, dz, ai, aj))) bond = bonded_ref(b, P, i, q);
     fl[k] = bond ? 1 : 0;
   }
 }

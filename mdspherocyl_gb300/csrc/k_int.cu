@@ -320,9 +320,11 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
 __global__ void __launch_bounds__(128) xi_mid_kernel(Batch b) {
   __shared__ double sh[2][128];
   const int s = blockIdx.x;
-  if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   SysState& S = b.st[s];
+  const bool off = at_limit(b, s);
+  if (threadIdx.x == 0) S.stepping = !off;
+  if (off) return;
   const int nb = cdiv(P.nw, 4), c = threadIdx.x;
   double K = 0.0, x1 = 0.0;
   if (c < 2) x1 = P.ex1 * S.xi[c] + P.cnoise * b.noise[((long long)S.iter * b.nsys + s) * 4 + 2 * c];
@@ -650,10 +652,13 @@ __global__ void __launch_bounds__(kRedThreads) reduce_obs_kernel(Batch b, int mo
   constexpr int NV = 12;
   __shared__ FF sh[NV][kRedThreads / 32];
   const int s = blockIdx.x / kRedGroups, grp = blockIdx.x % kRedGroups;
-  if (at_limit(b, s)) return;
   const SysDev& P = b.sys[s];
   SysState& S = b.st[s];
   SysObs& ob = b.obs[s];
+  // In a step not by the step count, which the kinetic block advances: a block
+  // of the same system that started behind it would take the last step before
+  // the limit for one beyond it.
+  if ((mode & kRedStep) ? !S.stepping : at_limit(b, s)) return;
   FF v[NV];
 #pragma unroll
   for (int c = 0; c < NV; ++c) v[c] = ff_of(0.f);

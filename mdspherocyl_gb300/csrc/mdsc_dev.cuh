@@ -181,6 +181,7 @@ struct SysState {
   int cell_ovf;      // this build: a cell held more than kCellSlots rods (all-pairs scan instead)
   int dmax;          // largest displacement measure of the configuration (FP32 bits; cleared by what reads the lists: finalize_kernel, cluster_bonds_kernel)
   long long stop;    // the step count at which the system stops taking steps (mdsc_set_step_limit)
+  int stepping;      // it takes this step (xi_mid_kernel; for reduce_obs_kernel, which counts the step)
   double K_first[2]; // kinetic energies after the first half kick
   double xi_mid[2];  // xi used by the second half kick
 };

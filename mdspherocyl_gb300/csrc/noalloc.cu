@@ -37,7 +37,6 @@
 
 #include "mdsc.h"
 #include "mdsc_dev.cuh"
-#include "reduce.cuh"
 
 namespace mdsc {
 void launch_real_pairs(const Batch& b, bool multi, cudaStream_t s);
@@ -101,48 +100,59 @@ __global__ void noalloc_prep_kernel(unsigned char* scr, SysDev sys, const double
   }
 }
 
-// Blocks of 256: the tile partials of a dipole's component over all partner
-// strips, a thread each, in float-float (48 bits; FP64 additions and
-// conversions hold a warp 64 cycles each: 3001 dipoles took 42 us in FP64 with
-// a thread per dipole, 6 this way) -> F and T in FP64; the last block sums the
-// tiles' energy and pressure tensor the same way.
-__global__ void __launch_bounds__(256) noalloc_reduce_kernel(const unsigned char* scr, int ndip,
+// The tile partials of a dipole's component over all partner strips, a thread
+// each, in strip order -> F and T; and kSums blocks behind them, a component each
+// of the tiles' energy and pressure tensor, in FP64.
+//
+// A dipole's sums are held in three FP32 numbers, each taking what the rounding
+// of the one before left out: 72 bits against FP64's 53.  An FP64 addition or
+// conversion holds a warp 64 cycles whatever its lanes do.  3001 dipoles, us a
+// launch: 42 with a thread per dipole and FP64, 9.5 with a thread per component
+// and FP64, 7.0 this way (6.1 in two FP32 numbers, 48 bits).  A sum that leaves
+// FP32's range is formed in FP64.
+constexpr int kSums = 10;
+constexpr int kRedBlock = 128;
+// s += v; returns what the rounding of the sum left out
+__device__ __forceinline__ float two_sum(float& s, float v) {
+  const float t = s + v, b = t - s, e = (s - (t - b)) + (v - b);
+  s = t;
+  return e;
+}
+__global__ void __launch_bounds__(kRedBlock) noalloc_reduce_kernel(const unsigned char* scr, int ndip,
                                                              double* __restrict__ F, double* __restrict__ T,
                                                              double* __restrict__ UPT) {
-  __shared__ FF sh[10][8];
-  const float* part = reinterpret_cast<const float*>(scr + kOffPart);
-  const float* tE = reinterpret_cast<const float*>(scr + kOffTileE);
-  const int ns = cdiv(ndip, kTile);
-  if (blockIdx.x + 1 < gridDim.x) {
-    const int k = blockIdx.x * 256 + threadIdx.x;
+  __shared__ double sh[kRedBlock / 32];
+  const int ns = cdiv(ndip, kTile), rows = (int)gridDim.x - kSums;
+  if ((int)blockIdx.x < rows) {
+    const int k = blockIdx.x * kRedBlock + threadIdx.x;
     if (k >= 6 * ndip) return;
     const int c = k / ndip, g = k - c * ndip;  // component-major: a warp reads consecutive dipoles
-    const float* p = part + ((size_t)(g / kTile) * ns * 6 + c) * kTile + g % kTile;
-    FF acc = ff_of(0.f);
+    const float* p = reinterpret_cast<const float*>(scr + kOffPart) + ((size_t)(g / kTile) * ns * 6 + c) * kTile +
+                     g % kTile;
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
 #pragma unroll 8
-    for (int Y = 0; Y < ns; ++Y) acc = ff_add(acc, ff_of(p[(size_t)Y * 6 * kTile]));
-    const double v = soft_f2d(acc.hi) + soft_f2d(acc.lo);
-    if (c < 3) F[3 * g + c] = v;
-    else T[3 * g + c - 3] = v;
+    for (int Y = 0; Y < ns; ++Y) s2 += two_sum(s1, two_sum(s0, p[(size_t)Y * 6 * kTile]));
+    double acc = (double)s0 + ((double)s1 + (double)s2);
+    if (!isfinite(s0)) {
+      acc = 0.0;
+      for (int Y = 0; Y < ns; ++Y) acc += (double)p[(size_t)Y * 6 * kTile];
+    }
+    if (c < 3) F[3 * g + c] = acc;
+    else T[3 * g + c - 3] = acc;
     return;
   }
-  const int ntile = ns * (ns + 1) / 2, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  FF v[10];
+  const float* tE = reinterpret_cast<const float*>(scr + kOffTileE) + (blockIdx.x - rows);
+  const int ntile = ns * (ns + 1) / 2;
+  double v = 0.0;
+#pragma unroll 8
+  for (int t = threadIdx.x; t < ntile; t += kRedBlock) v += (double)tE[(size_t)t * kSums];
 #pragma unroll
-  for (int c = 0; c < 10; ++c) v[c] = ff_of(0.f);
-  for (int t = threadIdx.x; t < ntile; t += 256)
-#pragma unroll
-    for (int c = 0; c < 10; ++c) v[c] = ff_add(v[c], ff_of(tE[(size_t)t * 10 + c]));
-#pragma unroll
-  for (int c = 0; c < 10; ++c) {
-    v[c] = ff_warp_sum(v[c]);
-    if (lane == 0) sh[c][w] = v[c];
-  }
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  if (threadIdx.x < 10) {
-    FF t = sh[threadIdx.x][0];
-    for (int q = 1; q < 8; ++q) t = ff_add(t, sh[threadIdx.x][q]);
-    UPT[threadIdx.x] = soft_f2d(t.hi) + soft_f2d(t.lo);
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < kRedBlock / 32; ++q) v += sh[q];
+    UPT[blockIdx.x - rows] = v;
   }
 }
 
@@ -234,6 +244,6 @@ extern "C" mdsc_status mdsc_force_dipR_noalloc(int ndip, const double* d_pos, co
   b.tileE = reinterpret_cast<float*>(base + kOffTileE);
   launch_real_pairs(b, false, st);
   if (cudaGetLastError() != cudaSuccess) return MDSC_ERR_CUDA;
-  noalloc_reduce_kernel<<<cdiv(6 * ndip, 256) + 1, 256, 0, st>>>(base, ndip, d_F, d_T, d_UPT);
+  noalloc_reduce_kernel<<<cdiv(6 * ndip, kRedBlock) + kSums, kRedBlock, 0, st>>>(base, ndip, d_F, d_T, d_UPT);
   return cudaGetLastError() == cudaSuccess ? MDSC_OK : MDSC_ERR_CUDA;
 }

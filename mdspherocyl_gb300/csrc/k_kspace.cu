@@ -56,33 +56,28 @@ __device__ __forceinline__ uint32_t phase_next(uint32_t ph, bool have, uint32_t 
 
 // The moment tensor of one particle chunk, sum of m m^T (one dipole per
 // particle), for the self terms of kenergy, by a warp of its own block (work
-// items of k tile -1).  Float-float: the products exact (one FMA each for the
-// low half), 48-bit sums -- in FP64 the six sums cost 64 cycles an instruction
-// and a warp (the FP64 unit's issue rate on this GPU, whatever the number of
-// independent chains).
+// items of k tile -1).  FP64: the products exact, the sums to 53 bits.  An FP64
+// instruction holds a warp 64 cycles, ~5000 cycles for a chunk, beside the waves
+// of the other items, which take longer: ksum1s of 256 rods 7.8 us a launch, 7.6
+// with float-float sums (48 bits); the step 31.4 us either way, of 4096 rods 75.5
+// and 77.3.
 __device__ __forceinline__ void chunk_tensor(const Batch& b, const SysDev& P, int chunk) {
   if (threadIdx.x >= 32) return;
   const int N = b.ndtot, p0 = chunk * kKChunk, np = min(kKChunk, P.n - p0);
-  FF g[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) g[c] = ff_of(0.f);
+  double g[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll 4
   for (int q = threadIdx.x; q < np; q += 32) {
     const int d = P.dip_off + p0 + q;
-    const float x = b.dm[d], y = b.dm[N + d], z = b.dm[2 * N + d];
-    const float u[6] = {x, x, x, y, y, z}, v[6] = {x, y, z, y, z, z};
+    const double x = soft_f2d(b.dm[d]), y = soft_f2d(b.dm[N + d]), z = soft_f2d(b.dm[2 * N + d]);
+    const double u[6] = {x, x, x, y, y, z}, v[6] = {x, y, z, y, z, z};
 #pragma unroll
-    for (int c = 0; c < 6; ++c) {
-      FF t;
-      t.hi = __fmul_rn(u[c], v[c]);
-      t.lo = __fmaf_rn(u[c], v[c], -t.hi);
-      g[c] = ff_add(g[c], t);
-    }
+    for (int c = 0; c < 6; ++c) g[c] = fma(u[c], v[c], g[c]);
   }
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
-    g[c] = ff_warp_sum(g[c]);
-    if (threadIdx.x == c) b.kG[((long long)P.gch_off + chunk) * 6 + c] = soft_f2d(g[c].hi) + soft_f2d(g[c].lo);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) g[c] += __shfl_xor_sync(0xffffffffu, g[c], off);
+    if (threadIdx.x == c) b.kG[((long long)P.gch_off + chunk) * 6 + c] = g[c];
   }
 }
 
@@ -453,19 +448,13 @@ __global__ void __launch_bounds__(kKBlock) kenergy_kernel(Batch b) {
   if (at_limit(b, kt.x)) return;
   const SysDev& P = b.sys[kt.x];
   const bool one = P.nd == 1;
-  if (one) {  // the moment tensor over the system's chunks
-    FF g[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) g[c] = ff_of(0.f);
-    for (int ch = threadIdx.x; ch < P.nkchunk; ch += kKBlock) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) g[c] = ff_add(g[c], ff_from(b.kG[((long long)P.gch_off + ch) * 6 + c]));
-    }
-    double tot[6];
-    block_sum<6, kKBlock>(g, sh, tot);
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int c = 0; c < 6; ++c) sG[c] = tot[c];
+  if (one) {  // the moment tensor over the system's chunks, in chunk order
+    if (threadIdx.x < 6) {
+      const double* in = b.kG + (long long)P.gch_off * 6 + threadIdx.x;
+      double g = 0.0;
+#pragma unroll 8
+      for (int ch = 0; ch < P.nkchunk; ++ch) g += in[6 * ch];
+      sG[threadIdx.x] = g;
     }
     __syncthreads();
   }

@@ -13,6 +13,7 @@ import numpy as np
 import pytest
 
 from mdspherocyl_gb300 import lib as L
+from mdspherocyl_gb300 import systems as S
 
 pytestmark = pytest.mark.gpu
 
@@ -118,3 +119,33 @@ def test_noalloc_keeps_what_is_not_a_number():
             assert not np.isfinite(T[bad]).any()
             rest = [i for i in range(n) if i not in bad]
             assert np.isfinite(F[rest]).all() and np.isfinite(T[rest]).all()
+
+
+@pytest.mark.parametrize("n", [32, 288, 600])
+def test_moment_tensor_of_the_self_terms_in_fp64(n):
+    """All rods at one place, moments in opposite pairs: the structure factor is
+    zero and the pressure tensor's xy term is the moment tensor's, whose terms
+    cancel within a chunk of 256 rods (n = 32), or between two and three."""
+    third = {32: 16, 288: 256, 600: 512}[n]  # where the opposite terms stand
+
+    def run(sizes):
+        m = np.zeros((n, 3))
+        for k, v in enumerate(sizes):
+            # products of the same sign in a pair, +-(v, 1) or +-(v, -1)
+            at = 4 * k if k < 3 else third + 1 + 4 * (k - 3)
+            m[at] = (abs(v), np.sign(v), 0.0)
+            m[at + 2] = -m[at]
+        dip = np.zeros((n, 1, 5))
+        dip[:, 0, 1:4] = m
+        dip[:, 0, 4] = 1.0
+        st = S.SystemState(np.zeros((n, 3)), np.zeros((n, 3)), np.stack([np.eye(3)] * n), np.zeros((n, 3)),
+                           np.full(n, 2.0), np.ones(n), np.ones(n), dip)
+        spec = S.SystemSpec(n=n, box=np.full(3, 16.0), alpha=0.4, K_max=2, ksq_max=1)
+        with L.Batch([spec], [st]) as bt:
+            bt.zero_forces()
+            return bt.force_dipK()[1][0]
+
+    alone = run([0.0, 0.0, TINY])
+    assert alone[0][1] != 0 and alone[0][1] == alone[1][0]
+    got = run([BIG, MIDDLE, TINY, -BIG, -MIDDLE])
+    assert got[0][1] == alone[0][1] and got[1][0] == alone[1][0]

@@ -1706,13 +1706,30 @@ static cudaError_t copy_state(bool to_device, int k, double* const* host, double
 // memory: one launch into pinned memory of the batch's own and from there by the
 // host (256 rods 81 us with a copy each, 41 this way; 1500 rods 83 and 54; 4096
 // 99 and 94, into arrays in use 68 and 76).  More: a copy each, into pages that
-// the host has touched first -- a copy into fresh pages takes a fault of the
-// device for each (32,768 rods into new arrays 4.4 ms, 0.51 this way).
+// the host has touched first (touch_pages) -- a copy into fresh pages takes a
+// fault of the device for each (32,768 rods into new arrays 4.4 ms, 0.51 this
+// way).
 constexpr int kStageRods = 2048;
+
+// A page for every part of n doubles of plain host memory, by writing a zero
+// over a zero: a page never written reads as zeros, and what is there stays --
+// an earlier upload may still be reading it, and a copy that fails must leave it.
+static void touch_pages(double* h, long long n) {
+  typedef unsigned long long __attribute__((__may_alias__)) Word;
+  const uintptr_t first = ((uintptr_t)h + 7) / 8 * 8, last = ((uintptr_t)(h + n) - 8) / 8 * 8;
+  const uintptr_t page = sysconf(_SC_PAGESIZE);
+  auto touch = [](uintptr_t at) {
+    Word zero = 0;
+    __atomic_compare_exchange_n((Word*)at, &zero, 0, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED);
+  };
+  for (uintptr_t at = first; at <= last; at += page) touch(at);
+  if (last >= first) touch(last);
+}
 static cudaError_t state_home(mdsc_batch* B, int k, double* const* host, double* const* dev, const int* width,
                               long long n) {
   cudaError_t e = cudaSuccess;
   bool plain = false;  // an array of plain host memory, and none that the host cannot write
+  bool fresh[6] = {};  // it is plain: its pages may not be there yet
   long long total = 0;
   for (int q = 0; q < k && n > 0; ++q)
     if (host[q]) {
@@ -1722,7 +1739,8 @@ static cudaError_t state_home(mdsc_batch* B, int k, double* const* host, double*
         plain = false;
         break;
       }
-      plain = plain || a.type == cudaMemoryTypeUnregistered;
+      fresh[q] = a.type == cudaMemoryTypeUnregistered;
+      plain = plain || fresh[q];
     }
   if (plain && n <= kStageRods) {
     if (total > B->stage_n) {
@@ -1745,15 +1763,9 @@ static cudaError_t state_home(mdsc_batch* B, int k, double* const* host, double*
       if (host[q]) memcpy(host[q], at[q], sizeof(double) * width[q] * n);
     return e;
   }
-  if (plain) {
-    const long long page = sysconf(_SC_PAGESIZE) / (long long)sizeof(double);
+  if (plain)
     for (int q = 0; q < k; ++q)
-      if (host[q]) {
-        volatile double* h = host[q];
-        for (long long i = 0; i < width[q] * n; i += page) h[i] = 0.0;
-        h[width[q] * n - 1] = 0.0;
-      }
-  }
+      if (host[q] && fresh[q]) touch_pages(host[q], width[q] * n);
   e = copy_state(false, k, host, dev, width, n, B->st);
   return e == cudaSuccess ? cudaStreamSynchronize(B->st) : e;
 }

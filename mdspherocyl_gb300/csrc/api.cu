@@ -1802,6 +1802,8 @@ mdsc_status mdsc_upload_all(mdsc_batch* B, const mdsc_host_state* h) {
   // arrays over several streams made the copies share the link and the whole no
   // faster (the same e2e within 1%, 175 GB/s for 4 concurrent copies against
   // 207 for one)
+  if (B->lo.ntot > 0 && (!h->r || !h->p || !h->O || !h->l))
+    return fail(B, MDSC_ERR_BAD_ARG, "r, p, O, l are required");
   Batch& b = B->b;
   const bool forces = h->F && h->T;
   double* const host[6] = {(double*)h->O, (double*)h->r, (double*)h->p, (double*)h->l, (double*)h->F, (double*)h->T};

@@ -1,5 +1,5 @@
 """State arrays on their way between host and device: arrays that an upload still
-reads are left alone by a download."""
+reads are left alone by a download, and arrays that are missing are refused."""
 import numpy as np
 import pytest
 
@@ -62,3 +62,25 @@ def test_a_download_into_the_plain_arrays_just_uploaded():
         bt.download_all(*host)
         for got, x in zip(host, want):
             assert np.array_equal(got, x)
+
+
+@pytest.mark.parametrize("missing", range(4), ids=["r", "p", "O", "l"])
+@pytest.mark.parametrize("n", [64, 9000])
+def test_missing_arrays_are_refused(n, missing):
+    """r, p, O and l are needed, in the upload of a state and in a step with one;
+    the batch's state and forces stay as they were."""
+    st, box = S.make_system(n=n, phi=0.05, lengths=np.full(n, 3.0), mu=np.full(n, 1.2), seed=8)
+    spec = S.SystemSpec(n=n, box=box, alpha=6.0 / float(box[0]), K_max=2, ksq_max=1)
+    arrays = [np.ascontiguousarray(np.asarray(a, dtype=np.float64)) + 0.5 for a in (st.r, st.p, st.O, st.l)]
+    arrays += [np.full((n, 3), 9.0), np.full((n, 3), 9.0)]
+    arrays[missing] = None
+    with L.Batch([spec], [st]) as bt:
+        bt.step(1)
+        before = bt.download(0)
+        with pytest.raises(L.MdscError):
+            bt.upload_all(*arrays)
+        with pytest.raises(L.MdscError):
+            bt.step_io(dict(zip("rpOlFT", arrays)), 1, None)
+        after = bt.download(0)
+    for k in ("r", "p", "O", "l", "F", "T"):
+        assert np.array_equal(before[k], after[k]), k

@@ -1705,26 +1705,12 @@ static cudaError_t copy_state(bool to_device, int k, double* const* host, double
 // State arrays of n rods to the host, there on return.  Few rods into plain host
 // memory: one launch into pinned memory of the batch's own and from there by the
 // host (256 rods 81 us with a copy each, 41 this way; 1500 rods 83 and 54; 4096
-// 99 and 94, into arrays in use 68 and 76).  More: a copy each, into pages that
-// the host has touched first (touch_pages) -- a copy into fresh pages takes a
-// fault of the device for each (32,768 rods into new arrays 4.4 ms, 0.51 this
-// way).
+// 99 and 94, into arrays in use 68 and 76).  More: a copy each, plain arrays into
+// pages that the host has touched first -- a copy into fresh pages takes a fault
+// of the device for each (32,768 rods into new arrays 4.4 ms, 0.50 this way) --
+// and not before the stream is idle: an upload may still be reading them.
 constexpr int kStageRods = 2048;
 
-// A page for every part of n doubles of plain host memory, by writing a zero
-// over a zero: a page never written reads as zeros, and what is there stays --
-// an earlier upload may still be reading it, and a copy that fails must leave it.
-static void touch_pages(double* h, long long n) {
-  typedef unsigned long long __attribute__((__may_alias__)) Word;
-  const uintptr_t first = ((uintptr_t)h + 7) / 8 * 8, last = ((uintptr_t)(h + n) - 8) / 8 * 8;
-  const uintptr_t page = sysconf(_SC_PAGESIZE);
-  auto touch = [](uintptr_t at) {
-    Word zero = 0;
-    __atomic_compare_exchange_n((Word*)at, &zero, 0, false, __ATOMIC_RELAXED, __ATOMIC_RELAXED);
-  };
-  for (uintptr_t at = first; at <= last; at += page) touch(at);
-  if (last >= first) touch(last);
-}
 static cudaError_t state_home(mdsc_batch* B, int k, double* const* host, double* const* dev, const int* width,
                               long long n) {
   cudaError_t e = cudaSuccess;
@@ -1763,9 +1749,17 @@ static cudaError_t state_home(mdsc_batch* B, int k, double* const* host, double*
       if (host[q]) memcpy(host[q], at[q], sizeof(double) * width[q] * n);
     return e;
   }
-  if (plain)
+  if (plain) {
+    e = cudaStreamSynchronize(B->st);
+    if (e != cudaSuccess) return e;
+    const long long page = sysconf(_SC_PAGESIZE) / (long long)sizeof(double);
     for (int q = 0; q < k; ++q)
-      if (host[q] && fresh[q]) touch_pages(host[q], width[q] * n);
+      if (host[q] && fresh[q]) {
+        volatile double* h = host[q];
+        for (long long i = 0; i < width[q] * n; i += page) h[i] = 0.0;
+        h[width[q] * n - 1] = 0.0;
+      }
+  }
   e = copy_state(false, k, host, dev, width, n, B->st);
   return e == cudaSuccess ? cudaStreamSynchronize(B->st) : e;
 }
@@ -1797,13 +1791,13 @@ mdsc_status mdsc_upload_all(mdsc_batch* B, const mdsc_host_state* h) {
     CU(cudaStreamSynchronize(B->st));
     return MDSC_OK;
   }
+  if (B->lo.ntot > 0 && (!h->r || !h->p || !h->O || !h->l))
+    return fail(B, MDSC_ERR_BAD_ARG, "r, p, O, l are required");
   // state only, one after another on the main stream.  Each copy runs at the
   // host link's rate (~205 GB/s to the device on this GB300); spreading the
   // arrays over several streams made the copies share the link and the whole no
   // faster (the same e2e within 1%, 175 GB/s for 4 concurrent copies against
   // 207 for one)
-  if (B->lo.ntot > 0 && (!h->r || !h->p || !h->O || !h->l))
-    return fail(B, MDSC_ERR_BAD_ARG, "r, p, O, l are required");
   Batch& b = B->b;
   const bool forces = h->F && h->T;
   double* const host[6] = {(double*)h->O, (double*)h->r, (double*)h->p, (double*)h->l, (double*)h->F, (double*)h->T};

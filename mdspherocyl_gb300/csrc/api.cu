@@ -1882,7 +1882,8 @@ mdsc_status mdsc_zero_forces(mdsc_batch* B) {
   if (st) return st;
   CU(cudaMemsetAsync(B->b.F, 0, sizeof(double) * 3 * B->lo.ntot, B->st));
   CU(cudaMemsetAsync(B->b.T, 0, sizeof(double) * 3 * B->lo.ntot, B->st));
-  return MDSC_OK;  // what reads the forces runs behind it on the stream
+  CU(cudaStreamSynchronize(B->st));
+  return MDSC_OK;
 }
 
 mdsc_status mdsc_force_sc(mdsc_batch* B, double* U, double* W, double* PT) {

@@ -1,5 +1,6 @@
 """State arrays on their way between host and device: arrays that an upload still
-reads are left alone by a download, and arrays that are missing are refused."""
+reads are left alone by a download, arrays that are missing are refused, and the
+call that zeroes the forces has done so when it returns."""
 import numpy as np
 import pytest
 
@@ -84,3 +85,20 @@ def test_missing_arrays_are_refused(n, missing):
         after = bt.download(0)
     for k in ("r", "p", "O", "l", "F", "T"):
         assert np.array_equal(before[k], after[k]), k
+
+
+def test_zero_forces_waits():
+    """The call returns with the forces zero, as the other function-level calls
+    return with their results."""
+    import torch
+
+    spec, st, host = _big()
+    with L.Batch([spec], [st]) as bt:
+        bt.upload_all(*host)
+        stream = torch.cuda.ExternalStream(bt.lib.mdsc_stream(bt.h))
+        _backlog(bt, host)
+        assert not stream.query()
+        bt.zero_forces()
+        assert stream.query()
+        d = bt.download(0)
+    assert not d["F"].any() and not d["T"].any()

@@ -29,7 +29,9 @@ void launch_real_sum(const Batch& b, cudaStream_t s);
 void launch_strip_energy(const Batch& b, cudaStream_t s);
 void launch_near_pass(const Batch& b, cudaStream_t s);  // the cutoff systems' real space
 void launch_kspace(const Batch& b, int maxnd, const int4* kwork, int nkwork, const int2* kowner, cudaStream_t s);
+// working copies of the state, with the displacement measure (derive) or without
 void launch_derive(const Batch& b, cudaStream_t s);
+void launch_copies(const Batch& b, cudaStream_t s);
 void launch_integrate_first(const Batch& b, cudaStream_t s);
 void launch_xi_mid(const Batch& b, cudaStream_t s);
 void launch_finalize(const Batch& b, int mode, cudaStream_t s);
@@ -676,6 +678,13 @@ Batch batch_with_noise(const mdsc_batch* B, int which) {
   return b;
 }
 
+// Clears the systems' displacement maxima behind a derive that no pass over the
+// lists clears it for: the next one counts up from its own configuration.
+cudaError_t forget_displacement(mdsc_batch* B) {
+  if (!B->nsys) return cudaSuccess;
+  return cudaMemset2DAsync((char*)B->b.st + offsetof(SysState, dmax), sizeof(SysState), 0, sizeof(int), B->nsys, B->st);
+}
+
 // every force term, F and T set from scratch, energies reduced; with a
 // skip mask (device, per system) the flagged systems are left as they are
 mdsc_status eval_forces(mdsc_batch* B, int force_list, const int* skip = nullptr) {
@@ -692,6 +701,7 @@ mdsc_status eval_forces(mdsc_batch* B, int force_list, const int* skip = nullptr
   launch_finalize_order(b, kMaskAll, B->st);
   launch_reduce_obs(b, kRedEnergies, B->st);
   CU(cudaGetLastError());
+  if (skip) CU(forget_displacement(B));  // the skipped systems'
   for (int s = 0; s < B->nsys; ++s) {
     B->built[s] = 1;
     B->have_forces[s] = 1;
@@ -1969,7 +1979,7 @@ mdsc_status mdsc_renorm(mdsc_batch* B) {
   mdsc_status st = need_state(B);
   if (st) return st;
   launch_renorm(B->b, B->st);
-  launch_derive(B->b, B->st);
+  launch_copies(B->b, B->st);
   CU(cudaGetLastError());
   CU(cudaStreamSynchronize(B->st));
   return MDSC_OK;
@@ -2007,6 +2017,7 @@ mdsc_status mdsc_neigh_list(mdsc_batch* B) {
   if (st) return st;
   launch_derive(B->b, B->st);
   launch_list_build(B->b, 1, B->st);
+  CU(forget_displacement(B));
   CU(cudaGetLastError());
   CU(cudaStreamSynchronize(B->st));
   for (int s = 0; s < B->nsys; ++s) B->built[s] = 1;
@@ -2017,6 +2028,7 @@ mdsc_status mdsc_check_list(mdsc_batch* B, int* rebuild) {
   mdsc_status st = need_state(B);
   if (st) return st;
   launch_derive(B->b, B->st);
+  CU(forget_displacement(B));
   std::vector<float> dm(std::max(B->b.nwblk, 1));
   CU(cudaMemcpyAsync(dm.data(), B->b.dmax, sizeof(float) * B->b.nwblk, cudaMemcpyDeviceToHost, B->st));
   CU(cudaStreamSynchronize(B->st));
@@ -2140,7 +2152,7 @@ mdsc_status mdsc_correlations(mdsc_batch* B, double bar_w, double* hist) {
   CU(cudaMemcpyAsync(dcs, cs.data(), cbytes, cudaMemcpyHostToDevice, B->st));
   CU(cudaMemcpyAsync(dsp, sp.data(), sp.size(), cudaMemcpyHostToDevice, B->st));
   CU(cudaMemsetAsync(dh, 0, hbytes, B->st));
-  launch_derive(B->b, B->st);
+  launch_copies(B->b, B->st);
   CU(launch_correlations(B->b, dcs, dsp, bar_w, ntiles, max_bins, dh, B->st));
   CU(cudaMemcpyAsync(h.data(), dh, hbytes, cudaMemcpyDeviceToHost, B->st));
   CU(give_scratch(B, d));
@@ -2164,7 +2176,7 @@ mdsc_status mdsc_order_params(mdsc_batch* B, double* G1, double* G2, double* M) 
   std::vector<double> part(12 * (size_t)nblk);
   char* d = nullptr;
   CU(take_scratch(B, sizeof(double) * part.size(), &d));
-  launch_derive(B->b, B->st);
+  launch_copies(B->b, B->st);
   launch_order_sums(B->b, reinterpret_cast<double*>(d), B->st);
   CU(cudaGetLastError());
   CU(cudaMemcpyAsync(part.data(), d, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, B->st));

@@ -215,14 +215,16 @@ __device__ __forceinline__ void rotor_row(const Batch& b, const Shared3& sh, int
 
 // ---------------------------------------------------------------------
 // first half of the step: moveTher(0), [renorm], moveP(first), moveX
-// (v25/functions.cpp:2071-2149); MOVE_ONLY: moveX alone; DERIVE: only the
-// working copies
+// (v25/functions.cpp:2071-2149); kPartMoveX: moveX alone; kPartDerive: only the
+// working copies and the displacement measure; kPartCopies: only the copies, for
+// calls that decide no list (the system's maximum counts up until a pass that
+// reads the lists clears it)
 // ---------------------------------------------------------------------
 // Measured against one lane per rod in blocks of 128 (with the force assembly
 // below and the per-system sums on lanes): a step of 256 rods 62.4 -> 51.8 us,
 // of 4096 rods 113 -> 93.7, of 32,768 rods 2205 -> 2135, of 64 systems 223 ->
 // 215, of 256 systems 688 -> 688 (FP64 throughput and the state's reads).
-enum : int { kPartDerive = 0, kPartMoveX = 1, kPartStep = 2 };
+enum : int { kPartDerive = 0, kPartMoveX = 1, kPartStep = 2, kPartCopies = 3 };
 
 template <int MODE>
 __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
@@ -256,7 +258,7 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) ax_built[c] = b.usave[3 * i + c];
   }
-  if constexpr (MODE != kPartDerive) {
+  if constexpr (MODE == kPartMoveX || MODE == kPartStep) {
     double p = b.p[3 * i + a], l = b.l[3 * i + a];
     const double im = b.invm[i];
     if constexpr (MODE == kPartStep) {
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(kRowBlock) particle_kernel(Batch b) {
     }
   }
   const float disp = derive_comp(b, P, sh, a, lane, i, ok, r, O, u_built, ax_built);
-  if constexpr (MODE != kPartMoveX) store_disp(b, S, row, a, disp);
+  if constexpr (MODE == kPartDerive || MODE == kPartStep) store_disp(b, S, row, a, disp);
   if constexpr (MODE == kPartStep) store_kin(b, sh, row, a, lane, i, ok);
 }
 
@@ -911,6 +913,9 @@ void launch_copy_arrays(const ArrayCopies& c, cudaStream_t s) {
 }
 void launch_derive(const Batch& b, cudaStream_t s) {
   if (b.nwblk) particle_kernel<kPartDerive><<<b.nwblk, kRowBlock, 0, s>>>(b);
+}
+void launch_copies(const Batch& b, cudaStream_t s) {
+  if (b.nwblk) particle_kernel<kPartCopies><<<b.nwblk, kRowBlock, 0, s>>>(b);
 }
 void launch_integrate_first(const Batch& b, cudaStream_t s) {
   if (b.nwblk) particle_kernel<kPartStep><<<b.nwblk, kRowBlock, 0, s>>>(b);

@@ -179,7 +179,7 @@ struct SysState {
   int force_list;    // rebuild the Verlet list at the next check regardless of the skin
   int list_ok;       // a list was built since force_list was last set
   int cell_ovf;      // this build: a cell held more than kCellSlots rods (all-pairs scan instead)
-  int dmax;          // largest displacement measure of the configuration (FP32 bits; cleared by what reads the lists: finalize_kernel, cluster_bonds_kernel)
+  int dmax;          // largest displacement measure of the configuration (FP32 bits; cleared by what reads the lists, finalize_kernel and cluster_bonds_kernel, else by forget_displacement)
   long long stop;    // the step count at which the system stops taking steps (mdsc_set_step_limit)
   int stepping;      // it takes this step (xi_mid_kernel; for reduce_obs_kernel, which counts the step)
   double K_first[2]; // kinetic energies after the first half kick

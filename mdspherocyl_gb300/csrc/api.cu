@@ -398,8 +398,6 @@ void make_layout(const mdsc_system_desc* descs, int nsys, Layout& Lo) {
     P.kt_off = (int)Lo.ktile.size();
     P.nkt = ktiles;
     for (int q = 0; q < ktiles; ++q) Lo.ktile.push_back(make_int2(s, q));
-    P.kgp_off = (int)Lo.kgsets;
-    Lo.kgsets += (long long)P.nblk * ktiles * d.nd;
     blk += P.nblk;
     P.cl_fr = d.cl_fr;
     for (int a = 0; a < 3; ++a) {
@@ -475,7 +473,12 @@ void make_layout(const mdsc_system_desc* descs, int nsys, Layout& Lo) {
   // one per particle block and k tile where they do not (and always for
   // systems that add their tiles in parts)
   const bool split = (int)Lo.blk.size() <= kGatherSplitMax;
-  for (int s = 0; s < nsys; ++s) Lo.sys[s].kgt = (split || Lo.sys[s].kgs > 1) ? std::max(Lo.sys[s].nkt, 1) : 1;
+  for (int s = 0; s < nsys; ++s) {
+    SysDev& P = Lo.sys[s];
+    P.kgt = (split || P.kgs > 1) ? std::max(P.nkt, 1) : 1;
+    P.kgp_off = (int)Lo.kgsets;  // sums of single tiles, where blocks leave them
+    if (P.kgt > 1) Lo.kgsets += (long long)P.nblk * P.nkt * P.nd;
+  }
   for (int g = 0; g < (int)Lo.blk.size(); ++g) {
     const SysDev& P = Lo.sys[Lo.blk[g].x];
     if (P.kgt == 1) Lo.kgwork.push_back(make_int2(g, -1));

@@ -159,3 +159,23 @@ def test_gsl_generator_files_have_the_reference_layout():
     import refdriver
 
     assert len(refdriver.mt_state_bytes(1)) == 5000
+
+
+def test_estimate_bytes_of_gather_sets_where_they_are_used():
+    """Batches whose particle blocks fill the GPU (above 300) gather whole walks and
+    hold no sums of single k tiles: what a wider k-vector set adds for a system
+    of 2048 rods is less there, by 16 particle blocks x 3 KB a tile."""
+
+    def added(copies):
+        d = []
+        for K, ksq in ((9, 64), (13, 144)):
+            st, box = S.make_system(n=2048, phi=0.1, lengths=np.full(2048, 3.0), mu=np.full(2048, 1.2), seed=1)
+            spec = S.SystemSpec(n=2048, box=box, alpha=0.3, K_max=K, ksq_max=ksq)
+            d.append(L.estimate_bytes([L.desc_from_spec(spec, 1)] * copies) / copies)
+        return d[1] - d[0]
+
+    kvecs = [sum(1 for x in range(-k, k + 1) for y in range(-k, k + 1) for z in range(-k, k + 1)
+                 if 0 < x * x + y * y + z * z <= q) // 2 for k, q in ((8, 64), (12, 144))]
+    tiles = [(v + 127) // 128 for v in kvecs]
+    sets = 16 * (tiles[1] - tiles[0]) * 128 * 6 * 4
+    assert abs((added(10) - added(40)) - sets) <= 0.02 * sets

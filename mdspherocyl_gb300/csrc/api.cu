@@ -766,7 +766,8 @@ mdsc_status autotune(mdsc_batch* B, int force, int reps) {
   Tuning best = b.tune;
   B->tune_log.clear();
   char line[160];
-  auto pick = [&](const char* what, const int* cand, int nc, int& field, auto&& launch) {
+  // the fastest candidate; a later one has to be below `need` times the best so far
+  auto pick = [&](const char* what, const int* cand, int nc, int& field, double need, auto&& launch) {
     double tbest = 1e30;
     int vbest = field;
     for (int k = 0; k < nc; ++k) {
@@ -774,11 +775,7 @@ mdsc_status autotune(mdsc_batch* B, int force, int reps) {
       const double t = time_launches(B, reps, launch);
       snprintf(line, sizeof line, "%s=%d %.4f ms; ", what, cand[k], t);
       B->tune_log += line;
-      // candidates ascend in what they hold of the SMs beside the step's other
-      // chains, which a kernel timed alone does not show (the WCA evaluation's
-      // grid on 608 blocks held every register of the GPU: 107 us per step of
-      // 4096 rods against 88 on 304): a larger one has to be clearly faster
-      if (t < (k ? 0.95 : 1.0) * tbest) {
+      if (t < (k ? need : 1.0) * tbest) {
         tbest = t;
         vbest = cand[k];
       }
@@ -789,21 +786,25 @@ mdsc_status autotune(mdsc_batch* B, int force, int reps) {
   {
     const int m = B->num_sms;
     const int cand[4] = {m * 2, m * 4, m * 8, m * 16};
-    pick("wca_blocks", cand, 4, b.tune.wca_blocks, [&] { launch_wca(b, true, B->st); });
+    // these candidates ascend in what they hold of the SMs beside the step's other
+    // chains, which a kernel timed alone does not show (608 blocks held every
+    // register of the GPU: 107 us per step of 4096 rods against 88 on 304): a
+    // larger one has to be clearly faster
+    pick("wca_blocks", cand, 4, b.tune.wca_blocks, 0.95, [&] { launch_wca(b, true, B->st); });
   }
   // real-space tiles per block, then the strip-sum block size
   if (b.ntiles > 0) {
     const int cand[3] = {1, 2, 4};
-    pick("rp_warps", cand, 3, b.tune.rp_warps, [&] { launch_real_pairs(b, B->lo.multi, B->st); });
+    pick("rp_warps", cand, 3, b.tune.rp_warps, 1.0, [&] { launch_real_pairs(b, B->lo.multi, B->st); });
     const int cand2[3] = {128, 256, 512};
-    pick("rsum_threads", cand2, 3, b.tune.rsum_threads, [&] { launch_real_sum(b, B->st); });
+    pick("rsum_threads", cand2, 3, b.tune.rsum_threads, 1.0, [&] { launch_real_sum(b, B->st); });
   }
   // k-space gather form (single-dipole systems)
   if (b.nktot > 0 && B->lo.maxnd <= 1) {
     launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 0, B->st);
     launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 1, B->st);
     const int cand[2] = {0, 1};
-    pick("kg_scalar", cand, 2, b.tune.kg_scalar, [&] {
+    pick("kg_scalar", cand, 2, b.tune.kg_scalar, 1.0, [&] {
       launch_kspace_parts(b, B->lo.maxnd, B->kwork, (int)B->lo.kwork.size(), B->kowner, 2, B->st);
     });
   }

@@ -580,7 +580,8 @@ __global__ void __launch_bounds__((TWO ? 2 : 1) * kRowBlock, TWO ? 5 : 10) final
         sv[a][lane] = m;
         sync_rows();
         t += sv[a1][lane] * P.B[a2] - sv[a2][lane] * P.B[a1];
-        uext -= m * P.B[a];
+        // by one warp: the three products cancel in FP64, not in the rows' 48 bits
+        if (a == 0) uext -= sv[0][lane] * P.B[0] + sv[1][lane] * P.B[1] + sv[2][lane] * P.B[2];
       }
       // lever arm of an off-centre dipole: d x f (v25/classes.hpp:135-136)
       sync_rows();

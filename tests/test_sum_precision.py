@@ -8,6 +8,7 @@ middle + tiny - big - middle with 24 bits each from 1 down to about 2^-51, which
 """
 import ctypes
 import math
+from fractions import Fraction
 
 import numpy as np
 import pytest
@@ -149,3 +150,25 @@ def test_moment_tensor_of_the_self_terms_in_fp64(n):
     assert alone[0][1] != 0 and alone[0][1] == alone[1][0]
     got = run([BIG, MIDDLE, TINY, -BIG, -MIDDLE])
     assert got[0][1] == alone[0][1] and got[1][0] == alone[1][0]
+
+
+def test_field_energy_of_a_moment_across_the_field():
+    """mu o . B of moments nearly across the field, where the components' products
+    cancel to 2^-44: within five FP64 roundings of the products."""
+    rng = np.random.default_rng(11)
+    for n in (1, 1, 1, 1, 1, 1, 1, 1, 33):
+        x, y = rng.uniform(0.3, 0.9, 2)
+        m = np.array([x, y, 0.0])
+        B = np.array([y, -x * (1.0 + 2.0 ** -44), 0.0])
+        dip = np.zeros((n, 1, 5))
+        dip[:, 0, 1:4] = m
+        dip[:, 0, 4] = 1.0
+        st = S.SystemState(np.arange(3.0 * n).reshape(n, 3) % 29.0, np.zeros((n, 3)), np.stack([np.eye(3)] * n),
+                           np.zeros((n, 3)), np.full(n, 2.0), np.ones(n), np.ones(n), dip)
+        spec = S.SystemSpec(n=n, box=np.full(3, 30.0), alpha=0.2, K_max=2, ksq_max=1, B=B)
+        with L.Batch([spec], [st]) as bt:
+            bt.zero_forces()
+            U = bt.ext_field()[0]
+        exact = -n * float(Fraction(m[0]) * Fraction(B[0]) + Fraction(m[1]) * Fraction(B[1]))
+        assert exact != 0.0
+        assert abs(U - exact) <= n * 5 * 2.0 ** -53 * (abs(m[0] * B[0]) + abs(m[1] * B[1])), (n, U, exact)

@@ -77,7 +77,7 @@ constexpr int kNoiseChunk = 256;  // steps of thermostat noise per upload
 // tiles came first and the other chains waited for them to end (its step ran
 // in 84 or in 100 us, by which was first), 89 behind it; 64 systems 195 and
 // 190; 2048 rods (528 tiles), where the tiles are the longest chain, 52 and 56.
-constexpr int kTilesAfter = 4 * 152;
+constexpr int kTilesAfter = 4 * kSMs;
 // Batches of at most this many tiles run each on four warps.  us per step on one
 // warp and on four: 256 rods (10 tiles) 39.4 and 33.4, 333 (21) 41.4 and 36.3,
 // 1000 (136) 43.9 and 39.3, 1200 (190) 43.2 and 39.9, 700 rods of two dipoles

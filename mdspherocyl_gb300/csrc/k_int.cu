@@ -910,7 +910,7 @@ void launch_reset_iter(const Batch& b, double* noise, const NoiseArgs& a, cudaSt
 void launch_copy_arrays(const ArrayCopies& c, cudaStream_t s) {
   long long most = 0;
   for (int q = 0; q < c.k; ++q) most = std::max(most, c.n[q]);
-  if (most) copy_arrays_kernel<<<dim3((unsigned)std::min<long long>((most + 255) / 256, 152), c.k), 256, 0, s>>>(c);
+  if (most) copy_arrays_kernel<<<dim3((unsigned)std::min<long long>((most + 255) / 256, kSMs), c.k), 256, 0, s>>>(c);
 }
 void launch_derive(const Batch& b, cudaStream_t s) {
   if (b.nwblk) particle_kernel<kPartDerive><<<b.nwblk, kRowBlock, 0, s>>>(b);

@@ -33,7 +33,7 @@ namespace mdsc {
 // a system of 256 rods 65.7 us per step with ksum1 and 62.4 with ksum1s, 24
 // systems of 128 to 2048 rods (330 blocks) 144 and 135; 64 systems (900) 229
 // and 226, 256 systems 693 and 696.
-constexpr int kKsumScalarMax = 4 * 152;
+constexpr int kKsumScalarMax = 4 * kSMs;
 
 // (int)ph * 2^-31 * pi: the phase, already reduced to [-pi, pi); the
 // hardware sine/cosine is accurate to ~4e-7 absolute on that range

@@ -230,7 +230,7 @@ cudaError_t launch_correlations(const Batch& b, const CorrSys* c, const unsigned
                                 int ntiles, int max_bins, unsigned long long* hist, cudaStream_t s) {
   if (ntiles <= 0) return cudaSuccess;
   // two blocks per SM: a run of tiles pays for a block's clearing and flush
-  const int grid = ntiles < 2 * 152 ? ntiles : 2 * 152;
+  const int grid = ntiles < 2 * kSMs ? ntiles : 2 * kSMs;
   if (max_bins <= kCorrSmemBins) {
     const int bytes = kCorrWords * max_bins * (int)sizeof(uint32_t);
     const cudaError_t e = cudaFuncSetAttribute(corr_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,

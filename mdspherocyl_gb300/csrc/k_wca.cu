@@ -88,7 +88,7 @@ __device__ __forceinline__ void sort_small(A& v, int n) {
 // A fixed grid looks through the rows for those that are due: most steps
 // rebuild few systems, and a block per row held the registers of the SMs from
 // the tiles that start at the same time.
-constexpr int kListBlocks = 4 * 152;
+constexpr int kListBlocks = 4 * kSMs;
 
 // The cell scan: blocks of two cells (two warps each), a thread per slot.
 __device__ void list_cells(const Batch& b, int force_all) {

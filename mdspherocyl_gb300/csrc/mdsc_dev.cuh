@@ -22,6 +22,7 @@ constexpr int kMaxNb = 64;       // Verlet-list capacity per particle
 constexpr int kMaxD = 4;         // dipoles per particle (MDSC_MAX_DIPOLES)
 constexpr int kPartBlock = 128;  // threads per block of the per-particle kernels
 constexpr int kKBlock = 128;     // k-vectors per block of the k-space kernels
+constexpr int kSMs = 152;        // multiprocessors of the GB300: the fixed grids and limits "per SM" are for it
 constexpr int kKChunk = 256;     // particles per block of the structure-factor kernel
 // Systems of more strips than this sum their tiles' partials and energies per
 // strip first (real_sum, strip_energy); in the others the force assembly adds

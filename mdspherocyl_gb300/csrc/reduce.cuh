@@ -174,19 +174,4 @@ __device__ __forceinline__ void ktile_sums(const float* in, int n, int stride, i
   for (int c = 0; c < NS; ++c) out[c] = parts == 1 ? FF{po[c], -pc[c]} : FF{fo[c], -__fadd_rn(fc[c], cs[c])};
 }
 
-// Per-block maximum of non-negative values.
-template <int NT>
-__device__ __forceinline__ float block_max(float v, float* sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, off));
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  float m = 0.f;
-  if (threadIdx.x == 0)
-    for (int k = 0; k < NT / 32; ++k) m = fmaxf(m, sh[k]);
-  __syncthreads();
-  return m;
-}
-
 }  // namespace mdsc

@@ -210,7 +210,9 @@ __global__ void __launch_bounds__(kRenderTile) render_kernel(RenderView v, const
   float d[3];
   pixel_ray(v, px, py, d);
   // the cone: its axis between two opposite corner rays, its angle that of the
-  // widest of the four (the others lie between them)
+  // widest of the four (the others lie between them, as long as that is below a
+  // right angle: a block of a low, wide picture can span more, and then its rays
+  // are tested against everything)
   float axis[3], sn = 0.f, cs = 1.f;
   {
     float c[4][3], nrm = 0.f;
@@ -227,6 +229,7 @@ __global__ void __launch_bounds__(kRenderTile) render_kernel(RenderView v, const
     }
     sn *= 1.0001f;
   }
+  const bool wide = !(cs > 0.1f);
   float tmin = 3.0e38f;
   int hit_k = -1, hit_list = 0;
   for (int list = 0; list < 2; ++list) {
@@ -246,7 +249,7 @@ __global__ void __launch_bounds__(kRenderTile) render_kernel(RenderView v, const
         const float r = s.w * 1.001f + 1e-5f * (fabsf(t) + perp);
         // outside: behind the eye, or further from the cone than its radius
         // (the distance to the cone's edge line is never above that to the cone)
-        in = s.w >= 0.f && !(t < -r || perp * cs - t * sn > r);
+        in = s.w >= 0.f && (wide || !(t < -r || perp * cs - t * sn > r));
       }
       const uint32_t m = __ballot_sync(0xffffffffu, in);
       if (lane == 0) wcnt[warp] = __popc(m);

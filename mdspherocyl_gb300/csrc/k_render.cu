@@ -72,13 +72,15 @@ __global__ void scene_kernel(Batch b, int sys, const unsigned char* __restrict__
                          images ? (float)(P.L[1] * ((m / 3) % 3 - 1)) : 0.f,
                          images ? (float)(P.L[2] * (m / 9 - 1)) : 0.f};
     const float c[3] = {(float)r[0] + sh[0], (float)r[1] + sh[1], (float)r[2] + sh[2]};
+    // the ends' roundings written out: which of two capsules that meet a pixel has
+    // hangs on their last bits, and the bounding spheres share their terms
     Capsule q;
-    q.ax = c[0] - h * u[0];
-    q.ay = c[1] - h * u[1];
-    q.az = c[2] - h * u[2];
-    q.bx = c[0] + h * u[0];
-    q.by = c[1] + h * u[1];
-    q.bz = c[2] + h * u[2];
+    q.ax = __fsub_rn(c[0], __fmul_rn(h, u[0]));
+    q.ay = __fsub_rn(c[1], __fmul_rn(h, u[1]));
+    q.az = __fsub_rn(c[2], __fmul_rn(h, u[2]));
+    q.bx = __fadd_rn(c[0], __fmul_rn(h, u[0]));
+    q.by = __fadd_rn(c[1], __fmul_rn(h, u[1]));
+    q.bz = __fadd_rn(c[2], __fmul_rn(h, u[2]));
     q.rad = rad;
     q.ex = (float)O[0];
     q.ey = (float)O[1];
@@ -112,12 +114,12 @@ __global__ void scene_kernel(Batch b, int sys, const unsigned char* __restrict__
       for (int s = 0; s < 2; ++s) {
         Capsule z;
         const float s0 = s == 0 ? -mlt : 0.f, s1 = s == 0 ? 0.f : mlt;
-        z.ax = p[0] + s0 * d[0];
-        z.ay = p[1] + s0 * d[1];
-        z.az = p[2] + s0 * d[2];
-        z.bx = p[0] + s1 * d[0];
-        z.by = p[1] + s1 * d[1];
-        z.bz = p[2] + s1 * d[2];
+        z.ax = __fmaf_rn(s0, d[0], p[0]);
+        z.ay = __fmaf_rn(s0, d[1], p[1]);
+        z.az = __fmaf_rn(s0, d[2], p[2]);
+        z.bx = __fmaf_rn(s1, d[0], p[0]);
+        z.by = __fmaf_rn(s1, d[1], p[1]);
+        z.bz = __fmaf_rn(s1, d[2], p[2]);
         z.rad = thick;
         z.ex = z.ey = z.ez = 0.f;
         z.tone = -1.f;

@@ -973,6 +973,7 @@ __global__ void __launch_bounds__(kPartBlock) kgather1s_kernel(Batch b) {
 
 template <int ND, bool TOTALS>
 static void launch_kgather(const Batch& b, cudaStream_t s) {
+  if (b.nkgwork == 0) return;  // k-vectors, but no rods
   if (b.ones) {
     if (b.tune.kg_scalar || TOTALS)  // the form that forms val S(k) itself is the one-rod one
       kgather1s_kernel<TOTALS><<<b.nkgwork, kPartBlock, 0, s>>>(b);
